@@ -13,8 +13,13 @@
 // The reference's semantics (AllPairsKernel.cl:47-135: P = sum over k of
 // A[i][k]*B[k][j], identity 0) are kept; only the order of the FP32 sums
 // differs from the sequential fold of the CUDA-core kernel.
+// Products of 256-column tiles are by default taken from two FP16 parts
+// instead, three products in place of six (gemm_pair_kernel, split_tile;
+// the FP16 split with a scaled residual is Ootomo & Yokota, "Recovering
+// single precision accuracy from Tensor Cores while surpassing the FP32
+// theoretical peak performance", IJHPCA 2022).
 //
-// Shape: 128 x 128 output tile per CTA.  Warp 0 (one thread) streams k-blocks
+// Shape of the bf16 kernel: 128 x 128 output tile per CTA.  Warp 0 (one thread) streams k-blocks
 // of 64 with TMA (3D tensor maps over the split parts, SWIZZLE_128B, one
 // mbarrier per stage); warp 1 allocates 2 x 128 TMEM columns and one thread
 // issues tcgen05.mma.kind::f16 (M=128, N=128, K=16; both operands K-major in
@@ -30,8 +35,10 @@
 // memory before it returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
+#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstdint>
 
 #include "internal.h"
@@ -39,7 +46,9 @@
 namespace scl {
 namespace tc {
 
+enum Format { kBf16 = 0, kF16 = 1 };  // of the operands' parts
 constexpr int BM = 128;
+constexpr int MPAD = 256;                        // M padding: whole tiles of CTA pairs
 constexpr int NPAD = 256;                        // N padding: fits both tile widths
 constexpr int KPAD = 64;                         // K padding: whole k-blocks of both shapes
 
@@ -60,19 +69,18 @@ struct Shape {
   static constexpr uint32_t SBO = 8 * BK * 2;    // bytes between 8-row groups
   static constexpr uint64_t LAYOUT = BK == 64 ? 2u : 4u;  // SWIZZLE_128B : SWIZZLE_64B
   // Instruction descriptor, kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16
-  // (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in bits
-  // 17-22, M >> 4 in bits 24-28.
+  // (bits 7-9 = 1, 10-12 = 1; 0: FP16), both K-major (bits 15, 16 = 0),
+  // N >> 3 in bits 17-22, M >> 4 in bits 24-28.
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) |
                                     ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 };
 
 // Shared-memory matrix descriptor for a K-major swizzled tile (rows of BK
-// bf16, 8-row groups SBO bytes apart): start address >> 4 (bits 0-13),
+// 16-bit parts, 8-row groups SBO bytes apart): start address >> 4 (bits 0-13),
 // leading-byte offset 1 (unused for swizzled K-major), stride-byte offset >> 4
 // (bits 32-45), descriptor version 1 (bits 46-47), layout (bits 61-63).
-template <int BN_T>
+template <typename SH>
 __device__ __forceinline__ uint64_t smem_desc(uint32_t saddr) {
-  using SH = Shape<BN_T>;
   uint64_t d = 0;
   d |= (uint64_t)((saddr >> 4) & 0x3FFFu);
   d |= (uint64_t)1u << 16;
@@ -105,102 +113,223 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, uint32_
   return true;
 }
 
+// 32 / 16 consecutive tensor-memory columns of this warp's 32 lanes (complete
+// after tcgen05.wait::ld).
+__device__ __forceinline__ void tmem_load32(uint32_t taddr, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10,"
+      " %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27,"
+      " %28, %29, %30, %31}, [%32];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+        "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
+        "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
+        "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
+        "=r"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10,"
+      " %11, %12, %13, %14, %15}, [%16];"
+      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
+        "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
+        "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+
 __device__ __forceinline__ void raise(unsigned int* err) {
   if (err) atomicOr(err, 1u);
 }
 
-// The split parts live in one [part][row][Kp] bf16 array per operand; rows and
-// Kp are padded to the tile sizes and zero-filled, so every TMA box is in
-// bounds.  Each thread splits 8 consecutive elements of a row and writes
-// each part's 8 bf16 with one 16-byte store.
-__device__ __forceinline__ void split8(const float (&x)[8], int parts, __nv_bfloat16* o0,
-                                       __nv_bfloat16* o1, __nv_bfloat16* o2) {
-  __align__(16) __nv_bfloat16 h[8], m[8], l[8];
-#pragma unroll
-  for (int e = 0; e < 8; ++e) {
-    h[e] = __float2bfloat16_rn(x[e]);
-    const float r1 = x[e] - __bfloat162float(h[e]);
-    m[e] = __float2bfloat16_rn(r1);
-    l[e] = __float2bfloat16_rn(r1 - __bfloat162float(m[e]));
-  }
-  *reinterpret_cast<uint4*>(o0) = *reinterpret_cast<const uint4*>(h);
-  *reinterpret_cast<uint4*>(o1) = *reinterpret_cast<const uint4*>(m);
-  if (parts > 2) *reinterpret_cast<uint4*>(o2) = *reinterpret_cast<const uint4*>(l);
-}
+// One operand of the split pass: X, `rows` x K row-major (kmajor) or K x
+// `rows` row-major, into planes [part][rp][Kp] of 16-bit parts; FP16 parts
+// come with one unscale factor per row and 128-wide k-block ([k-block][rp]).
+// Only the first `rows` rows of a plane are written (the rest only reach
+// outputs that are not stored); k is zero-filled to Kp.
+struct Operand {
+  const float* x;
+  void* out;
+  float* unscale;
+  uint32_t rows, rp;
+  int kmajor;
+};
 
-// X (R x C row-major) -> parts of X ([part][Rp][Cp]): rows over blockIdx.y
-// (grid-stride), 8-element chunks of a row over x.  Cp is a multiple of 64.
-__global__ void __launch_bounds__(256) split_rows_kernel(const float* __restrict__ X, uint32_t R,
-                                                         uint32_t C, uint32_t Rp, uint32_t Cp, int parts,
-                                                         __nv_bfloat16* __restrict__ out) {
-  const uint64_t plane = (uint64_t)Rp * Cp;
-  const uint32_t chunks = Cp / 8;
-  const bool vec = (C % 4u) == 0 && (reinterpret_cast<uintptr_t>(X) & 15u) == 0;
-  for (uint32_t r = blockIdx.y; r < Rp; r += gridDim.y) {
-    for (uint32_t ch = blockIdx.x * blockDim.x + threadIdx.x; ch < chunks; ch += gridDim.x * blockDim.x) {
-      const uint32_t c0 = ch * 8;
-      float x[8];
-      if (r < R && vec && c0 + 8 <= C) {
-        const float4 a = *reinterpret_cast<const float4*>(X + (uint64_t)r * C + c0);
-        const float4 b = *reinterpret_cast<const float4*>(X + (uint64_t)r * C + c0 + 4);
-        x[0] = a.x; x[1] = a.y; x[2] = a.z; x[3] = a.w;
-        x[4] = b.x; x[5] = b.y; x[6] = b.z; x[7] = b.w;
-      } else {
+// FP16 parts of a 128-wide k-block.  A power of two brings the block's largest
+// |x| into [2^14, 2^15); hi = fp16(x s), lo = fp16((x s - hi) 2^11), so that
+// hi + 2^-11 lo holds 23 bits of every |x s| >= 2^-13 and every smaller
+// element to 2^-36, 2^-50 of the block's largest.  The products hi*hi + 2^-11
+// (lo*hi + hi*lo) then carry a relative error of at most about 2^-22 per term,
+// except where an element below 2^-13 meets an operand element that is itself
+// small or zero (with every element of the other block at least 2^-28 of its
+// largest, the 2^-50 is below 2^-22 of the block's sum of |a b|).  Those
+// k-blocks, non-finite elements and blocks whose largest |x| lies outside
+// [2^-45, 2^46) are reported in `flags`, and the launch takes the bf16 parts
+// instead.  flags: eight words per k-block, set to the launch's epoch: 0 / 2
+// a non-zero element of A / B below 2^-13, 1 / 3 any element below it (zeros
+// included), 4 out of range.
+constexpr int kScaleK = 128;
+constexpr int kFlagWords = 8;
+constexpr uint32_t kMaxKBlocks = 4096;  // k-blocks the flag area has room for
+constexpr int kMinExp = 82, kMaxExp = 172;  // biased exponents of 2^-45, 2^45
+
+// X tile of 64 rows x 128 k at (r0, k0): thread i handles rows i / 16 (+ 16,
+// + 32, + 48), k (i % 16) * 8 .. + 7, so sixteen neighbouring lanes hold a
+// row's k-block and store 256 contiguous bytes per part.
+template <int FMT>
+__device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32_t Kp, uint32_t r0, uint32_t k0,
+                                           int parts, float (*tile)[65], unsigned int* flags,
+                                           unsigned int epoch, int flag0) {
+  const uint64_t plane = (uint64_t)op.rp * Kp;
+  const uint32_t R = op.rows;
+  if (!op.kmajor) {
+    // K x R: through shared memory, [k][row]; 16-byte loads when rows allow
+    // it (r0 and R multiples of 4: a load is wholly in or out)
+    if ((R % 4u) == 0 && (reinterpret_cast<uintptr_t>(op.x) & 15u) == 0) {
+      const uint32_t c4 = threadIdx.x % 16, kr = threadIdx.x / 16;
+      float4 q[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) x[e] = (r < R && c0 + e < C) ? X[(uint64_t)r * C + c0 + e] : 0.0f;
+      for (int i = 0; i < 8; ++i) {
+        const uint32_t k = k0 + kr + 16 * i, n = r0 + c4 * 4;
+        q[i] = (k < K && n < R) ? *reinterpret_cast<const float4*>(op.x + (uint64_t)k * R + n)
+                                : make_float4(0.f, 0.f, 0.f, 0.f);
       }
-      const uint64_t o = (uint64_t)r * Cp + c0;
-      split8(x, parts, out + o, out + plane + o, out + 2 * plane + o);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        float* t = &tile[kr + 16 * i][c4 * 4];
+        t[0] = q[i].x;
+        t[1] = q[i].y;
+        t[2] = q[i].z;
+        t[3] = q[i].w;
+      }
+    } else {
+#pragma unroll 8
+      for (int i = threadIdx.x; i < 128 * 64; i += 256) {
+        const uint32_t kk = (uint32_t)i / 64, nn = (uint32_t)i % 64;
+        const uint32_t k = k0 + kk, n = r0 + nn;
+        tile[kk][nn] = (k < K && n < R) ? op.x[(uint64_t)k * R + n] : 0.0f;
+      }
+    }
+    __syncthreads();
+  }
+  const bool vec = op.kmajor && (K % 4u) == 0 && (reinterpret_cast<uintptr_t>(op.x) & 15u) == 0;
+  const uint32_t kc = (threadIdx.x % 16) * 8, k = k0 + kc;
+  float x[4][8];
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const uint32_t rr = threadIdx.x / 16 + 16 * c, row = r0 + rr;
+    if (!op.kmajor) {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[c][e] = tile[kc + e][rr];
+    } else if (vec && row < R && k + 8 <= K) {
+      const float4 a = *reinterpret_cast<const float4*>(op.x + (uint64_t)row * K + k);
+      const float4 b = *reinterpret_cast<const float4*>(op.x + (uint64_t)row * K + k + 4);
+      x[c][0] = a.x; x[c][1] = a.y; x[c][2] = a.z; x[c][3] = a.w;
+      x[c][4] = b.x; x[c][5] = b.y; x[c][6] = b.z; x[c][7] = b.w;
+    } else {
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[c][e] = (row < R && k + e < K) ? op.x[(uint64_t)row * K + k + e] : 0.0f;
+    }
+  }
+#pragma unroll
+  for (int c = 0; c < 4; ++c) {
+    const uint32_t row = r0 + threadIdx.x / 16 + 16 * c;
+    const bool stored = row < R && k < Kp;
+    const uint64_t o = (uint64_t)row * Kp + k;
+    if constexpr (FMT == kBf16) {
+      __align__(16) __nv_bfloat16 h[8], m[8], l[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        h[e] = __float2bfloat16_rn(x[c][e]);
+        const float r1 = x[c][e] - __bfloat162float(h[e]);
+        m[e] = __float2bfloat16_rn(r1);
+        l[e] = __float2bfloat16_rn(r1 - __bfloat162float(m[e]));
+      }
+      if (stored) {
+        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(op.out) + o;
+        *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
+        *reinterpret_cast<uint4*>(out + plane) = *reinterpret_cast<const uint4*>(m);
+        if (parts > 2) *reinterpret_cast<uint4*>(out + 2 * plane) = *reinterpret_cast<const uint4*>(l);
+      }
+    } else {
+      unsigned int mb = 0;  // largest |x| of the row's k-block, as bits (NaN above infinity)
+#pragma unroll
+      for (int e = 0; e < 8; ++e) mb = max(mb, __float_as_uint(x[c][e]) & 0x7fffffffu);
+      mb = __reduce_max_sync(0xffffu << (threadIdx.x & 16), mb);  // over the row's 16 lanes
+      const int eb = (int)(mb >> 23);
+      const bool in_range = mb == 0u || (eb >= kMinExp && eb <= kMaxExp);
+      const bool scaled = mb != 0u && in_range;
+      const float s = scaled ? __uint_as_float((unsigned int)(268 - eb) << 23) : 1.0f;  // 2^(14 - e)
+      __align__(16) __half h[8], l[8];
+      bool small_nz = false, small = false;
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float v = x[c][e] * s;
+        h[e] = __float2half_rn(v);
+        l[e] = __float2half_rn((v - __half2float(h[e])) * 2048.0f);
+        const bool below = fabsf(v) < 0x1p-13f && row < R && k + e < K;
+        small |= below;
+        small_nz |= below && x[c][e] != 0.0f;
+      }
+      if (stored) {
+        __half* out = static_cast<__half*>(op.out) + o;
+        *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
+        *reinterpret_cast<uint4*>(out + plane) = *reinterpret_cast<const uint4*>(l);
+        if (kc == 0)
+          op.unscale[(uint64_t)(k0 / kScaleK) * op.rp + row] =
+              scaled ? __uint_as_float((unsigned int)(eb - 14) << 23) : 1.0f;
+      }
+      const bool any_nz = __any_sync(0xffffffffu, small_nz), any = __any_sync(0xffffffffu, small);
+      const bool out_of_range = __any_sync(0xffffffffu, !in_range);
+      if ((threadIdx.x & 31) == 0) {
+        unsigned int* f = flags + (uint64_t)(k0 / kScaleK) * kFlagWords;
+        if (any_nz) f[flag0] = epoch;
+        if (any) f[flag0 + 1] = epoch;
+        if (out_of_range) f[4] = epoch;
+      }
     }
   }
 }
 
-// B (K x N row-major) -> parts of B^T ([part][Np][Kp]) through 64 x 64 tiles
-// in shared memory: coalesced row reads of B (16 bytes at a time when rows
-// allow it), 16-byte stores of 8 consecutive k per part.  Np and Kp are
-// multiples of 64.
-__global__ void __launch_bounds__(256) split_transpose_kernel(const float* __restrict__ B, uint32_t K,
-                                                              uint32_t N, uint32_t Np, uint32_t Kp,
-                                                              int parts, __nv_bfloat16* __restrict__ out) {
-  __shared__ float tile[64][65];  // [k][n]
-  const uint32_t k0 = blockIdx.y * 64, n0 = blockIdx.x * 64;
-  const uint64_t plane = (uint64_t)Np * Kp;
-  if ((N % 4u) == 0 && (reinterpret_cast<uintptr_t>(B) & 15u) == 0) {
-    // 16-byte loads, four rows per thread in flight (a full row of 64 is 16
-    // loads; n0 and N are multiples of 4, so a load is wholly in or out)
-    const uint32_t c4 = threadIdx.x % 16, r0 = threadIdx.x / 16;
-    float4 q[4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint32_t k = k0 + r0 + 16 * i, n = n0 + c4 * 4;
-      q[i] = (k < K && n < N) ? *reinterpret_cast<const float4*>(B + (uint64_t)k * N + n)
-                              : make_float4(0.f, 0.f, 0.f, 0.f);
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+// Splits both operands, one 64 x 128 tile per step (grid-stride over A's
+// tiles, then B's).  Bound by memory: reads 4 bytes, writes 4 (FP16) or 6
+// (bf16, three parts) per element.  A row-major operand's tiles are taken
+// along k, a transposed one's along its rows, so neighbouring blocks read
+// neighbouring memory.  With `verdict` (bf16 parts after an FP16 split) the
+// kernel first looks through the flags and leaves unless some k-block needs
+// the bf16 parts, which it reports to the contraction as *verdict = epoch.
+template <int FMT>
+__global__ void __launch_bounds__(256)
+split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int parts, unsigned int* flags,
+             unsigned int epoch, unsigned int* verdict) {
+  __shared__ float tile[128][65];
+  dependency_wait();
+  const uint32_t kt = (Kp + 127) / 128;
+  if (FMT == kBf16 && verdict) {
+    bool bad = false;
+    for (uint32_t i = threadIdx.x; i < kt; i += 256) {
+      const uint4 f = *reinterpret_cast<const uint4*>(flags + (uint64_t)i * kFlagWords);
+      const unsigned int range = flags[(uint64_t)i * kFlagWords + 4];
+      bad |= (f.x == epoch && f.w == epoch) || (f.z == epoch && f.y == epoch) || range == epoch;
     }
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      float* t = &tile[r0 + 16 * i][c4 * 4];
-      t[0] = q[i].x;
-      t[1] = q[i].y;
-      t[2] = q[i].z;
-      t[3] = q[i].w;
-    }
-  } else {
-    for (int i = threadIdx.x; i < 64 * 64; i += 256) {
-      const uint32_t kk = (uint32_t)i / 64, nn = (uint32_t)i % 64;
-      const uint32_t k = k0 + kk, n = n0 + nn;
-      tile[kk][nn] = (k < K && n < N) ? B[(uint64_t)k * N + n] : 0.0f;
-    }
+    if (!__syncthreads_or(bad ? 1 : 0)) return;
+    if (blockIdx.x == 0 && threadIdx.x == 0) *verdict = epoch;
   }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 64 * 8; i += 256) {
-    const uint32_t nn = (uint32_t)i / 8, kc = ((uint32_t)i % 8) * 8;
-    const uint32_t n = n0 + nn, k = k0 + kc;
-    if (n >= Np || k >= Kp) continue;
-    float x[8];
-#pragma unroll
-    for (int e = 0; e < 8; ++e) x[e] = tile[kc + e][nn];
-    const uint64_t o = (uint64_t)n * Kp + k;
-    split8(x, parts, out + o, out + plane + o, out + 2 * plane + o);
+  const uint32_t rta = (a.rows + 63) / 64, rtb = (b.rows + 63) / 64;
+  const uint64_t na = (uint64_t)rta * kt, n = na + (uint64_t)rtb * kt;
+  for (uint64_t t = blockIdx.x; t < n; t += gridDim.x) {
+    const bool second = t >= na;
+    const Operand& op = second ? b : a;
+    const uint64_t i = second ? t - na : t;
+    const uint32_t rt = second ? rtb : rta;
+    const uint32_t r0 = (uint32_t)(op.kmajor ? i / kt : i % rt) * 64;
+    const uint32_t k0 = (uint32_t)(op.kmajor ? i % kt : i / rt) * 128;
+    split_tile<FMT>(op, K, Kp, r0, k0, parts, tile, flags, epoch, second ? 2 : 0);
+    if (n > gridDim.x) __syncthreads();  // (block-uniform: the tile is filled again)
   }
 }
 
@@ -234,6 +363,7 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __shared__ uint32_t tmem_slot;
   __shared__ int s_fail;
 
+  dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // 1024-aligned stage ring
   uint32_t n0, m0;
@@ -342,9 +472,9 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         const uint32_t dtm = tmem + (uint32_t)(acc_i * BN);
 #pragma unroll
         for (int q = 0; q < NPROD; ++q) {
-          const uint64_t ad = smem_desc<BN_T>(stage + (uint32_t)prod_a[q] * SH::A_TILE);
+          const uint64_t ad = smem_desc<SH>(stage + (uint32_t)prod_a[q] * SH::A_TILE);
           const uint64_t bd =
-              smem_desc<BN_T>(stage + (uint32_t)(PARTS * SH::A_TILE + prod_b[q] * SH::B_TILE));
+              smem_desc<SH>(stage + (uint32_t)(PARTS * SH::A_TILE + prod_b[q] * SH::B_TILE));
 #pragma unroll
           for (int ks = 0; ks < BK / 16; ++ks) {
             // advance 16 bf16 = 32 bytes along K inside the swizzle row
@@ -396,20 +526,7 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 #pragma unroll
       for (int c = 0; c < CW / 32; ++c) {
         uint32_t r[32];
-        const uint32_t taddr =
-            tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc_i * BN + h * CW + c * 32);
-        asm volatile(
-            "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10,"
-            " %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27,"
-            " %28, %29, %30, %31}, [%32];"
-            : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-              "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]),
-              "=r"(r[13]), "=r"(r[14]), "=r"(r[15]), "=r"(r[16]), "=r"(r[17]), "=r"(r[18]),
-              "=r"(r[19]), "=r"(r[20]), "=r"(r[21]), "=r"(r[22]), "=r"(r[23]), "=r"(r[24]),
-              "=r"(r[25]), "=r"(r[26]), "=r"(r[27]), "=r"(r[28]), "=r"(r[29]), "=r"(r[30]),
-              "=r"(r[31])
-            : "r"(taddr)
-            : "memory");
+        tmem_load32(tmem + ((uint32_t)(q * 32) << 16) + (uint32_t)(acc_i * BN + h * CW + c * 32), r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r[j]);
@@ -462,14 +579,435 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   }
 }
 
+// ---- CTA pairs --------------------------------------------------------------------
+// The default form: 256 x 256 output tiles, one per pair of CTAs
+// (cta_group::2, M = 256, N = 256, K = 16).  Each CTA of the pair holds 128
+// rows of A and 128 of the 256 columns of B per stage and the accumulators of
+// its 128 rows x 256 columns; the pair's first CTA issues the MMAs.  Two
+// 256-column accumulators in tensor memory alternate (ping-pong), drained by
+// 8 epilogue warps of 32 rows x 128 columns into FP32 registers.
+// FP16 parts (three products): k-blocks of 64, three stages of 64 KB per CTA,
+//   a drain per k-block that applies the rows' and columns' unscale factors
+//   (copied into a ring in shared memory beside the operands; products with
+//   powers of two, so exact).  The cross products go first, 2^11 too large;
+//   the first hi*hi MMA scales them down (scale-input-d = 11).
+// bf16 parts (six products, where the split reported values FP16 parts do not
+//   hold): k-blocks of 32, four stages of 48 KB, a drain every 64 of K.
+// 8192 x 4096 x 8192, split included: 1.11 ms against 1.85 ms for six products
+// in gemm_3xbf16_kernel; without the drains' work 1.04 ms, at K = 16384 4.31
+// and 3.88 ms (three products at 1.54 and 1.71 of the 1.74 PFLOP/s bf16 a
+// long run sustains).  Bound by the tensor cores, then by the way round an
+// accumulator (MMAs, commit, drain, arrival from the other CTA).  A drain
+// every 128 of K ran 1.07 ms but doubled the error of positive operands
+// (4.6e-7 against 2.5e-7 for six products); two half-tiles of N = 128 with
+// their own accumulators 1.34 ms; 16 epilogue warps of 64 columns 1.25 ms;
+// release / acquire at cluster scope on the accumulators' barriers 1.69 ms
+// (the tcgen05 fences order what they hand over).
+// Normwise error against FP64 (2560 x K x 2048), here and with six bf16
+// products: normal operands K = 48 1.2e-7 / 2.1e-7, 128 1.4e-7 / 3.2e-7, 1024
+// 1.5e-7 / 3.2e-7, 4096 2.0e-7 / 3.5e-7; uniform in (0, 1) K = 48 1.4e-7 /
+// 1.9e-7, 4096 2.1e-7 / 2.6e-7.  Below K = 48 the six products are the more
+// exact (K = 32: 1.0e-7 / 0.6e-7), and stay.
+constexpr int kPairMinK = 48;
+constexpr int kPairCols = 256;  // tile columns; the tile has 2 * BM rows
+constexpr int kPairCW = 128;    // columns per epilogue warp
+constexpr int kPairThreads = 64 + 32 * 4 * (kPairCols / kPairCW);
+constexpr int kRing = 8;        // unscale slots: more than stages + accumulators in flight
+constexpr int kSlotBytes = (BM + kPairCols) * 4;
+
+template <int FMT>
+struct PairShape {
+  static constexpr int PARTS = FMT == kF16 ? 2 : 3;
+  static constexpr int STAGES = FMT == kF16 ? 3 : 4;
+  static constexpr int G = FMT == kF16 ? 1 : 2;  // k-blocks per drain
+  static constexpr int GS = 128 / (FMT == kF16 ? 64 : 32);  // k-blocks per unscale slot
+  static constexpr int BK = FMT == kF16 ? 64 : 32;
+  static constexpr int TILE = BM * BK * 2;       // bytes of one part of either operand per CTA
+  static constexpr int STAGE_BYTES = 2 * PARTS * TILE;
+  static constexpr uint32_t SBO = 8 * BK * 2;
+  static constexpr uint64_t LAYOUT = BK == 64 ? 2u : 4u;
+  static constexpr uint32_t IDESC = (1u << 4) | (FMT == kBf16 ? (1u << 7) | (1u << 10) : 0u) |
+                                    ((uint32_t)(kPairCols >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+};
+constexpr size_t kPairSmem = (size_t)3 * 64 * 1024 + kRing * kSlotBytes + 1024;
+static_assert(PairShape<kF16>::STAGES * PairShape<kF16>::STAGE_BYTES == 3 * 64 * 1024 &&
+                  PairShape<kBf16>::STAGES * PairShape<kBf16>::STAGE_BYTES == 3 * 64 * 1024,
+              "both formats use the same stage ring");
+
+struct PairArgs {
+  float* P;
+  const float* unscale_a;  // [k-block][Mp]
+  const float* unscale_b;  // [k-block][Np]
+  const unsigned int* verdict;
+  unsigned int* err;
+  uint32_t M, N, Kp, Mp, Np, epoch, spin_limit, tiles_n, tiles_m, group_m;
+};
+
+// The address of `addr` (shared memory) in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned; barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// Bounded wait for arrivals from both CTAs.
+__device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t limit) {
+  uint32_t polls = 0;
+  for (;;) {
+    uint32_t ok;
+    asm volatile(
+        "{ .reg .pred p; mbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;"
+        " selp.u32 %0, 1, 0, p; }"
+        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ok) return true;
+    if (++polls > limit) return false;
+    if (polls > 64) __nanosleep(32);
+  }
+}
+// Arrives on `bar` of both CTAs of the pair once every MMA issued so far has
+// completed.
+__device__ __forceinline__ void commit_pair(uint32_t bar) {
+  asm volatile(
+      "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+      :: "r"(bar), "h"((uint16_t)3) : "memory");
+}
+__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
+  uint64_t d;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
+  return d;
+}
+__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
+  uint64_t d;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
+  return d;
+}
+__device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
+  uint64_t d;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
+  return d;
+}
+
+struct PairBarriers {
+  uint64_t full[4];       // operands of a stage landed, both CTAs' (used in the first CTA)
+  uint64_t empty[4];      // the MMAs reading a stage completed (each CTA)
+  uint64_t acc_full[2];   // accumulator ready (each CTA)
+  uint64_t acc_empty[2];  // accumulator drained by both CTAs' epilogues (first CTA)
+  uint64_t ring[kRing];   // unscale slot landed (each CTA)
+  uint64_t drain;         // all issued MMAs completed (each CTA)
+};
+
+template <int FMT>
+__device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const PairArgs& g,
+                                          uint32_t base, uint32_t ring, PairBarriers* bars, uint32_t tmem,
+                                          uint32_t rank, uint32_t m0, uint32_t n0, int* s_fail) {
+  using SH = PairShape<FMT>;
+  constexpr int EPI_WARPS = 4 * (kPairCols / kPairCW);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t nk = g.Kp / SH::BK;
+  if (warp == 0) {
+    // ---- TMA producer (both CTAs): its 128 rows of A and of B's columns, counted
+    //      on the first CTA's barrier, and the unscale factors of its outputs
+    if (lane == 0) {
+      for (uint32_t kb = 0; kb < nk; ++kb) {
+        const uint32_t s = kb % SH::STAGES, round = kb / SH::STAGES;
+        if (round > 0 && !mbar_wait(smem_u32(&bars->empty[s]), (round - 1) & 1u, g.spin_limit)) {
+          raise(g.err);
+          *s_fail = 1;
+          break;
+        }
+        const uint32_t fb = smem_u32(&bars->full[s]);
+        if (rank == 0)
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                       :: "r"(fb), "r"((uint32_t)(2 * SH::STAGE_BYTES)) : "memory");
+        const uint32_t first_fb = cluster_addr(fb, 0);
+        const uint32_t stage = base + s * SH::STAGE_BYTES;
+        const int kx = (int)(kb * SH::BK);
+#pragma unroll
+        for (int p = 0; p < SH::PARTS; ++p) {
+          asm volatile(
+              "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+              " [%0], [%1, {%2, %3, %4}], [%5];"
+              :: "r"(stage + (uint32_t)(p * SH::TILE)), "l"(&tmA), "r"(kx), "r"((int)m0), "r"(p), "r"(first_fb)
+              : "memory");
+          asm volatile(
+              "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+              " [%0], [%1, {%2, %3, %4}], [%5];"
+              :: "r"(stage + (uint32_t)((SH::PARTS + p) * SH::TILE)), "l"(&tmB), "r"(kx),
+                 "r"((int)(n0 + rank * 128u)), "r"(p), "r"(first_fb)
+              : "memory");
+        }
+        if (FMT == kF16 && kb % SH::GS == 0) {
+          // slot grp % kRing was read for slot-group grp - kRing, long drained:
+          // the MMAs of k-block kb - STAGES, just waited for, began after the
+          // drain of k-block kb - STAGES - 2
+          static_assert(kRing * SH::GS >= SH::STAGES + 2 + SH::GS, "a slot is reused after its drain");
+          const uint32_t grp = kb / SH::GS;
+          const uint32_t slot = ring + (grp % kRing) * kSlotBytes, rb = smem_u32(&bars->ring[grp % kRing]);
+          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                       :: "r"(rb), "r"((uint32_t)kSlotBytes) : "memory");
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+              :: "r"(slot), "l"(g.unscale_a + (uint64_t)grp * g.Mp + m0), "r"((uint32_t)(BM * 4)), "r"(rb)
+              : "memory");
+          asm volatile(
+              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+              :: "r"(slot + BM * 4), "l"(g.unscale_b + (uint64_t)grp * g.Np + n0),
+                 "r"((uint32_t)(kPairCols * 4)), "r"(rb)
+              : "memory");
+        }
+      }
+    }
+  } else if (warp == 1) {
+    // ---- MMA issuer (first CTA)
+    if (lane == 0) {
+      if (rank == 0) {
+        // the products of one k-block: part pa of A times part pb of B
+        auto mma = [&](uint32_t dtm, uint32_t stage, int pa, int pb, bool fresh, bool scale_down) {
+          const uint64_t ad = smem_desc<SH>(stage + (uint32_t)(pa * SH::TILE));
+          const uint64_t bd = smem_desc<SH>(stage + (uint32_t)((SH::PARTS + pb) * SH::TILE));
+#pragma unroll
+          for (int ks = 0; ks < SH::BK / 16; ++ks) {
+            // 16 elements = 32 bytes along K inside the swizzle row
+            const uint64_t a = ad + (uint64_t)(ks * 2), b = bd + (uint64_t)(ks * 2);
+            const uint32_t acc = fresh && ks == 0 ? 0u : 1u;
+            if (scale_down && ks == 0)
+              asm volatile(
+                  "{ .reg .pred p; setp.ne.b32 p, %4, 0;"
+                  " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, 11; }"
+                  :: "r"(dtm), "l"(a), "l"(b), "r"(SH::IDESC), "r"(acc)
+                  : "memory");
+            else
+              asm volatile(
+                  "{ .reg .pred p; setp.ne.b32 p, %4, 0;"
+                  " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }"
+                  :: "r"(dtm), "l"(a), "l"(b), "r"(SH::IDESC), "r"(acc)
+                  : "memory");
+          }
+        };
+        bool landed = true;
+        for (uint32_t kb = 0; landed && kb < nk; kb += SH::G) {  // one drain group
+          const uint32_t grp = kb / SH::G, acc_i = grp & 1u, use = grp >> 1;
+          const uint32_t dtm = tmem + acc_i * kPairCols;
+          if (use > 0)
+            landed = mbar_wait_cluster(smem_u32(&bars->acc_empty[acc_i]), (use - 1) & 1u, g.spin_limit);
+#pragma unroll
+          for (int j = 0; j < SH::G; ++j) {
+            const uint32_t s = (kb + j) % SH::STAGES, stage = base + s * SH::STAGE_BYTES;
+            landed = landed && mbar_wait_cluster(smem_u32(&bars->full[s]), ((kb + j) / SH::STAGES) & 1u,
+                                                 g.spin_limit);
+            if (!landed) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            if (FMT == kF16) {  // lo*hi, hi*lo, hi*hi
+              mma(dtm, stage, 1, 0, true, false);
+              mma(dtm, stage, 0, 1, false, false);
+              mma(dtm, stage, 0, 0, false, true);
+            } else {  // lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi: smallest first
+              mma(dtm, stage, 2, 0, j == 0, false);
+              mma(dtm, stage, 0, 2, false, false);
+              mma(dtm, stage, 1, 1, false, false);
+              mma(dtm, stage, 1, 0, false, false);
+              mma(dtm, stage, 0, 1, false, false);
+              mma(dtm, stage, 0, 0, false, false);
+            }
+            commit_pair(smem_u32(&bars->empty[s]));
+          }
+          if (landed) commit_pair(smem_u32(&bars->acc_full[acc_i]));
+        }
+        if (!landed) {
+          raise(g.err);
+          *s_fail = 1;
+        }
+        // no MMA may still run when the tensor memory is freed (also after a
+        // failed wait above)
+        commit_pair(smem_u32(&bars->drain));
+      }
+      if (!mbar_wait(smem_u32(&bars->drain), 0, g.spin_limit)) raise(g.err);
+    }
+  } else {
+    // ---- epilogue (both CTAs): warp w (2 .. 9) owns tensor-memory lanes
+    //      32 * (w % 4) .. and columns 128 * ((w - 2) / 4) ..
+    const int q = warp & 3;
+    const uint32_t tile_col = (uint32_t)(((warp - 2) >> 2) * kPairCW);
+    uint64_t sum[kPairCW / 2];  // pairs of neighbouring columns
+#pragma unroll
+    for (int j = 0; j < kPairCW / 2; ++j) sum[j] = 0ull;
+    bool ok = true;
+    const uint32_t ngrp = nk / SH::G;
+    for (uint32_t grp = 0; grp < ngrp; ++grp) {
+      const uint32_t acc_i = grp & 1u;
+      uint64_t sa = 0;
+      uint32_t sb = 0;
+      if (FMT == kF16) {
+        const uint32_t sg = grp * SH::G / SH::GS;
+        const uint32_t slot = ring + (sg % kRing) * kSlotBytes;
+        if (!mbar_wait(smem_u32(&bars->ring[sg % kRing]), (sg / kRing) & 1u, g.spin_limit)) {
+          if (lane == 0) raise(g.err);
+          ok = false;
+          break;
+        }
+        uint32_t v;
+        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(slot + (uint32_t)(q * 32 + lane) * 4u));
+        sa = pack2(v, v);
+        sb = slot + BM * 4 + tile_col * 4;
+      }
+      if (!mbar_wait(smem_u32(&bars->acc_full[acc_i]), (grp >> 1) & 1u, g.spin_limit)) {
+        if (lane == 0) raise(g.err);
+        ok = false;
+        break;
+      }
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint32_t tm = tmem + ((uint32_t)(q * 32) << 16) + acc_i * kPairCols + tile_col;
+#pragma unroll
+      for (int c = 0; c < kPairCW / 16; ++c) {
+        uint32_t r[16];
+        tmem_load16(tm + (uint32_t)(c * 16), r);
+        if (FMT == kF16) {
+          uint64_t f[8];
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];"
+                         : "=l"(f[2 * j]), "=l"(f[2 * j + 1]) : "r"(sb + (uint32_t)(c * 64 + j * 16)));
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            sum[c * 8 + j] = fma2(pack2(r[2 * j], r[2 * j + 1]), mul2(sa, f[j]), sum[c * 8 + j]);
+        } else {
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int j = 0; j < 8; ++j)
+            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[c * 8 + j]) : "l"(pack2(r[2 * j], r[2 * j + 1])));
+        }
+      }
+      // accumulator drained: hand it back to the MMA issuer (one arrive per warp)
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0)
+        asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];"
+                     :: "r"(cluster_addr(smem_u32(&bars->acc_empty[acc_i]), 0)) : "memory");
+    }
+    const uint32_t row = m0 + (uint32_t)(q * 32 + lane), col0 = n0 + tile_col;
+    if (ok && row < g.M) {
+      float* dst = g.P + (uint64_t)row * g.N + col0;
+      if ((g.N % 4u) == 0u && col0 + kPairCW <= g.N) {
+#pragma unroll
+        for (int j = 0; j < kPairCW / 4; ++j)
+          *reinterpret_cast<ulonglong2*>(dst + j * 4) = make_ulonglong2(sum[2 * j], sum[2 * j + 1]);
+      } else {
+#pragma unroll
+        for (int j = 0; j < kPairCW / 2; ++j) {
+          uint32_t lo, hi;
+          asm("mov.b64 {%0, %1}, %2;" : "=r"(lo), "=r"(hi) : "l"(sum[j]));
+          if (col0 + 2 * j < g.N) dst[2 * j] = __uint_as_float(lo);
+          if (col0 + 2 * j + 1 < g.N) dst[2 * j + 1] = __uint_as_float(hi);
+        }
+      }
+    }
+  }
+  static_assert(EPI_WARPS * 32 + 64 == kPairThreads, "");
+}
+
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
+gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
+                 const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB3,
+                 const PairArgs g) {
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ __align__(8) PairBarriers bars;
+  __shared__ uint32_t tmem_slot;
+  __shared__ int s_fail;
+  const int warp = threadIdx.x >> 5;
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // 1024-aligned stage ring
+  const uint32_t ring = base + 3 * 64 * 1024;
+  uint32_t rank;
+  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  uint32_t m0, n0;
+  {
+    // tiles in groups of group_m tile rows (see gemm_3xbf16_kernel)
+    const uint32_t t = blockIdx.x / 2, per_group = g.group_m * g.tiles_n;
+    const uint32_t grp = t / per_group, r = t % per_group, first = grp * g.group_m;
+    const uint32_t rows = g.tiles_m - first < g.group_m ? g.tiles_m - first : g.group_m;
+    m0 = ((first + r % rows) * 2 + rank) * BM;
+    n0 = (r / rows) * kPairCols;
+  }
+  if (threadIdx.x == 0) {
+    s_fail = 0;
+    auto init = [](uint64_t* b, uint32_t count) {
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" :: "r"(smem_u32(b)), "r"(count));
+    };
+    for (int s = 0; s < 4; ++s) {
+      init(&bars.full[s], 1);
+      init(&bars.empty[s], 1);
+    }
+    for (int a = 0; a < 2; ++a) {
+      init(&bars.acc_full[a], 1);
+      init(&bars.acc_empty[a], 2 * 4 * (kPairCols / kPairCW));
+    }
+    for (int s = 0; s < kRing; ++s) init(&bars.ring[s], 1);
+    init(&bars.drain, 1);
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::2.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_u32(&tmem_slot)), "r"(512u) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
+  }
+  dependency_wait();
+  const bool f16 = *g.verdict != g.epoch;
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  cluster_sync();  // both CTAs' barriers are initialised, both hold tensor memory
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+  if (f16)
+    pair_body<kF16>(tmA, tmB, g, base, ring, &bars, tmem, rank, m0, n0, &s_fail);
+  else
+    pair_body<kBf16>(tmA3, tmB3, g, base, ring, &bars, tmem, rank, m0, n0, &s_fail);
+
+  // ---- teardown: wait for the copies a failed pipeline may still have in
+  //      flight (bounded), then, both CTAs together, free the tensor memory
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (s_fail && threadIdx.x == 0) {
+    for (int s = 0; s < 4; ++s) {
+      mbar_wait(smem_u32(&bars.full[s]), 0, g.spin_limit);
+      mbar_wait(smem_u32(&bars.full[s]), 1, g.spin_limit);
+    }
+    for (int s = 0; s < kRing; ++s) {
+      mbar_wait(smem_u32(&bars.ring[s]), 0, g.spin_limit);
+      mbar_wait(smem_u32(&bars.ring[s]), 1, g.spin_limit);
+    }
+  }
+  __syncthreads();
+  cluster_sync();  // neither CTA leaves while the other may still signal it
+  if (warp == 1) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(512u) : "memory");
+  }
+}
+
 inline uint32_t round_up(uint32_t v, uint32_t m) { return (v + m - 1) / m * m; }
 
 }  // namespace tc
 
 size_t allpairs_tc_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int parts) {
-  const uint64_t Mp = tc::round_up(M, tc::BM), Np = tc::round_up(N, tc::NPAD),
+  const uint64_t Mp = tc::round_up(M, tc::MPAD), Np = tc::round_up(N, tc::NPAD),
                  Kp = tc::round_up(K, tc::KPAD);
   return (size_t)parts * (Mp + Np) * Kp * 2 + 1024;
+}
+
+// Head of the workspace, before the scratch: [verdict | flags], zero when the
+// workspace is made and written only with launch epochs.
+size_t allpairs_tc_head_bytes() { return 256 + (size_t)tc::kMaxKBlocks * tc::kFlagWords * 4; }
+// Scratch of the CTA-pair form: the planes of either format, then the unscale
+// factors.
+size_t allpairs_pair_scratch_bytes(uint32_t M, uint32_t N, uint32_t K) {
+  const uint64_t Mp = tc::round_up(M, tc::MPAD), Np = tc::round_up(N, tc::NPAD),
+                 Kp = tc::round_up(K, tc::kScaleK);
+  return (size_t)3 * (Mp + Np) * Kp * 2 + 1024 + (size_t)(Mp + Np) * (Kp / tc::kScaleK) * 4;
+}
+bool allpairs_pair_supported(uint32_t K) {
+  return K >= tc::kPairMinK && (K - 1) / tc::kScaleK < tc::kMaxKBlocks;
 }
 
 bool allpairs_tc_supported(uint32_t M, uint32_t N, uint32_t K, const void*, const void*,
@@ -480,94 +1018,118 @@ bool allpairs_tc_supported(uint32_t M, uint32_t N, uint32_t K, const void*, cons
   return (uint64_t)M * N >= 128ull * 128ull && K >= 16 && rt().cc_major == 10;
 }
 
-static int encode_parts(CUtensorMap* tm, void* base, uint64_t rows, uint64_t Kp, int parts,
-                        uint32_t box_rows, uint32_t box_k) {
+static int encode_parts(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t Kp, int parts,
+                        uint32_t box_rows, uint32_t box_k, tc::Format fmt) {
   cuuint64_t dims[3] = {Kp, rows, (cuuint64_t)parts};
   cuuint64_t strides[2] = {Kp * 2, rows * Kp * 2};
   cuuint32_t box[3] = {box_k, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = rt().drv.cuTensorMapEncodeTiled(
-      tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, base, dims, strides, box, estr,
-      CU_TENSOR_MAP_INTERLEAVE_NONE,
+      tm, fmt == tc::kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
+      const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
       box_k == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
-  if (r != CUDA_SUCCESS) return cu_fail(r, "cuTensorMapEncodeTiled(3xbf16 parts)");
+  if (r != CUDA_SUCCESS) return cu_fail(r, "cuTensorMapEncodeTiled(split parts)");
   return SCL_OK;
 }
 
 namespace {
+// Launch on the library stream, overlapped like the skeleton kernels (every
+// kernel here starts with dependency_wait()).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, unsigned threads, size_t smem,
+                              cudaStream_t stream, const Args&... args) {
+  if (smem > 32 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = rt().pdl ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+  if (e == cudaSuccess) ++rt().launches;
+  return e;
+}
+
 template <int PARTS, int STAGES, int G, int BN_T>
 cudaError_t launch_gemm(dim3 grid, cudaStream_t stream, const CUtensorMap& tmA, const CUtensorMap& tmB,
                         float* P, uint32_t M, uint32_t N, uint32_t Kp, uint32_t spin_limit,
                         unsigned int* err, uint32_t tiles_n, uint32_t group_m) {
   using SH = tc::Shape<BN_T>;
   const size_t smem = (size_t)STAGES * PARTS * (SH::A_TILE + SH::B_TILE) + 1024;
-  auto kern = tc::gemm_3xbf16_kernel<PARTS, STAGES, G, BN_T>;
-  cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  if (e != cudaSuccess) return e;
-  kern<<<grid, SH::THREADS, smem, stream>>>(tmA, tmB, P, M, N, Kp, spin_limit, err, tiles_n, group_m);
-  return cudaGetLastError();
+  return launch_overlapped(tc::gemm_3xbf16_kernel<PARTS, STAGES, G, BN_T>, grid, SH::THREADS, smem, stream,
+                           tmA, tmB, P, M, N, Kp, spin_limit, err, tiles_n, group_m);
+}
+
+// Both operands' split descriptors for planes of `parts` parts from `scratch`
+// (1024-aligned inside it).
+struct Split {
+  uint32_t Mp, Np, Kp;
+  tc::Operand a, b;
+};
+Split split_of(const float* A, const float* B, uint32_t M, uint32_t N, uint32_t K, uint32_t kpad, int parts,
+               int trans, void* scratch) {
+  Split s;
+  s.Mp = tc::round_up(M, tc::MPAD);
+  s.Np = tc::round_up(N, tc::NPAD);
+  s.Kp = tc::round_up(K, kpad);
+  uint16_t* base = reinterpret_cast<uint16_t*>(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
+  s.a = {A, base, nullptr, M, s.Mp, (trans & 1) ? 0 : 1};
+  s.b = {B, base + (size_t)parts * s.Mp * s.Kp, nullptr, N, s.Np, (trans & 2) ? 1 : 0};
+  return s;
+}
+uint64_t split_tiles(const Split& s) {
+  return (uint64_t)((s.a.rows + 63) / 64 + (s.b.rows + 63) / 64) * ((s.Kp + 127) / 128);
+}
+dim3 split_grid(const Split& s) { return dim3((unsigned)std::min<uint64_t>(split_tiles(s), 0x7fffffffull)); }
+
+// The output tiles (rows x cols each), numbered in groups of tile rows; the
+// default is a group whose rows of A and columns of B for one wave of one
+// block per SM fit in L2 together.
+struct Tiles {
+  uint32_t m, n, group;
+};
+int tiles_of(uint32_t M, uint32_t N, uint32_t rows, uint32_t cols, uint32_t group_rows, Tiles* t) {
+  const uint64_t tn = ((uint64_t)N + cols - 1) / cols, tm = ((uint64_t)M + rows - 1) / rows;
+  if (tn * tm * (rows / tc::BM) > 0x7fffffffull) return fail(SCL_ERR_ARG, "tensor-core AllPairs: too many output tiles");
+  uint32_t g = (group_rows ? group_rows : 16) / (rows / tc::BM);
+  if (g < 1) g = 1;
+  if (g > tm) g = (uint32_t)tm;
+  *t = {(uint32_t)tm, (uint32_t)tn, g};
+  return SCL_OK;
 }
 }  // namespace
 
-// The split pass: both operands into `parts` bf16 planes, K-major ([row][k]
-// and [col][k]), zero-padded to Mp / Np / Kp, in `scratch` (1024-aligned
-// inside it).  A transposed operand (trans bit 0: A stored K x M, bit 1: B
-// stored N x K) swaps which of the two split kernels produces it.
-void split_operands(const float* A, const float* B, uint32_t M, uint32_t N, uint32_t K, int parts,
-                    int trans, void* scratch, cudaStream_t stream, __nv_bfloat16** a_out,
-                    __nv_bfloat16** b_out) {
-  const uint32_t Mp = tc::round_up(M, tc::BM), Np = tc::round_up(N, tc::NPAD),
-                 Kp = tc::round_up(K, tc::KPAD);
-  uint8_t* s = reinterpret_cast<uint8_t*>(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
-  __nv_bfloat16* a_parts = reinterpret_cast<__nv_bfloat16*>(s);
-  __nv_bfloat16* b_parts = a_parts + (size_t)parts * Mp * Kp;
-  auto rows_grid = [](uint32_t Rp, uint32_t Cp) {
-    return dim3((Cp / 8 + 255) / 256, Rp < 65535u ? Rp : 65535u);
-  };
-  if (trans & 1) {
-    tc::split_transpose_kernel<<<dim3(Mp / 64, Kp / 64), 256, 0, stream>>>(A, K, M, Mp, Kp, parts, a_parts);
-  } else {
-    tc::split_rows_kernel<<<rows_grid(Mp, Kp), 256, 0, stream>>>(A, M, K, Mp, Kp, parts, a_parts);
-  }
-  if (trans & 2) {
-    tc::split_rows_kernel<<<rows_grid(Np, Kp), 256, 0, stream>>>(B, N, K, Np, Kp, parts, b_parts);
-  } else {
-    tc::split_transpose_kernel<<<dim3(Np / 64, Kp / 64), 256, 0, stream>>>(B, K, N, Np, Kp, parts, b_parts);
-  }
-  rt().launches += 2;
-  *a_out = a_parts;
-  *b_out = b_parts;
-}
-
+// bf16 parts: `parts` 3 (six products) or 2 (three), each drained every
+// `drain` k-blocks.
 int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N,
                        uint32_t K, int parts, int trans, int drain, int wide, uint32_t group_rows,
                        void* scratch, size_t scratch_bytes, cudaStream_t stream, uint32_t spin_limit,
                        unsigned int* err) {
   if (parts != 2 && parts != 3) return fail(SCL_ERR_ARG, "3xBF16: parts must be 2 or 3");
-  const uint32_t Mp = tc::round_up(M, tc::BM), Np = tc::round_up(N, tc::NPAD),
-                 Kp = tc::round_up(K, tc::KPAD);
   if (scratch_bytes < allpairs_tc_scratch_bytes(M, N, K, parts))
     return fail(SCL_ERR_ARG, "3xBF16: scratch too small");
-  __nv_bfloat16 *a_parts = nullptr, *b_parts = nullptr;
-  split_operands(A, B, M, N, K, parts, trans, scratch, stream, &a_parts, &b_parts);
-
-  alignas(64) CUtensorMap tmA, tmB;
+  const Split sp = split_of(A, B, M, N, K, tc::KPAD, parts, trans, scratch);
+  const uint32_t Kp = sp.Kp;
   const uint32_t bn = wide ? 256 : 128, bk = wide ? 32 : 64;
-  if (int st = encode_parts(&tmA, a_parts, Mp, Kp, parts, tc::BM, bk)) return st;
-  if (int st = encode_parts(&tmB, b_parts, Np, Kp, parts, bn, bk)) return st;
-
-  // one 1D grid over the output tiles, grouped by `group_m` tile rows; the
-  // default is a group whose rows of A and columns of B for one wave of one
-  // block per SM fit in L2 together
-  const uint64_t tiles_n = (N + bn - 1) / bn, tiles_m = Mp / tc::BM;
-  if (tiles_n * tiles_m > 0x7fffffffull) return fail(SCL_ERR_ARG, "3xBF16: too many output tiles");
-  uint32_t group_m = group_rows;
-  if (group_m == 0) group_m = 16;
-  if (group_m > tiles_m) group_m = (uint32_t)tiles_m;
-  dim3 grid((unsigned)(tiles_n * tiles_m));
-  const uint32_t tn = (uint32_t)tiles_n;
-  cudaError_t e;
+  Tiles tiles;
+  if (int st = tiles_of(M, N, tc::BM, bn, group_rows, &tiles)) return st;
+  const dim3 grid(tiles.m * tiles.n);
+  const uint32_t tn = tiles.n, group_m = tiles.group;
+  alignas(64) CUtensorMap tmA, tmB;
+  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, parts, tc::BM, bk, tc::kBf16)) return st;
+  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, parts, bn, bk, tc::kBf16)) return st;
+  unsigned int* none = nullptr;
+  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), 256, 0, stream, sp.a, sp.b, K, Kp,
+                                    parts, none, 0u, none);
+  if (e != cudaSuccess) return cuda_fail(e, "split launch");
   if (wide) {
     // 128 x 256 tiles, k-blocks of 32: drains every 2 k-blocks (64 K, as the
     // narrow shape's default); parts 3: 3 stages of 72 KB; parts 2: 4 of 48 KB
@@ -584,7 +1146,45 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
                    : launch_gemm<2, 3, 1, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m);
   }
   if (e != cudaSuccess) return cuda_fail(e, "3xBF16 launch");
-  rt().launches += 1;
+  return SCL_OK;
+}
+
+// CTA pairs: FP16 parts, with the bf16 parts as the device's fallback.
+// `head` (allpairs_tc_head_bytes) precedes the scratch; `epoch` differs from
+// every earlier launch's on this head, or the head was cleared before.
+int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
+                         uint32_t group_rows, void* head, void* scratch, size_t scratch_bytes, unsigned int epoch,
+                         cudaStream_t stream, uint32_t spin_limit, unsigned int* err) {
+  if (scratch_bytes < allpairs_pair_scratch_bytes(M, N, K) || !allpairs_pair_supported(K))
+    return fail(SCL_ERR_ARG, "tensor-core AllPairs: scratch too small");
+  Split sp = split_of(A, B, M, N, K, tc::kScaleK, 2, trans, scratch);
+  const Split sp3 = split_of(A, B, M, N, K, tc::kScaleK, 3, trans, scratch);
+  const uint32_t Kp = sp.Kp;
+  float* unscale = reinterpret_cast<float*>(static_cast<uint16_t*>(sp3.b.out) + (size_t)3 * sp.Np * Kp);
+  sp.a.unscale = unscale;
+  sp.b.unscale = unscale + (size_t)sp.Mp * (Kp / tc::kScaleK);
+  unsigned int* verdict = static_cast<unsigned int*>(head);
+  unsigned int* flags = verdict + 64;
+  Tiles tiles;
+  if (int st = tiles_of(M, N, 2 * tc::BM, tc::kPairCols, group_rows, &tiles)) return st;
+  alignas(64) CUtensorMap tmA, tmB, tmA3, tmB3;
+  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, 2, tc::BM, 64, tc::kF16)) return st;
+  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, 2, 128, 64, tc::kF16)) return st;
+  if (int st = encode_parts(&tmA3, sp3.a.out, sp.Mp, Kp, 3, tc::BM, 32, tc::kBf16)) return st;
+  if (int st = encode_parts(&tmB3, sp3.b.out, sp.Np, Kp, 3, 128, 32, tc::kBf16)) return st;
+  unsigned int* none = nullptr;
+  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kF16>, split_grid(sp), 256, 0, stream, sp.a, sp.b, K, Kp, 2,
+                                    flags, epoch, none);
+  if (e != cudaSuccess) return cuda_fail(e, "split launch");
+  const unsigned few = (unsigned)std::min<uint64_t>(split_tiles(sp), (uint64_t)rt().sm_count * 4);
+  e = launch_overlapped(tc::split_kernel<tc::kBf16>, dim3(few), 256, 0, stream, sp3.a, sp3.b, K, Kp, 3, flags, epoch,
+                        verdict);
+  if (e != cudaSuccess) return cuda_fail(e, "split launch");
+  const tc::PairArgs args = {P,     sp.a.unscale, sp.b.unscale, verdict, err,        M,       N,      Kp,
+                             sp.Mp, sp.Np,        epoch,        spin_limit, tiles.n, tiles.m, tiles.group};
+  e = launch_overlapped(tc::gemm_pair_kernel, dim3(2 * tiles.m * tiles.n), tc::kPairThreads, tc::kPairSmem, stream,
+                        tmA, tmB, tmA3, tmB3, args);
+  if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
   return SCL_OK;
 }
 
@@ -601,8 +1201,9 @@ extern "C" int scl_debug_allpairs_split(const float* A, const float* B, uint32_t
   if (!scratch) return SCL_OK;
   if (int st = require_init()) return st;
   if (!A || !B || scratch_bytes < need) return fail(SCL_ERR_ARG, "split: null operand or scratch too small");
-  __nv_bfloat16 *a = nullptr, *b = nullptr;
-  split_operands(A, B, M, N, K, parts, trans, scratch, rt().stream, &a, &b);
-  SCL_CUDA(cudaGetLastError());
+  const Split sp = split_of(A, B, M, N, K, tc::KPAD, parts, trans, scratch);
+  unsigned int* none = nullptr;
+  SCL_CUDA(launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), 256, 0, rt().stream, sp.a, sp.b, K, sp.Kp,
+                             parts, none, 0u, none));
   return SCL_OK;
 }
