@@ -323,8 +323,10 @@ int scl_launch_scan_noalloc(scl_program* prog, const scl_shape* shape,
  *      same n_segments, and n at least the plan's) runs its segmented Scan or
  *      Reduce as ONE
  *      launch: the tiles of the long segments first, then one block per
- *      window of segments of up to 4096 elements (a thread per segment of up
- *      to 256 elements, a warp per longer one).  The plan keeps, per tile
+ *      window of short segments (up to 2048 four-byte elements for a Scan,
+ *      which scans a window's segments together; up to 4096 for a Reduce,
+ *      which gives each segment a share of the block's threads).  The plan
+ *      keeps, per tile
  *      shape, which tiles belong to which segment (and each tile's segment)
  *      and the windows; the first launch with a tile shape builds them (four
  *      small launches and a read-back of the offsets), so make it before
@@ -335,7 +337,8 @@ int scl_segplan_create(const uint64_t* seg_offsets, uint64_t n_segments, uint64_
 int scl_segplan_release(uint32_t plan);
 /* The window records a segment plan makes of its short segments (host only,
  * no device): for HOST offsets (n_segments + 1, clamped, non-decreasing)
- * and short_max > 0 (a plan uses half a scan tile), *count receives the
+ * and short_max > 0, with windows of short_max elements (a Reduce's plan; a
+ * Scan's windows are wider than its longest short segment), *count receives the
  * number of records and, when `records` is not NULL, up to `capacity`
  * records of four words {first segment, end segment, first element,
  * elements}.  For tests of the plan's host logic. */

@@ -234,15 +234,21 @@ int segments_prepare(const uint64_t* seg_offsets, uint64_t n_seg, uint64_t n_tot
 // tile shape the tile numbering with its exact tile count and the window
 // records of the short segments.
 struct SegPlanCfg {
-  uint64_t tile = 0, vg = 1, a = 0, short_max = 0;
+  uint64_t tile = 0, vg = 1, a = 0, short_max = 0, window = 0;
   int reverse = 0;
   unsigned int* tile_start = nullptr;  // device, n_seg + 1
   uint64_t tiles = 0;                  // tile_start[n_seg]
   unsigned int* tile_seg = nullptr;    // device, `tiles` entries: each tile's segment
-  // window records of the short segments (device, 4 words each: first
-  // segment, end segment, first element, elements), one block each
+  // window records of the short segments (the plan's, one block each)
   uint64_t n_rec = 0;
   uint64_t* win_rec = nullptr;
+};
+// The window records of one pair of limits, shared by the tile shapes that
+// use it (device, 4 words each: first segment, end segment, first element,
+// elements).
+struct SegPlanRecords {
+  uint64_t short_max = 0, window = 0, n_rec = 0;
+  uint64_t* rec = nullptr;
 };
 struct SegPlan {
   uint32_t id = 0;
@@ -251,18 +257,19 @@ struct SegPlan {
   unsigned int* tickets = nullptr;
   uint64_t* scratch = nullptr;
   std::deque<SegPlanCfg> cfgs;  // (stable addresses)
+  std::vector<SegPlanRecords> records;
+  std::vector<uint64_t> host_off;  // the clamped offsets, read back once
 };
 // The window records a segment plan makes of its short segments (four words
 // each: first segment, end segment, first element, elements).
-void segplan_window_records(const uint64_t* off, uint64_t n_seg, uint64_t short_max,
+void segplan_window_records(const uint64_t* off, uint64_t n_seg, uint64_t short_max, uint64_t window,
                             std::vector<uint64_t>* rec);
-
 SegPlan* segplan_find(uint32_t id);
 // The plan's tile numbering for one tile shape, built on first use (three
 // small launches and a read-back of the tile count; refused inside a stream
 // capture).
 int segplan_config(SegPlan* p, uint64_t tile, uint64_t vg, uint64_t a, int reverse, uint64_t short_max,
-                   const SegPlanCfg** out);
+                   uint64_t window, const SegPlanCfg** out);
 // Autotuner (tune.cpp): lookup/store of the (device, program, skeleton, size
 // bucket) cache, and the launch wrapper that times `cands` on a miss.
 bool tune_lookup(const std::string& key, scl_tuning* out);

@@ -376,7 +376,7 @@ static int launch_reduce_impl(scl_program* p, const scl_shape* sh, void* const* 
     const uint64_t wt = (uint64_t)8 * 256 * V;
     uint64_t short_max = wt / 2;
     const SegPlanCfg* cfg = nullptr;
-    if (int st = segplan_config(pl, tile, 1, 0, 0, short_max, &cfg)) return st;
+    if (int st = segplan_config(pl, tile, 1, 0, 0, short_max, short_max, &cfg)) return st;
     const std::string kname = "scl_reduce_seg<" + std::to_string(R) + ", 1>";
     CUfunction fn = find_kernel(p, kname);
     if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname + " missing");
@@ -625,10 +625,14 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
   uint64_t tiles;
   const SegPlanCfg* pcfg = nullptr;
   if (plan) {
-    // the plan's exact tile count; windows of tile / 2 elements and short
-    // segments of at most tile / 2, so a window's segments fit in one staged
-    // tile
-    if (int st = segplan_config(plan, tile, vg, ga, reverse ? 1 : 0, tile / 2, &pcfg)) return st;
+    // the plan's exact tile count; short segments of at most tile / 4 and
+    // windows of 47/64 of a tile: a window's segments fit in one staged tile,
+    // and a record of short vectors fills 24 rows of the window scan, three
+    // per warp (10^6 vectors of 1..199 floats 133 us; windows and segments of
+    // half a tile, 17 rows, 154 us; segments of 3000 floats, now tiles, 333
+    // against 388 us)
+    if (int st = segplan_config(plan, tile, vg, ga, reverse ? 1 : 0, tile / 4, tile * 47 / 64,
+                                &pcfg)) return st;
     tiles = pcfg->tiles;
   } else if (n_seg) {
     // an upper bound (the pre-pass has the count): tiles exist only for
@@ -701,12 +705,12 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
   uint64_t grid = tiles;
   if (plan) {
     // the blocks past the tiles take one window record of short segments
-    // each; a record keeps its 16-byte phase in shared memory, so it needs
-    // one vector more than a tile
+    // each; a record keeps its 16-byte phase in shared memory and is read in
+    // whole lane chunks, so it needs up to three vectors more than a tile
     grid = tiles + pcfg->n_rec;
     if (grid == 0) return SCL_OK;  // (every vector is either a tile's or in a record)
     if (grid > 0x7fffffffull) return fail(SCL_ERR_ARG, "segmented scan: too many tiles");
-    smem += 16;
+    smem += 48;
   }
   if (prepass) {
     uint64_t* scratch = reinterpret_cast<uint64_t*>((char*)p->ws.ptr + total + seg_of + seg_ts);

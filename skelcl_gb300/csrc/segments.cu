@@ -299,38 +299,81 @@ void free_plan(SegPlan* p) {
   cudaFree(p->scratch);
   for (auto& c : p->cfgs) {
     cudaFree(c.tile_start);
-    cudaFree(c.win_rec);
     cudaFree(c.tile_seg);
   }
+  for (auto& r : p->records) cudaFree(r.rec);
 }
 }  // namespace
 
-// Window records of the short segments: consecutive segments starting in the
-// same window of short_max elements form one record {first segment, end
-// segment, first element, elements}; a last segment longer than short_max
-// belongs to the tiles and is left out (its start ends the record's
-// elements).  All but the last segment of a record end inside its window, so
-// a record spans at most 2 * short_max elements.  Records whose segments are
-// all empty stay (the Reduce writes their identities); windows that own no
-// segment get none.  `off` holds n_seg + 1 clamped offsets.
-void segplan_window_records(const uint64_t* off, uint64_t n_seg, uint64_t short_max,
+// Window records of the short segments: consecutive segments of at most
+// short_max elements that start in the same window of `window` >= short_max
+// elements form one record {first segment, end segment, first element,
+// elements}; longer segments belong to the tiles and end the record before
+// them.  All but the last segment of a record end inside its window, so a
+// record spans less than window + short_max elements.  Records whose segments
+// are all empty stay (the Reduce writes their identities); windows that own
+// no segment get none.  `off` holds n_seg + 1 clamped offsets.
+void segplan_window_records(const uint64_t* off, uint64_t n_seg, uint64_t short_max, uint64_t window,
                             std::vector<uint64_t>* rec) {
   rec->clear();
   for (uint64_t sg = 0; sg < n_seg;) {
-    const uint64_t w = off[sg] / short_max, w0 = w * short_max, w1 = w0 + short_max;
-    uint64_t hi = sg + 1;
-    while (hi < n_seg && off[hi] >= w0 && off[hi] < w1) ++hi;
-    const uint64_t la = off[hi - 1], lb = std::max(la, off[hi]);
-    const uint64_t top = lb - la > short_max ? hi - 1 : hi;
-    if (top > sg) {
-      const uint64_t e0 = off[sg];
-      uint64_t e1 = top == hi ? lb : off[top];
-      if (e1 < e0) e1 = e0;
-      rec->insert(rec->end(), {sg, top, e0, e1 - e0});
+    const uint64_t e0 = off[sg];
+    uint64_t lo = e0, hi = off[sg + 1];  // the segment at hand
+    if (hi > lo && hi - lo > short_max) {
+      ++sg;
+      continue;
     }
-    sg = hi;
+    const uint64_t w0 = e0 / window * window;
+    uint64_t top = sg + 1, last = hi > lo ? hi : lo;
+    while (top < n_seg) {
+      lo = hi;
+      hi = off[top + 1];
+      if (lo - w0 >= window || (hi > lo && hi - lo > short_max)) break;
+      last = hi > lo ? hi : lo;
+      ++top;
+    }
+    rec->insert(rec->end(), {sg, top, e0, last > e0 ? last - e0 : 0});
+    sg = top;
   }
 }
+
+namespace {
+// The plan's records for these limits, built on the host at first use.
+int segplan_records(SegPlan* p, uint64_t short_max, uint64_t window, const SegPlanRecords** out) {
+  for (auto& r : p->records)
+    if (r.short_max == short_max && r.window == window) {
+      *out = &r;
+      return SCL_OK;
+    }
+  if (p->host_off.empty()) {
+    std::vector<uint64_t> off(p->n_seg + 1);
+    SCL_CUDA(cudaMemcpyAsync(off.data(), p->off, off.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost,
+                             rt().stream));
+    SCL_CUDA(cudaStreamSynchronize(rt().stream));
+    p->host_off.swap(off);
+  }
+  std::vector<uint64_t> rec;
+  segplan_window_records(p->host_off.data(), p->n_seg, short_max, window, &rec);
+  SegPlanRecords r;
+  r.short_max = short_max;
+  r.window = window;
+  r.n_rec = rec.size() / 4;
+  if (r.n_rec) {
+    rt().device_allocs++;
+    cudaError_t e = cudaMalloc(&r.rec, rec.size() * sizeof(uint64_t));
+    if (e == cudaSuccess)
+      e = cudaMemcpyAsync(r.rec, rec.data(), rec.size() * sizeof(uint64_t), cudaMemcpyHostToDevice, rt().stream);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(rt().stream);
+    if (e != cudaSuccess) {
+      cudaFree(r.rec);
+      return cuda_fail(e, "segment plan: window records");
+    }
+  }
+  p->records.push_back(r);
+  *out = &p->records.back();
+  return SCL_OK;
+}
+}  // namespace
 
 SegPlan* segplan_find(uint32_t id) {
   std::lock_guard<std::mutex> g(g_plan_mu);
@@ -339,9 +382,10 @@ SegPlan* segplan_find(uint32_t id) {
 }
 
 int segplan_config(SegPlan* p, uint64_t tile, uint64_t vg, uint64_t a, int reverse, uint64_t short_max,
-                   const SegPlanCfg** out) {
+                   uint64_t window, const SegPlanCfg** out) {
   for (auto& c : p->cfgs)
-    if (c.tile == tile && c.vg == vg && c.a == a && c.reverse == reverse && c.short_max == short_max) {
+    if (c.tile == tile && c.vg == vg && c.a == a && c.reverse == reverse && c.short_max == short_max &&
+        c.window == window) {
       *out = &c;
       return SCL_OK;
     }
@@ -357,33 +401,17 @@ int segplan_config(SegPlan* p, uint64_t tile, uint64_t vg, uint64_t a, int rever
   c.a = a;
   c.reverse = reverse;
   c.short_max = short_max;
+  c.window = window;
+  const SegPlanRecords* rec = nullptr;
+  if (int st = segplan_records(p, short_max, window, &rec)) return st;
+  c.n_rec = rec->n_rec;
+  c.win_rec = rec->rec;
   rt().device_allocs++;
   SCL_CUDA(cudaMalloc(&c.tile_start, (p->n_seg + 1) * sizeof(unsigned int)));
   if (int st = segments_prepare(p->off, p->n_seg, p->n_total, tile, vg, a, reverse, short_max, p->off,
                                 c.tile_start, p->scratch, rt().stream)) {
     cudaFree(c.tile_start);
     return st;
-  }
-  // the window records of the short segments (on the host, once)
-  std::vector<uint64_t> off(p->n_seg + 1);
-  SCL_CUDA(cudaMemcpyAsync(off.data(), p->off, off.size() * sizeof(uint64_t), cudaMemcpyDeviceToHost,
-                           rt().stream));
-  SCL_CUDA(cudaStreamSynchronize(rt().stream));
-  std::vector<uint64_t> rec;
-  segplan_window_records(off.data(), p->n_seg, short_max, &rec);
-  c.n_rec = rec.size() / 4;
-  if (c.n_rec) {
-    rt().device_allocs++;
-    cudaError_t e = cudaMalloc(&c.win_rec, rec.size() * sizeof(uint64_t));
-    if (e == cudaSuccess)
-      e = cudaMemcpyAsync(c.win_rec, rec.data(), rec.size() * sizeof(uint64_t), cudaMemcpyHostToDevice,
-                          rt().stream);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(rt().stream);
-    if (e != cudaSuccess) {
-      cudaFree(c.tile_start);
-      cudaFree(c.win_rec);
-      return cuda_fail(e, "segment plan: window records");
-    }
   }
   unsigned int tiles = 0;
   SCL_CUDA(cudaMemcpyAsync(&tiles, c.tile_start + p->n_seg, sizeof(tiles), cudaMemcpyDeviceToHost,
@@ -401,7 +429,6 @@ int segplan_config(SegPlan* p, uint64_t tile, uint64_t vg, uint64_t a, int rever
     }
     if (e != cudaSuccess) {
       cudaFree(c.tile_start);
-      cudaFree(c.win_rec);
       cudaFree(c.tile_seg);
       return cuda_fail(e, "segment plan: tile owners");
     }
@@ -494,7 +521,7 @@ extern "C" int scl_debug_window_records(const uint64_t* offsets, uint64_t n_segm
   if (!offsets || !count) return fail(SCL_ERR_ARG, "scl_debug_window_records: null argument");
   if (short_max == 0) return fail(SCL_ERR_ARG, "scl_debug_window_records: short_max must be positive");
   std::vector<uint64_t> rec;
-  segplan_window_records(offsets, n_segments, short_max, &rec);
+  segplan_window_records(offsets, n_segments, short_max, short_max, &rec);
   *count = rec.size() / 4;
   if (records) {
     if (capacity < *count) return fail(SCL_ERR_ARG, "scl_debug_window_records: capacity too small");

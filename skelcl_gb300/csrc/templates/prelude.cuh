@@ -327,10 +327,6 @@ struct scl_vec_width {
                                 16 % S1 == 0 && 16 % S2 == 0) ? 16 / S : 1;
 };
 
-// Segment-plan windows: a vector of at most this many elements is folded or
-// scanned by one thread, a longer one by a warp.
-#define SCL_WIN_THREAD 256
-
 // Device-side status word: bit 0 = a bounded wait gave up.
 #define SCL_DEV_ERR_TIMEOUT 1u
 __device__ __forceinline__ void scl_raise(unsigned int* err, unsigned int bit) {

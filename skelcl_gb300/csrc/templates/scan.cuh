@@ -463,45 +463,73 @@ __device__ __forceinline__ void scl_scan_short_run(const scl_T* in, scl_O* out, 
   }
 }
 
-// Window role of a planned segmented scan (the blocks past the tiles): block
-// r takes window record r of the plan, {first vector, end vector, first
-// element, elements}: consecutive vectors of at most short_max elements that
-// start in one window of short_max elements (all but the last end inside
-// it, so the record spans at most 2 * short_max = TILE elements, one staged
-// tile).  The record's elements are brought into shared memory by bulk
-// asynchronous copies (element e0 + p at ts[p + shift]; bounded wait) while
-// each thread reads its first vector's offsets, and every vector is scanned
-// in place there: one of at most SCL_WIN_THREAD elements by
-// one thread, in element order; a longer one by a warp, in rounds of 32 x U
-// logical elements (lane l holds U consecutive ones; a reverse scan reads the
-// vector from its end), the lanes' totals scanned across the warp and rounds
-// chained by a carry.  Then the block stores the record's elements in order
-// (the vectors cover them).  f(earlier, later) throughout, in the element
-// type; the exclusive form starts from SCL_IDENTITY (neutral, as for the
-// tiles' padding).
-template <int TILE>
-__device__ __forceinline__ void scl_scan_window_run(const scl_T* in, scl_O* out, const scl_u64* seg_off,
-                                                    const scl_u64* win_rec, scl_u64 r,
-                                                    unsigned int flags, scl_T* ts, unsigned int bar_s,
-                                                    unsigned int spin_limit,
-                                                    unsigned int* err SCL_USER_PARAMS) {
-  constexpr int B = SCL_SCAN_B, NW = B / 32, U = 4;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const bool inclusive = (flags & 1u) != 0, reverse = (flags & 2u) != 0;
-  const scl_T ident = (scl_T)(SCL_IDENTITY);
-  const scl_u64 lo = win_rec[4 * r], top = win_rec[4 * r + 1], e0 = win_rec[4 * r + 2];
-  const scl_u64 ln = win_rec[4 * r + 3];
-  const int len = (int)(ln < (scl_u64)TILE ? ln : (scl_u64)TILE);  // (more only for bad offsets)
-  if (len == 0) return;  // (block-uniform) nothing to write for empty vectors
+// ---- windows of short segments (planned segmented Scan) --------------------
+// One block takes one window record r of the plan, {first vector, end vector,
+// first element, elements}: consecutive vectors of at most a quarter of a
+// tile that start in one window of 47/64 of a tile, all but the last ending
+// inside it, so that the record fits in one staged tile.
+// The record's elements come into shared memory by bulk asynchronous copies
+// (element e0 + p at ts[p + shift]; bounded wait) while the threads mark, in
+// a bit mask, where the vectors start in logical order (their last elements
+// for a reverse scan).  Then the whole record is scanned at once as one
+// segmented scan, whatever the vectors' lengths: rows of 32 x E elements, one
+// per warp at a time, E consecutive ones per lane (two 16-byte vectors), a
+// start bit cutting the running fold; the lanes' tails are scanned across
+// the warp back to the nearest lane that holds a start, the rows' tails
+// across one warp, and an element before its row's first start takes the
+// row's carry when it is read back.  f(earlier, later) throughout, in the
+// element type; the identity only fills positions outside the record.
+// Bound by memory (8 bytes an element), then by issue: 10^6 vectors of 1..199
+// floats 0.211 -> 0.133 ms (flat 0.142), 10^7 of 0..2 0.352 -> 0.048 ms,
+// 66,666 of 1000..1999 0.284 -> 0.133 ms against one thread per vector of up
+// to 256 elements (about 40 busy threads of a block's 256, each a chain of
+// shared-memory round trips) and a warp per longer one.
+template <typename T, int TILE>
+struct scl_win {
+  static constexpr int V = scl_vec_width<sizeof(T)>::value;
+  static constexpr int E = 2 * V;           // elements per lane and row
+  static constexpr int ROW = 32 * E;
+  static constexpr int ROWS = TILE / ROW + 1;  // (a record keeps its 16-byte phase)
+  unsigned int mask[ROWS * ROW / 32];       // bit p: a vector starts at ts[p]
+  T carry[ROWS];                            // a row's tail, then the carry into it
+  int head[ROWS];                           // the row's first start (ROW: none)
+};
+
+// The block's record in shared memory, its starts marked; false after a
+// wait that gave up.  Ends with a block barrier.
+template <typename T, int TILE, int B>
+__device__ __forceinline__ bool scl_win_open(const T* in, const scl_u64* seg_off, scl_u64 lo, scl_u64 top,
+                                             scl_u64 e0, int len, bool reverse, const T& ident, T* ts,
+                                             scl_win<T, TILE>& w, unsigned int bar_s, unsigned int spin_limit,
+                                             unsigned int* err, int* shift_out) {
+  typedef scl_win<T, TILE> W;
   __shared__ int s_ok;
   unsigned int tx;
-  const int shift = scl_stage_bulk<scl_T, B>(in + e0, len, ts, bar_s, &tx);
+  const int shift = scl_stage_bulk<T, B>(in + e0, len, ts, bar_s, &tx);
+  *shift_out = shift;
   // this thread's first vector's offsets are read while the copy lands
   scl_u64 sg = lo + threadIdx.x;
-  scl_u64 a_n = 0, b_n = 0;
+  scl_u64 a = 0, b = 0;
   if (sg < top) {
-    a_n = seg_off[sg];
-    b_n = seg_off[sg + 1];
+    a = seg_off[sg];
+    b = seg_off[sg + 1];
+  }
+  for (int i = threadIdx.x; i < W::ROWS * W::ROW / 32; i += B) w.mask[i] = 0u;
+  const int P = shift + len, PT = (P + W::E - 1) / W::E * W::E;
+  if ((int)threadIdx.x < shift) ts[threadIdx.x] = ident;
+  if ((int)threadIdx.x < PT - P) ts[P + threadIdx.x] = ident;
+  __syncthreads();
+  while (sg < top) {
+    // (outside the record only for offsets changed since the plan)
+    if (b > a && a >= e0 && b <= e0 + (scl_u64)len) {
+      const int p = (int)((reverse ? b - 1 : a) - e0) + shift;
+      atomicOr(&w.mask[p >> 5], 1u << (p & 31));
+    }
+    sg += B;
+    if (sg < top) {
+      a = seg_off[sg];
+      b = seg_off[sg + 1];
+    }
   }
   if (threadIdx.x == 0) {
     bool ok = tx == 0u || scl_mbar_wait(bar_s, spin_limit);
@@ -512,74 +540,192 @@ __device__ __forceinline__ void scl_scan_window_run(const scl_T* in, scl_O* out,
     s_ok = ok ? 1 : 0;
   }
   __syncthreads();
-  if (!s_ok) return;
-  // short vectors: a thread each, in place
-  for (; sg < top; sg += B) {
-    const scl_u64 a = a_n, b = b_n;
-    if (sg + B < top) {
-      a_n = seg_off[sg + B];
-      b_n = seg_off[sg + B + 1];
-    }
-    if (b <= a || b - a > SCL_WIN_THREAD || a < e0 || b > e0 + (scl_u64)len) continue;
-    const int nv = (int)(b - a);
-    scl_T* v = ts + (int)(a - e0) + shift;
-    const int step = reverse ? -1 : 1;
-    if (reverse) v += nv - 1;
-    scl_T acc = v[0];
-    if (!inclusive) v[0] = ident;
-#pragma unroll 4
-    for (int e = 1; e < nv; ++e) {
-      const scl_T x = v[e * step];
-      if (inclusive) {
-        acc = SCL_FUNC(acc, x SCL_OP_ARGS);
-        v[e * step] = acc;
-      } else {
-        v[e * step] = acc;
-        acc = SCL_FUNC(acc, x SCL_OP_ARGS);
-      }
-    }
+  return s_ok != 0;
+}
+
+// Segmented scan across a warp: lane l's t becomes the fold of the t of lanes
+// start .. l, start = the nearest lane at or below l whose bit is set in
+// `starts` (0 if none).
+template <typename T>
+__device__ __forceinline__ T scl_warp_segscan(T t, unsigned int starts SCL_USER_PARAMS) {
+  const int lane = threadIdx.x & 31;
+  const unsigned int below = starts & (0xffffffffu >> (31 - lane));
+  const int start = below ? 31 - __clz((int)below) : 0;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const T o = scl_shfl_up(t, off);
+    if (lane - off >= start) t = SCL_FUNC(o, t SCL_OP_ARGS);
   }
-  // longer vectors: warp w takes vectors lo + w, lo + w + NW, ... (its next
-  // 32 offset pairs read at once, one per lane)
-  for (scl_u64 g = lo + warp; g < top; g += (scl_u64)NW * 32) {
-    const scl_u64 mine = g + (scl_u64)NW * lane;
-    scl_u64 a_l = 0, b_l = 0;
-    if (mine < top) {
-      a_l = seg_off[mine];
-      b_l = seg_off[mine + 1];
-    }
-    const int cnt = (int)((top - g + NW - 1) / NW < 32 ? (top - g + NW - 1) / NW : 32);
-    for (int k = 0; k < cnt; ++k) {
-      const scl_u64 a = __shfl_sync(0xffffffffu, a_l, k), b = __shfl_sync(0xffffffffu, b_l, k);
-      if (b <= a || b - a <= SCL_WIN_THREAD) continue;  // (empty, or a thread's above)
-      if (a < e0 || b > e0 + (scl_u64)len) continue;  // (only for offsets changed since the plan)
-      const int pa = (int)(a - e0) + shift, nv = (int)(b - a);
-      // logical element e of the vector sits at ts[at(e)]
-      auto at = [&](int e) { return reverse ? pa + nv - 1 - e : pa + e; };
-      scl_T carry = ident;
-      for (int b0 = 0; b0 < nv; b0 += 32 * U) {
-        const int eb = b0 + lane * U;
-        scl_T v[U];
+  return t;
+}
+
+// Scans positions 0 .. P - 1 of the record in place (REV: from the end), up
+// to the carries into the rows (scl_win_at applies them).  Ends with a block
+// barrier.
+template <int REV, typename T, int TILE, int B>
+__device__ __forceinline__ void scl_win_scan(T* ts, unsigned int P, const T& ident,
+                                             scl_win<T, TILE>& w SCL_USER_PARAMS) {
+  typedef scl_win<T, TILE> W;
+  constexpr int V = W::V, E = W::E;
+  const unsigned int lane = threadIdx.x & 31u, warp = threadIdx.x >> 5;
+  const unsigned int chunks = (P + E - 1) / E, rows = (chunks + 31u) / 32u;
+  for (unsigned int row = warp; row < rows; row += B / 32) {
+    const unsigned int j = row * 32u + lane;
+    const unsigned int pos = (REV ? chunks - 1u - j : j) * E;
+    T x[E];  // in logical order
+    unsigned int hd = 0;
+    if (j < chunks) {
+      const scl_pack<T, V> p0 = scl_load<T, V>(ts + pos);
+      const scl_pack<T, V> p1 = scl_load<T, V>(ts + pos + V);
 #pragma unroll
-        for (int u = 0; u < U; ++u) v[u] = eb + u < nv ? ts[at(eb + u)] : ident;
-#pragma unroll
-        for (int u = 1; u < U; ++u) v[u] = SCL_FUNC(v[u - 1], v[u] SCL_OP_ARGS);
-        const scl_T tot = scl_warp_incl(v[U - 1] SCL_EXTRA_ARGS);
-        scl_T lane_excl = scl_shfl_up(tot, 1);
-        if (lane == 0) lane_excl = ident;
-        const scl_T pre = SCL_FUNC(carry, lane_excl SCL_OP_ARGS);
-#pragma unroll
-        for (int u = 0; u < U; ++u) {
-          if (eb + u < nv)
-            ts[at(eb + u)] = inclusive ? SCL_FUNC(pre, v[u] SCL_OP_ARGS)
-                                       : (u == 0 ? pre : SCL_FUNC(pre, v[u - 1] SCL_OP_ARGS));
-        }
-        carry = SCL_FUNC(carry, scl_shfl_idx(tot, 31) SCL_OP_ARGS);
+      for (int e = 0; e < V; ++e) {
+        x[REV ? E - 1 - e : e] = p0.v[e];
+        x[REV ? V - 1 - e : V + e] = p1.v[e];
       }
+      hd = w.mask[pos >> 5] >> (pos & 31u);
+      if (REV) hd = __brev(hd << (32 - E));
+      else if (E < 32) hd &= (1u << (E & 31)) - 1u;
+    } else {
+#pragma unroll
+      for (int e = 0; e < E; ++e) x[e] = ident;
+    }
+#pragma unroll
+    for (int e = 1; e < E; ++e)
+      if (!((hd >> e) & 1u)) x[e] = SCL_FUNC(x[e - 1], x[e] SCL_OP_ARGS);
+    const unsigned int starts = __ballot_sync(0xffffffffu, hd != 0u);
+    const T t = scl_warp_segscan(x[E - 1], starts SCL_EXTRA_ARGS);
+    const T cin = scl_shfl_up(t, 1);
+    const int first = hd ? __ffs((int)hd) - 1 : E;  // elements the lanes before reach into
+    if (lane != 0) {
+#pragma unroll
+      for (int e = 0; e < E; ++e)
+        if (e < first) x[e] = SCL_FUNC(cin, x[e] SCL_OP_ARGS);
+    }
+    if (j < chunks) {
+      scl_pack<T, V> p0, p1;
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        p0.v[e] = x[REV ? E - 1 - e : e];
+        p1.v[e] = x[REV ? V - 1 - e : V + e];
+      }
+      scl_store<T, V>(ts + pos, p0);
+      scl_store<T, V>(ts + pos + V, p1);
+    }
+    const int fl = starts ? __ffs((int)starts) - 1 : 0;
+    const int fe = __shfl_sync(0xffffffffu, first, fl);
+    if (lane == 31u) {
+      w.carry[row] = t;
+      w.head[row] = starts ? fl * E + fe : W::ROW;
     }
   }
   __syncthreads();
-  for (int p = threadIdx.x; p < len; p += B) out[e0 + p] = SCL_EPILOGUE(ts[p + shift]);
+  if (warp == 0) {
+    T carry = ident;
+    for (unsigned int r0 = 0; r0 < rows; r0 += 32) {
+      const unsigned int r = r0 + lane;
+      const bool in_row = r < rows;
+      T t = in_row ? w.carry[r] : ident;
+      const unsigned int starts = __ballot_sync(0xffffffffu, in_row && w.head[in_row ? r : 0] < W::ROW);
+      t = scl_warp_segscan(t, starts SCL_EXTRA_ARGS);
+      const unsigned int below = starts & (0xffffffffu >> (31u - lane));
+      if (r0 > 0 && below == 0u) t = SCL_FUNC(carry, t SCL_OP_ARGS);
+      const T prev = scl_shfl_up(t, 1);
+      if (in_row) w.carry[r] = lane == 0 ? carry : prev;
+      carry = scl_shfl_idx(t, 31);
+    }
+  }
+  __syncthreads();
+}
+
+// The scanned value at ts[p].
+template <int REV, typename T, int TILE>
+__device__ __forceinline__ T scl_win_at(const T* ts, unsigned int p, unsigned int P,
+                                        const scl_win<T, TILE>& w SCL_USER_PARAMS) {
+  typedef scl_win<T, TILE> W;
+  const unsigned int l = REV ? (P + W::E - 1) / W::E * W::E - 1 - p : p;
+  const unsigned int row = l / W::ROW;
+  T v = ts[p];
+  if ((int)(l % W::ROW) < w.head[row]) v = SCL_FUNC(w.carry[row], v SCL_OP_ARGS);
+  return v;
+}
+
+// Scans the opened record and stores it: out[e0 - shift + p] for position p,
+// 16 bytes at a time where `out` shares the input's 16-byte phase.
+template <int REV, int TILE>
+__device__ __forceinline__ void scl_scan_window_store(scl_T* ts, scl_u64 e0, int shift, int len, bool inclusive,
+                                                      scl_win<scl_T, TILE>& w, scl_O* out SCL_USER_PARAMS) {
+  constexpr int B = SCL_SCAN_B;
+  typedef scl_win<scl_T, TILE> W;
+  constexpr int V = W::V;
+  const scl_T ident = (scl_T)(SCL_IDENTITY);
+  const unsigned int P = (unsigned int)(shift + len), PT = (P + W::E - 1) / W::E * W::E;
+  scl_win_scan<REV, scl_T, TILE, B>(ts, P, ident, w SCL_EXTRA_ARGS);
+  const scl_u64 ob = (scl_u64)out + e0 * sizeof(scl_O) - (scl_u64)shift * sizeof(scl_O);
+  const bool ovec = sizeof(scl_O) == sizeof(scl_T) && (ob & 15u) == 0;
+  for (unsigned int p0 = threadIdx.x * V; p0 < P; p0 += B * V) {
+    // (V positions of one lane's chunk: one row; they take the row's carry
+    // up to its first start)
+    const unsigned int l0 = REV ? PT - 1u - p0 : p0, row = l0 / W::ROW;
+    const int d = w.head[row] - (int)(l0 % W::ROW);
+    scl_pack<scl_T, V> v = scl_load<scl_T, V>(ts + p0);
+    if (REV ? d > 1 - V : d > 0) {
+      const scl_T c = w.carry[row];
+#pragma unroll
+      for (int e = 0; e < V; ++e)
+        if (REV ? d > -e : d > e) v.v[e] = SCL_FUNC(c, v.v[e] SCL_OP_ARGS);
+    }
+    scl_pack<scl_O, V> m;
+    if (inclusive) {
+#pragma unroll
+      for (int e = 0; e < V; ++e) m.v[e] = SCL_EPILOGUE(v.v[e]);
+    } else {
+      // the value before (after, for a reverse scan), or the identity at a start
+      scl_T prev = ident;
+      if (REV ? p0 + V < P : p0 > 0)
+        prev = scl_win_at<REV>(ts, REV ? p0 + V : p0 - 1u, P, w SCL_EXTRA_ARGS);
+      const unsigned int bits = w.mask[p0 >> 5] >> (p0 & 31u);
+#pragma unroll
+      for (int e = 0; e < V; ++e) {
+        const scl_T before = REV ? (e + 1 < V ? v.v[e + 1 < V ? e + 1 : e] : prev)
+                                 : (e > 0 ? v.v[e > 0 ? e - 1 : 0] : prev);
+        const scl_T val = (bits >> e) & 1u ? ident : before;
+        m.v[e] = SCL_EPILOGUE(val);
+      }
+    }
+    if (ovec && p0 >= (unsigned int)shift && p0 + V <= P) {
+      scl_store<scl_O, V>(reinterpret_cast<scl_O*>(ob) + p0, m);
+    } else {
+#pragma unroll
+      for (int e = 0; e < V; ++e)
+        if (p0 + e >= (unsigned int)shift && p0 + e < P) out[e0 + (p0 + e - (unsigned int)shift)] = m.v[e];
+    }
+  }
+}
+
+// Window role of a planned segmented scan (the blocks past the tiles; see
+// scl_win): the record's vectors are scanned in place and stored in order
+// (they cover the record).  The exclusive form starts from SCL_IDENTITY.
+template <int TILE>
+__device__ __forceinline__ void scl_scan_window_run(const scl_T* in, scl_O* out, const scl_u64* seg_off,
+                                                    const scl_u64* win_rec, scl_u64 r,
+                                                    unsigned int flags, scl_T* ts, unsigned int bar_s,
+                                                    unsigned int spin_limit,
+                                                    unsigned int* err SCL_USER_PARAMS) {
+  constexpr int B = SCL_SCAN_B;
+  typedef scl_win<scl_T, TILE> W;
+  const bool inclusive = (flags & 1u) != 0, reverse = (flags & 2u) != 0;
+  const scl_T ident = (scl_T)(SCL_IDENTITY);
+  __shared__ W w;
+  const scl_u64 lo = win_rec[4 * r], top = win_rec[4 * r + 1], e0 = win_rec[4 * r + 2];
+  const scl_u64 ln = win_rec[4 * r + 3];
+  const int len = (int)(ln < (scl_u64)TILE ? ln : (scl_u64)TILE);  // (more only for bad offsets)
+  if (len == 0) return;  // (block-uniform) nothing to write for empty vectors
+  int shift;
+  if (!scl_win_open<scl_T, TILE, B>(in, seg_off, lo, top, e0, len, reverse, ident, ts, w, bar_s, spin_limit,
+                                    err, &shift))
+    return;
+  if (reverse) scl_scan_window_store<1, TILE>(ts, e0, shift, len, inclusive, w, out SCL_EXTRA_ARGS);
+  else scl_scan_window_store<0, TILE>(ts, e0, shift, len, inclusive, w, out SCL_EXTRA_ARGS);
 }
 
 // The warp-per-segment kernel on its own (segmented launches without a
