@@ -27,6 +27,7 @@ template <typename T>
 __global__ void broadcast_kernel(const T* __restrict__ g, T* __restrict__ gx, uint64_t n, int acc,
                                  int aligned) {
   constexpr int V = 16 / sizeof(T);
+  dependency_wait();
   const T v = *g;
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
@@ -54,6 +55,7 @@ template <typename T>
 __global__ void accumulate_kernel(T* __restrict__ dst, const T* __restrict__ src, uint64_t n,
                                   int aligned) {
   constexpr int V = 16 / sizeof(T);
+  dependency_wait();
   const uint64_t tid = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   const uint64_t nth = (uint64_t)gridDim.x * blockDim.x;
   const uint64_t nvec = aligned ? n / V : 0;
@@ -76,29 +78,14 @@ __global__ void accumulate_kernel(T* __restrict__ dst, const T* __restrict__ src
 // in[clamp(y+dy)][clamp(x+dx)]; every read position p' outside the matrix
 // was served by the edge pixel clamp(p').  Its adjoint therefore adds, to each
 // edge pixel p, the zero-padded transposed stencil of g evaluated at every
-// outside position p' with clamp(p') = p.  One warp per edge pixel: the lanes
-// share the taps, loop over the outside positions, and add their sums with
-// shuffles.
-__global__ void stencil_edges_kernel(const float* __restrict__ g, const float* __restrict__ w,
-                                     float* __restrict__ gin, int64_t rows, int64_t cols, int R,
-                                     int64_t n_edge) {
-  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+// outside position p' with clamp(p') = p.
+
+// One edge pixel (y, x), any of them, by one warp: the lanes share the taps,
+// loop over the outside positions, and add their sums with shuffles.
+__device__ __forceinline__ void edge_pixel(const float* __restrict__ g, const float* __restrict__ w,
+                                           float* __restrict__ gin, int64_t rows, int64_t cols, int R, int64_t y,
+                                           int64_t x) {
   const int lane = threadIdx.x & 31;
-  if (e >= n_edge) return;  // whole warps leave together (blockDim is a multiple of 32)
-  int64_t y, x;
-  // top row, bottom row (rows > 1), left column, right column (cols > 1),
-  // the columns without their first and last pixels
-  const int64_t inner = rows > 2 ? rows - 2 : 0;
-  if (e < cols) {
-    y = 0; x = e;
-  } else if (rows > 1 && e < 2 * cols) {
-    y = rows - 1; x = e - cols;
-  } else {
-    const int64_t base = rows > 1 ? 2 * cols : cols;
-    const int64_t k = e - base;
-    if (k < inner) { y = 1 + k; x = 0; }
-    else { y = 1 + (k - inner); x = cols - 1; }
-  }
   const int64_t y0 = (y == 0) ? -R : y, y1 = (y == rows - 1) ? rows - 1 + R : y;
   const int64_t x0 = (x == 0) ? -R : x, x1 = (x == cols - 1) ? cols - 1 + R : x;
   const int W = 2 * R + 1;
@@ -121,6 +108,65 @@ __global__ void stencil_edges_kernel(const float* __restrict__ g, const float* _
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) acc += __shfl_down_sync(0xffffffffu, acc, o);
   if (lane == 0) gin[y * cols + x] += acc;
+}
+
+// A matrix of one row or one column: every pixel is an edge pixel.
+__global__ void line_edges_kernel(const float* __restrict__ g, const float* __restrict__ w,
+                                  float* __restrict__ gin, int64_t rows, int64_t cols, int R) {
+  dependency_wait();
+  const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  if (e >= rows * cols) return;  // whole warps leave together (blockDim is a multiple of 32)
+  edge_pixel(g, w, gin, rows, cols, R, e / cols, e % cols);
+}
+
+// Rows and columns >= 2.  An edge pixel that is no corner has its outside
+// positions on one line, 1 .. R steps out, and of g only the R lines nearest
+// the edge reach them; line k enters with the weights of steps 1 .. R - k
+// added up, R x (2R+1) sums that each block makes once in shared memory (for
+// R = 5, 55 taps a pixel instead of 165 products over 605 positions).  One
+// thread per pixel of the side (blockIdx.y: top, bottom, left, right), the
+// four corners by a warp each.  Bound by latency: 8192 x 8192, R = 5, 41 ->
+// 7 us of a 629 us blur with its gradient, against a warp per pixel.
+constexpr int kEdgeThreads = 128;
+__global__ void __launch_bounds__(kEdgeThreads)
+stencil_edges_kernel(const float* __restrict__ g, const float* __restrict__ w, float* __restrict__ gin,
+                     int64_t rows, int64_t cols, int R) {
+  extern __shared__ float sums[];  // [line k][step along the edge]
+  const int W = 2 * R + 1, side = blockIdx.y;
+  dependency_wait();
+  if (side == 4) {  // corners
+    const int warp = threadIdx.x >> 5;
+    if (blockIdx.x == 0 && warp < 4)
+      edge_pixel(g, w, gin, rows, cols, R, (warp & 1) ? rows - 1 : 0, (warp & 2) ? cols - 1 : 0);
+    return;
+  }
+  const int64_t n = side < 2 ? cols : rows, depth = side < 2 ? rows : cols;
+  if ((int64_t)blockIdx.x * kEdgeThreads >= n) return;  // (block-uniform)
+  // the tap from step d outside to line k inside is k + d lines (columns)
+  // forward, backward on the bottom and the right
+  for (int i = threadIdx.x; i < R * W; i += kEdgeThreads) {
+    const int k = i / W, t = i % W;
+    float s = 0.0f;
+    for (int d = 1; d <= R - k; ++d) {
+      const int far = (side & 1) ? R - (k + d) : R + (k + d);
+      s += side < 2 ? w[far * W + t] : w[t * W + far];
+    }
+    sums[i] = s;
+  }
+  __syncthreads();
+  const int64_t e = (int64_t)blockIdx.x * kEdgeThreads + threadIdx.x;
+  if (e == 0 || e >= n - 1) return;  // a corner, or past the side
+  const int64_t along = side < 2 ? 1 : cols, inward = (side & 1) ? (side < 2 ? -cols : -1) : (side < 2 ? cols : 1);
+  const int64_t edge = ((side & 1) ? (side < 2 ? (rows - 1) * cols : cols - 1) : 0) + e * along;
+  const int lines = depth < R ? (int)depth : R;
+  const int t0 = e < R ? (int)(R - e) : 0, t1 = n - 1 - e < R ? (int)(R + (n - 1 - e)) : 2 * R;
+  float acc = 0.0f;
+  for (int k = 0; k < lines; ++k) {
+    const float* line = g + edge + k * inward - R * along;
+#pragma unroll 4
+    for (int t = t0; t <= t1; ++t) acc += sums[k * W + t] * line[t * along];
+  }
+  gin[edge] += acc;
 }
 
 template <typename T>
@@ -172,12 +218,11 @@ extern "C" int scl_adjoint_broadcast(const void* g, void* gx, uint64_t n, int dt
   const int V = 16 / dtype_size(dtype);
   const int grid = grid_for(aligned ? (n + V - 1) / V : n);
   const int acc = accumulate ? 1 : 0;
-  if (dtype == SCL_DTYPE_F32)
-    broadcast_kernel<float><<<grid, kBlock, 0, rt().stream>>>((const float*)g, (float*)gx, n, acc, aligned);
-  else
-    broadcast_kernel<double><<<grid, kBlock, 0, rt().stream>>>((const double*)g, (double*)gx, n, acc, aligned);
-  SCL_CUDA(cudaGetLastError());
-  ++rt().launches;
+  SCL_CUDA(dtype == SCL_DTYPE_F32
+               ? launch_overlapped(broadcast_kernel<float>, dim3(grid), dim3(kBlock), 0, rt().stream,
+                                   (const float*)g, (float*)gx, n, acc, aligned)
+               : launch_overlapped(broadcast_kernel<double>, dim3(grid), dim3(kBlock), 0, rt().stream,
+                                   (const double*)g, (double*)gx, n, acc, aligned));
   return SCL_OK;
 }
 
@@ -189,12 +234,11 @@ extern "C" int scl_adjoint_accumulate(void* dst, const void* src, uint64_t n, in
   const int aligned = (aligned16(dst) && aligned16(src)) ? 1 : 0;
   const int V = 16 / dtype_size(dtype);
   const int grid = grid_for(aligned ? (n + V - 1) / V : n);
-  if (dtype == SCL_DTYPE_F32)
-    accumulate_kernel<float><<<grid, kBlock, 0, rt().stream>>>((float*)dst, (const float*)src, n, aligned);
-  else
-    accumulate_kernel<double><<<grid, kBlock, 0, rt().stream>>>((double*)dst, (const double*)src, n, aligned);
-  SCL_CUDA(cudaGetLastError());
-  ++rt().launches;
+  SCL_CUDA(dtype == SCL_DTYPE_F32
+               ? launch_overlapped(accumulate_kernel<float>, dim3(grid), dim3(kBlock), 0, rt().stream, (float*)dst,
+                                   (const float*)src, n, aligned)
+               : launch_overlapped(accumulate_kernel<double>, dim3(grid), dim3(kBlock), 0, rt().stream,
+                                   (double*)dst, (const double*)src, n, aligned));
   return SCL_OK;
 }
 
@@ -207,11 +251,16 @@ extern "C" int scl_mapoverlap_adjoint_edges(const float* g, const float* w, floa
   if (rows > (1ull << 40) || cols > (1ull << 40)) return fail(SCL_ERR_ARG, "stencil adjoint: matrix too large");
   if (R == 0) return SCL_OK;
   const int64_t r = (int64_t)rows, c = (int64_t)cols;
-  const int64_t n_edge = c + (r > 1 ? c : 0) + (r > 2 ? r - 2 : 0) * (c > 1 ? 2 : 1);
-  const int64_t grid = (n_edge + 7) / 8;  // 8 warps (edge pixels) per block
+  if (r < 2 || c < 2) {
+    const int64_t grid = (r * c + 7) / 8;  // 8 warps (edge pixels) per block
+    if (grid > 0x7fffffffll) return fail(SCL_ERR_ARG, "stencil adjoint: matrix too large");
+    SCL_CUDA(launch_overlapped(line_edges_kernel, dim3((unsigned)grid), dim3(256), 0, rt().stream, g, w, gin, r, c,
+                               R));
+    return SCL_OK;
+  }
+  const int64_t grid = ((r > c ? r : c) + kEdgeThreads - 1) / kEdgeThreads;
   if (grid > 0x7fffffffll) return fail(SCL_ERR_ARG, "stencil adjoint: matrix too large");
-  stencil_edges_kernel<<<(unsigned)grid, 256, 0, rt().stream>>>(g, w, gin, r, c, R, n_edge);
-  SCL_CUDA(cudaGetLastError());
-  ++rt().launches;
+  SCL_CUDA(launch_overlapped(stencil_edges_kernel, dim3((unsigned)grid, 5), dim3(kEdgeThreads),
+                             (size_t)R * (2 * R + 1) * sizeof(float), rt().stream, g, w, gin, r, c, R));
   return SCL_OK;
 }

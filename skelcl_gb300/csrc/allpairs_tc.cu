@@ -293,8 +293,6 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
   }
 }
 
-__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
 // Splits both operands, one 64 x 128 tile per step (grid-stride over A's
 // tiles, then B's).  Bound by memory: reads 4 bytes, writes 4 (FP16) or 6
 // (bf16, three parts) per element.  A row-major operand's tiles are taken
@@ -1034,37 +1032,13 @@ static int encode_parts(CUtensorMap* tm, const void* base, uint64_t rows, uint64
 }
 
 namespace {
-// Launch on the library stream, overlapped like the skeleton kernels (every
-// kernel here starts with dependency_wait()).
-template <typename... KArgs, typename... Args>
-cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, unsigned threads, size_t smem,
-                              cudaStream_t stream, const Args&... args) {
-  if (smem > 32 * 1024) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    if (e != cudaSuccess) return e;
-  }
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(threads);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = rt().pdl ? 1 : 0;
-  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
-  if (e == cudaSuccess) ++rt().launches;
-  return e;
-}
-
 template <int PARTS, int STAGES, int G, int BN_T>
 cudaError_t launch_gemm(dim3 grid, cudaStream_t stream, const CUtensorMap& tmA, const CUtensorMap& tmB,
                         float* P, uint32_t M, uint32_t N, uint32_t Kp, uint32_t spin_limit,
                         unsigned int* err, uint32_t tiles_n, uint32_t group_m) {
   using SH = tc::Shape<BN_T>;
   const size_t smem = (size_t)STAGES * PARTS * (SH::A_TILE + SH::B_TILE) + 1024;
-  return launch_overlapped(tc::gemm_3xbf16_kernel<PARTS, STAGES, G, BN_T>, grid, SH::THREADS, smem, stream,
+  return launch_overlapped(tc::gemm_3xbf16_kernel<PARTS, STAGES, G, BN_T>, grid, dim3(SH::THREADS), smem, stream,
                            tmA, tmB, P, M, N, Kp, spin_limit, err, tiles_n, group_m);
 }
 
@@ -1127,7 +1101,7 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
   if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, parts, tc::BM, bk, tc::kBf16)) return st;
   if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, parts, bn, bk, tc::kBf16)) return st;
   unsigned int* none = nullptr;
-  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), 256, 0, stream, sp.a, sp.b, K, Kp,
+  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp,
                                     parts, none, 0u, none);
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
   if (wide) {
@@ -1173,16 +1147,16 @@ int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, u
   if (int st = encode_parts(&tmA3, sp3.a.out, sp.Mp, Kp, 3, tc::BM, 32, tc::kBf16)) return st;
   if (int st = encode_parts(&tmB3, sp3.b.out, sp.Np, Kp, 3, 128, 32, tc::kBf16)) return st;
   unsigned int* none = nullptr;
-  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kF16>, split_grid(sp), 256, 0, stream, sp.a, sp.b, K, Kp, 2,
+  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kF16>, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp, 2,
                                     flags, epoch, none);
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
   const unsigned few = (unsigned)std::min<uint64_t>(split_tiles(sp), (uint64_t)rt().sm_count * 4);
-  e = launch_overlapped(tc::split_kernel<tc::kBf16>, dim3(few), 256, 0, stream, sp3.a, sp3.b, K, Kp, 3, flags, epoch,
+  e = launch_overlapped(tc::split_kernel<tc::kBf16>, dim3(few), dim3(256), 0, stream, sp3.a, sp3.b, K, Kp, 3, flags, epoch,
                         verdict);
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
   const tc::PairArgs args = {P,     sp.a.unscale, sp.b.unscale, verdict, err,        M,       N,      Kp,
                              sp.Mp, sp.Np,        epoch,        spin_limit, tiles.n, tiles.m, tiles.group};
-  e = launch_overlapped(tc::gemm_pair_kernel, dim3(2 * tiles.m * tiles.n), tc::kPairThreads, tc::kPairSmem, stream,
+  e = launch_overlapped(tc::gemm_pair_kernel, dim3(2 * tiles.m * tiles.n), dim3(tc::kPairThreads), tc::kPairSmem, stream,
                         tmA, tmB, tmA3, tmB3, args);
   if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
   return SCL_OK;
@@ -1203,7 +1177,7 @@ extern "C" int scl_debug_allpairs_split(const float* A, const float* B, uint32_t
   if (!A || !B || scratch_bytes < need) return fail(SCL_ERR_ARG, "split: null operand or scratch too small");
   const Split sp = split_of(A, B, M, N, K, tc::KPAD, parts, trans, scratch);
   unsigned int* none = nullptr;
-  SCL_CUDA(launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), 256, 0, rt().stream, sp.a, sp.b, K, sp.Kp,
+  SCL_CUDA(launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), dim3(256), 0, rt().stream, sp.a, sp.b, K, sp.Kp,
                              parts, none, 0u, none));
   return SCL_OK;
 }

@@ -214,6 +214,33 @@ int pack_extra(scl_program* p, CUfunction fn, size_t fixed, const unsigned char*
 // cuLaunchKernel on the library stream.
 int launch(CUfunction fn, dim3 grid, dim3 block, size_t smem, ArgPack& pack);
 
+// Launch of a precompiled kernel, overlapped like the skeleton kernels (with
+// scl::dependency_wait() ahead of its first access to memory).
+template <typename... KArgs, typename... Args>
+cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              const Args&... args) {
+  if (smem > 32 * 1024) {
+    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (e != cudaSuccess) return e;
+  }
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cfg.attrs = &attr;
+  cfg.numAttrs = rt().pdl ? 1 : 0;
+  cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
+  if (e == cudaSuccess) ++rt().launches;
+  return e;
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // Device status word bits (bit 0: a bounded wait gave up, set by the
 // generated kernels).
 constexpr unsigned int kDevErrSegments = 2u;  // segment offsets decreasing or past the end
