@@ -164,17 +164,188 @@ seg_tile_start_kernel(const uint64_t* off, uint64_t n_seg, uint64_t tile, uint64
 }
 
 // gx[i] (+)= g[s] for every element i of segment s (elements outside every
-// segment are left alone).  Each warp takes a chunk of CH elements: it finds
+// segment are left alone).  A block takes a run of consecutive chunks of CH
+// elements.  It finds the last segment starting at or before the run (256
+// probes per round) and then walks the segments from chunk to chunk: it marks
+// in a bit mask where the chunk's non-empty segments start, keeps their values
+// in order, and gives every element the value of the last start at or below
+// it: the mask's running count, one count per word and a popcount.  The next
+// chunk's first 256 segments are read while this one is stored.  Bound by
+// memory (4 bytes an element): 10^6 vectors of 1..199 floats 0.123 -> 0.081 ms,
+// 10^7 of 0..2 0.651 -> 0.116 ms, against broadcast_long_segments_kernel (a
+// search per chunk instead of per run: 0.107 and 0.137 ms).
+template <typename T>
+struct BroadcastChunk {
+  static constexpr int WORDS = 1024 / sizeof(T);  // mask words, one per thread at most
+  static constexpr int CH = WORDS * 32 - 32;      // a word to spare for gx's 16-byte phase
+};
+template <typename T>
+__global__ void __launch_bounds__(256)
+broadcast_segments_kernel(const T* __restrict__ g, T* __restrict__ gx, const uint64_t* __restrict__ off,
+                          uint64_t n_seg, uint64_t n_total, int acc, uint64_t run) {
+  constexpr int WORDS = BroadcastChunk<T>::WORDS, CH = BroadcastChunk<T>::CH, V = 16 / sizeof(T);
+  __shared__ unsigned int mask[WORDS];  // bit p: a segment starts at position p
+  __shared__ int before[WORDS];         // starts below the word
+  __shared__ int warp_sum[8];
+  __shared__ int cov_lo, cov_hi;        // positions covered by segments
+  __shared__ unsigned long long last;   // last segment that starts in or before the chunk
+  __shared__ T val[CH];                 // the segments' values, in order
+  const int tid = threadIdx.x, lane = tid & 31;
+  // position p = element c0 + p - phase, so that positions and gx share
+  // their 16-byte phase (CH is a multiple of V)
+  const int phase = (int)((reinterpret_cast<uintptr_t>(gx) & 15u) / sizeof(T));
+  dependency_wait();
+  uint64_t c0 = (uint64_t)blockIdx.x * run * CH;
+  const uint64_t end = c0 + run * CH < n_total ? c0 + run * CH : n_total;
+  if (c0 >= end) return;  // (block-uniform)
+  // last segment with off[s] <= c0 (0 if none): each round 256 offsets spread
+  // over [lo, hi] are probed and the count at or below c0 narrows it
+  // (decreasing offsets still end the search)
+  uint64_t lo = 0, hi = n_seg - 1;
+  while (lo < hi) {  // (block-uniform)
+    const uint64_t span = hi - lo;
+    const int below = __syncthreads_count(off[lo + 1 + span * (uint64_t)tid / 256] <= c0);
+    if (below == 0) {
+      hi = lo;
+    } else {
+      const uint64_t at = lo + 1 + span * (uint64_t)(below - 1) / 256;
+      hi = below < 256 ? lo + span * (uint64_t)below / 256 : hi;
+      lo = at;
+    }
+  }
+  // segment lo + tid: its offsets and value
+  uint64_t a = ~0ull, b = 0;
+  T v = T(0);
+  auto fetch = [&](uint64_t s) {
+    a = ~0ull;
+    if (s < n_seg) {
+      a = off[s];
+      b = off[s + 1];
+      v = g[s];
+    }
+  };
+  fetch(lo + tid);
+  for (; c0 < end; c0 += CH) {  // (block-uniform)
+    const uint64_t c1 = c0 + CH < end ? c0 + CH : end;
+    if (tid < WORDS) mask[tid] = 0u;
+    if (tid == 0) {
+      cov_lo = CH + V;
+      cov_hi = 0;
+      last = lo;
+    }
+    __syncthreads();
+    // the part [i0, i1) of the chunk, as positions, of the segment at hand
+    auto part = [&](int* i0, int* i1) {
+      *i0 = *i1 = 0;
+      if (a >= c1) return;
+      const uint64_t x0 = a > c0 ? a : c0, x1 = b < c1 ? b : c1;
+      if (x0 < x1) {
+        *i0 = (int)(x0 - c0) + phase;
+        *i1 = (int)(x1 - c0) + phase;
+      }
+    };
+    int f0 = 0, f1 = 0;  // this thread's first segment
+    const T fv = v;
+    bool many = false;   // more than 256 segments
+    for (uint64_t base = lo;; base += 256) {  // (block-uniform)
+      int i0, i1;
+      part(&i0, &i1);
+      if (base == lo) {
+        f0 = i0;
+        f1 = i1;
+      }
+      if (i0 < i1) atomicOr(&mask[i0 >> 5], 1u << (i0 & 31));
+      const int wl = __reduce_min_sync(0xffffffffu, i0 < i1 ? i0 : CH + V);
+      const int wh = __reduce_max_sync(0xffffffffu, i1);
+      const unsigned int starts = __ballot_sync(0xffffffffu, a < c1);
+      if (lane == 0) {
+        if (wh > 0) {
+          atomicMin(&cov_lo, wl);
+          atomicMax(&cov_hi, wh);
+        }
+        if (starts) atomicMax(&last, (unsigned long long)(base + tid + 31 - __clz((int)starts)));
+      }
+      if (!__syncthreads_or(tid == 255 && a < c1)) break;
+      many = true;
+      fetch(base + 256 + tid);
+    }
+    // starts below each word
+    const int cnt = tid < WORDS ? __popc(mask[tid]) : 0;
+    int incl = cnt;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+      const int o = __shfl_up_sync(0xffffffffu, incl, d);
+      if (lane >= d) incl += o;
+    }
+    if (lane == 31) warp_sum[tid >> 5] = incl;
+    __syncthreads();
+    int base_cnt = 0;
+    for (int w = 0; w < (tid >> 5); ++w) base_cnt += warp_sum[w];
+    if (tid < WORDS) before[tid] = base_cnt + incl - cnt;
+    __syncthreads();
+    // the last start at or below position p
+    auto rank = [&](int p) { return before[p >> 5] + __popc(mask[p >> 5] & (0xffffffffu >> (31 - (p & 31)))) - 1; };
+    if (f0 < f1) val[rank(f0)] = fv;
+    const uint64_t next = last;
+    if (many) {
+      for (uint64_t base = lo + 256; base <= next; base += 256) {  // (block-uniform)
+        fetch(base + tid);
+        int i0, i1;
+        part(&i0, &i1);
+        if (i0 < i1) val[rank(i0)] = v;
+      }
+    }
+    lo = next;
+    fetch(lo + tid);  // the next chunk's
+    __syncthreads();
+    T* const out = gx + c0 - phase;
+    const int lo_p = cov_lo, hi_p = cov_hi;
+    for (int p = (lo_p / V + tid) * V; p < hi_p; p += 256 * V) {
+      if (p >= lo_p && p + V <= hi_p) {
+        int r = rank(p);
+        const unsigned int starts = (mask[p >> 5] >> (p & 31)) >> 1;  // at p + 1 ..
+        T x[V];
+        x[0] = val[r];
+#pragma unroll
+        for (int e = 1; e < V; ++e) {
+          r += (int)((starts >> (e - 1)) & 1u);
+          x[e] = val[r];
+        }
+        if (acc) {
+          const uint4 w = *reinterpret_cast<const uint4*>(out + p);
+          T y[V];
+          memcpy(y, &w, 16);
+#pragma unroll
+          for (int e = 0; e < V; ++e) x[e] += y[e];
+        }
+        uint4 w;
+        memcpy(&w, x, 16);
+        *reinterpret_cast<uint4*>(out + p) = w;
+      } else {
+        for (int e = 0; e < V; ++e)
+          if (p + e >= lo_p && p + e < hi_p) {
+            const T u = val[rank(p + e)];
+            out[p + e] = acc ? out[p + e] + u : u;
+          }
+      }
+    }
+    __syncthreads();
+  }
+}
+
+// The same for long segments: each warp takes a chunk of CH elements: it finds
 // the last segment starting at or before the chunk (a search of the warp, 32
 // probes per round), then walks the segments that start before the chunk's
 // end, the offsets and values of 32 of them read at once, and writes each
 // one's part of the chunk with lane-strided stores (16 bytes at a time when
 // gx is 16-byte aligned, single elements at the part's ragged ends).
+constexpr int kBroadcastWarp = 1024;
 template <typename T>
 __global__ void __launch_bounds__(256)
-broadcast_segments_kernel(const T* __restrict__ g, T* __restrict__ gx, const uint64_t* __restrict__ off,
+broadcast_long_segments_kernel(const T* __restrict__ g, T* __restrict__ gx, const uint64_t* __restrict__ off,
                           uint64_t n_seg, uint64_t n_total, int acc, int aligned) {
-  constexpr int CH = 1024, V = 16 / sizeof(T);
+  constexpr int CH = kBroadcastWarp, V = 16 / sizeof(T);
+  dependency_wait();
   const int lane = threadIdx.x & 31;
   const uint64_t c0 = (((uint64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5) * CH;
   if (c0 >= n_total) return;  // (warp-uniform)
@@ -501,18 +672,34 @@ extern "C" int scl_adjoint_broadcast_segments(const void* g, void* gx, const uin
     return fail(SCL_ERR_ARG, "segmented broadcast: dtype must be SCL_DTYPE_F32 or _F64");
   if (n == 0 || n_segments == 0) return SCL_OK;
   if (!g || !gx || !seg_offsets) return fail(SCL_ERR_ARG, "segmented broadcast: null pointer");
-  const uint64_t blocks = (n + 8191) / 8192;  // 8 warps of 1024 elements each
-  if (blocks > 0x7fffffffull) return fail(SCL_ERR_ARG, "segmented broadcast: vector too large");
   const int acc = accumulate ? 1 : 0;
-  const int aligned = (reinterpret_cast<uintptr_t>(gx) & 15u) == 0 ? 1 : 0;
-  if (dtype == SCL_DTYPE_F32)
-    broadcast_segments_kernel<float><<<(unsigned)blocks, 256, 0, rt().stream>>>(
-        (const float*)g, (float*)gx, seg_offsets, n_segments, n, acc, aligned);
-  else
-    broadcast_segments_kernel<double><<<(unsigned)blocks, 256, 0, rt().stream>>>(
-        (const double*)g, (double*)gx, seg_offsets, n_segments, n, acc, aligned);
-  SCL_CUDA(cudaGetLastError());
-  ++rt().launches;
+  // a warp per 1024 elements walks long segments at the speed of plain stores,
+  // but spends 40 instructions an element on short ones: 10^8 floats in
+  // vectors of 100 on average 123 us against 81 for the chunks, of 300 64
+  // against 70, of 1500 62 against 70
+  const bool long_segments = n / n_segments >= 200;
+  if (long_segments) {
+    const uint64_t blocks = (n + 8 * kBroadcastWarp - 1) / (8 * kBroadcastWarp);
+    if (blocks > 0x7fffffffull) return fail(SCL_ERR_ARG, "segmented broadcast: vector too large");
+    const dim3 grid((unsigned)blocks);
+    const int aligned = (reinterpret_cast<uintptr_t>(gx) & 15u) == 0 ? 1 : 0;
+    SCL_CUDA(dtype == SCL_DTYPE_F32
+                 ? launch_overlapped(broadcast_long_segments_kernel<float>, grid, dim3(256), 0, rt().stream,
+                                     (const float*)g, (float*)gx, seg_offsets, n_segments, n, acc, aligned)
+                 : launch_overlapped(broadcast_long_segments_kernel<double>, grid, dim3(256), 0, rt().stream,
+                                     (const double*)g, (double*)gx, seg_offsets, n_segments, n, acc, aligned));
+    return SCL_OK;
+  }
+  // one wave of blocks (6 per SM by their shared memory), each a run of chunks
+  const uint64_t chunk = dtype == SCL_DTYPE_F32 ? BroadcastChunk<float>::CH : BroadcastChunk<double>::CH;
+  const uint64_t chunks = (n + chunk - 1) / chunk, wave = (uint64_t)rt().sm_count * 6;
+  const uint64_t run = (chunks + wave - 1) / wave, blocks = (chunks + run - 1) / run;
+  const dim3 grid((unsigned)blocks);
+  SCL_CUDA(dtype == SCL_DTYPE_F32
+               ? launch_overlapped(broadcast_segments_kernel<float>, grid, dim3(256), 0, rt().stream,
+                                   (const float*)g, (float*)gx, seg_offsets, n_segments, n, acc, run)
+               : launch_overlapped(broadcast_segments_kernel<double>, grid, dim3(256), 0, rt().stream,
+                                   (const double*)g, (double*)gx, seg_offsets, n_segments, n, acc, run));
   return SCL_OK;
 }
 
