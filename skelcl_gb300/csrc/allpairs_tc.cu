@@ -140,6 +140,16 @@ __device__ __forceinline__ void tmem_load16(uint32_t taddr, uint32_t (&r)[16]) {
       : "memory");
 }
 
+// The address of `addr` (shared memory) in CTA `rank` of the cluster.
+__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
+  uint32_t r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
+  return r;
+}
+__device__ __forceinline__ void cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned; barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+
 __device__ __forceinline__ void raise(unsigned int* err) {
   if (err) atomicOr(err, 1u);
 }
@@ -305,6 +315,9 @@ __global__ void __launch_bounds__(256)
 split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int parts, unsigned int* flags,
              unsigned int epoch, unsigned int* verdict) {
   __shared__ float tile[128][65];
+  // the contraction's blocks may start setting up once every block here runs
+  // (they wait for this grid's end before they read): 2-4 % of a small product
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   dependency_wait();
   const uint32_t kt = (Kp + 127) / 128;
   if (FMT == kBf16 && verdict) {
@@ -342,7 +355,10 @@ split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int part
 // block per SM then reads about group_m rows of A and SMs / group_m columns
 // of B, which stay in L2 for the whole wave (row-major order read every
 // column of B in every wave: at 4096^3, 2.5x the parts' bytes from DRAM).
-template <int PARTS, int STAGES, int G, int BN_T>
+// SPLIT: the blocks of a cluster share one output tile, each taking a share of
+// its k-blocks; their sums meet in shared memory, where every block adds up
+// its share of the tile's rows, in block order.
+template <int PARTS, int STAGES, int G, int BN_T, bool SPLIT = false>
 __global__ void __launch_bounds__(Shape<BN_T>::THREADS, 1)
 gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                    float* __restrict__ P, uint32_t M, uint32_t N, uint32_t Kp, uint32_t spin_limit,
@@ -361,19 +377,24 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
   __shared__ uint32_t tmem_slot;
   __shared__ int s_fail;
 
-  dependency_wait();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // 1024-aligned stage ring
-  uint32_t n0, m0;
+  uint32_t n0, m0, ranks = 1, rank = 0;
+  if constexpr (SPLIT) {
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  }
   {
-    const uint32_t tiles_m = gridDim.x / tiles_n, per_group = group_m * tiles_n;
-    const uint32_t grp = blockIdx.x / per_group, r = blockIdx.x % per_group;
+    const uint32_t tile = blockIdx.x / ranks;
+    const uint32_t tiles_m = gridDim.x / ranks / tiles_n, per_group = group_m * tiles_n;
+    const uint32_t grp = tile / per_group, r = tile % per_group;
     const uint32_t first = grp * group_m;
     const uint32_t rows = tiles_m - first < group_m ? tiles_m - first : group_m;
     m0 = (first + r % rows) * BM;
     n0 = (r / rows) * BN;
   }
-  const uint32_t nk = Kp / BK;
+  // this block's k-blocks: nk from k0 on
+  const uint32_t all_k = Kp / BK, k0 = all_k * rank / ranks, nk = all_k * (rank + 1) / ranks - k0;
 
   if (threadIdx.x == 0) {
     s_fail = 0;
@@ -397,6 +418,7 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  dependency_wait();  // (the barriers and tensor memory above need nothing of the split)
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
@@ -416,7 +438,7 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
                      :: "r"(fb), "r"((uint32_t)STAGE_BYTES) : "memory");
         const uint32_t stage = base + (uint32_t)s * STAGE_BYTES;
-        const int kx = (int)(kb * BK);
+        const int kx = (int)((k0 + kb) * BK);
 #pragma unroll
         for (int p = 0; p < PARTS; ++p) {
           asm volatile(
@@ -536,7 +558,17 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];"
                      :: "r"(smem_u32(&acc_empty[acc_i])) : "memory");
     }
-    if (ok) {
+    if (SPLIT) {
+      // (every MMA that reads the stages has completed)  16-byte chunk c of
+      // row r at chunk c ^ (r % 32): a warp's accesses meet all banks
+      const uint32_t r = (uint32_t)(q * 32 + lane);
+#pragma unroll
+      for (int c = 0; c < CW / 4; ++c)
+        asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
+                     :: "r"(base + r * (CW * 4) + (((uint32_t)c ^ (r & 31u)) * 16u)), "f"(sum[c * 4]),
+                        "f"(sum[c * 4 + 1]), "f"(sum[c * 4 + 2]), "f"(sum[c * 4 + 3])
+                     : "memory");
+    } else if (ok) {
       const uint32_t row = m0 + (uint32_t)(q * 32 + lane);
       if (row < M) {
         const bool vec = (N % 4u) == 0u;
@@ -558,6 +590,41 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         }
       }
     }
+  }
+
+  if constexpr (SPLIT) {
+    static_assert(!SPLIT || BN == 128, "one epilogue warp per 32 rows: its sums are whole rows");
+    __syncthreads();
+    cluster_sync();
+    const uint32_t rows = BM / ranks, first = rank * rows;
+    for (uint32_t i = threadIdx.x; i < rows * 32u; i += SH::THREADS) {
+      const uint32_t r = first + i / 32u, c = i % 32u;
+      const uint32_t at = base + r * 512u + ((c ^ (r & 31u)) * 16u);
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      for (uint32_t p = 0; p < ranks; ++p) {
+        float4 o;
+        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                     : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(cluster_addr(at, p)) : "memory");
+        v.x += o.x;
+        v.y += o.y;
+        v.z += o.z;
+        v.w += o.w;
+      }
+      const uint32_t row = m0 + r, col = n0 + c * 4u;
+      if (row < M) {
+        float* dst = P + (uint64_t)row * N + col;
+        if ((N % 4u) == 0u && col + 4u <= N) {
+          *reinterpret_cast<float4*>(dst) = v;
+        } else {
+          if (col < N) dst[0] = v.x;
+          if (col + 1u < N) dst[1] = v.y;
+          if (col + 2u < N) dst[2] = v.z;
+          if (col + 3u < N) dst[3] = v.w;
+        }
+      }
+    }
+    __syncthreads();
+    cluster_sync();  // no block leaves while another may still read its sums
   }
 
   // ---- teardown: wait for the copies a failed pipeline may still have in
@@ -641,15 +708,6 @@ struct PairArgs {
   uint32_t M, N, Kp, Mp, Np, epoch, spin_limit, tiles_n, tiles_m, group_m;
 };
 
-// The address of `addr` (shared memory) in CTA `rank` of the cluster.
-__device__ __forceinline__ uint32_t cluster_addr(uint32_t addr, uint32_t rank) {
-  uint32_t r;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(addr), "r"(rank));
-  return r;
-}
-__device__ __forceinline__ void cluster_sync() {
-  asm volatile("barrier.cluster.arrive.release.aligned; barrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
 // Bounded wait for arrivals from both CTAs.
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t limit) {
   uint32_t polls = 0;
@@ -1032,6 +1090,19 @@ static int encode_parts(CUtensorMap* tm, const void* base, uint64_t rows, uint64
 }
 
 namespace {
+// Blocks that share an output tile of 128 x 128 (a cluster): as many as leave
+// no SM without a block, with at least four k-blocks of 64 each.  Splitting
+// the operands included, with one block per tile and so: 1000 x 500 x 1100 (72
+// tiles on 152 SMs) 16.5 -> 15.9 us, 1000 x 1100 x 500 (32 tiles) 27.9 -> 16.3
+// us, 64 x 4096 x 512 (4 tiles) 72.9 -> 19.0 us; 256 x 256 x 256 with two
+// k-blocks each 11.2 -> 12.1 us.
+uint32_t split_of_k(uint64_t tiles, uint32_t Kp) {
+  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  uint32_t s = 1;
+  while (s < 8 && tiles * s * 2 <= sms && Kp / 64 >= 8 * s) s *= 2;
+  return s;
+}
+
 template <int PARTS, int STAGES, int G, int BN_T>
 cudaError_t launch_gemm(dim3 grid, cudaStream_t stream, const CUtensorMap& tmA, const CUtensorMap& tmB,
                         float* P, uint32_t M, uint32_t N, uint32_t Kp, uint32_t spin_limit,
@@ -1111,9 +1182,14 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
                    : launch_gemm<2, 4, 2, 256>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m);
   } else if (parts == 3) {
     // parts 3: 2 stages of 96 KB; parts 2: 3 stages of 64 KB
-    e = drain >= 4 ? launch_gemm<3, 2, 4, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m)
-      : drain == 2 ? launch_gemm<3, 2, 2, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m)
-                   : launch_gemm<3, 2, 1, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m);
+    const uint32_t split = drain >= 2 ? 1 : split_of_k(grid.x, Kp);
+    e = drain >= 4  ? launch_gemm<3, 2, 4, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m)
+      : drain == 2  ? launch_gemm<3, 2, 2, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m)
+      : split == 1  ? launch_gemm<3, 2, 1, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m)
+                    : launch_clustered(tc::gemm_3xbf16_kernel<3, 2, 1, 128, true>, split, dim3(grid.x * split),
+                                       dim3(tc::Shape<128>::THREADS),
+                                       (size_t)2 * 3 * (tc::Shape<128>::A_TILE + tc::Shape<128>::B_TILE) + 1024,
+                                       stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m);
   } else {
     e = drain >= 4 ? launch_gemm<2, 3, 4, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m)
       : drain == 2 ? launch_gemm<2, 3, 2, 128>(grid, stream, tmA, tmB, P, M, N, Kp, spin_limit, err, tn, group_m)

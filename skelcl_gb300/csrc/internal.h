@@ -217,25 +217,39 @@ int launch(CUfunction fn, dim3 grid, dim3 block, size_t smem, ArgPack& pack);
 // Launch of a precompiled kernel, overlapped like the skeleton kernels (with
 // scl::dependency_wait() ahead of its first access to memory).
 template <typename... KArgs, typename... Args>
-cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
-                              const Args&... args) {
+cudaError_t launch_clustered(void (*kern)(KArgs...), unsigned cluster, dim3 grid, dim3 block, size_t smem,
+                             cudaStream_t stream, const Args&... args) {
   if (smem > 32 * 1024) {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e != cudaSuccess) return e;
   }
-  cudaLaunchAttribute attr{};
-  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr.val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2] = {};
+  unsigned n = 0;
+  if (rt().pdl) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {  // (blocks per cluster, along x)
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = 1;
+    attr[n++].val.clusterDim.z = 1;
+  }
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cfg.attrs = &attr;
-  cfg.numAttrs = rt().pdl ? 1 : 0;
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
   cudaError_t e = cudaLaunchKernelEx(&cfg, kern, KArgs(args)...);
   if (e == cudaSuccess) ++rt().launches;
   return e;
+}
+template <typename... KArgs, typename... Args>
+cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream,
+                              const Args&... args) {
+  return launch_clustered(kern, 1u, grid, block, smem, stream, args...);
 }
 #ifdef __CUDACC__
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -1,5 +1,6 @@
-"""AllPairs zip(x*y)/reduce(x+y) on 256-column tiles: CTA pairs with FP16
-parts, and the bf16 parts the device falls back to."""
+"""AllPairs zip(x*y)/reduce(x+y) on the tensor cores: 256-column tiles on CTA
+pairs with FP16 parts and the bf16 parts the device falls back to, and
+128-column tiles shared by the blocks of a cluster."""
 import numpy as np
 import pytest
 
@@ -18,14 +19,14 @@ def program():
                      source2="float func(float x, float y){ return x*y; }", identity="0")
 
 
-def run(p, A, B, items=0, flags=0):
+def run(p, A, B, items=0, flags=0, cols=256):
     M, K = A.shape
     N = B.shape[1]
     a = np.ascontiguousarray(A.T if flags & S.SHAPE_TRANS_LEFT else A)
     b = np.ascontiguousarray(B.T if flags & S.SHAPE_TRANS_RIGHT else B)
     dA, dB, dP = S.DeviceArray.from_numpy(a), S.DeviceArray.from_numpy(b), S.DeviceArray(M * N, np.float32)
     p.launch([dA, dB, dP], rows=M, cols=N, dim=K, flags=flags,
-             tuning=S.Tuning(variant=S.VARIANT_TC3XBF16, items=items, tile_h=256))
+             tuning=S.Tuning(variant=S.VARIANT_TC3XBF16, items=items, tile_h=cols))
     return dP.to_numpy().reshape(M, N)
 
 
@@ -111,3 +112,19 @@ def test_pair_in_a_graph(scl, orc):
         S.check(L.scl_graph_launch(g))
         assert np.array_equal(dP.to_numpy(), ref, equal_nan=True)
     S.check(L.scl_graph_destroy(g))
+
+
+@pytest.mark.parametrize("flags", [0, S.SHAPE_TRANS_LEFT, S.SHAPE_TRANS_RIGHT])
+@pytest.mark.parametrize("shape", [(128, 448, 128), (128, 512, 128), (127, 640, 131), (130, 1024, 129), (257, 1000, 72),
+                                   (300, 2100, 258), (1000, 500, 1100), (640, 2100, 500)])
+def test_split_k_against_fp64(scl, orc, shape, flags):
+    """One, two, four and eight blocks to a tile; their k-blocks shared out
+    evenly and unevenly."""
+    M, K, N = shape
+    A = orc.normal_f32(M * K, 71).reshape(M, K)
+    B = orc.normal_f32(K * N, 72).reshape(K, N)
+    p = program()
+    P = run(p, A, B, flags=flags, cols=128)
+    bound = C * (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64))
+    assert np.all(np.abs(P - A.astype(np.float64) @ B.astype(np.float64)) <= bound)
+    assert np.array_equal(P, run(p, A, B, flags=flags, cols=128))  # summed in one order
