@@ -8,6 +8,7 @@
 #include <cstdint>
 #include <deque>
 #include <functional>
+#include <initializer_list>
 #include <map>
 #include <memory>
 #include <mutex>
@@ -190,6 +191,19 @@ struct scl_program {
   std::set<std::string> lazy;               // variants compiled on first use
   scl::Workspace ws;
   uint32_t last_variant = 0;
+  bool has_func2 = false;                   // the source defines the second derivative (Zip adjoint)
+  // what every launch would otherwise ask again: kernels by a small id, and
+  // the blocks of a kernel the device holds at once (several threads may
+  // launch one program)
+  std::mutex hot_mu;
+  std::vector<std::pair<uint32_t, CUfunction>> hot_kernels;
+  struct Resident {
+    CUfunction fn;
+    int block;
+    size_t smem;
+    int blocks;
+  };
+  std::vector<Resident> hot_resident;
 };
 
 namespace scl {
@@ -199,9 +213,39 @@ CUfunction find_kernel(scl_program* p, const std::string& name);
 // uses the allocation; growing there is refused.
 int ensure_workspace(scl_program* p, size_t bytes, bool fresh = false);
 
+// Kernel parameter pointers of one launch, kept off the heap up to 48.
+class PtrList {
+public:
+  PtrList() = default;
+  PtrList& operator=(std::initializer_list<void*> l) {
+    n_ = 0;
+    more_.clear();
+    for (void* p : l) push_back(p);
+    return *this;
+  }
+  void push_back(void* p) {
+    if (n_ < kInline) {
+      in_[n_] = p;
+    } else {
+      if (n_ == kInline) more_.assign(in_, in_ + kInline);
+      more_.push_back(p);
+    }
+    ++n_;
+  }
+  size_t size() const { return n_; }
+  bool empty() const { return n_ == 0; }
+  void** data() { return n_ <= kInline ? in_ : more_.data(); }
+
+private:
+  static constexpr size_t kInline = 48;
+  void* in_[kInline];
+  size_t n_ = 0;
+  std::vector<void*> more_;
+};
+
 // Kernel parameters of one launch (launch.cpp)
 struct ArgPack {
-  std::vector<void*> ptrs;
+  PtrList ptrs;
   uint32_t vals[64];  // storage for values built here (Local offsets)
   int nvals = 0;
   size_t local_bytes = 0;

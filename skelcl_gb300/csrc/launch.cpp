@@ -183,7 +183,12 @@ int launch(CUfunction fn, dim3 grid, dim3 block, size_t smem, ArgPack& pack) {
 
 namespace {
 
-int max_resident_blocks(CUfunction fn, int block, size_t smem) {
+int max_resident_blocks(scl_program* p, CUfunction fn, int block, size_t smem) {
+  {
+    std::lock_guard<std::mutex> g(p->hot_mu);
+    for (const auto& r : p->hot_resident)
+      if (r.fn == fn && r.block == block && r.smem == smem) return r.blocks;
+  }
   int per_sm = 0;
   // the query counts only what the function may use: raise its dynamic limit
   // first, as launch() does
@@ -192,7 +197,26 @@ int max_resident_blocks(CUfunction fn, int block, size_t smem) {
   if (rt().drv.cuOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, fn, block, smem) != CUDA_SUCCESS ||
       per_sm < 1)
     per_sm = 1;
-  return per_sm * rt().sm_count;
+  const int blocks = per_sm * rt().sm_count;
+  std::lock_guard<std::mutex> g(p->hot_mu);
+  if (p->hot_resident.size() < 64) p->hot_resident.push_back({fn, block, smem, blocks});
+  return blocks;
+}
+
+// find_kernel() by an id that stands for its name within the program.
+template <typename Name>
+CUfunction hot_kernel(scl_program* p, uint32_t id, Name name) {
+  {
+    std::lock_guard<std::mutex> g(p->hot_mu);
+    for (const auto& k : p->hot_kernels)
+      if (k.first == id) return k.second;
+  }
+  CUfunction fn = find_kernel(p, name());
+  if (fn) {
+    std::lock_guard<std::mutex> g(p->hot_mu);
+    p->hot_kernels.emplace_back(id, fn);
+  }
+  return fn;
 }
 
 int vec_width(size_t s0, size_t s1 = 1, size_t s2 = 1) {
@@ -258,7 +282,7 @@ static int launch_map_impl(scl_program* p, const scl_shape* sh, void* const* buf
   int acc = 0;
   if (kind == SCL_KIND_ZIP_ADJOINT) {
     if (!b[3] && !b[4]) return fail(SCL_ERR_ARG, "Zip adjoint: both gradient buffers are null");
-    if (b[4] && p->source.find("#define SCL_HAS_FUNC2") == std::string::npos)
+    if (b[4] && !p->has_func2)
       return fail(SCL_ERR_ARG, "Zip adjoint: a right gradient needs the right derivative (func2)");
     acc = ((sh->flags & SCL_SHAPE_ACCUMULATE) ? 1 : 0) | ((sh->flags & SCL_SHAPE_ACCUMULATE_RIGHT) ? 2 : 0);
   } else if (kind == SCL_KIND_MAP_ADJOINT) {
@@ -273,12 +297,11 @@ static int launch_map_impl(scl_program* p, const scl_shape* sh, void* const* buf
   for (int i = 0; i < nbuf; ++i) aligned &= (!b[i] || aligned16(b[i])) ? 1 : 0;
   uint32_t items = (tu && tu->items) ? tu->items : 4;
   if (items != 1 && items != 2 && items != 4) items = 4;
-  std::string kname = simple ? "scl_map_simple" : "scl_map_k<" + std::to_string(items) + ">";
-  CUfunction fn = find_kernel(p, kname);
-  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname + " missing from the program");
+  auto kname = [&] { return simple ? std::string("scl_map_simple") : "scl_map_k<" + std::to_string(items) + ">"; };
+  CUfunction fn = hot_kernel(p, simple ? 0u : items, kname);
+  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname() + " missing from the program");
 
   ArgPack pack;
-  pack.ptrs.reserve(32);
   for (int i = 0; i < nbuf; ++i) pack.ptrs.push_back(&b[i]);
   if (point) {
     pack.ptrs.push_back(&rows);
@@ -312,7 +335,7 @@ static int launch_map_impl(scl_program* p, const scl_shape* sh, void* const* buf
     }
     p->last_variant = SCL_VARIANT_SIMPLE;
   } else {
-    const int maxb = max_resident_blocks(fn, (int)wg, pack.local_bytes);
+    const int maxb = max_resident_blocks(p, fn, (int)wg, pack.local_bytes);
     if (point) {
       uint32_t bx = 256;
       block = dim3(bx, 1, 1);
@@ -445,7 +468,7 @@ static int launch_reduce_impl(scl_program* p, const scl_shape* sh, void* const* 
                             &spack))
       return st;
     uint64_t sblocks = (n_seg + 7) / 8;  // 8 warps per block
-    const uint64_t smax = (uint64_t)max_resident_blocks(fn_short, 256, spack.local_bytes);
+    const uint64_t smax = (uint64_t)max_resident_blocks(p, fn_short, 256, spack.local_bytes);
     if (sblocks > smax) sblocks = smax;
     if (int st = launch(fn_short, dim3((unsigned)sblocks), dim3(256), 0, spack)) return st;
     // longer segments: tiles (blocks past the last tile return at once)
@@ -465,12 +488,12 @@ static int launch_reduce_impl(scl_program* p, const scl_shape* sh, void* const* 
   // faster than 4 at 2^24 and 2^26 f32)
   uint32_t items = (tu && tu->items) ? tu->items : 8;
   if (items != 1 && items != 2 && items != 4 && items != 8) items = 8;
-  std::string kname = "scl_reduce_k<" + std::to_string(items) + ">";
-  CUfunction fn = find_kernel(p, kname);
-  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname + " missing");
+  auto kname = [&] { return "scl_reduce_k<" + std::to_string(items) + ">"; };
+  CUfunction fn = hot_kernel(p, items, kname);
+  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname() + " missing");
   uint32_t wg = pick_block(tu, 256);
   wg = (wg + 31) / 32 * 32;
-  const int maxb = max_resident_blocks(fn, (int)wg, 0);
+  const int maxb = max_resident_blocks(p, fn, (int)wg, 0);
   uint64_t units = aligned ? n / V : n;
   uint64_t g = units == 0 ? 1 : (units + wg - 1) / wg;
   if (g > (uint64_t)maxb) g = (uint64_t)maxb;
@@ -504,12 +527,12 @@ static int launch_zipreduce(scl_program* p, const scl_shape* sh, void* const* bu
   int aligned = (aligned16(l) && aligned16(r)) ? 1 : 0;
   uint32_t items = (tu && tu->items) ? tu->items : 4;
   if (items != 1 && items != 2 && items != 4) items = 4;
-  const std::string kname = "scl_zipreduce_k<" + std::to_string(items) + ">";
-  CUfunction fn = find_kernel(p, kname);
-  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname + " missing");
+  auto kname = [&] { return "scl_zipreduce_k<" + std::to_string(items) + ">"; };
+  CUfunction fn = hot_kernel(p, items, kname);
+  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname() + " missing");
   uint32_t wg = pick_block(tu, 256);
   wg = (wg + 31) / 32 * 32;
-  const int maxb = max_resident_blocks(fn, (int)wg, 0);
+  const int maxb = max_resident_blocks(p, fn, (int)wg, 0);
   uint64_t units = aligned ? n / V : n;
   uint64_t g = units == 0 ? 1 : (units + wg - 1) / wg;
   if (g > (uint64_t)maxb) g = (uint64_t)maxb;
@@ -654,10 +677,13 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
     minb = R == 16 ? 2 : (R == 8 ? 4 : (R == 4 ? 6 : 8));
   }
   if (n_seg) minb = R == 16 ? 3 : 6;
-  const std::string kname = std::string(staged ? "scl_scan_s<" : "scl_scan_k<") + std::to_string(R) +
-                            ", " + std::to_string(minb) + (plan ? ", 2>" : (n_seg ? ", 1>" : ">"));
-  CUfunction fn = find_kernel(p, kname);
-  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname + " missing");
+  auto kname = [&] {
+    return std::string(staged ? "scl_scan_s<" : "scl_scan_k<") + std::to_string(R) + ", " + std::to_string(minb) +
+           (plan ? ", 2>" : (n_seg ? ", 1>" : ">"));
+  };
+  CUfunction fn = hot_kernel(p, R | minb << 8 | (staged ? 1u << 16 : 0u) | (plan ? 2u << 17 : n_seg ? 1u << 17 : 0u),
+                             kname);
+  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname() + " missing");
   // workspace: three status regions (scan_region_bytes); segmented launches
   // add [clamped offsets | tile numbering | pre-pass scratch] after them
   auto up = [](size_t b) { return (b + 255) / 256 * 256; };
@@ -726,7 +752,7 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
                             &spack))
       return st;
     uint64_t sblocks = (n_seg + 7) / 8;  // 8 warps per block
-    const uint64_t smax = (uint64_t)max_resident_blocks(fn_short, 256, spack.local_bytes);
+    const uint64_t smax = (uint64_t)max_resident_blocks(p, fn_short, 256, spack.local_bytes);
     if (sblocks > smax) sblocks = smax;
     if (int st = launch(fn_short, dim3((unsigned)sblocks), dim3(256), 0, spack)) return st;
   }
@@ -787,12 +813,14 @@ static int launch_mapoverlap_impl(scl_program* p, const scl_shape* sh, void* con
   dim3 grid((unsigned)((cols + TW - 1) / TW), (unsigned)((rows + TH - 1) / TH)), block(32, 8);
   if (grid.y > 65535) return fail(SCL_ERR_ARG, "matrix has too many rows for one launch");
   const bool tma_ok = tma_shape_ok && win_h <= 256;
-  const std::string py = "<" + std::to_string(PY) + ">";
+  auto kname = [&](bool tma) {
+    return std::string(tma ? "scl_mapoverlap_tma<" : "scl_mapoverlap_ldst<") + std::to_string(PY) + ">";
+  };
   unsigned int spin = spin_of(tu);
   unsigned int* err = rt().dev_err;
   if (want_tma && tma_ok) {
-    CUfunction fn = find_kernel(p, "scl_mapoverlap_tma" + py);
-    if (!fn) return fail(SCL_ERR_LAUNCH, "kernel scl_mapoverlap_tma" + py + " missing");
+    CUfunction fn = hot_kernel(p, (uint32_t)PY | 1u << 16, [&] { return kname(true); });
+    if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname(true) + " missing");
     alignas(64) CUtensorMap tmap;
     CUtensorMapDataType dt = tsz == 1 ? CU_TENSOR_MAP_DATA_TYPE_UINT8
                            : tsz == 2 ? CU_TENSOR_MAP_DATA_TYPE_UINT16
@@ -814,8 +842,8 @@ static int launch_mapoverlap_impl(scl_program* p, const scl_shape* sh, void* con
     p->last_variant = SCL_VARIANT_TMA;
     return launch(fn, grid, block, win_bytes, pack);
   }
-  CUfunction fn = find_kernel(p, "scl_mapoverlap_ldst" + py);
-  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel scl_mapoverlap_ldst" + py + " missing");
+  CUfunction fn = hot_kernel(p, (uint32_t)PY, [&] { return kname(false); });
+  if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname(false) + " missing");
   ArgPack pack;
   pack.ptrs = {&in, &out, &rows, &cols};
   if (int st = pack_extra(p, fn, pack.ptrs.size(), (const unsigned char*)extra, extra_bytes, &pack))
@@ -970,7 +998,7 @@ scl_tuning shape(uint32_t workgroup, uint32_t items, uint32_t tile_w, uint32_t t
 extern "C" int scl_launch_map(scl_program* p, const scl_shape* sh, void* const* bufs,
                               const void* extra, size_t extra_bytes, const scl_tuning* tu) {
   auto run = [&](const scl_tuning* t) { return launch_map_impl(p, sh, bufs, extra, extra_bytes, t); };
-  if (!p || !sh || !bufs || untuned(tu) == false || p->uses_workitem) return run(tu);
+  if (!p || !sh || !bufs || untuned(tu) == false || p->uses_workitem || !autotune_enabled()) return run(tu);
   const uint64_t n = (p->kind == SCL_KIND_MAP_POINT || p->kind == SCL_KIND_MAP_POINT_VOID) ? sh->rows * sh->cols
                                                                                           : sh->n;
   const auto& ts = p->type_sizes;
@@ -999,7 +1027,7 @@ extern "C" int scl_launch_map(scl_program* p, const scl_shape* sh, void* const* 
 extern "C" int scl_launch_reduce(scl_program* p, const scl_shape* sh, void* const* bufs,
                                  const void* extra, size_t extra_bytes, const scl_tuning* tu) {
   auto run = [&](const scl_tuning* t) { return launch_reduce_impl(p, sh, bufs, extra, extra_bytes, t); };
-  if (!p || !sh || !bufs || !bufs[0] || !bufs[1] || p->type_sizes.empty()) return run(tu);
+  if (!p || !sh || !bufs || !bufs[0] || !bufs[1] || p->type_sizes.empty() || !autotune_enabled()) return run(tu);
   if (p->kind == SCL_KIND_ZIP_REDUCE) {
     if (!bufs[2] || p->type_sizes.size() < 3) return run(tu);
     const bool safe = extras_are_values(p) &&
@@ -1026,7 +1054,7 @@ extern "C" int scl_launch_reduce(scl_program* p, const scl_shape* sh, void* cons
 extern "C" int scl_launch_scan(scl_program* p, const scl_shape* sh, void* const* bufs,
                                const void* extra, size_t extra_bytes, const scl_tuning* tu) {
   auto run = [&](const scl_tuning* t) { return launch_scan_impl(p, sh, bufs, extra, extra_bytes, t); };
-  if (!p || !sh || !bufs || !bufs[0] || !bufs[1] || p->type_sizes.empty()) return run(tu);
+  if (!p || !sh || !bufs || !bufs[0] || !bufs[1] || p->type_sizes.empty() || !autotune_enabled()) return run(tu);
   const size_t bytes = sh->n * p->type_sizes[0];
   const bool safe = extras_are_values(p) && !overlaps(bufs[0], bytes, bufs[1], bytes);
   std::vector<scl_tuning> cands;
@@ -1042,7 +1070,7 @@ extern "C" int scl_launch_scan(scl_program* p, const scl_shape* sh, void* const*
 extern "C" int scl_launch_mapoverlap(scl_program* p, const scl_shape* sh, void* const* bufs,
                                      const void* extra, size_t extra_bytes, const scl_tuning* tu) {
   auto run = [&](const scl_tuning* t) { return launch_mapoverlap_impl(p, sh, bufs, extra, extra_bytes, t); };
-  if (!p || !sh || !bufs) return run(tu);
+  if (!p || !sh || !bufs || !autotune_enabled()) return run(tu);
   const bool safe = extras_are_values(p) || [&] {
     // weights passed as Vector / Matrix arguments are read by the stencil, not written
     for (const Param& e : p->extra)

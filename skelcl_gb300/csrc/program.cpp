@@ -778,6 +778,7 @@ extern "C" int scl_program_build(const scl_program_desc* desc, scl_program** out
   }
   p->f64_carry = f64;
   p->source = a.source;
+  p->has_func2 = a.source.find("#define SCL_HAS_FUNC2") != std::string::npos;
   for (auto& k : a.lazy) p->lazy.insert(k);
   if (int st = require_init()) {
     copy_log("scl_init() has not been called", log, log_cap);
