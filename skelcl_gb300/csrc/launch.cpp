@@ -812,6 +812,13 @@ static int launch_mapoverlap_impl(scl_program* p, const scl_shape* sh, void* con
   if (win_bytes > rt().smem_optin) return fail(SCL_ERR_ARG, "overlap range too large for shared memory");
   dim3 grid((unsigned)((cols + TW - 1) / TW), (unsigned)((rows + TH - 1) / TH)), block(32, 8);
   if (grid.y > 65535) return fail(SCL_ERR_ARG, "matrix has too many rows for one launch");
+  // a thread's adjacent outputs in one store: 4, 8 or 16 bytes that every row
+  // of `out` is aligned to
+  const size_t obytes = (p->type_sizes.size() > 1 ? p->type_sizes[1] : tsz) * (size_t)p->stencil_px;
+  int ovec = (obytes == 4 || obytes == 8 || obytes == 16) && cols % (uint64_t)p->stencil_px == 0 &&
+                     reinterpret_cast<uintptr_t>(out) % obytes == 0
+                 ? 1
+                 : 0;
   const bool tma_ok = tma_shape_ok && win_h <= 256;
   auto kname = [&](bool tma) {
     return std::string(tma ? "scl_mapoverlap_tma<" : "scl_mapoverlap_ldst<") + std::to_string(PY) + ">";
@@ -836,7 +843,7 @@ static int launch_mapoverlap_impl(scl_program* p, const scl_shape* sh, void* con
         CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
     if (r != CUDA_SUCCESS) return cu_fail(r, "cuTensorMapEncodeTiled");
     ArgPack pack;
-    pack.ptrs = {&tmap, &out, &rows, &cols, &spin, &err};
+    pack.ptrs = {&tmap, &out, &rows, &cols, &spin, &err, &ovec};
     if (int st = pack_extra(p, fn, pack.ptrs.size(), (const unsigned char*)extra, extra_bytes, &pack))
       return st;
     p->last_variant = SCL_VARIANT_TMA;
@@ -849,7 +856,8 @@ static int launch_mapoverlap_impl(scl_program* p, const scl_shape* sh, void* con
   if (int st = pack_extra(p, fn, pack.ptrs.size(), (const unsigned char*)extra, extra_bytes, &pack))
     return st;
   p->last_variant = SCL_VARIANT_LDST;
-  return launch(fn, grid, block, win_bytes, pack);
+  // the tile's outputs pass through the window's place
+  return launch(fn, grid, block, std::max(win_bytes, (size_t)TH * 32 * obytes), pack);
 }
 
 // ---- AllPairs -------------------------------------------------------------------

@@ -27,25 +27,33 @@ __device__ __forceinline__ scl_u64 scl_clampi(long long v, long long hi) {
   return (scl_u64)(v < 0 ? 0 : (v > hi ? hi : v));
 }
 
-// Fill the positions of the window that lie outside the matrix.
+// Fill the positions of the window that lie outside the matrix: a warp takes a
+// row of the window at a time, all of it for a row outside, else the columns
+// left and right of the matrix.
 template <int WIN_H>
 __device__ __forceinline__ void scl_patch_border(SCL_TYPE_0* win, long long x_org, long long y_org,
                                                  scl_u64 rows, scl_u64 cols) {
-  const int nthreads = blockDim.x * blockDim.y;
-  const int t = threadIdx.y * blockDim.x + threadIdx.x;
-  for (int k = t; k < WIN_H * SCL_WIN_W; k += nthreads) {
-    const int ly = k / SCL_WIN_W, lx = k % SCL_WIN_W;
-    const long long gy = y_org + ly, gx = x_org + lx;
-    const bool inside = gy >= 0 && gy < (long long)rows && gx >= 0 && gx < (long long)cols;
-    if (inside) continue;
+  // (the window overlaps the matrix: these fit in an int)
+  const int left = x_org < 0 ? (int)-x_org : 0, top = y_org < 0 ? (int)-y_org : 0;
+  const int right = (long long)cols - x_org < SCL_WIN_W ? (int)((long long)cols - x_org) : SCL_WIN_W;
+  const int bottom = (long long)rows - y_org < WIN_H ? (int)((long long)rows - y_org) : WIN_H;
+#pragma unroll 1
+  for (int ly = threadIdx.y; ly < WIN_H; ly += 8) {
+    const bool inside = ly >= top && ly < bottom;
+    SCL_TYPE_0* row = win + ly * SCL_WIN_W;
 #if SCL_PADDING == 1
-    const long long cy = (long long)scl_clampi(gy, (long long)rows - 1);
-    const long long cx = (long long)scl_clampi(gx, (long long)cols - 1);
-    // the clamped position lies inside both the matrix and the window
-    win[k] = win[(cy - y_org) * SCL_WIN_W + (cx - x_org)];
-#else
-    win[k] = (SCL_TYPE_0)(SCL_NEUTRAL);
+    // (the clamped positions lie inside both the matrix and the window)
+    const SCL_TYPE_0* from = win + (inside ? ly : (ly < top ? top : bottom - 1)) * SCL_WIN_W;
 #endif
+#pragma unroll 1
+    for (int lx = threadIdx.x; lx < SCL_WIN_W; lx += 32) {
+      if (inside && lx >= left && lx < right) continue;
+#if SCL_PADDING == 1
+      row[lx] = from[lx < left ? left : (lx >= right ? right - 1 : lx)];
+#else
+      row[lx] = (SCL_TYPE_0)(SCL_NEUTRAL);
+#endif
+    }
   }
 }
 
@@ -53,11 +61,9 @@ __device__ __forceinline__ void scl_patch_border(SCL_TYPE_0* win, long long x_or
 // adjacent columns: with the user loops unrolled, the taps those outputs
 // share are read once.
 template <int PY>
-__device__ __forceinline__ void scl_compute_tile(const SCL_TYPE_0* win, SCL_TYPE_1* out,
-                                                 scl_u64 rows, scl_u64 cols, scl_u64 x0,
-                                                 scl_u64 y0 SCL_USER_PARAMS) {
+__device__ __forceinline__ void scl_compute_tile(const SCL_TYPE_0* win,
+                                                 SCL_TYPE_1 (&res)[PY][SCL_PX] SCL_USER_PARAMS) {
   const int tx = threadIdx.x, ty = threadIdx.y;
-  SCL_TYPE_1 res[PY][SCL_PX];
 #pragma unroll
   for (int p = 0; p < PY; ++p) {
     const int ly = ty * PY + p;
@@ -71,18 +77,59 @@ __device__ __forceinline__ void scl_compute_tile(const SCL_TYPE_0* win, SCL_TYPE
       res[p][c] = USR_FUNC(m SCL_EXTRA_ARGS);
     }
   }
+}
+
+// One element to shared memory, ASYNC: asynchronously (complete after
+// cp.async.wait_all), for elements of 4 or 8 bytes that sit on their size.
+template <bool ASYNC>
+__device__ __forceinline__ void scl_stage_element(SCL_TYPE_0* dst, const SCL_TYPE_0* src) {
+  if constexpr (ASYNC)
+    asm volatile("cp.async.ca.shared.global [%0], [%1], %2;"
+                 :: "r"((unsigned int)__cvta_generic_to_shared(dst)), "l"(src), "n"((int)sizeof(SCL_TYPE_0))
+                 : "memory");
+  else
+    *dst = *src;
+}
+
+// The window at (x_org, y_org), a warp per row, padded outside the matrix.
+template <int WIN_H, bool ASYNC>
+__device__ __forceinline__ void scl_stage_window(SCL_TYPE_0* win, const SCL_TYPE_0* in, long long x_org,
+                                                 long long y_org, scl_u64 rows, scl_u64 cols) {
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  if (x_org >= 0 && y_org >= 0 && x_org + SCL_WIN_W <= (long long)cols && y_org + WIN_H <= (long long)rows) {
+    const SCL_TYPE_0* src = in + (scl_u64)(y_org + ty) * cols + (scl_u64)(x_org + tx);
+    SCL_TYPE_0* dst = win + ty * SCL_WIN_W + tx;
+    for (int ly = ty; ly < WIN_H; ly += 8, src += 8 * cols, dst += 8 * SCL_WIN_W) {
 #pragma unroll
-  for (int p = 0; p < PY; ++p) {
-    const scl_u64 y = y0 + ty * PY + p;
-#pragma unroll
-    for (int c = 0; c < SCL_PX; ++c) {
-      const scl_u64 x = x0 + (scl_u64)tx * SCL_PX + c;
-      if (y < rows && x < cols) out[y * cols + x] = res[p][c];
+      for (int c = 0; c < SCL_WIN_W; c += 32)
+        if (c + 32 <= SCL_WIN_W || tx < SCL_WIN_W - c) scl_stage_element<ASYNC>(dst + c, src + c);
+    }
+    return;
+  }
+  for (int ly = ty; ly < WIN_H; ly += 8) {
+    const long long gy = y_org + ly;
+    const bool row_in = gy >= 0 && gy < (long long)rows;
+    const SCL_TYPE_0* row = in + scl_clampi(gy, (long long)rows - 1) * cols;
+    for (int lx = tx; lx < SCL_WIN_W; lx += 32) {
+      const long long gx = x_org + lx;
+      const bool inside = row_in && gx >= 0 && gx < (long long)cols;
+#if SCL_PADDING == 1
+      (void)inside;
+      scl_stage_element<ASYNC>(win + ly * SCL_WIN_W + lx, row + scl_clampi(gx, (long long)cols - 1));
+#else
+      if (inside) scl_stage_element<ASYNC>(win + ly * SCL_WIN_W + lx, row + gx);
+      else win[ly * SCL_WIN_W + lx] = (SCL_TYPE_0)(SCL_NEUTRAL);
+#endif
     }
   }
 }
 
-// Cooperative-load variant: any shape, any alignment.
+// Cooperative-load variant: any shape, any alignment.  A warp brings a row of
+// the window at a time, coalesced; the outputs go back through shared memory
+// (the window's place, once every thread has read it) so that a warp stores
+// rows as well, not every SCL_PX-th element.  6000 x 5999 floats, clamped, R =
+// 1 108.4 -> 59.6 us, R = 5 280.5 -> 171.3 us against staging by a division per
+// element and stores SCL_PX elements apart.
 template <int PY>
 __global__ void __launch_bounds__(256)
 scl_mapoverlap_ldst(const SCL_TYPE_0* in, SCL_TYPE_1* out, scl_u64 rows, scl_u64 cols
@@ -92,37 +139,54 @@ scl_mapoverlap_ldst(const SCL_TYPE_0* in, SCL_TYPE_1* out, scl_u64 rows, scl_u64
   SCL_TYPE_0* win = reinterpret_cast<SCL_TYPE_0*>(scl_dyn_smem);  // WIN_H x SCL_WIN_W
   const scl_u64 x0 = (scl_u64)blockIdx.x * SCL_TW, y0 = (scl_u64)blockIdx.y * TH;
   const long long x_org = (long long)x0 - SCL_XLEAD, y_org = (long long)y0 - SCL_R;
-  const int nthreads = blockDim.x * blockDim.y;
-  const int t = threadIdx.y * blockDim.x + threadIdx.x;
-  for (int k = t; k < WIN_H * SCL_WIN_W; k += nthreads) {
-    const int ly = k / SCL_WIN_W, lx = k % SCL_WIN_W;
-    const long long gy = y_org + ly, gx = x_org + lx;
-    SCL_TYPE_0 v;
-    if (gy >= 0 && gy < (long long)rows && gx >= 0 && gx < (long long)cols) {
-      v = in[(scl_u64)gy * cols + (scl_u64)gx];
-    } else {
-#if SCL_PADDING == 1
-      v = in[scl_clampi(gy, (long long)rows - 1) * cols + scl_clampi(gx, (long long)cols - 1)];
-#else
-      v = (SCL_TYPE_0)(SCL_NEUTRAL);
-#endif
-    }
-    win[k] = v;
-  }
+  const int tx = threadIdx.x, ty = threadIdx.y;
+  constexpr bool sized = sizeof(SCL_TYPE_0) == 4 || sizeof(SCL_TYPE_0) == 8;
+  if (sized && (scl_u64)in % sizeof(SCL_TYPE_0) == 0)
+    scl_stage_window<WIN_H, sized>(win, in, x_org, y_org, rows, cols);
+  else
+    scl_stage_window<WIN_H, false>(win, in, x_org, y_org, rows, cols);
+  asm volatile("cp.async.wait_all;" ::: "memory");
   __syncthreads();
-  scl_compute_tile<PY>(win, out, rows, cols, x0, y0 SCL_EXTRA_ARGS);
+  SCL_TYPE_1 res[PY][SCL_PX];
+  scl_compute_tile<PY>(win, res SCL_EXTRA_ARGS);
+  __syncthreads();
+  SCL_TYPE_1* mine = reinterpret_cast<SCL_TYPE_1*>(scl_dyn_smem) + ty * PY * SCL_TW;  // this warp's rows
+#pragma unroll
+  for (int p = 0; p < PY; ++p) {
+    scl_pack<SCL_TYPE_1, SCL_PX> v;
+#pragma unroll
+    for (int c = 0; c < SCL_PX; ++c) v.v[c] = res[p][c];
+    scl_store<SCL_TYPE_1, SCL_PX>(mine + p * SCL_TW + tx * SCL_PX, v);
+  }
+  __syncwarp();
+#pragma unroll
+  for (int p = 0; p < PY; ++p) {
+    const scl_u64 y = y0 + ty * PY + p;
+    if (y >= rows) break;
+#pragma unroll
+    for (int c = 0; c < SCL_PX; ++c) {
+      const scl_u64 x = x0 + c * 32 + tx;
+      if (x < cols) out[y * cols + x] = mine[p * SCL_TW + c * 32 + tx];
+    }
+  }
 }
 
 // TMA variant: one elected thread loads the whole window with
 // cp.async.bulk.tensor.2d (zero fill outside the matrix); border tiles are
 // patched afterwards.  Requires cols * sizeof(T) % 16 == 0 (tensor-map stride
-// rule) and a 16-byte aligned base; the host checks both.
+// rule) and a 16-byte aligned base; the host checks both.  With `ovec` (the
+// host's word that rows of `out` sit on the size of SCL_PX elements) a thread
+// stores its adjacent columns at once.  8192^2 floats, with that and the border
+// patched by rows: clamped R = 1 91.3 -> 78.7 us, R = 2 100.6 -> 87.6, R = 5
+// 299.8 -> 283.2; neutral R = 5 287.4 -> 276.2 us (79 us are the transfer).
+// (A resident grid whose blocks fetch their next window while computing took
+// 100.6 and 327 us clamped: tiles are best handed out as blocks end.)
 struct __align__(64) scl_tmap { unsigned long long v[16]; };
 
 template <int PY>
 __global__ void __launch_bounds__(256)
 scl_mapoverlap_tma(const __grid_constant__ scl_tmap tmap, SCL_TYPE_1* out, scl_u64 rows,
-                   scl_u64 cols, unsigned int spin_limit, unsigned int* err SCL_EXTRA_PARAMS) {
+                   scl_u64 cols, unsigned int spin_limit, unsigned int* err, int ovec SCL_EXTRA_PARAMS) {
   SCL_EXTRA_SETUP
   constexpr int TH = 8 * PY, WIN_H = TH + 2 * SCL_R;
   SCL_TYPE_0* win = reinterpret_cast<SCL_TYPE_0*>(scl_dyn_smem);  // WIN_H x SCL_WIN_W
@@ -181,6 +245,22 @@ scl_mapoverlap_tma(const __grid_constant__ scl_tmap tmap, SCL_TYPE_1* out, scl_u
   if (border) scl_patch_border<WIN_H>(win, x_org, y_org, rows, cols);
 #endif
   __syncthreads();
-  scl_compute_tile<PY>(win, out, rows, cols, x0, y0 SCL_EXTRA_ARGS);
+  SCL_TYPE_1 res[PY][SCL_PX];
+  scl_compute_tile<PY>(win, res SCL_EXTRA_ARGS);
+#pragma unroll
+  for (int p = 0; p < PY; ++p) {
+    const scl_u64 y = y0 + threadIdx.y * PY + p, x = x0 + (scl_u64)threadIdx.x * SCL_PX;
+    if (y >= rows) break;
+    if (ovec) {
+      scl_pack<SCL_TYPE_1, SCL_PX> v;
+#pragma unroll
+      for (int c = 0; c < SCL_PX; ++c) v.v[c] = res[p][c];
+      if (x < cols) scl_store<SCL_TYPE_1, SCL_PX>(out + y * cols + x, v);
+    } else {
+#pragma unroll
+      for (int c = 0; c < SCL_PX; ++c)
+        if (x + c < cols) out[y * cols + x + c] = res[p][c];
+    }
+  }
 }
 #endif
