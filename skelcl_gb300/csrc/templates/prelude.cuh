@@ -353,6 +353,16 @@ __device__ __forceinline__ bool scl_mbar_wait(unsigned int bar_s, unsigned int s
   return true;
 }
 
+// Asks for [lo, hi) (addresses) to be brought into L2: the 16-byte-aligned
+// interior, under 4 GB.
+__device__ __forceinline__ void scl_prefetch_l2(scl_u64 lo, scl_u64 hi) {
+  lo = (lo + 15) & ~(scl_u64)15;
+  hi &= ~(scl_u64)15;
+  if (hi > lo)
+    asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;"
+                 :: "l"((const void*)lo), "r"((unsigned int)(hi - lo)) : "memory");
+}
+
 // Starts bringing src[0 .. len) into shared memory so that src[p] lands at
 // ts[p + shift] (ts 16-byte aligned, room for len + 16 / sizeof(T)
 // elements); returns shift, the elements between src and the 16-byte
