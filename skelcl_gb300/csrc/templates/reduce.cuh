@@ -280,10 +280,11 @@ scl_reduce_short(const scl_T* in, scl_T* out, const scl_u64* seg_off, scl_u64 n_
 // floats 0.143 -> 0.095 ms, 10^7 of 0..2 0.323 -> 0.049 ms, 3 * 10^5 of 200..399
 // 0.123 -> 0.079 ms against a thread per vector of up to 256 elements (about 40
 // busy threads of a block's 256) and a warp per longer one.
+#define SCL_REDUCE_AHEAD 304
 template <int WT>
 __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* out, const scl_u64* seg_off,
-                                                      const scl_u64* win_rec, scl_u64 r, scl_T* ts,
-                                                      unsigned int spin_limit,
+                                                      const scl_u64* win_rec, scl_u64 r, scl_u64 n_rec,
+                                                      scl_T* ts, unsigned int spin_limit,
                                                       unsigned int* err SCL_USER_PARAMS) {
   constexpr int B = 256;
   const scl_T ident = (scl_T)(SCL_IDENTITY);
@@ -298,6 +299,15 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
   const scl_u64 lo = win_rec[4 * r], top = win_rec[4 * r + 1], e0 = win_rec[4 * r + 2];
   const scl_u64 ln = win_rec[4 * r + 3];
   const int len = (int)(ln < (scl_u64)WT ? ln : (scl_u64)WT);  // (more only for bad offsets)
+  // the record two per SM further on is asked into L2 ahead of its block, which
+  // makes two dependent trips there (the record, then what it names): 10^6
+  // vectors of 1..199 floats 95.4 -> 87.1 us (152 records ahead 89.1, 912 87.7)
+  if (threadIdx.x == 32 && r + SCL_REDUCE_AHEAD < n_rec) {
+    const scl_u64* nr = win_rec + 4 * (r + SCL_REDUCE_AHEAD);
+    const scl_u64 a0 = (scl_u64)in + nr[2] * sizeof(scl_T), l0 = nr[3] < (scl_u64)WT ? nr[3] : (scl_u64)WT;
+    scl_prefetch_l2(a0, a0 + l0 * sizeof(scl_T));
+    scl_prefetch_l2((scl_u64)(seg_off + nr[0]), (scl_u64)(seg_off + nr[1] + 1));
+  }
   unsigned int tx;
   const int shift = scl_stage_bulk<scl_T, B>(in + e0, len, ts, bar_s, &tx);
   const scl_u64 nvec = top - lo;
@@ -383,7 +393,7 @@ scl_reduce_seg(const scl_T* in, scl_T* out, const scl_u64* seg_off,
   if constexpr (MERGED != 0) {
     if (blockIdx.x >= nt) {  // (block-uniform: the whole block takes the window role)
       constexpr int WT = 8 * 256 * scl_vec_width<sizeof(scl_T)>::value;  // 32 KB of elements
-      scl_reduce_window_run<WT>(in, out, seg_off, win_rec, blockIdx.x - nt,
+      scl_reduce_window_run<WT>(in, out, seg_off, win_rec, blockIdx.x - nt, gridDim.x - nt,
                                 reinterpret_cast<scl_T*>(scl_dyn_smem), spin_limit, err SCL_EXTRA_ARGS);
       return;
     }
