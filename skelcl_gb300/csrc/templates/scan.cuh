@@ -82,6 +82,36 @@ template <typename C> struct scl_status_mode {
 // faster; for 4-byte carries keeping them is 1 % faster).
 constexpr bool kLocalPrefix = !scl_same<scl_C, scl_T>::value;
 
+// Adjacent 16-byte vectors of a lane in one row of a staged tile.  A row costs
+// every lane five folds across the warp and two more for its prefix; doubles,
+// whose additions this device does at a sixty-fourth of the rate of single
+// precision, take four vectors a lane (2.75 folds an element instead of 5, for
+// four-way bank conflicts): 2^25 doubles 344.5 -> 204.2 us (two vectors 243.7,
+// eight 260.3; floats with two 94.5 -> 102.8 at 2^26).
+constexpr int kLaneVectors = scl_same<scl_T, double>::value ? 4 : 1;
+// A lane's vectors in shared memory.
+template <typename T, int V, int M>
+__device__ __forceinline__ scl_pack<T, V * M> scl_load_lane(const T* p) {
+  scl_pack<T, V * M> r;
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    const scl_pack<T, V> q = scl_load<T, V>(p + m * V);
+#pragma unroll
+    for (int e = 0; e < V; ++e) r.v[m * V + e] = q.v[e];
+  }
+  return r;
+}
+template <typename T, int V, int M>
+__device__ __forceinline__ void scl_store_lane(T* p, const scl_pack<T, V * M>& r) {
+#pragma unroll
+  for (int m = 0; m < M; ++m) {
+    scl_pack<T, V> q;
+#pragma unroll
+    for (int e = 0; e < V; ++e) q.v[e] = r.v[m * V + e];
+    scl_store<T, V>(p + m * V, q);
+  }
+}
+
 __device__ __forceinline__ unsigned long long scl_ld_relaxed64(const unsigned long long* p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -796,6 +826,8 @@ scl_scan_s(const scl_T* in, scl_O* out, scl_u64 n, unsigned int flags, int align
   constexpr int B = SCL_SCAN_B, W = SCL_SCAN_W;
   constexpr int V = scl_vec_width<sizeof(scl_T)>::value;
   constexpr int TILE = R * B * V;
+  // rows of the in-tile scan and a lane's elements in each
+  constexpr int M = R % kLaneVectors == 0 ? kLaneVectors : 1, RR = R / M, VV = V * M;
   constexpr unsigned int ROW_BYTES = B * V * sizeof(scl_T);
   constexpr bool natural = sizeof(scl_T) == 4 || sizeof(scl_T) == 8 || sizeof(scl_T) == 16;
   const bool inclusive = (flags & 1u) != 0, reverse = (flags & 2u) != 0;
@@ -806,7 +838,7 @@ scl_scan_s(const scl_T* in, scl_O* out, scl_u64 n, unsigned int flags, int align
   __shared__ __align__(8) unsigned long long bar;
   __shared__ unsigned int s_tile;
   __shared__ int s_ok;
-  __shared__ scl_T s_wsum[R * W];
+  __shared__ scl_T s_wsum[RR * W];
   __shared__ scl_T s_carry;  // the tile's prefix, converted once to the element type
   const unsigned int bar_s = (unsigned int)__cvta_generic_to_shared(&bar);
   if (threadIdx.x == 0) {
@@ -939,43 +971,43 @@ scl_scan_s(const scl_T* in, scl_O* out, scl_u64 n, unsigned int flags, int align
   }
   const bool mask = bulk && !full;  // positions outside [c_lo, c_hi) hold other data
 
-  // ---- in-thread inclusive scan of each logical vector (written back to its
-  //      slot in logical order), warp scans of the vector totals.  Logical
-  //      vector q sits at q*V, or at TILE-(q+1)*V reversed for a reverse scan.
-  scl_T wincl[R];  // (unused with local prefixes)
+  // ---- in-thread inclusive scan of each lane's VV elements (written back to
+  //      their slots in logical order), warp scans of the totals.  Logical
+  //      group q sits at q*VV, or at TILE-(q+1)*VV reversed for a reverse scan.
+  scl_T wincl[RR];  // (unused with local prefixes)
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
+  for (int r = 0; r < RR; ++r) {
     const int q = r * B + threadIdx.x;
-    const int pos = reverse ? TILE - (q + 1) * V : q * V;
-    scl_pack<scl_T, V> p = scl_load<scl_T, V>(ts + pos);
+    const int pos = reverse ? TILE - (q + 1) * VV : q * VV;
+    scl_pack<scl_T, VV> p = scl_load_lane<scl_T, V, M>(ts + pos);
     if (mask) {
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
+      for (int e = 0; e < VV; ++e) {
         const long long i = tile_lo + pos + e;
         if (i < c_lo || i >= c_hi) p.v[e] = ident;
       }
     }
     if (reverse) {
 #pragma unroll
-      for (int e = 0; e < V / 2; ++e) {
+      for (int e = 0; e < VV / 2; ++e) {
         const scl_T t = p.v[e];
-        p.v[e] = p.v[V - 1 - e];
-        p.v[V - 1 - e] = t;
+        p.v[e] = p.v[VV - 1 - e];
+        p.v[VV - 1 - e] = t;
       }
     }
 #pragma unroll
-    for (int e = 1; e < V; ++e) p.v[e] = SCL_FUNC(p.v[e - 1], p.v[e] SCL_OP_ARGS);
+    for (int e = 1; e < VV; ++e) p.v[e] = SCL_FUNC(p.v[e - 1], p.v[e] SCL_OP_ARGS);
     if constexpr (kLocalPrefix) {
-      const scl_T tot = scl_warp_incl(p.v[V - 1] SCL_EXTRA_ARGS);
+      const scl_T tot = scl_warp_incl(p.v[VV - 1] SCL_EXTRA_ARGS);
       scl_T lx = scl_shfl_up(tot, 1);
       if (lane == 0) lx = ident;
       if (lane == 31) s_wsum[r * W + warp] = tot;
 #pragma unroll
-      for (int e = 0; e < V; ++e) p.v[e] = SCL_FUNC(lx, p.v[e] SCL_OP_ARGS);
-      scl_store<scl_T, V>(ts + pos, p);
+      for (int e = 0; e < VV; ++e) p.v[e] = SCL_FUNC(lx, p.v[e] SCL_OP_ARGS);
+      scl_store_lane<scl_T, V, M>(ts + pos, p);
     } else {
-      scl_store<scl_T, V>(ts + pos, p);
-      wincl[r] = scl_warp_incl(p.v[V - 1] SCL_EXTRA_ARGS);
+      scl_store_lane<scl_T, V, M>(ts + pos, p);
+      wincl[r] = scl_warp_incl(p.v[VV - 1] SCL_EXTRA_ARGS);
       if (lane == 31) s_wsum[r * W + warp] = wincl[r];
     }
   }
@@ -985,13 +1017,13 @@ scl_scan_s(const scl_T* in, scl_O* out, scl_u64 n, unsigned int flags, int align
   if (warp == 0) {
     scl_T carry = ident;
 #pragma unroll
-    for (int c = 0; c < (R * W + 31) / 32; ++c) {
+    for (int c = 0; c < (RR * W + 31) / 32; ++c) {
       const int q = c * 32 + lane;
-      scl_T v = q < R * W ? s_wsum[q] : ident;
+      scl_T v = q < RR * W ? s_wsum[q] : ident;
       scl_T vi = scl_warp_incl(v SCL_EXTRA_ARGS);
       scl_T ve = scl_shfl_up(vi, 1);
       if (lane == 0) ve = ident;
-      if (q < R * W) s_wsum[q] = SCL_FUNC(carry, ve SCL_OP_ARGS);
+      if (q < RR * W) s_wsum[q] = SCL_FUNC(carry, ve SCL_OP_ARGS);
       scl_T total = scl_shfl_idx(vi, 31);
       carry = SCL_FUNC(carry, total SCL_OP_ARGS);
     }
@@ -1012,22 +1044,22 @@ scl_scan_s(const scl_T* in, scl_O* out, scl_u64 n, unsigned int flags, int align
   const bool ovec = sizeof(scl_O) == sizeof(scl_T) && full &&
                     (((scl_u64)out + (scl_u64)(tile_lo * (long long)sizeof(scl_O))) & 15u) == 0;
 #pragma unroll
-  for (int r = 0; r < R; ++r) {
+  for (int r = 0; r < RR; ++r) {
     const int q = r * B + threadIdx.x;
-    const int pos = reverse ? TILE - (q + 1) * V : q * V;
-    scl_pack<scl_T, V> p = scl_load<scl_T, V>(ts + pos);
-    scl_pack<scl_T, V> o;  // logical order
+    const int pos = reverse ? TILE - (q + 1) * VV : q * VV;
+    scl_pack<scl_T, VV> p = scl_load_lane<scl_T, V, M>(ts + pos);
+    scl_pack<scl_T, VV> o;  // logical order
     if constexpr (kLocalPrefix) {
       // the slot holds the warp-local inclusive values
       const scl_T pre = SCL_FUNC(tile_carry, s_wsum[r * W + warp] SCL_OP_ARGS);
       if (inclusive) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) o.v[e] = SCL_FUNC(pre, p.v[e] SCL_OP_ARGS);
+        for (int e = 0; e < VV; ++e) o.v[e] = SCL_FUNC(pre, p.v[e] SCL_OP_ARGS);
       } else {
-        const scl_T lx = scl_shfl_up(p.v[V - 1], 1);  // the previous lane's last value
+        const scl_T lx = scl_shfl_up(p.v[VV - 1], 1);  // the previous lane's last value
         o.v[0] = lane == 0 ? pre : SCL_FUNC(pre, lx SCL_OP_ARGS);
 #pragma unroll
-        for (int e = 1; e < V; ++e) o.v[e] = SCL_FUNC(pre, p.v[e - 1] SCL_OP_ARGS);
+        for (int e = 1; e < VV; ++e) o.v[e] = SCL_FUNC(pre, p.v[e - 1] SCL_OP_ARGS);
       }
     } else {
       scl_T lane_excl = scl_shfl_up(wincl[r], 1);
@@ -1036,29 +1068,29 @@ scl_scan_s(const scl_T* in, scl_O* out, scl_u64 n, unsigned int flags, int align
                                  lane_excl SCL_OP_ARGS);
       if (inclusive) {
 #pragma unroll
-        for (int e = 0; e < V; ++e) o.v[e] = SCL_FUNC(pre, p.v[e] SCL_OP_ARGS);
+        for (int e = 0; e < VV; ++e) o.v[e] = SCL_FUNC(pre, p.v[e] SCL_OP_ARGS);
       } else {
         o.v[0] = pre;
 #pragma unroll
-        for (int e = 1; e < V; ++e) o.v[e] = SCL_FUNC(pre, p.v[e - 1] SCL_OP_ARGS);
+        for (int e = 1; e < VV; ++e) o.v[e] = SCL_FUNC(pre, p.v[e - 1] SCL_OP_ARGS);
       }
     }
     if (reverse) {  // back to physical order
 #pragma unroll
-      for (int e = 0; e < V / 2; ++e) {
+      for (int e = 0; e < VV / 2; ++e) {
         const scl_T t = o.v[e];
-        o.v[e] = o.v[V - 1 - e];
-        o.v[V - 1 - e] = t;
+        o.v[e] = o.v[VV - 1 - e];
+        o.v[VV - 1 - e] = t;
       }
     }
-    scl_pack<scl_O, V> m;
+    scl_pack<scl_O, VV> m;
 #pragma unroll
-    for (int e = 0; e < V; ++e) m.v[e] = SCL_EPILOGUE(o.v[e]);
+    for (int e = 0; e < VV; ++e) m.v[e] = SCL_EPILOGUE(o.v[e]);
     if (ovec) {
-      scl_store<scl_O, V>(out + (tile_lo + pos), m);
+      scl_store_lane<scl_O, V, M>(out + (tile_lo + pos), m);
     } else {
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
+      for (int e = 0; e < VV; ++e) {
         const long long i = tile_lo + pos + e;
         if (i >= c_lo && i < c_hi) out[i] = m.v[e];
       }
