@@ -175,6 +175,10 @@ __global__ void scl_reduce_k(const scl_T* in, scl_T* out, scl_u64 n, int aligned
   if (have) c = (scl_C)acc;
   scl_block_fold(have, c SCL_EXTRA_ARGS);
 
+  if (gridDim.x == 1) {  // no other block's partials to wait for
+    if (threadIdx.x == 0) out[0] = (scl_T)c;
+    return;
+  }
   __shared__ int s_last;
   if (threadIdx.x == 0) {
     // every block holds at least one element (the host sizes the grid so)
@@ -561,6 +565,10 @@ __global__ void scl_zipreduce_k(const SCL_TYPE_0* left, const SCL_TYPE_1* right,
   if (have) c = (scl_C)acc;
   scl_block_fold(have, c SCL_EXTRA_ARGS);
 
+  if (gridDim.x == 1) {
+    if (threadIdx.x == 0) out[0] = (scl_T)c;
+    return;
+  }
   __shared__ int s_last;
   if (threadIdx.x == 0) {
     scl_st_cg(&partials[blockIdx.x], c);  // every block holds at least one element
