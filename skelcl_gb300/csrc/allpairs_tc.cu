@@ -645,7 +645,7 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ---- CTA pairs --------------------------------------------------------------------
-// The default form: 256 x 256 output tiles, one per pair of CTAs
+// The default form: 256 x 256 output tiles, each by a pair of CTAs
 // (cta_group::2, M = 256, N = 256, K = 16).  Each CTA of the pair holds 128
 // rows of A and 128 of the 256 columns of B per stage and the accumulators of
 // its 128 rows x 256 columns; the pair's first CTA issues the MMAs.  Two
@@ -668,6 +668,9 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 // their own accumulators 1.34 ms; 16 epilogue warps of 64 columns 1.25 ms;
 // release / acquire at cluster scope on the accumulators' barriers 1.69 ms
 // (the tcgen05 fences order what they hand over).
+// WALK: as many pairs as the device holds, each over several tiles, so that one
+// tile's way out overlaps the next one's products (allpairs_pair_launch says
+// when).
 // Normwise error against FP64 (2560 x K x 2048), here and with six bf16
 // products: normal operands K = 48 1.2e-7 / 2.1e-7, 128 1.4e-7 / 3.2e-7, 1024
 // 1.5e-7 / 3.2e-7, 4096 2.0e-7 / 3.5e-7; uniform in (0, 1) K = 48 1.4e-7 /
@@ -755,64 +758,84 @@ struct PairBarriers {
   uint64_t drain;         // all issued MMAs completed (each CTA)
 };
 
-template <int FMT>
+template <int FMT, bool WALK>
 __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const PairArgs& g,
                                           uint32_t base, uint32_t ring, uint32_t stage_out, PairBarriers* bars,
-                                          uint32_t tmem, uint32_t rank, uint32_t m0, uint32_t n0, int* s_fail) {
+                                          uint32_t tmem, uint32_t rank, int* s_fail) {
   using SH = PairShape<FMT>;
   constexpr int EPI_WARPS = 4 * (kPairCols / kPairCW);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const uint32_t nk = g.Kp / SH::BK;
+  const uint32_t nk = g.Kp / SH::BK, tiles = g.tiles_m * g.tiles_n;
+  // WALK: the pair takes tiles pair, pair + pairs, ... of all; else tile `pair`
+  const uint32_t pair = blockIdx.x / 2, pairs = WALK ? gridDim.x / 2 : 1, end = WALK ? tiles : pair + 1;
+  // this CTA's rows m0 .. and the tile's columns n0 .. of tile t: tiles in
+  // groups of group_m tile rows (see gemm_3xbf16_kernel)
+  auto place = [&](uint32_t t, uint32_t* m0, uint32_t* n0) {
+    const uint32_t per_group = g.group_m * g.tiles_n;
+    const uint32_t grp = t / per_group, r = t % per_group, first = grp * g.group_m;
+    const uint32_t rows = g.tiles_m - first < g.group_m ? g.tiles_m - first : g.group_m;
+    *m0 = ((first + r % rows) * 2 + rank) * BM;
+    *n0 = (r / rows) * kPairCols;
+  };
+  // the roles' counters run on across the tiles, so that a tile's first operands
+  // and MMAs overlap the last one's way out
   if (warp == 0) {
     // ---- TMA producer (both CTAs): its 128 rows of A and of B's columns, counted
     //      on the first CTA's barrier, and the unscale factors of its outputs
     if (lane == 0) {
-      for (uint32_t kb = 0; kb < nk; ++kb) {
-        const uint32_t s = kb % SH::STAGES, round = kb / SH::STAGES;
-        if (round > 0 && !mbar_wait(smem_u32(&bars->empty[s]), (round - 1) & 1u, g.spin_limit)) {
-          raise(g.err);
-          *s_fail = 1;
-          break;
-        }
-        const uint32_t fb = smem_u32(&bars->full[s]);
-        if (rank == 0)
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                       :: "r"(fb), "r"((uint32_t)(2 * SH::STAGE_BYTES)) : "memory");
-        const uint32_t first_fb = cluster_addr(fb, 0);
-        const uint32_t stage = base + s * SH::STAGE_BYTES;
-        const int kx = (int)(kb * SH::BK);
+      uint32_t m0, n0, it = 0;  // k-blocks so far
+      bool landed = true;
+      for (uint32_t t = pair; landed && t < end; t += pairs) {
+        place(t, &m0, &n0);
+        for (uint32_t kb = 0; kb < nk; ++kb, ++it) {
+          const uint32_t s = it % SH::STAGES, round = it / SH::STAGES;
+          if (round > 0 && !mbar_wait(smem_u32(&bars->empty[s]), (round - 1) & 1u, g.spin_limit)) {
+            raise(g.err);
+            *s_fail = 1;
+            landed = false;
+            break;
+          }
+          const uint32_t fb = smem_u32(&bars->full[s]);
+          if (rank == 0)
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                         :: "r"(fb), "r"((uint32_t)(2 * SH::STAGE_BYTES)) : "memory");
+          const uint32_t first_fb = cluster_addr(fb, 0);
+          const uint32_t stage = base + s * SH::STAGE_BYTES;
+          const int kx = (int)(kb * SH::BK);
 #pragma unroll
-        for (int p = 0; p < SH::PARTS; ++p) {
-          asm volatile(
-              "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-              " [%0], [%1, {%2, %3, %4}], [%5];"
-              :: "r"(stage + (uint32_t)(p * SH::TILE)), "l"(&tmA), "r"(kx), "r"((int)m0), "r"(p), "r"(first_fb)
-              : "memory");
-          asm volatile(
-              "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
-              " [%0], [%1, {%2, %3, %4}], [%5];"
-              :: "r"(stage + (uint32_t)((SH::PARTS + p) * SH::TILE)), "l"(&tmB), "r"(kx),
-                 "r"((int)(n0 + rank * 128u)), "r"(p), "r"(first_fb)
-              : "memory");
-        }
-        if (FMT == kF16 && kb % SH::GS == 0) {
-          // slot grp % kRing was read for slot-group grp - kRing, long drained:
-          // the MMAs of k-block kb - STAGES, just waited for, began after the
-          // drain of k-block kb - STAGES - 2
-          static_assert(kRing * SH::GS >= SH::STAGES + 2 + SH::GS, "a slot is reused after its drain");
-          const uint32_t grp = kb / SH::GS;
-          const uint32_t slot = ring + (grp % kRing) * kSlotBytes, rb = smem_u32(&bars->ring[grp % kRing]);
-          asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                       :: "r"(rb), "r"((uint32_t)kSlotBytes) : "memory");
-          asm volatile(
-              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-              :: "r"(slot), "l"(g.unscale_a + (uint64_t)grp * g.Mp + m0), "r"((uint32_t)(BM * 4)), "r"(rb)
-              : "memory");
-          asm volatile(
-              "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-              :: "r"(slot + BM * 4), "l"(g.unscale_b + (uint64_t)grp * g.Np + n0),
-                 "r"((uint32_t)(kPairCols * 4)), "r"(rb)
-              : "memory");
+          for (int p = 0; p < SH::PARTS; ++p) {
+            asm volatile(
+                "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                " [%0], [%1, {%2, %3, %4}], [%5];"
+                :: "r"(stage + (uint32_t)(p * SH::TILE)), "l"(&tmA), "r"(kx), "r"((int)m0), "r"(p), "r"(first_fb)
+                : "memory");
+            asm volatile(
+                "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.tile.mbarrier::complete_tx::bytes"
+                " [%0], [%1, {%2, %3, %4}], [%5];"
+                :: "r"(stage + (uint32_t)((SH::PARTS + p) * SH::TILE)), "l"(&tmB), "r"(kx),
+                   "r"((int)(n0 + rank * 128u)), "r"(p), "r"(first_fb)
+                : "memory");
+          }
+          if (FMT == kF16 && kb % SH::GS == 0) {
+            // the slot was last read kRing slots ago, long drained: the MMAs of
+            // k-block it - STAGES, just waited for, began after the drain of
+            // k-block it - STAGES - 2
+            static_assert(kRing * SH::GS >= SH::STAGES + 2 + SH::GS, "a slot is reused after its drain");
+            const uint32_t grp = kb / SH::GS;
+            const uint32_t sg = it / SH::GS;  // a tile is a whole number of slots
+            const uint32_t slot = ring + (sg % kRing) * kSlotBytes, rb = smem_u32(&bars->ring[sg % kRing]);
+            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
+                         :: "r"(rb), "r"((uint32_t)kSlotBytes) : "memory");
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                :: "r"(slot), "l"(g.unscale_a + (uint64_t)grp * g.Mp + m0), "r"((uint32_t)(BM * 4)), "r"(rb)
+                : "memory");
+            asm volatile(
+                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+                :: "r"(slot + BM * 4), "l"(g.unscale_b + (uint64_t)grp * g.Np + n0),
+                   "r"((uint32_t)(kPairCols * 4)), "r"(rb)
+                : "memory");
+          }
         }
       }
     }
@@ -844,33 +867,36 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
           }
         };
         bool landed = true;
-        for (uint32_t kb = 0; landed && kb < nk; kb += SH::G) {  // one drain group
-          const uint32_t grp = kb / SH::G, acc_i = grp & 1u, use = grp >> 1;
-          const uint32_t dtm = tmem + acc_i * kPairCols;
-          if (use > 0)
-            landed = mbar_wait_cluster(smem_u32(&bars->acc_empty[acc_i]), (use - 1) & 1u, g.spin_limit);
+        uint32_t it = 0, grp = 0;  // k-blocks and drain groups so far
+        for (uint32_t t = pair; landed && t < end; t += pairs) {
+          for (uint32_t kb = 0; landed && kb < nk; kb += SH::G, it += SH::G, ++grp) {  // one drain group
+            const uint32_t acc_i = grp & 1u, use = grp >> 1;
+            const uint32_t dtm = tmem + acc_i * kPairCols;
+            if (use > 0)
+              landed = mbar_wait_cluster(smem_u32(&bars->acc_empty[acc_i]), (use - 1) & 1u, g.spin_limit);
 #pragma unroll
-          for (int j = 0; j < SH::G; ++j) {
-            const uint32_t s = (kb + j) % SH::STAGES, stage = base + s * SH::STAGE_BYTES;
-            landed = landed && mbar_wait_cluster(smem_u32(&bars->full[s]), ((kb + j) / SH::STAGES) & 1u,
-                                                 g.spin_limit);
-            if (!landed) break;
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (FMT == kF16) {  // lo*hi, hi*lo, hi*hi
-              mma(dtm, stage, 1, 0, true, false);
-              mma(dtm, stage, 0, 1, false, false);
-              mma(dtm, stage, 0, 0, false, true);
-            } else {  // lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi: smallest first
-              mma(dtm, stage, 2, 0, j == 0, false);
-              mma(dtm, stage, 0, 2, false, false);
-              mma(dtm, stage, 1, 1, false, false);
-              mma(dtm, stage, 1, 0, false, false);
-              mma(dtm, stage, 0, 1, false, false);
-              mma(dtm, stage, 0, 0, false, false);
+            for (int j = 0; j < SH::G; ++j) {
+              const uint32_t s = (it + j) % SH::STAGES, stage = base + s * SH::STAGE_BYTES;
+              landed = landed && mbar_wait_cluster(smem_u32(&bars->full[s]), ((it + j) / SH::STAGES) & 1u,
+                                                   g.spin_limit);
+              if (!landed) break;
+              asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+              if (FMT == kF16) {  // lo*hi, hi*lo, hi*hi
+                mma(dtm, stage, 1, 0, true, false);
+                mma(dtm, stage, 0, 1, false, false);
+                mma(dtm, stage, 0, 0, false, true);
+              } else {  // lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi: smallest first
+                mma(dtm, stage, 2, 0, j == 0, false);
+                mma(dtm, stage, 0, 2, false, false);
+                mma(dtm, stage, 1, 1, false, false);
+                mma(dtm, stage, 1, 0, false, false);
+                mma(dtm, stage, 0, 1, false, false);
+                mma(dtm, stage, 0, 0, false, false);
+              }
+              commit_pair(smem_u32(&bars->empty[s]));
             }
-            commit_pair(smem_u32(&bars->empty[s]));
+            if (landed) commit_pair(smem_u32(&bars->acc_full[acc_i]));
           }
-          if (landed) commit_pair(smem_u32(&bars->acc_full[acc_i]));
         }
         if (!landed) {
           raise(g.err);
@@ -887,107 +913,113 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
     //      32 * (w % 4) .. and columns 128 * ((w - 2) / 4) ..
     const int q = warp & 3;
     const uint32_t tile_col = (uint32_t)(((warp - 2) >> 2) * kPairCW);
-    uint64_t sum[kPairCW / 2];  // pairs of neighbouring columns
-#pragma unroll
-    for (int j = 0; j < kPairCW / 2; ++j) sum[j] = 0ull;
     bool ok = true;
-    const uint32_t ngrp = nk / SH::G;
-    for (uint32_t grp = 0; grp < ngrp; ++grp) {
-      const uint32_t acc_i = grp & 1u;
-      uint64_t sa = 0;
-      uint32_t sb = 0;
-      if (FMT == kF16) {
-        const uint32_t sg = grp * SH::G / SH::GS;
-        const uint32_t slot = ring + (sg % kRing) * kSlotBytes;
-        if (!mbar_wait(smem_u32(&bars->ring[sg % kRing]), (sg / kRing) & 1u, g.spin_limit)) {
+    uint32_t grp = 0;  // drain groups so far
+    for (uint32_t t = pair; ok && t < end; t += pairs) {
+      uint64_t sum[kPairCW / 2];  // pairs of neighbouring columns
+#pragma unroll
+      for (int j = 0; j < kPairCW / 2; ++j) sum[j] = 0ull;
+      const uint32_t last = grp + nk / SH::G;
+      for (; grp != last; ++grp) {
+        const uint32_t acc_i = grp & 1u;
+        uint64_t sa = 0;
+        uint32_t sb = 0;
+        if (FMT == kF16) {
+          const uint32_t sg = grp / (SH::GS / SH::G);
+          const uint32_t slot = ring + (sg % kRing) * kSlotBytes;
+          if (!mbar_wait(smem_u32(&bars->ring[sg % kRing]), (sg / kRing) & 1u, g.spin_limit)) {
+            if (lane == 0) raise(g.err);
+            ok = false;
+            break;
+          }
+          uint32_t v;
+          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(slot + (uint32_t)(q * 32 + lane) * 4u));
+          sa = pack2(v, v);
+          sb = slot + BM * 4 + tile_col * 4;
+        }
+        if (!mbar_wait(smem_u32(&bars->acc_full[acc_i]), (grp >> 1) & 1u, g.spin_limit)) {
           if (lane == 0) raise(g.err);
           ok = false;
           break;
         }
-        uint32_t v;
-        asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(slot + (uint32_t)(q * 32 + lane) * 4u));
-        sa = pack2(v, v);
-        sb = slot + BM * 4 + tile_col * 4;
-      }
-      if (!mbar_wait(smem_u32(&bars->acc_full[acc_i]), (grp >> 1) & 1u, g.spin_limit)) {
-        if (lane == 0) raise(g.err);
-        ok = false;
-        break;
-      }
-      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-      const uint32_t tm = tmem + ((uint32_t)(q * 32) << 16) + acc_i * kPairCols + tile_col;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const uint32_t tm = tmem + ((uint32_t)(q * 32) << 16) + acc_i * kPairCols + tile_col;
 #pragma unroll
-      for (int c = 0; c < kPairCW / 16; ++c) {
-        uint32_t r[16];
-        tmem_load16(tm + (uint32_t)(c * 16), r);
-        if (FMT == kF16) {
-          uint64_t f[8];
+        for (int c = 0; c < kPairCW / 16; ++c) {
+          uint32_t r[16];
+          tmem_load16(tm + (uint32_t)(c * 16), r);
+          if (FMT == kF16) {
+            uint64_t f[8];
 #pragma unroll
-          for (int j = 0; j < 4; ++j)
-            asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];"
-                         : "=l"(f[2 * j]), "=l"(f[2 * j + 1]) : "r"(sb + (uint32_t)(c * 64 + j * 16)));
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int j = 0; j < 4; ++j)
+              asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];"
+                           : "=l"(f[2 * j]), "=l"(f[2 * j + 1]) : "r"(sb + (uint32_t)(c * 64 + j * 16)));
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            sum[c * 8 + j] = fma2(pack2(r[2 * j], r[2 * j + 1]), mul2(sa, f[j]), sum[c * 8 + j]);
-        } else {
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+            for (int j = 0; j < 8; ++j)
+              sum[c * 8 + j] = fma2(pack2(r[2 * j], r[2 * j + 1]), mul2(sa, f[j]), sum[c * 8 + j]);
+          } else {
+            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-          for (int j = 0; j < 8; ++j)
-            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[c * 8 + j]) : "l"(pack2(r[2 * j], r[2 * j + 1])));
-        }
-      }
-      // accumulator drained: hand it back to the MMA issuer (one arrive per warp)
-      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-      __syncwarp();
-      if (lane == 0)
-        asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];"
-                     :: "r"(cluster_addr(smem_u32(&bars->acc_empty[acc_i]), 0)) : "memory");
-    }
-    // The sums leave 16 columns at a time through shared memory (16-byte chunk
-    // c of row r at chunk c ^ (r / 2 % 4)), four lanes to a row, so that a
-    // store covers 64 bytes of eight rows instead of 16 bytes of 32 (8192 x 256
-    // x 8192 245 -> 171 us, K = 4096 1.14 -> 1.11 ms).
-    if (ok) {
-      const uint32_t st = stage_out + (uint32_t)(warp - 2) * 2048u;
-      const bool vec = (g.N % 4u) == 0u;
-#pragma unroll
-      for (int c = 0; c < kPairCW / 16; ++c) {
-#pragma unroll
-        for (int j = 0; j < 4; ++j)
-          asm volatile("st.shared.v2.u64 [%0], {%1, %2};"
-                       :: "r"(st + (uint32_t)lane * 64u + (((uint32_t)j ^ ((uint32_t)lane >> 1 & 3u)) * 16u)),
-                          "l"(sum[c * 8 + 2 * j]), "l"(sum[c * 8 + 2 * j + 1])
-                       : "memory");
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          const uint32_t r = (uint32_t)(i * 8 + (lane >> 2)), ch = (uint32_t)(lane & 3);
-          float4 v;
-          asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                       : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                       : "r"(st + r * 64u + ((ch ^ (r >> 1 & 3u)) * 16u))
-                       : "memory");
-          const uint32_t row = m0 + (uint32_t)(q * 32) + r, col = n0 + tile_col + (uint32_t)(c * 16) + ch * 4u;
-          if (row < g.M) {
-            float* dst = g.P + (uint64_t)row * g.N + col;
-            if (vec && col + 4u <= g.N) {
-              *reinterpret_cast<float4*>(dst) = v;
-            } else {
-              if (col < g.N) dst[0] = v.x;
-              if (col + 1u < g.N) dst[1] = v.y;
-              if (col + 2u < g.N) dst[2] = v.z;
-              if (col + 3u < g.N) dst[3] = v.w;
-            }
+            for (int j = 0; j < 8; ++j)
+              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[c * 8 + j]) : "l"(pack2(r[2 * j], r[2 * j + 1])));
           }
         }
+        // accumulator drained: hand it back to the MMA issuer (one arrive per warp)
+        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
         __syncwarp();
+        if (lane == 0)
+          asm volatile("mbarrier.arrive.relaxed.cluster.shared::cluster.b64 _, [%0];"
+                       :: "r"(cluster_addr(smem_u32(&bars->acc_empty[acc_i]), 0)) : "memory");
+      }
+      // The sums leave 16 columns at a time through shared memory (16-byte chunk
+      // c of row r at chunk c ^ (r / 2 % 4)), four lanes to a row, so that a
+      // store covers 64 bytes of eight rows instead of 16 bytes of 32 (8192 x 256
+      // x 8192 245 -> 171 us, K = 4096 1.14 -> 1.11 ms).
+      if (ok) {
+        const uint32_t st = stage_out + (uint32_t)(warp - 2) * 2048u;
+        const bool vec = (g.N % 4u) == 0u;
+        uint32_t m0, n0;
+        place(t, &m0, &n0);
+#pragma unroll
+        for (int c = 0; c < kPairCW / 16; ++c) {
+#pragma unroll
+          for (int j = 0; j < 4; ++j)
+            asm volatile("st.shared.v2.u64 [%0], {%1, %2};"
+                         :: "r"(st + (uint32_t)lane * 64u + (((uint32_t)j ^ ((uint32_t)lane >> 1 & 3u)) * 16u)),
+                            "l"(sum[c * 8 + 2 * j]), "l"(sum[c * 8 + 2 * j + 1])
+                         : "memory");
+          __syncwarp();
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            const uint32_t r = (uint32_t)(i * 8 + (lane >> 2)), ch = (uint32_t)(lane & 3);
+            float4 v;
+            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                         : "r"(st + r * 64u + ((ch ^ (r >> 1 & 3u)) * 16u))
+                         : "memory");
+            const uint32_t row = m0 + (uint32_t)(q * 32) + r, col = n0 + tile_col + (uint32_t)(c * 16) + ch * 4u;
+            if (row < g.M) {
+              float* dst = g.P + (uint64_t)row * g.N + col;
+              if (vec && col + 4u <= g.N) {
+                *reinterpret_cast<float4*>(dst) = v;
+              } else {
+                if (col < g.N) dst[0] = v.x;
+                if (col + 1u < g.N) dst[1] = v.y;
+                if (col + 2u < g.N) dst[2] = v.z;
+                if (col + 3u < g.N) dst[3] = v.w;
+              }
+            }
+          }
+          __syncwarp();
+        }
       }
     }
   }
   static_assert(EPI_WARPS * 32 + 64 == kPairThreads, "");
 }
 
+template <bool WALK>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB3,
@@ -1001,15 +1033,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   const uint32_t ring = base + 3 * 64 * 1024, stage_out = ring + kRing * kSlotBytes;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
-  uint32_t m0, n0;
-  {
-    // tiles in groups of group_m tile rows (see gemm_3xbf16_kernel)
-    const uint32_t t = blockIdx.x / 2, per_group = g.group_m * g.tiles_n;
-    const uint32_t grp = t / per_group, r = t % per_group, first = grp * g.group_m;
-    const uint32_t rows = g.tiles_m - first < g.group_m ? g.tiles_m - first : g.group_m;
-    m0 = ((first + r % rows) * 2 + rank) * BM;
-    n0 = (r / rows) * kPairCols;
-  }
   if (threadIdx.x == 0) {
     s_fail = 0;
     auto init = [](uint64_t* b, uint32_t count) {
@@ -1040,9 +1063,9 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
   if (f16)
-    pair_body<kF16>(tmA, tmB, g, base, ring, stage_out, &bars, tmem, rank, m0, n0, &s_fail);
+    pair_body<kF16, WALK>(tmA, tmB, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
   else
-    pair_body<kBf16>(tmA3, tmB3, g, base, ring, stage_out, &bars, tmem, rank, m0, n0, &s_fail);
+    pair_body<kBf16, WALK>(tmA3, tmB3, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
 
   // ---- teardown: wait for the copies a failed pipeline may still have in
   //      flight (bounded), then, both CTAs together, free the tensor memory
@@ -1223,6 +1246,34 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
   return SCL_OK;
 }
 
+namespace {
+// CTA pairs the device holds at once.
+uint64_t resident_pairs() {
+  int n = rt().pair_clusters;
+  if (n == 0) {
+    const int half = (rt().sm_count > 0 ? rt().sm_count : 148) / 2;
+    cudaLaunchAttribute attr{};
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = 2;
+    attr.val.clusterDim.y = attr.val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg{};
+    cfg.gridDim = dim3((unsigned)(2 * half));
+    cfg.blockDim = dim3(tc::kPairThreads);
+    cfg.dynamicSmemBytes = tc::kPairSmem;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    if (cudaFuncSetAttribute(tc::gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                             (int)tc::kPairSmem) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, tc::gemm_pair_kernel<true>, &cfg) != cudaSuccess || n < 1) {
+      cudaGetLastError();
+      n = half;
+    }
+    rt().pair_clusters = n;
+  }
+  return (uint64_t)n;
+}
+}  // namespace
+
 // CTA pairs: FP16 parts, with the bf16 parts as the device's fallback.
 // `head` (allpairs_tc_head_bytes) precedes the scratch; `epoch` differs from
 // every earlier launch's on this head, or the head was cleared before.
@@ -1256,8 +1307,17 @@ int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, u
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
   const tc::PairArgs args = {P,     sp.a.unscale, sp.b.unscale, verdict, err,        M,       N,      Kp,
                              sp.Mp, sp.Np,        epoch,        spin_limit, tiles.n, tiles.m, tiles.group};
-  e = launch_overlapped(tc::gemm_pair_kernel, dim3(2 * tiles.m * tiles.n), dim3(tc::kPairThreads), tc::kPairSmem, stream,
-                        tmA, tmB, tmA3, tmB3, args);
+  // With few k-blocks to a tile, its start and its way out weigh more than its
+  // products: each pair then walks over the tiles.  us, one tile per pair and
+  // walking, 8192 x K x 8192: K = 64 134 / 101, 256 171 / 146, 1000 347 / 328,
+  // 2048 579 / 579, 4096 1085 / 1100, 16384 4500 / 4680 (dealt out in advance,
+  // the tiles do not follow the pairs' speeds); 5000 x 100 x 5000 57 / 50; with
+  // 2.5 tiles to a pair (4000 x K x 3000) at K = 1000 81.5 / 82.5.
+  const uint64_t all = (uint64_t)tiles.m * tiles.n;
+  const bool walk = Kp <= 1024 && all > resident_pairs() * (Kp <= 512 ? 1 : 4);
+  e = launch_overlapped(walk ? tc::gemm_pair_kernel<true> : tc::gemm_pair_kernel<false>,
+                        dim3((unsigned)(2 * (walk ? resident_pairs() : all))), dim3(tc::kPairThreads), tc::kPairSmem,
+                        stream, tmA, tmB, tmA3, tmB3, args);
   if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
   return SCL_OK;
 }

@@ -5,6 +5,7 @@
 #include <cuda.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
 #include <deque>
 #include <functional>
@@ -82,6 +83,7 @@ struct Runtime {
   uint64_t pdl_launches = 0;
   uint64_t device_allocs = 0;  // device allocations made by the library (scl_alloc included)
   uint64_t module_loads = 0;   // cubins loaded
+  std::atomic<int> pair_clusters{0};  // resident CTA pairs of the tensor-core AllPairs (0: not asked yet)
   bool capturing = false;
   Driver drv;
 };

@@ -162,6 +162,7 @@ extern "C" int scl_init(int device) {
   SCL_CUDA(cudaGetDeviceProperties(&prop, device));
   g_rt.device = device;
   g_rt.sm_count = prop.multiProcessorCount;
+  g_rt.pair_clusters = 0;
   g_rt.cc_major = prop.major;
   g_rt.cc_minor = prop.minor;
   g_rt.smem_optin = prop.sharedMemPerBlockOptin;

@@ -42,6 +42,21 @@ def test_pair_against_fp64(scl, orc, shape, flags):
     assert np.all(np.abs(P - A.astype(np.float64) @ B.astype(np.float64)) <= bound)
 
 
+# more tiles than a GPU holds pairs: each pair walks over several
+@pytest.mark.parametrize("shape", [(2300, 48, 2600), (2500, 130, 2305), (2561, 500, 2048), (4600, 1000, 4370),
+                                   (4100, 1100, 1300)])
+def test_pair_walk_against_fp64(scl, orc, shape):
+    M, K, N = shape
+    A = orc.normal_f32(M * K, 81).reshape(M, K)
+    B = orc.normal_f32(K * N, 82).reshape(K, N)
+    p = program()
+    P = run(p, A, B)
+    bound = C * (np.abs(A).astype(np.float64) @ np.abs(B).astype(np.float64))
+    assert np.all(np.abs(P - A.astype(np.float64) @ B.astype(np.float64)) <= bound)
+    A[M - 1, 3] = np.inf  # bf16 parts
+    assert np.array_equal(run(p, A, B), run(p, A, B, items=3), equal_nan=True)
+
+
 @pytest.mark.parametrize("exp", [-10, -26, -27, -30, -45, -70])
 def test_pair_small_elements(scl, exp):
     """A small element of A that meets the only non-zero element of B's column
