@@ -90,6 +90,18 @@ struct Runtime {
 Runtime& rt();
 int require_init();
 
+// ---- CUDA-core AllPairs (templates/allpairs.cuh): its tiles, small to large ----
+struct AllPairsTile {
+  const char* kernel;
+  unsigned int rows, cols, threads;
+};
+constexpr AllPairsTile kAllPairsTiles[] = {
+    {"scl_allpairs_simt<16, 16, 1, 1, 64, 3, 4>", 16, 16, 256},
+    {"scl_allpairs_simt<32, 32, 2, 2, 32, 3, 4>", 32, 32, 256},
+    {"scl_allpairs_simt<64, 64, 4, 4, 32, 2, 4>", 64, 64, 256},
+    {"scl_allpairs_simt<64, 128, 8, 8, 16, 2, 4>", 64, 128, 128},
+};
+
 // ---- splicer ----------------------------------------------------------------
 enum class ParamKind { Value, Buffer, Matrix, Local };
 struct Param {

@@ -254,6 +254,34 @@ uint64_t reduce_grid(uint64_t units, uint32_t wg, uint32_t items, uint64_t maxb)
   return std::min(maxb, std::max(full, std::min(most, sms)));
 }
 
+// Tile of the CUDA-core AllPairs for M x N outputs.  A block takes its K steps
+// whatever its size, so the smallest tile whose blocks the SMs (152) still hold
+// without queueing wins: us, |x - y| of floats, K = 255, by tile 16 / 32 / 64 /
+// 64 x 128:   193^2  8.4 / 11.0 / 22.2 / 33.0     240^2  7.0 / 7.5 / 15.1 / 28.4
+//   301^2  10.4 / 9.5 / 17.2 / 35.3               500^2  20.9 / 11.4 / 15.2 / 29.9
+//   600^2  28.6 / 16.0 / 15.9 / 29.8              1001^2  76 / 37 / 30.4 / 30.9
+//   2001^2  292 / 125 / 86.5 / 93.0               2700^2  508 / 216 / 143.8 / 146.6
+//   4001^2  1142 / 481 / 306.1 / 304.5            4096^2 (K = 256)  - / - / 293.2 / 287.0
+// Operands narrower than 4 bytes are staged through registers, which the large
+// tile's 8 x 8 outputs pay for sooner (unsigned char, K = 128, tiles 64 / 64 x
+// 128: 1400^2 25.5 / 22.9, 3000^2 91 / 80).  Of wider values the two small
+// tiles alone: their arithmetic (FP64 1/64, 64-bit integers several
+// instructions) is what counts, and an even share of it (double x * y, K = 128,
+// tiles 16 / 32 / 64: 97^2 10.6 / 35 / 132, 1400^2 409 / 417 / 513, 3000^2 1857
+// / 1876 / 1909; long 3000^2 478 / 314 / 317).
+int allpairs_tile(const scl_program* p, unsigned int M, unsigned int N) {
+  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  auto waves = [&](int tile) {
+    const AllPairsTile& t = kAllPairsTiles[tile];
+    return (((uint64_t)M + t.rows - 1) / t.rows * (((uint64_t)N + t.cols - 1) / t.cols) + sms - 1) / sms;
+  };
+  const size_t l = p->type_sizes[0], r = p->type_sizes[1], o = p->type_sizes[2];
+  if (waves(0) <= 2) return 0;
+  if (waves(1) <= 3 || l > 4 || r > 4 || o > 4) return 1;
+  if (l < 4 || r < 4) return 10 * waves(2) >= 17 * waves(3) ? 3 : 2;
+  return waves(2) >= 24 ? 3 : 2;
+}
+
 uint32_t pick_block(const scl_tuning* t, uint32_t dflt) {
   uint32_t b = (t && t->workgroup) ? t->workgroup : dflt;
   if (b > 1024) b = 1024;
@@ -956,8 +984,13 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
     if (want == SCL_VARIANT_TC3XBF16)
       return fail(SCL_ERR_UNSUPPORTED, "the tensor-core AllPairs needs zip x*y, reduce x+y, identity 0, "
                                        "float operands, no extra arguments and supported shapes");
-    CUfunction fn = find_kernel(p, "scl_allpairs_simt");
-    if (!fn) return fail(SCL_ERR_LAUNCH, "kernel scl_allpairs_simt missing");
+    int tile = allpairs_tile(p, M, N);
+    CUfunction fn = nullptr;
+    auto get_kernel = [&] {
+      fn = hot_kernel(p, (uint32_t)tile, [&] { return std::string(kAllPairsTiles[tile].kernel); });
+      return fn ? SCL_OK : fail(SCL_ERR_LAUNCH, std::string("kernel ") + kAllPairsTiles[tile].kernel + " missing");
+    };
+    if (int st = get_kernel()) return st;
     if (trans) {
       // CUDA-core kernel: transposed operands are first stored row-major in
       // the program's workspace
@@ -975,16 +1008,26 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
         B = ws + a_bytes;
       }
     }
-    int vec_a = (p->type_sizes[0] == 4 && K % 4 == 0 && aligned16(A)) ? 1 : 0;
     int vec_b = (p->type_sizes[1] == 4 && N % 4 == 0 && aligned16(B)) ? 1 : 0;
     ArgPack pack;
-    pack.ptrs = {&A, &B, &P, &M, &N, &K, &vec_a, &vec_b};
+    unsigned int tiles_n = 0;
+    pack.ptrs = {&A, &B, &P, &M, &N, &K, &tiles_n, &vec_b};
     if (int st = pack_extra(p, fn, pack.ptrs.size(), (const unsigned char*)extra, extra_bytes, &pack))
       return st;
-    dim3 grid((N + 127) / 128, (M + 127) / 128);
-    if (grid.y > 65535) return fail(SCL_ERR_ARG, "too many rows");
+    if (((uint64_t)M + 127) / 128 > 65535) return fail(SCL_ERR_ARG, "too many rows");
+    // 34 KB of static shared memory leave 14 KB for Local arguments, less than
+    // the 16 KB that a launch may ask for without more ado: the next tile's 25
+    // KB are enough
+    if (tile == 2 && pack.local_bytes > 12 * 1024) {
+      tile = 3;
+      if (int st = get_kernel()) return st;
+    }
+    const AllPairsTile& t = kAllPairsTiles[tile];
+    tiles_n = (unsigned)(((uint64_t)N + t.cols - 1) / t.cols);
+    const uint64_t blocks = ((uint64_t)M + t.rows - 1) / t.rows * tiles_n;
+    if (blocks > 0x7fffffffull) return fail(SCL_ERR_ARG, "too many outputs");
     p->last_variant = SCL_VARIANT_SIMT;
-    return launch(fn, grid, dim3(256), 0, pack);
+    return launch(fn, dim3((unsigned)blocks), dim3(t.threads), 0, pack);
   }
   if (trans) return fail(SCL_ERR_UNSUPPORTED, "transposed operands: only the Reduce/Zip AllPairs");
   CUfunction fn = find_kernel(p, "scl_allpairs_generic");

@@ -380,7 +380,7 @@ int assemble(const scl_program_desc* d, scl_program* p, bool want_f64, Assembly*
       break;
     case SCL_KIND_ALLPAIRS:
       s << scl_tpl_allpairs;
-      out->kernels = {"scl_allpairs_simt"};
+      for (const AllPairsTile& t : kAllPairsTiles) out->kernels.push_back(t.kernel);
       break;
     case SCL_KIND_ALLPAIRS_GENERIC:
       s << scl_tpl_allpairs;

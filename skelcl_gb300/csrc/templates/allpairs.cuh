@@ -6,11 +6,20 @@
 // folded strictly in k order (AllPairsKernel.cl:89-91); the right operand is
 // K x N row-major (AllPairsKernel.cl:72).  Extra arguments: the Reduce's
 // first, then the Zip's (AllPairsDef.h:265-269).
-// Shape: 128 x 128 output tile per 256-thread block, 8 x 8 register
-// accumulators per thread, k-tiles of 16 double-buffered in shared memory
-// with the next tile prefetched into registers.  Unlike the reference, P is
-// written once (the reference re-reads and re-writes P every 32-wide k
+// Shape: BM x BN outputs per block, TM x TN accumulators per thread, k-tiles
+// copied into a ring in shared memory with cp.async.  Unlike the reference, P
+// is written once (the reference re-reads and re-writes P every 32-wide k
 // segment, AllPairsKernel.cl:77-78,95-96).
+// A fold runs along k in one thread, so a block's time is that of its K steps
+// whatever the size of the output: small outputs are bound by how many blocks
+// share them and by a step's latency, large ones by the arithmetic (FP32: two
+// instructions per pair of |x - y| and +).  Hence four tiles, chosen by the
+// number of blocks (scl_launch_allpairs).  us against one tile of 128 x 128
+// with register prefetch: |x - y|, K = 255 97 x 97 46.7 -> 5.9, 500 x 500
+// 46.7 -> 11.4, 1001 x 1001 51 -> 30, 2700 x 2700 170 -> 144, 4096 x 4096 (K =
+// 256) 289 -> 287 (bound by issue; 3.8 % of it the last wave); double x * y,
+// K = 128 97 x 97 517 -> 10.6, 1400 x 1400 524 -> 417, 3000 x 3000 2086 ->
+// 1876 (FP64 pipe: 1840).
 //
 // SCL_KIND 13 (user f(lmatrix_t*, rmatrix_t*, dim, ...),
 // include/SkelCL/detail/AllPairsKernel2.cl:42-65): one output per thread in
@@ -18,132 +27,172 @@
 // they are staged there and the accessors read the staged copies.
 // ---------------------------------------------------------------------------
 #if SCL_KIND == 12
-#define SCL_AP_BM 128
-#define SCL_AP_BN 128
-// k-tile: 16 for 4-byte operands, 8 for wider ones (48 KB of static shared memory)
-#define SCL_AP_BK ((sizeof(SCL_TYPE_0) <= 4 && sizeof(SCL_TYPE_1) <= 4) ? 16 : 8)
 typedef SCL_TYPE_0 scl_L;
 typedef SCL_TYPE_1 scl_Rt;
 typedef SCL_TYPE_2 scl_O;
 
-// Thread (tx, ty) of the 16 x 16 block owns rows {ty*4 .. +3, 64 + ty*4 .. +3}
-// and columns {tx*4 .. +3, 64 + tx*4 .. +3} of the 128 x 128 tile: its
-// shared-memory reads are 16-byte loads that a warp spreads over all banks.
-// two blocks per SM when the accumulators are 4-byte values
-extern "C" __global__ void __launch_bounds__(256, sizeof(SCL_TYPE_2) <= 4 ? 2 : 1)
+template <typename T> struct scl_ap_real { static constexpr bool value = false; };
+template <> struct scl_ap_real<float> { static constexpr bool value = true; };
+template <> struct scl_ap_real<double> { static constexpr bool value = true; };
+
+// BYTES to shared memory, complete after cp.async.wait_group.
+template <int BYTES>
+__device__ __forceinline__ void scl_ap_copy(void* dst, const void* src) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], %2;"
+               :: "r"((unsigned int)__cvta_generic_to_shared(dst)), "l"(src), "n"(BYTES) : "memory");
+}
+
+// k-tiles of BK4 in STAGES buffers, BK4 / 2 where an operand is wider than 4
+// bytes.  Thread (tx, ty) owns groups of four (or all) consecutive rows and
+// columns, the groups spread over the tile: its shared-memory reads are
+// 16-byte loads that a warp spreads over all banks.  The block's tile is
+// blockIdx.x in rows of tiles_n.
+template <int BM, int BN, int TM, int TN, int BK4, int STAGES, int PER_SM>
+__global__ void __launch_bounds__(BM / TM * (BN / TN), PER_SM)
 scl_allpairs_simt(const scl_L* A, const scl_Rt* B, scl_O* P, unsigned int M, unsigned int N,
-                  unsigned int K, int vec_a, int vec_b SCL_EXTRA_PARAMS) {
+                  unsigned int K, unsigned int tiles_n, int vec_b SCL_EXTRA_PARAMS) {
   SCL_EXTRA_SETUP
-  __shared__ __align__(16) scl_L As[2][SCL_AP_BK][SCL_AP_BM];
-  __shared__ __align__(16) scl_Rt Bs[2][SCL_AP_BK][SCL_AP_BN];
+  // wider values take tiles of at most four outputs per thread
+  if constexpr (TM * TN > 4 && (sizeof(scl_L) > 4 || sizeof(scl_Rt) > 4 || sizeof(scl_O) > 4)) return;
+  constexpr int BK = sizeof(scl_L) <= 4 && sizeof(scl_Rt) <= 4 ? BK4 : BK4 / 2;
+  constexpr int TX = BN / TN, TY = BM / TM, THREADS = TX * TY;
+  constexpr int VA = TM < 4 ? TM : 4, VB = TN < 4 ? TN : 4;
+  constexpr bool ASYNC = (sizeof(scl_L) == 4 || sizeof(scl_L) == 8) && (sizeof(scl_Rt) == 4 || sizeof(scl_Rt) == 8);
+  constexpr int AHEAD = ASYNC ? STAGES - 1 : 1;
+  constexpr int LDA = BM + 4;  // (the transposed stores of A meet two to a bank)
+  // 8 x 8 accumulators: 64 x 128 of |x - y| at 4096 x 256 x 4096 307 us with all
+  // 16 steps unrolled, 287 with four; int x * y at 4001 x 255 x 4001 264 and 269
+  constexpr int UNR = TM == 8 && scl_ap_real<scl_O>::value ? 4 : BK;
+  constexpr int TAIL = TM * TN >= 32 ? 1 : 4;
+  __shared__ __align__(16) scl_L As[STAGES][BK][LDA];
+  __shared__ __align__(16) scl_Rt Bs[STAGES][BK][BN];
   const int tid = threadIdx.x;
-  const int tx = tid & 15, ty = tid >> 4;
-  const unsigned int m0 = blockIdx.y * SCL_AP_BM, n0 = blockIdx.x * SCL_AP_BN;
-  // global -> register mapping: A tile 128 rows x BK k (row = tid/2, AE
-  // consecutive k per thread), B tile BK k x 128 cols (BE consecutive columns)
-  constexpr int BK = SCL_AP_BK, AE = BK / 2, TPR = 256 / BK, BE = SCL_AP_BN / TPR;
-  const int a_row = tid >> 1, a_k = (tid & 1) * AE;
-  const int b_k = tid / TPR, b_col = (tid % TPR) * BE;
-  scl_L ra[AE];
-  scl_Rt rb[BE];
-  auto load_tile = [&](unsigned int k0) {
-    const unsigned int gm = m0 + a_row;
+  const int tx = tid % TX, ty = tid / TX;
+  const unsigned int m0 = blockIdx.x / tiles_n * BM, n0 = blockIdx.x % tiles_n * BN;
+  // global -> shared: a thread brings A[row ra + i * RS][k ka] and
+  // B[k kb + i * KS][column cb]; rows and columns past the matrix are read from
+  // its last, for outputs that are not stored, and k past K are left out
+  static_assert(THREADS % BK == 0 && THREADS % BN == 0, "");
+  constexpr int RS = THREADS / BK, AE = BM / RS, KS = THREADS / BN, BE = BK / KS, KSV = THREADS / (BN / 4);
+  const int ra = tid / BK, ka = tid % BK;
+  const bool rows_in = m0 + BM <= M;
+  scl_L va[ASYNC ? 1 : AE];
+  scl_Rt vb[ASYNC ? 1 : BE];
+  auto fetch = [&](unsigned int kt) {
+    const unsigned int k0 = kt * BK;
+    const int buf = (int)(kt % STAGES);
+    if (k0 + ka < K) {
+      const scl_L* src = A + (scl_u64)(m0 + ra) * K + (k0 + ka);
 #pragma unroll
-    for (int h = 0; h < AE / 4; ++h) {
-      const unsigned int gk = k0 + a_k + h * 4;
-      if (vec_a && gm < M && gk + 3 < K) {
-        scl_pack<scl_L, 4> p = scl_load<scl_L, 4>(A + (scl_u64)gm * K + gk);
-#pragma unroll
-        for (int i = 0; i < 4; ++i) ra[h * 4 + i] = p.v[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          ra[h * 4 + i] = (gm < M && gk + i < K) ? A[(scl_u64)gm * K + gk + i] : (scl_L)0;
+      for (int i = 0; i < AE; ++i) {
+        if (!rows_in) src = A + (scl_u64)min(m0 + ra + i * RS, M - 1) * K + (k0 + ka);
+        if constexpr (ASYNC) scl_ap_copy<(int)sizeof(scl_L)>(&As[buf][ka][ra + i * RS], src);
+        else va[i] = *src;
+        src += (scl_u64)RS * K;
       }
     }
-    const unsigned int bk = k0 + b_k;
+    if constexpr (ASYNC && sizeof(scl_Rt) == 4) {
+      if (vec_b) {
+        const int c = tid % (BN / 4) * 4, k = tid / (BN / 4);
+        const scl_Rt* src = B + (scl_u64)(k0 + k) * N + (n0 + c < N ? n0 + c : 0);
 #pragma unroll
-    for (int h = 0; h < BE / 4; ++h) {
-      const unsigned int bn = n0 + b_col + h * 4;
-      if (vec_b && bk < K && bn + 3 < N) {
-        scl_pack<scl_Rt, 4> p = scl_load<scl_Rt, 4>(B + (scl_u64)bk * N + bn);
+        for (int i = 0; i < (BK + KSV - 1) / KSV; ++i, src += (scl_u64)KSV * N)
+          if (k + i * KSV < BK && k0 + k + i * KSV < K) scl_ap_copy<16>(&Bs[buf][k + i * KSV][c], src);
+        return;
+      }
+    }
+    const int cb = tid % BN, kb = tid / BN;
+    const scl_Rt* src = B + (scl_u64)(k0 + kb) * N + min(n0 + cb, N - 1);
 #pragma unroll
-        for (int i = 0; i < 4; ++i) rb[h * 4 + i] = p.v[i];
-      } else {
-#pragma unroll
-        for (int i = 0; i < 4; ++i)
-          rb[h * 4 + i] = (bk < K && bn + i < N) ? B[(scl_u64)bk * N + bn + i] : (scl_Rt)0;
+    for (int i = 0; i < BE; ++i, src += (scl_u64)KS * N) {
+      if (k0 + kb + i * KS < K) {
+        if constexpr (ASYNC) scl_ap_copy<(int)sizeof(scl_Rt)>(&Bs[buf][kb + i * KS][cb], src);
+        else vb[i] = *src;
       }
     }
   };
-  auto store_tile = [&](int buf) {
+  auto put = [&](unsigned int kt) {
+    if constexpr (!ASYNC) {
+      const int buf = (int)(kt % STAGES);
 #pragma unroll
-    for (int i = 0; i < AE; ++i) As[buf][a_k + i][a_row] = ra[i];
+      for (int i = 0; i < AE; ++i) As[buf][ka][ra + i * RS] = va[i];
 #pragma unroll
-    for (int i = 0; i < BE; ++i) Bs[buf][b_k][b_col + i] = rb[i];
+      for (int i = 0; i < BE; ++i) Bs[buf][tid / BN + i * KS][tid % BN] = vb[i];
+    }
   };
-  auto step = [&](scl_O (&acc)[8][8], int cur, int kk) {
-    scl_L a[8];
-    scl_Rt b[8];
-    const scl_pack<scl_L, 4> a0 = scl_load<scl_L, 4>(&As[cur][kk][ty * 4]);
-    const scl_pack<scl_L, 4> a1 = scl_load<scl_L, 4>(&As[cur][kk][64 + ty * 4]);
-    const scl_pack<scl_Rt, 4> b0 = scl_load<scl_Rt, 4>(&Bs[cur][kk][tx * 4]);
-    const scl_pack<scl_Rt, 4> b1 = scl_load<scl_Rt, 4>(&Bs[cur][kk][64 + tx * 4]);
+  auto commit = [&]() {
+    if constexpr (ASYNC) asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  auto step = [&](scl_O (&acc)[TM][TN], int cur, int kk) {
+    scl_L a[TM];
+    scl_Rt b[TN];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      a[i] = a0.v[i];
-      a[4 + i] = a1.v[i];
-      b[i] = b0.v[i];
-      b[4 + i] = b1.v[i];
+    for (int g = 0; g < TM / VA; ++g) {
+      const scl_pack<scl_L, VA> q = scl_load<scl_L, VA>(&As[cur][kk][g * (BM / (TM / VA)) + ty * VA]);
+#pragma unroll
+      for (int i = 0; i < VA; ++i) a[g * VA + i] = q.v[i];
     }
 #pragma unroll
-    for (int i = 0; i < 8; ++i)
+    for (int g = 0; g < TN / VB; ++g) {
+      const scl_pack<scl_Rt, VB> q = scl_load<scl_Rt, VB>(&Bs[cur][kk][g * (BN / (TN / VB)) + tx * VB]);
 #pragma unroll
-      for (int j = 0; j < 8; ++j)
+      for (int i = 0; i < VB; ++i) b[g * VB + i] = q.v[i];
+    }
+#pragma unroll
+    for (int i = 0; i < TM; ++i)
+#pragma unroll
+      for (int j = 0; j < TN; ++j)
         acc[i][j] = USR_REDUCE(acc[i][j], USR_ZIP(a[i], b[j] SCL_ZIP_ARGS) SCL_REDUCE_ARGS);
   };
 
-  scl_O acc[8][8];
+  scl_O acc[TM][TN];
 #pragma unroll
-  for (int i = 0; i < 8; ++i)
+  for (int i = 0; i < TM; ++i)
 #pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = (scl_O)(SCL_IDENTITY);
+    for (int j = 0; j < TN; ++j) acc[i][j] = (scl_O)(SCL_IDENTITY);
 
-  const unsigned int ktiles = (K + SCL_AP_BK - 1) / SCL_AP_BK;
-  load_tile(0);
-  store_tile(0);
-  __syncthreads();
-  for (unsigned int kt = 0; kt < ktiles; ++kt) {
-    const int cur = kt & 1;
-    if (kt + 1 < ktiles) load_tile((kt + 1) * SCL_AP_BK);
-    const unsigned int kmax = min((unsigned int)SCL_AP_BK, K - kt * SCL_AP_BK);
-    if (kmax == SCL_AP_BK) {
+  const unsigned int ktiles = (K + BK - 1) / BK;
 #pragma unroll
-      for (int kk = 0; kk < SCL_AP_BK; ++kk) step(acc, cur, kk);
+  for (int t = 0; t < AHEAD; ++t) {
+    if (t < ktiles) {
+      fetch(t);
+      put(t);
+    }
+    commit();
+  }
+  for (unsigned int kt = 0; kt < ktiles; ++kt) {
+    if constexpr (ASYNC) asm volatile("cp.async.wait_group %0;" :: "n"(AHEAD - 1) : "memory");
+    __syncthreads();
+    if (kt + AHEAD < ktiles) fetch(kt + AHEAD);
+    commit();
+    const int cur = (int)(kt % STAGES);
+    const unsigned int kmax = min((unsigned int)BK, K - kt * BK);
+    if (kmax == BK) {
+#pragma unroll UNR
+      for (int kk = 0; kk < BK; ++kk) step(acc, cur, kk);
     } else {
+#pragma unroll TAIL
       for (unsigned int kk = 0; kk < kmax; ++kk) step(acc, cur, (int)kk);
     }
-    if (kt + 1 < ktiles) store_tile(cur ^ 1);
-    __syncthreads();
+    if (kt + AHEAD < ktiles) put(kt + AHEAD);
   }
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const unsigned int gm = m0 + (i < 4 ? ty * 4 + i : 64 + ty * 4 + (i - 4));
+  for (int i = 0; i < TM; ++i) {
+    const unsigned int gm = m0 + (i / VA) * (BM / (TM / VA)) + ty * VA + i % VA;
     if (gm >= M) continue;
 #pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const unsigned int gn = n0 + h * 64 + tx * 4;
+    for (int h = 0; h < TN / VB; ++h) {
+      const unsigned int gn = n0 + h * (BN / (TN / VB)) + tx * VB;
       scl_O* dst = P + (scl_u64)gm * N + gn;
-      if (sizeof(scl_O) == 4 && (N % 4u) == 0 && gn + 3 < N &&
-          (((scl_u64)dst) & 15u) == 0) {
-        scl_pack<scl_O, 4> o;
+      if (sizeof(scl_O) == 4 && (N % VB) == 0 && gn + VB - 1 < N && (((scl_u64)dst) & (VB * 4 - 1u)) == 0) {
+        scl_pack<scl_O, VB> o;
 #pragma unroll
-        for (int j = 0; j < 4; ++j) o.v[j] = acc[i][h * 4 + j];
-        scl_store<scl_O, 4>(dst, o);
+        for (int j = 0; j < VB; ++j) o.v[j] = acc[i][h * VB + j];
+        scl_store<scl_O, VB>(dst, o);
       } else {
 #pragma unroll
-        for (int j = 0; j < 4; ++j)
-          if (gn + j < N) dst[j] = acc[i][h * 4 + j];
+        for (int j = 0; j < VB; ++j)
+          if (gn + j < N) dst[j] = acc[i][h * VB + j];
       }
     }
   }
