@@ -657,7 +657,9 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 //   powers of two, so exact).  The cross products go first, 2^11 too large;
 //   the first hi*hi MMA scales them down (scale-input-d = 11).
 // bf16 parts (six products, where the split reported values FP16 parts do not
-//   hold): k-blocks of 32, four stages of 48 KB, a drain every 64 of K.
+//   hold): k-blocks of 32, four stages of 48 KB, a drain every 64 of K; the
+//   products of a k-block together, or (SMALLEST_FIRST) of a drain's two, which
+//   is the order and so the bits of gemm_3xbf16_kernel's k-blocks of 64.
 // 8192 x 4096 x 8192, split included: 1.11 ms against 1.85 ms for six products
 // in gemm_3xbf16_kernel; without the drains' work 1.04 ms, at K = 16384 4.31
 // and 3.88 ms (three products at 1.54 and 1.71 of the 1.74 PFLOP/s bf16 a
@@ -758,7 +760,7 @@ struct PairBarriers {
   uint64_t drain;         // all issued MMAs completed (each CTA)
 };
 
-template <int FMT, bool WALK>
+template <int FMT, bool WALK, bool SMALLEST_FIRST = false>
 __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const PairArgs& g,
                                           uint32_t base, uint32_t ring, uint32_t stage_out, PairBarriers* bars,
                                           uint32_t tmem, uint32_t rank, int* s_fail) {
@@ -874,26 +876,45 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
             const uint32_t dtm = tmem + acc_i * kPairCols;
             if (use > 0)
               landed = mbar_wait_cluster(smem_u32(&bars->acc_empty[acc_i]), (use - 1) & 1u, g.spin_limit);
+            if constexpr (SMALLEST_FIRST) {
+              // the whole drain group product by product, the smallest first,
+              // as gemm_3xbf16_kernel does with its k-blocks of 64
 #pragma unroll
-            for (int j = 0; j < SH::G; ++j) {
-              const uint32_t s = (it + j) % SH::STAGES, stage = base + s * SH::STAGE_BYTES;
-              landed = landed && mbar_wait_cluster(smem_u32(&bars->full[s]), ((it + j) / SH::STAGES) & 1u,
-                                                   g.spin_limit);
+              for (int j = 0; j < SH::G; ++j)
+                landed = landed && mbar_wait_cluster(smem_u32(&bars->full[(it + j) % SH::STAGES]),
+                                                     ((it + j) / SH::STAGES) & 1u, g.spin_limit);
               if (!landed) break;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              if (FMT == kF16) {  // lo*hi, hi*lo, hi*hi
-                mma(dtm, stage, 1, 0, true, false);
-                mma(dtm, stage, 0, 1, false, false);
-                mma(dtm, stage, 0, 0, false, true);
-              } else {  // lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi: smallest first
-                mma(dtm, stage, 2, 0, j == 0, false);
-                mma(dtm, stage, 0, 2, false, false);
-                mma(dtm, stage, 1, 1, false, false);
-                mma(dtm, stage, 1, 0, false, false);
-                mma(dtm, stage, 0, 1, false, false);
-                mma(dtm, stage, 0, 0, false, false);
+              constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
+#pragma unroll
+              for (int q = 0; q < 6; ++q)
+#pragma unroll
+                for (int j = 0; j < SH::G; ++j)
+                  mma(dtm, base + (it + j) % SH::STAGES * SH::STAGE_BYTES, pa[q], pb[q], q == 0 && j == 0, false);
+#pragma unroll
+              for (int j = 0; j < SH::G; ++j) commit_pair(smem_u32(&bars->empty[(it + j) % SH::STAGES]));
+            } else {
+#pragma unroll
+              for (int j = 0; j < SH::G; ++j) {
+                const uint32_t s = (it + j) % SH::STAGES, stage = base + s * SH::STAGE_BYTES;
+                landed = landed && mbar_wait_cluster(smem_u32(&bars->full[s]), ((it + j) / SH::STAGES) & 1u,
+                                                     g.spin_limit);
+                if (!landed) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                if (FMT == kF16) {  // lo*hi, hi*lo, hi*hi
+                  mma(dtm, stage, 1, 0, true, false);
+                  mma(dtm, stage, 0, 1, false, false);
+                  mma(dtm, stage, 0, 0, false, true);
+                } else {  // lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi: smallest first
+                  mma(dtm, stage, 2, 0, j == 0, false);
+                  mma(dtm, stage, 0, 2, false, false);
+                  mma(dtm, stage, 1, 1, false, false);
+                  mma(dtm, stage, 1, 0, false, false);
+                  mma(dtm, stage, 0, 1, false, false);
+                  mma(dtm, stage, 0, 0, false, false);
+                }
+                commit_pair(smem_u32(&bars->empty[s]));
               }
-              commit_pair(smem_u32(&bars->empty[s]));
             }
             if (landed) commit_pair(smem_u32(&bars->acc_full[acc_i]));
           }
@@ -1019,7 +1040,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
   static_assert(EPI_WARPS * 32 + 64 == kPairThreads, "");
 }
 
-template <bool WALK>
+// WALK: see pair_body.  BF16: bf16 parts alone, without a verdict of the split.
+template <bool WALK, bool BF16 = false>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
                  const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB3,
@@ -1056,13 +1078,15 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   dependency_wait();
-  const bool f16 = *g.verdict != g.epoch;
+  const bool f16 = !BF16 && *g.verdict != g.epoch;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   cluster_sync();  // both CTAs' barriers are initialised, both hold tensor memory
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  if (f16)
+  if (BF16)
+    pair_body<kBf16, WALK, true>(tmA3, tmB3, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
+  else if (f16)
     pair_body<kF16, WALK>(tmA, tmB, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
   else
     pair_body<kBf16, WALK>(tmA3, tmB3, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
@@ -1318,6 +1342,43 @@ int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, u
   e = launch_overlapped(walk ? tc::gemm_pair_kernel<true> : tc::gemm_pair_kernel<false>,
                         dim3((unsigned)(2 * (walk ? resident_pairs() : all))), dim3(tc::kPairThreads), tc::kPairSmem,
                         stream, tmA, tmB, tmA3, tmB3, args);
+  if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
+  return SCL_OK;
+}
+
+// CTA pairs, bf16 parts: where 128 x 128 tiles take two waves of the SMs and 256
+// x 256 tiles one of the pairs.  A k-block of 64 takes 1.2 us in the former
+// (its 96 KB per SM come at 12 TB/s, from L2) and 1.9 us in the latter, for
+// twice the outputs per SM, with the same products in the same order and so the
+// same bits.  us, 128 x 128 tiles and so, the split included: 2000 x K x 2000
+// K = 64 15.3 / 11.9, 500 32.1 / 24.8, 2000 90.1 / 71.8, 4000 166 / 132; 300 x
+// 1000 x 8000 55.8 / 47.3.
+bool allpairs_pair3_wins(uint32_t M, uint32_t N) {
+  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u, pairs = resident_pairs();
+  const uint64_t small = (uint64_t)((M + 127) / 128) * ((N + 127) / 128);
+  const uint64_t large = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
+  return small > sms && large <= pairs;
+}
+int allpairs_pair3_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
+                          uint32_t group_rows, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                          uint32_t spin_limit, unsigned int* err) {
+  if (scratch_bytes < allpairs_tc_scratch_bytes(M, N, K, 3))
+    return fail(SCL_ERR_ARG, "tensor-core AllPairs: scratch too small");
+  const Split sp = split_of(A, B, M, N, K, tc::KPAD, 3, trans, scratch);
+  const uint32_t Kp = sp.Kp;
+  Tiles tiles;
+  if (int st = tiles_of(M, N, 2 * tc::BM, tc::kPairCols, group_rows, &tiles)) return st;
+  alignas(64) CUtensorMap tmA, tmB;
+  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, 3, tc::BM, 32, tc::kBf16)) return st;
+  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, 3, 128, 32, tc::kBf16)) return st;
+  unsigned int* none = nullptr;
+  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp,
+                                    3, none, 0u, none);
+  if (e != cudaSuccess) return cuda_fail(e, "split launch");
+  const tc::PairArgs args = {P,     nullptr, nullptr, none,       err,     M,       N,      Kp,
+                             sp.Mp, sp.Np,   0u,      spin_limit, tiles.n, tiles.m, tiles.group};
+  e = launch_overlapped(tc::gemm_pair_kernel<false, true>, dim3(2 * tiles.m * tiles.n), dim3(tc::kPairThreads),
+                        tc::kPairSmem, stream, tmA, tmB, tmA, tmB, args);
   if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
   return SCL_OK;
 }

@@ -19,6 +19,10 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
 int transpose_launch(const void* src, void* dst, uint64_t rows, uint64_t cols, size_t elem,
                      cudaStream_t stream);
 size_t allpairs_tc_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int parts);
+bool allpairs_pair3_wins(uint32_t M, uint32_t N);
+int allpairs_pair3_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
+                          uint32_t group_rows, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                          uint32_t spin_limit, unsigned int* err);
 int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
                          uint32_t group_rows, void* head, void* scratch, size_t scratch_bytes, unsigned int epoch,
                          cudaStream_t stream, uint32_t spin_limit, unsigned int* err);
@@ -977,6 +981,11 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
                                     p->ws.ptr, scratch, p->ws.bytes - tc_head, epoch, rt().stream, spin_of(tu),
                                     rt().dev_err);
       }
+      // 128-column tiles in two waves, CTA pairs in one: the same products, the
+      // same bits (allpairs_pair3_launch)
+      if (!wide && parts == 3 && cols == 0 && !(tu && (tu->items || tu->tile_w)) && allpairs_pair3_wins(M, N))
+        return allpairs_pair3_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans, group_rows, scratch,
+                                     p->ws.bytes - tc_head, rt().stream, spin_of(tu), rt().dev_err);
       return allpairs_tc_launch((const float*)A, (const float*)B, (float*)P, M, N, K, parts, trans,
                                 drain, wide, group_rows, scratch, p->ws.bytes - tc_head, rt().stream,
                                 spin_of(tu), rt().dev_err);

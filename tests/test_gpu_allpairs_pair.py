@@ -57,6 +57,20 @@ def test_pair_walk_against_fp64(scl, orc, shape):
     assert np.array_equal(run(p, A, B), run(p, A, B, items=3), equal_nan=True)
 
 
+# 128-column tiles in two waves, CTA pairs in one
+@pytest.mark.parametrize("flags", [0, S.SHAPE_TRANS_LEFT, S.SHAPE_TRANS_RIGHT])
+@pytest.mark.parametrize("shape", [(2000, 16, 2000), (2050, 64, 2047), (1665, 130, 1700), (2431, 65, 1537),
+                                   (257, 500, 9000), (2000, 1001, 1930)])
+def test_bf16_pairs_same_bits_as_small_tiles(scl, orc, shape, flags):
+    M, K, N = shape
+    A = orc.normal_f32(M * K, 91).reshape(M, K)
+    A[M - 1, 0] = np.inf
+    A[M // 2, K // 2] = 2.0 ** -100
+    B = orc.normal_f32(K * N, 92).reshape(K, N)
+    p = program()
+    assert np.array_equal(run(p, A, B, flags=flags, cols=0), run(p, A, B, flags=flags, cols=128), equal_nan=True)
+
+
 @pytest.mark.parametrize("exp", [-10, -26, -27, -30, -45, -70])
 def test_pair_small_elements(scl, exp):
     """A small element of A that meets the only non-zero element of B's column
