@@ -675,6 +675,14 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
   // the register kernel
   bool staged = !(tu && tu->variant == SCL_VARIANT_VECTOR) || p->kind == SCL_KIND_SCAN_MAP;
   if (staged && R == 2) R = 4;
+  // tiles of half the size while the whole ones are at most one to two SMs: a
+  // tile's own steps are what such a call waits for (us, floats 1000 4.2 ->
+  // 3.3, 100,000 5.6 -> 4.5, 620,000 6.5 -> 6.0, 800,000 6.5 and 6.5; doubles
+  // 1000 6.0 -> 4.3, 300,000 8.4 -> 7.2, 400,000 8.7 and 8.9; unsigned char
+  // 1000 8.6 -> 4.9)
+  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  if (staged && !(tu && (tu->items || tu->tile_w)) && sh->n_segments == 0 &&
+      (n + 2048ull * V - 1) / (2048ull * V) <= sms / 2) R = 4;
   if (!staged && R == 6) R = 8;
   size_t smem = staged ? (size_t)R * 256 * V * tsz : 0;
   if (staged && smem + 2048 > rt().smem_optin) {

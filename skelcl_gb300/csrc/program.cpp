@@ -347,10 +347,10 @@ int assemble(const scl_program_desc* d, scl_program* p, bool want_f64, Assembly*
       break;
     case SCL_KIND_SCAN:
       s << scl_tpl_reduce << "\n" << scl_tpl_scan;
-      out->kernels = {"scl_scan_s<8, 6>", "scl_scan_k<8, 4>"};
+      out->kernels = {"scl_scan_s<8, 6>", "scl_scan_s<4, 8>", "scl_scan_k<8, 4>"};
       out->lazy = {"scl_scan_k<8, 3>", "scl_scan_k<8, 2>", "scl_scan_k<4, 4>", "scl_scan_k<4, 6>",
                    "scl_scan_k<2, 8>", "scl_scan_k<16, 2>", "scl_scan_k<16, 1>",
-                   "scl_scan_s<8, 5>", "scl_scan_s<8, 4>", "scl_scan_s<4, 8>", "scl_scan_s<6, 8>",
+                   "scl_scan_s<8, 5>", "scl_scan_s<8, 4>", "scl_scan_s<6, 8>",
                    "scl_scan_s<16, 3>", "scl_scan_s<8, 6, 1>", "scl_scan_s<16, 3, 1>",
                    "scl_scan_s<8, 6, 2>", "scl_scan_s<16, 3, 2>", "scl_scan_short<8>"};
       break;
@@ -360,8 +360,8 @@ int assemble(const scl_program_desc* d, scl_program* p, bool want_f64, Assembly*
       break;
     case SCL_KIND_SCAN_MAP:
       s << scl_tpl_reduce << "\n" << scl_tpl_scan;
-      out->kernels = {"scl_scan_s<8, 6>"};
-      out->lazy = {"scl_scan_s<8, 5>", "scl_scan_s<8, 4>", "scl_scan_s<4, 8>", "scl_scan_s<6, 8>",
+      out->kernels = {"scl_scan_s<8, 6>", "scl_scan_s<4, 8>"};
+      out->lazy = {"scl_scan_s<8, 5>", "scl_scan_s<8, 4>", "scl_scan_s<6, 8>",
                    "scl_scan_s<16, 3>", "scl_scan_s<8, 6, 1>", "scl_scan_s<16, 3, 1>",
                    "scl_scan_s<8, 6, 2>", "scl_scan_s<16, 3, 2>", "scl_scan_short<8>"};
       break;
