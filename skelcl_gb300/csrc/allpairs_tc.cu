@@ -344,6 +344,44 @@ split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int part
   }
 }
 
+// A 128 x 128 tile's sums lie in the shared memory of the cluster's `ranks`
+// blocks (16-byte chunk c of row r at chunk c ^ (r % 32) of the row's 512
+// bytes): this block adds up its share of the rows, in block order, and stores
+// them, a warp per row.  us, against a thread storing its own row's 128 sums:
+// 1400 x 300 x 1400 14.7 -> 13.5, x 1401 23.7 -> 14.4, 1500 x 2000 x 1499 57.7 ->
+// 48.8.
+template <int THREADS>
+__device__ __forceinline__ void store_sums(uint32_t base, uint32_t ranks, uint32_t rank, uint32_t m0, uint32_t n0,
+                                           uint32_t M, uint32_t N, float* P) {
+  const uint32_t rows = BM / ranks, first = rank * rows;
+  for (uint32_t i = threadIdx.x; i < rows * 32u; i += THREADS) {
+    const uint32_t r = first + i / 32u, c = i % 32u;
+    const uint32_t at = base + r * 512u + ((c ^ (r & 31u)) * 16u);
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    for (uint32_t p = 0; p < ranks; ++p) {
+      float4 o;
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
+                   : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(cluster_addr(at, p)) : "memory");
+      v.x += o.x;
+      v.y += o.y;
+      v.z += o.z;
+      v.w += o.w;
+    }
+    const uint32_t row = m0 + r, col = n0 + c * 4u;
+    if (row < M) {
+      float* dst = P + (uint64_t)row * N + col;
+      if ((N % 4u) == 0u && col + 4u <= N) {
+        *reinterpret_cast<float4*>(dst) = v;
+      } else {
+        if (col < N) dst[0] = v.x;
+        if (col + 1u < N) dst[1] = v.y;
+        if (col + 2u < N) dst[2] = v.z;
+        if (col + 3u < N) dst[3] = v.w;
+      }
+    }
+  }
+}
+
 // G = k-blocks accumulated in tensor memory between two drains into the
 // epilogue's FP32 registers (1: every k-block; larger G drains less often at
 // a longer in-TMEM accumulation chain).
@@ -558,7 +596,7 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
         asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];"
                      :: "r"(smem_u32(&acc_empty[acc_i])) : "memory");
     }
-    if (SPLIT) {
+    if (BN == 128) {
       // (every MMA that reads the stages has completed)  16-byte chunk c of
       // row r at chunk c ^ (r % 32): a warp's accesses meet all banks
       const uint32_t r = (uint32_t)(q * 32 + lane);
@@ -592,39 +630,15 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     }
   }
 
-  if constexpr (SPLIT) {
-    static_assert(!SPLIT || BN == 128, "one epilogue warp per 32 rows: its sums are whole rows");
+  static_assert(!SPLIT || BN == 128, "one epilogue warp per 32 rows: its sums are whole rows");
+  if constexpr (BN == 128) {
     __syncthreads();
-    cluster_sync();
-    const uint32_t rows = BM / ranks, first = rank * rows;
-    for (uint32_t i = threadIdx.x; i < rows * 32u; i += SH::THREADS) {
-      const uint32_t r = first + i / 32u, c = i % 32u;
-      const uint32_t at = base + r * 512u + ((c ^ (r & 31u)) * 16u);
-      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-      for (uint32_t p = 0; p < ranks; ++p) {
-        float4 o;
-        asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];"
-                     : "=f"(o.x), "=f"(o.y), "=f"(o.z), "=f"(o.w) : "r"(cluster_addr(at, p)) : "memory");
-        v.x += o.x;
-        v.y += o.y;
-        v.z += o.z;
-        v.w += o.w;
-      }
-      const uint32_t row = m0 + r, col = n0 + c * 4u;
-      if (row < M) {
-        float* dst = P + (uint64_t)row * N + col;
-        if ((N % 4u) == 0u && col + 4u <= N) {
-          *reinterpret_cast<float4*>(dst) = v;
-        } else {
-          if (col < N) dst[0] = v.x;
-          if (col + 1u < N) dst[1] = v.y;
-          if (col + 2u < N) dst[2] = v.z;
-          if (col + 3u < N) dst[3] = v.w;
-        }
-      }
+    if constexpr (SPLIT) cluster_sync();
+    store_sums<SH::THREADS>(base, ranks, rank, m0, n0, M, N, P);
+    if constexpr (SPLIT) {
+      __syncthreads();
+      cluster_sync();  // no block leaves while another may still read its sums
     }
-    __syncthreads();
-    cluster_sync();  // no block leaves while another may still read its sums
   }
 
   // ---- teardown: wait for the copies a failed pipeline may still have in
