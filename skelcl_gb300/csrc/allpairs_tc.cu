@@ -1127,6 +1127,225 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   }
 }
 
+// ---- One wave of 128 x 128 tiles, the split fused -----------------------------------
+// Blocks that read the operands themselves: 512 threads load a k-block of 64 as
+// FP32 into registers, split it into three bf16 parts and store those where
+// gemm_3xbf16_kernel's TMA would have put them, while the tensor cores work on
+// the k-block before and the sums of the one before that are drained.  No split
+// pass, no planes written and read back, 64 instead of 96 KB per k-block from
+// L2; but every tile splits its own rows and columns, at 1.7 us per k-block (2.1
+// with an operand whose k are not contiguous, 2.5 with both) against 1.2 of
+// the kernel that reads parts: bound by the conversions, and by shared memory,
+// which the tensor cores' operand reads alone keep at 90 %.  It wins while the
+// k-blocks are few.  us, split pass and kernel / fused: 500 x K x 600 K = 40
+// 9.4 / 6.1, 128 10.9 / 7.9, 190 11.7 / 10.7, 256 12.7 / 11.9, 300 14.0 / 14.1;
+// 1000 x K x 1100 K = 128 10.2 / 8.0, 256 12.2 / 12.0, 300 13.4 / 14.4; left
+// operand transposed K = 190 11.3 / 11.3, 256 12.4 / 13.7.  (256 threads: 2.4
+// us per k-block.)  The same parts in the same order: the same bits.
+struct Fused {
+  Operand a, b;
+  float* P;
+  unsigned int* err;
+  uint32_t M, N, K, spin_limit, tiles_n, group_m;
+};
+constexpr int kFusedThreads = 512;
+constexpr int kFusedChunks = 1024 / kFusedThreads;     // of either operand per thread
+constexpr int kFusedCols = 128 * 128 / kFusedThreads;  // of sums per thread
+
+// The operand's k-block of 64 at k0, rows r0 .. + 127, 8 consecutive k (a
+// 16-byte chunk of a part) at a time: chunk c of row
+// c / 8 where k is contiguous, else of row c % 128, so that lanes read
+// neighbouring memory.
+struct FusedPlace {
+  uint32_t row, kc;
+};
+__device__ __forceinline__ FusedPlace fused_place(int kmajor, int i) {
+  const uint32_t c = threadIdx.x + (uint32_t)i * kFusedThreads;
+  return kmajor ? FusedPlace{c / 8u, c % 8u} : FusedPlace{c % 128u, c / 128u};
+}
+__device__ __forceinline__ void fused_load(const Operand& op, uint32_t K, uint32_t r0, uint32_t k0, bool vec,
+                                           float (&x)[kFusedChunks][8]) {
+#pragma unroll
+  for (int i = 0; i < kFusedChunks; ++i) {
+    const FusedPlace at = fused_place(op.kmajor, i);
+    const uint32_t row = r0 + at.row, k = k0 + at.kc * 8u;
+    const bool in = row < op.rows;
+    if (op.kmajor) {
+      const float* src = op.x + (in ? (uint64_t)row * K + k : 0u);
+      if (vec && in && k + 8u <= K) {
+        const float4 u = *reinterpret_cast<const float4*>(src), v = *reinterpret_cast<const float4*>(src + 4);
+        x[i][0] = u.x; x[i][1] = u.y; x[i][2] = u.z; x[i][3] = u.w;
+        x[i][4] = v.x; x[i][5] = v.y; x[i][6] = v.z; x[i][7] = v.w;
+      } else {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) x[i][e] = in && k + e < K ? src[e] : 0.0f;
+      }
+    } else {
+      const float* src = op.x + (in ? (uint64_t)k * op.rows + row : 0u);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) x[i][e] = in && k + e < K ? src[(uint64_t)e * op.rows] : 0.0f;
+    }
+  }
+}
+__device__ __forceinline__ void fused_store(int kmajor, const float (&x)[kFusedChunks][8], uint32_t tile) {
+#pragma unroll
+  for (int i = 0; i < kFusedChunks; ++i) {
+    const FusedPlace at = fused_place(kmajor, i);
+    uint32_t part[3][4];
+#pragma unroll
+    for (int e = 0; e < 8; e += 2) {
+      float u = x[i][e], v = x[i][e + 1];
+#pragma unroll
+      for (int p = 0; p < 3; ++p) {
+        const __nv_bfloat162 h = __floats2bfloat162_rn(u, v);
+        part[p][e / 2] = *reinterpret_cast<const uint32_t*>(&h);
+        u -= __low2float(h);
+        v -= __high2float(h);
+      }
+    }
+    // (SWIZZLE_128B: 16-byte chunk kc of row r at chunk kc ^ (r % 8))
+    const uint32_t dst = tile + at.row * 128u + ((at.kc ^ (at.row & 7u)) * 16u);
+#pragma unroll
+    for (int p = 0; p < 3; ++p)
+      asm volatile("st.shared.v4.b32 [%0], {%1, %2, %3, %4};"
+                   :: "r"(dst + (uint32_t)p * Shape<128>::A_TILE), "r"(part[p][0]), "r"(part[p][1]), "r"(part[p][2]),
+                      "r"(part[p][3])
+                   : "memory");
+  }
+}
+
+// SPLIT: the blocks of a cluster share an output tile's k-blocks.
+template <bool SPLIT>
+__global__ void __launch_bounds__(kFusedThreads, 1) gemm_fused_kernel(const Fused g) {
+  using SH = Shape<128>;
+  constexpr int STAGE_BYTES = 3 * (SH::A_TILE + SH::B_TILE);
+  extern __shared__ __align__(1024) uint8_t smem_raw[];
+  __shared__ __align__(8) uint64_t done[2];  // the MMAs of k-blocks 0, 2, ... / 1, 3, ... completed
+  __shared__ uint32_t tmem_slot;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  uint32_t ranks = 1, rank = 0;
+  if constexpr (SPLIT) {
+    asm volatile("mov.u32 %0, %%cluster_nctarank;" : "=r"(ranks));
+    asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
+  }
+  uint32_t m0, n0;
+  {
+    // tiles in groups of group_m tile rows (see gemm_3xbf16_kernel)
+    const uint32_t tile = blockIdx.x / ranks, tiles_m = gridDim.x / ranks / g.tiles_n, per_group = g.group_m * g.tiles_n;
+    const uint32_t grp = tile / per_group, r = tile % per_group, first = grp * g.group_m;
+    const uint32_t rows = tiles_m - first < g.group_m ? tiles_m - first : g.group_m;
+    m0 = (first + r % rows) * BM;
+    n0 = (r / rows) * 128u;
+  }
+  const uint32_t all_k = (g.K + 63u) / 64u, k0 = all_k * rank / ranks, nk = all_k * (rank + 1) / ranks - k0;
+  if (threadIdx.x == 0) {
+    for (int a = 0; a < 2; ++a)
+      asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(smem_u32(&done[a])));
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;"
+                 :: "r"(smem_u32(&tmem_slot)), "r"(SH::TMEM_COLS) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  dependency_wait();
+  const bool vec = (g.K % 4u) == 0u;
+  const bool vec_a = vec && (reinterpret_cast<uintptr_t>(g.a.x) & 15u) == 0,
+             vec_b = vec && (reinterpret_cast<uintptr_t>(g.b.x) & 15u) == 0;
+  float xa[kFusedChunks][8], xb[kFusedChunks][8];
+  fused_load(g.a, g.K, m0, k0 * 64u, vec_a, xa);
+  fused_load(g.b, g.K, n0, k0 * 64u, vec_b, xb);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = tmem_slot;
+
+  // warp w owns tensor-memory lanes 32 * (w % 4) .. (rows) and columns kFusedCols * (w / 4) ..
+  const int q = warp & 3, h = warp >> 2;
+  float sum[kFusedCols];
+#pragma unroll
+  for (int j = 0; j < kFusedCols; ++j) sum[j] = 0.0f;
+  bool ok = true;
+  auto drain = [&](uint32_t kb) {  // adds k-block kb's products to the sums
+    const uint32_t a = kb & 1u;
+    if (ok && !mbar_wait(smem_u32(&done[a]), (kb >> 1) & 1u, g.spin_limit)) {
+      ok = false;
+      if (lane == 0) raise(g.err);
+    }
+    __syncwarp();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+    for (int c = 0; c < kFusedCols / 32; ++c) {
+      uint32_t r[32];
+      tmem_load32(tmem + ((uint32_t)(q * 32) << 16) + a * 128u + (uint32_t)(h * kFusedCols + c * 32), r);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+      for (int j = 0; j < 32; ++j) sum[c * 32 + j] += __uint_as_float(r[j]);
+    }
+  };
+  for (uint32_t kb = 0; kb < nk; ++kb) {
+    // Stage and accumulator kb % 2 were last used for k-block kb - 2, whose
+    // MMAs this thread has seen complete (drain).
+    const uint32_t stage = base + (kb & 1u) * STAGE_BYTES;
+    fused_store(g.a.kmajor, xa, stage);
+    fused_store(g.b.kmajor, xb, stage + 3 * SH::A_TILE);
+    if (kb + 1 < nk) {
+      fused_load(g.a, g.K, m0, (k0 + kb + 1) * 64u, vec_a, xa);
+      fused_load(g.b, g.K, n0, (k0 + kb + 1) * 64u, vec_b, xb);
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (threadIdx.x == 0) {
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};  // smallest first
+#pragma unroll
+      for (int p = 0; p < 6; ++p) {
+        const uint64_t ad = smem_desc<SH>(stage + (uint32_t)pa[p] * SH::A_TILE);
+        const uint64_t bd = smem_desc<SH>(stage + (uint32_t)(3 * SH::A_TILE + pb[p] * SH::B_TILE));
+#pragma unroll
+        for (int ks = 0; ks < 4; ++ks) {
+          const uint32_t acc = p > 0 || ks > 0 ? 1u : 0u;
+          asm volatile(
+              "{ .reg .pred p; setp.ne.b32 p, %4, 0;"
+              " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p; }"
+              :: "r"(tmem + (kb & 1u) * 128u), "l"(ad + (uint64_t)(ks * 2)), "l"(bd + (uint64_t)(ks * 2)),
+                 "r"(SH::IDESC), "r"(acc)
+              : "memory");
+        }
+      }
+      asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];"
+                   :: "r"(smem_u32(&done[kb & 1u])) : "memory");
+    }
+    __syncwarp();
+    if (kb > 0) drain(kb - 1);
+  }
+  if (nk > 0) drain(nk - 1);
+
+  // the sums through shared memory: no MMA reads the stages any more (after a
+  // wait that gave up, another one is made: the status says the outputs are void)
+  if (!ok) mbar_wait(smem_u32(&done[(nk - 1) & 1u]), ((nk - 1) >> 1) & 1u, g.spin_limit);
+  __syncwarp();
+  const uint32_t r = (uint32_t)(q * 32 + lane);
+#pragma unroll
+  for (int c = 0; c < kFusedCols / 4; ++c)
+    asm volatile("st.shared.v4.f32 [%0], {%1, %2, %3, %4};"
+                 :: "r"(base + r * 512u + (((uint32_t)(h * (kFusedCols / 4) + c) ^ (r & 31u)) * 16u)), "f"(sum[c * 4]),
+                    "f"(sum[c * 4 + 1]), "f"(sum[c * 4 + 2]), "f"(sum[c * 4 + 3])
+                 : "memory");
+  __syncthreads();
+  if constexpr (SPLIT) cluster_sync();
+  store_sums<kFusedThreads>(base, ranks, rank, m0, n0, g.M, g.N, g.P);
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if constexpr (SPLIT) cluster_sync();  // no block leaves while another may still read its sums
+  if (warp == 0) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" :: "r"(tmem), "r"(SH::TMEM_COLS) : "memory");
+  }
+}
+
 inline uint32_t round_up(uint32_t v, uint32_t m) { return (v + m - 1) / m * m; }
 
 }  // namespace tc
@@ -1311,6 +1530,32 @@ uint64_t resident_pairs() {
   return (uint64_t)n;
 }
 }  // namespace
+
+// One wave of 128 x 128 tiles (or of clusters that share one), few k-blocks a
+// block: the operands split where they are used (gemm_fused_kernel).
+bool allpairs_fused_wins(uint32_t M, uint32_t N, uint32_t K, int trans) {
+  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  const uint64_t tiles = (uint64_t)((M + 127) / 128) * ((N + 127) / 128);
+  const uint32_t all_k = (K + 63) / 64, split = split_of_k(tiles, tc::round_up(K, tc::KPAD));
+  const bool strided = trans == 1;  // both operands
+  return tiles <= sms && (all_k + split - 1) / split <= (strided ? 3u : 4u);
+}
+int allpairs_fused_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
+                          uint32_t group_rows, cudaStream_t stream, uint32_t spin_limit, unsigned int* err) {
+  Tiles tiles;
+  if (int st = tiles_of(M, N, tc::BM, 128, group_rows, &tiles)) return st;
+  const tc::Fused args = {{A, nullptr, nullptr, M, M, (trans & 1) ? 0 : 1},
+                          {B, nullptr, nullptr, N, N, (trans & 2) ? 1 : 0},
+                          P, err, M, N, K, spin_limit, tiles.n, tiles.group};
+  const uint32_t split = split_of_k((uint64_t)tiles.m * tiles.n, tc::round_up(K, tc::KPAD));
+  const dim3 grid(tiles.m * tiles.n * split);
+  const size_t smem = (size_t)2 * 3 * (tc::Shape<128>::A_TILE + tc::Shape<128>::B_TILE) + 1024;
+  const cudaError_t e =
+      split == 1 ? launch_overlapped(tc::gemm_fused_kernel<false>, grid, dim3(tc::kFusedThreads), smem, stream, args)
+                 : launch_clustered(tc::gemm_fused_kernel<true>, split, grid, dim3(tc::kFusedThreads), smem, stream, args);
+  if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
+  return SCL_OK;
+}
 
 // CTA pairs: FP16 parts, with the bf16 parts as the device's fallback.
 // `head` (allpairs_tc_head_bytes) precedes the scratch; `epoch` differs from

@@ -19,6 +19,9 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
 int transpose_launch(const void* src, void* dst, uint64_t rows, uint64_t cols, size_t elem,
                      cudaStream_t stream);
 size_t allpairs_tc_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int parts);
+bool allpairs_fused_wins(uint32_t M, uint32_t N, uint32_t K, int trans);
+int allpairs_fused_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
+                          uint32_t group_rows, cudaStream_t stream, uint32_t spin_limit, unsigned int* err);
 bool allpairs_pair3_wins(uint32_t M, uint32_t N);
 int allpairs_pair3_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
                           uint32_t group_rows, void* scratch, size_t scratch_bytes, cudaStream_t stream,
@@ -963,6 +966,13 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
       // 1.1e-7, is below what FP16 parts gave there, 1.6e-7)
       const bool pair = wide && !(tu && (tu->items || tu->tile_w > 1)) && allpairs_pair_supported(K);
       const int parts = (tu && tu->items == 2) ? 2 : 3;
+      // (the fused form takes no workspace)
+      const bool plain = cols == 0 && parts == 3 && !(tu && (tu->items || tu->tile_w));
+      if (!wide && plain && allpairs_fused_wins(M, N, K, trans)) {
+        p->last_variant = SCL_VARIANT_TC3XBF16;
+        return allpairs_fused_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans,
+                                     tu ? tu->workgroup : 0u, rt().stream, spin_of(tu), rt().dev_err);
+      }
       const size_t need = pair ? allpairs_pair_scratch_bytes(M, N, K) : allpairs_tc_scratch_bytes(M, N, K, parts);
       if (int st = ensure_workspace(p, tc_head + need)) return st;
       char* scratch = static_cast<char*>(p->ws.ptr) + tc_head;
@@ -991,7 +1001,7 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
       }
       // 128-column tiles in two waves, CTA pairs in one: the same products, the
       // same bits (allpairs_pair3_launch)
-      if (!wide && parts == 3 && cols == 0 && !(tu && (tu->items || tu->tile_w)) && allpairs_pair3_wins(M, N))
+      if (!wide && plain && allpairs_pair3_wins(M, N))
         return allpairs_pair3_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans, group_rows, scratch,
                                      p->ws.bytes - tc_head, rt().stream, spin_of(tu), rt().dev_err);
       return allpairs_tc_launch((const float*)A, (const float*)B, (float*)P, M, N, K, parts, trans,

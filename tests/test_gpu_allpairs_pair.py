@@ -71,6 +71,35 @@ def test_bf16_pairs_same_bits_as_small_tiles(scl, orc, shape, flags):
     assert np.array_equal(run(p, A, B, flags=flags, cols=0), run(p, A, B, flags=flags, cols=128), equal_nan=True)
 
 
+# one wave, few k-blocks: the operands split in the contraction itself
+@pytest.mark.parametrize("flags", [0, S.SHAPE_TRANS_LEFT, S.SHAPE_TRANS_RIGHT,
+                                   S.SHAPE_TRANS_LEFT | S.SHAPE_TRANS_RIGHT])
+@pytest.mark.parametrize("shape", [(128, 16, 128), (129, 63, 131), (300, 64, 301), (130, 65, 1029), (1400, 128, 1401),
+                                   (500, 190, 600), (1, 17, 16400), (257, 256, 384), (1000, 500, 1100),
+                                   (512, 1000, 640)])
+def test_fused_split_same_bits(scl, orc, shape, flags):
+    M, K, N = shape
+    A = orc.normal_f32(M * K, 95).reshape(M, K)
+    A[M - 1, 0] = np.inf
+    A[M // 2, K // 2] = 2.0 ** -100
+    B = orc.normal_f32(K * N, 96).reshape(K, N)
+    B[K - 1, N - 1] = np.nan
+    p = program()
+    assert np.array_equal(run(p, A, B, flags=flags, cols=0), run(p, A, B, flags=flags, cols=128), equal_nan=True)
+
+
+def test_fused_split_unaligned_operands(scl, orc):
+    M, K, N = 200, 64, 260
+    a, b = orc.normal_f32(M * K + 1, 97), orc.normal_f32(K * N + 1, 98)
+    p, out = program(), []
+    for cols in (0, 128):
+        dA, dB, dP = S.DeviceArray.from_numpy(a), S.DeviceArray.from_numpy(b), S.DeviceArray(M * N, np.float32)
+        p.launch([dA.view(1, M * K), dB.view(1, K * N), dP], rows=M, cols=N, dim=K, flags=S.SHAPE_TRANS_RIGHT,
+                 tuning=S.Tuning(variant=S.VARIANT_TC3XBF16, tile_h=cols))
+        out.append(dP.to_numpy())
+    assert np.array_equal(out[0], out[1])
+
+
 @pytest.mark.parametrize("exp", [-10, -26, -27, -30, -45, -70])
 def test_pair_small_elements(scl, exp):
     """A small element of A that meets the only non-zero element of B's column
