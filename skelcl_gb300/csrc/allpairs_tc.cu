@@ -1025,25 +1025,31 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
                             "l"(sum[c * 8 + 2 * j]), "l"(sum[c * 8 + 2 * j + 1])
                          : "memory");
           __syncwarp();
+          const uint32_t col0 = n0 + tile_col + (uint32_t)(c * 16);
+          if (vec) {
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            const uint32_t r = (uint32_t)(i * 8 + (lane >> 2)), ch = (uint32_t)(lane & 3);
-            float4 v;
-            asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
-                         : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
-                         : "r"(st + r * 64u + ((ch ^ (r >> 1 & 3u)) * 16u))
-                         : "memory");
-            const uint32_t row = m0 + (uint32_t)(q * 32) + r, col = n0 + tile_col + (uint32_t)(c * 16) + ch * 4u;
-            if (row < g.M) {
-              float* dst = g.P + (uint64_t)row * g.N + col;
-              if (vec && col + 4u <= g.N) {
-                *reinterpret_cast<float4*>(dst) = v;
-              } else {
-                if (col < g.N) dst[0] = v.x;
-                if (col + 1u < g.N) dst[1] = v.y;
-                if (col + 2u < g.N) dst[2] = v.z;
-                if (col + 3u < g.N) dst[3] = v.w;
-              }
+            for (int i = 0; i < 4; ++i) {
+              const uint32_t r = (uint32_t)(i * 8 + (lane >> 2)), ch = (uint32_t)(lane & 3);
+              float4 v;
+              asm volatile("ld.shared.v4.f32 {%0, %1, %2, %3}, [%4];"
+                           : "=f"(v.x), "=f"(v.y), "=f"(v.z), "=f"(v.w)
+                           : "r"(st + r * 64u + ((ch ^ (r >> 1 & 3u)) * 16u))
+                           : "memory");
+              const uint32_t row = m0 + (uint32_t)(q * 32) + r, col = col0 + ch * 4u;
+              if (row < g.M && col < g.N) *reinterpret_cast<float4*>(g.P + (uint64_t)row * g.N + col) = v;
+            }
+          } else {
+            // sixteen lanes to a row: 8000 x 256 x 8001 212 -> 166 us, 2001 x 1000
+            // x 2003 48 -> 41 against four 4-byte stores of four lanes to a row
+            const uint32_t cc = (uint32_t)(lane & 15), col = col0 + cc;
+#pragma unroll 4
+            for (int i = 0; i < 16; ++i) {
+              const uint32_t r = (uint32_t)(i * 2 + (lane >> 4)), row = m0 + (uint32_t)(q * 32) + r;
+              float v;
+              asm volatile("ld.shared.f32 %0, [%1];"
+                           : "=f"(v) : "r"(st + r * 64u + (((cc >> 2) ^ (r >> 1 & 3u)) * 16u) + (cc & 3u) * 4u)
+                           : "memory");
+              if (row < g.M && col < g.N) g.P[(uint64_t)row * g.N + col] = v;
             }
           }
           __syncwarp();
@@ -1592,7 +1598,7 @@ int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, u
                              sp.Mp, sp.Np,        epoch,        spin_limit, tiles.n, tiles.m, tiles.group};
   // With few k-blocks to a tile, its start and its way out weigh more than its
   // products: each pair then walks over the tiles.  us, one tile per pair and
-  // walking, 8192 x K x 8192: K = 64 134 / 101, 256 171 / 146, 1000 347 / 328,
+  // walking, 8192 x K x 8192: K = 64 134 / 101, 256 171 / 126, 1000 347 / 328,
   // 2048 579 / 579, 4096 1085 / 1100, 16384 4500 / 4680 (dealt out in advance,
   // the tiles do not follow the pairs' speeds); 5000 x 100 x 5000 57 / 50; with
   // 2.5 tiles to a pair (4000 x K x 3000) at K = 1000 81.5 / 82.5.
