@@ -741,7 +741,7 @@ def segmented_short(S, oracle, hbm_peak):
             "broadcast_adjoint": {"ms": round(seg_bc, 4), "GBps": round(4 * n / seg_bc / 1e6, 1),
                                   "flat_ms": round(flat_bc, 4), "exact": bc_ok},
             "note": "with a segment plan: one launch per call, the short vectors' window records "
-                    "bulk-copied into shared memory, a thread per vector of up to 256 elements; without "
+                    "bulk-copied into shared memory, scanned as one segmented scan; without "
                     "it the offsets pre-pass runs on every call and each short vector takes a warp"}
 
 
