@@ -174,12 +174,19 @@ struct Operand {
 // (lo*hi + hi*lo) then carry a relative error of at most about 2^-22 per term,
 // except where an element below 2^-13 meets an operand element that is itself
 // small or zero (with every element of the other block at least 2^-28 of its
-// largest, the 2^-50 is below 2^-22 of the block's sum of |a b|).  Those
-// k-blocks, non-finite elements and blocks whose largest |x| lies outside
-// [2^-45, 2^46) are reported in `flags`, and the launch takes the bf16 parts
-// instead.  flags: eight words per k-block, set to the launch's epoch: 0 / 2
-// a non-zero element of A / B below 2^-13, 1 / 3 any element below it (zeros
-// included), 4 out of range.
+// largest, the 2^-50 is below 2^-22 of the block's sum of |a b|).  Nor there,
+// if at some k of every output both elements are at least 2, so that the sum
+// is at least 4 and the 2^-36 2^15 below 2^-23 of it: so it is where fewer
+// than an eighth of any row's elements, and fewer than seven eighths of any
+// column's, are below 2, or the other way round (zeros beside a few tiny
+// elements: 8192 x 4096 x 8192 with one of each 1.84 -> 1.10 ms).  The
+// remaining k-blocks, non-finite elements and blocks whose largest |x| lies
+// outside [2^-45, 2^46) are reported in `flags`, and the launch takes the bf16
+// parts instead.  flags: eight words per k-block, set to the launch's epoch, of
+// A (0 ..) and B (4 ..): a non-zero element below 2^-13, any element below it
+// (zeros included), a row with an eighth of its elements below 2, a row with
+// seven eighths of them (a row of zeros counts as neither); all of them where
+// out of range.
 constexpr int kScaleK = 128;
 constexpr int kFlagWords = 8;
 constexpr uint32_t kMaxKBlocks = 4096;  // k-blocks the flag area has room for
@@ -273,16 +280,26 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
       const bool scaled = mb != 0u && in_range;
       const float s = scaled ? __uint_as_float((unsigned int)(268 - eb) << 23) : 1.0f;  // 2^(14 - e)
       __align__(16) __half h[8], l[8];
-      bool small_nz = false, small = false;
+      float least = 0x1p126f;
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         const float v = x[c][e] * s;
         h[e] = __float2half_rn(v);
         l[e] = __float2half_rn((v - __half2float(h[e])) * 2048.0f);
-        const bool below = fabsf(v) < 0x1p-13f && row < R && k + e < K;
-        small |= below;
-        small_nz |= below && x[c][e] != 0.0f;
+        if (k + 8 <= K || k + e < K) least = fminf(least, fabsf(v));
       }
+      const bool small = row < R && least < 0x1p-13f;
+      // the row's elements below 2 (2^-13 to 2^-14 of its largest), zeros past K
+      // taken off; a row of zeros has exact products
+      __half2 under = __float2half2_rn(0.0f);
+#pragma unroll
+      for (int e = 0; e < 8; e += 2)
+        under = __hadd2(under, __hlt2(__habs2(*reinterpret_cast<const __half2*>(h + e)), __float2half2_rn(2.0f)));
+      int low = (int)(__low2float(under) + __high2float(under));
+      if (k + 8 > K) low -= k < K ? (int)(k + 8 - K) : 8;
+      low = __reduce_add_sync(0xffffu << (threadIdx.x & 16), low);
+      if (mb == 0u) low = 0;
+      const int len = (int)(K - k0 < (uint32_t)kScaleK ? K - k0 : (uint32_t)kScaleK), eighth = len / 8;
       if (stored) {
         __half* out = static_cast<__half*>(op.out) + o;
         *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
@@ -291,13 +308,25 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
           op.unscale[(uint64_t)(k0 / kScaleK) * op.rp + row] =
               scaled ? __uint_as_float((unsigned int)(eb - 14) << 23) : 1.0f;
       }
-      const bool any_nz = __any_sync(0xffffffffu, small_nz), any = __any_sync(0xffffffffu, small);
+      const bool any = __any_sync(0xffffffffu, small);
+      bool any_nz = false;
+      if (any) {
+        bool small_nz = false;
+#pragma unroll
+        for (int e = 0; e < 8; ++e) small_nz |= x[c][e] != 0.0f && fabsf(x[c][e] * s) < 0x1p-13f;
+        any_nz = __any_sync(0xffffffffu, small_nz);
+      }
       const bool out_of_range = __any_sync(0xffffffffu, !in_range);
+      const bool some = __any_sync(0xffffffffu, low >= (eighth > 1 ? eighth : 1));
+      const bool many = __any_sync(0xffffffffu, low >= len - eighth);
       if ((threadIdx.x & 31) == 0) {
         unsigned int* f = flags + (uint64_t)(k0 / kScaleK) * kFlagWords;
         if (any_nz) f[flag0] = epoch;
         if (any) f[flag0 + 1] = epoch;
-        if (out_of_range) f[4] = epoch;
+        if (some) f[flag0 + 2] = epoch;
+        if (many) f[flag0 + 3] = epoch;
+        if (out_of_range)
+          for (int i = 0; i < kFlagWords; ++i) f[i] = epoch;
       }
     }
   }
@@ -310,8 +339,11 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
 // neighbouring memory.  With `verdict` (bf16 parts after an FP16 split) the
 // kernel first looks through the flags and leaves unless some k-block needs
 // the bf16 parts, which it reports to the contraction as *verdict = epoch.
+// (FP16: three blocks per SM, 80 registers; left to itself 128 and two blocks:
+// 8192 x 4096 x 8192 1.152 against 1.136 ms, 2560 x 512 x 2560 37.4 and 36.4 us.
+// bf16 parts: 64 registers by themselves.)
 template <int FMT>
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, FMT == kF16 ? 3 : 0)
 split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int parts, unsigned int* flags,
              unsigned int epoch, unsigned int* verdict) {
   __shared__ float tile[128][65];
@@ -324,8 +356,10 @@ split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int part
     bool bad = false;
     for (uint32_t i = threadIdx.x; i < kt; i += 256) {
       const uint4 f = *reinterpret_cast<const uint4*>(flags + (uint64_t)i * kFlagWords);
-      const unsigned int range = flags[(uint64_t)i * kFlagWords + 4];
-      bad |= (f.x == epoch && f.w == epoch) || (f.z == epoch && f.y == epoch) || range == epoch;
+      const uint4 g = *reinterpret_cast<const uint4*>(flags + (uint64_t)i * kFlagWords + 4);
+      const bool meet = (f.x == epoch && g.y == epoch) || (g.x == epoch && f.y == epoch);
+      const bool both_large = (f.z != epoch && g.w != epoch) || (f.w != epoch && g.z != epoch);
+      bad |= meet && !both_large;
     }
     if (!__syncthreads_or(bad ? 1 : 0)) return;
     if (blockIdx.x == 0 && threadIdx.x == 0) *verdict = epoch;
@@ -339,7 +373,7 @@ split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int part
     const uint32_t rt = second ? rtb : rta;
     const uint32_t r0 = (uint32_t)(op.kmajor ? i / kt : i % rt) * 64;
     const uint32_t k0 = (uint32_t)(op.kmajor ? i % kt : i / rt) * 128;
-    split_tile<FMT>(op, K, Kp, r0, k0, parts, tile, flags, epoch, second ? 2 : 0);
+    split_tile<FMT>(op, K, Kp, r0, k0, parts, tile, flags, epoch, second ? 4 : 0);
     if (n > gridDim.x) __syncthreads();  // (block-uniform: the tile is filled again)
   }
 }

@@ -135,11 +135,29 @@ def test_pair_falls_back_to_bf16_parts(scl, orc, what):
     else:
         A[8, 130] = np.float32(2.0 ** -40)
         B = B.copy()
-        B[150, 9] = 0.0
+        B[129:, 9] = 0.0
     P = run(p, A, B)
     assert np.array_equal(P, run(p, A, B, items=3), equal_nan=True)
     if what != "small_times_zero":
         assert np.array_equal(run(p, A0, B), clean)
+
+
+@pytest.mark.parametrize("shape", [(300, 200, 520), (300, 137, 520), (130, 53, 300)])
+@pytest.mark.parametrize("zeros", [1, 10, 80, 100])
+def test_pair_tiny_elements_beside_zeros(scl, orc, zeros, shape):
+    """Tiny elements on one side, zeros (`zeros` of 128 per column) on the
+    other: as exact as without them, whichever parts the launch takes."""
+    M, K, N = shape
+    A = orc.normal_f32(M * K, 55).reshape(M, K)
+    B = orc.normal_f32(K * N, 56).reshape(K, N)
+    rng = np.random.default_rng(zeros)
+    A[rng.integers(0, M, 40), rng.integers(0, K, 40)] = 2.0 ** -40
+    A[:, 7] *= np.float32(2.0 ** -33)
+    B[rng.permuted(np.tile(np.arange(K)[:, None], (1, N)), axis=0) % 128 < zeros] = 0.0
+    for a, b in ((A, B), (np.ascontiguousarray(B.T), np.ascontiguousarray(A.T))):
+        P = run(program(), a, b).astype(np.float64)
+        bound = C * (np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64))
+        assert np.all(np.abs(P - a.astype(np.float64) @ b.astype(np.float64)) <= bound)
 
 
 def test_pair_in_a_graph(scl, orc):
