@@ -464,7 +464,12 @@ static int launch_reduce_impl(scl_program* p, const scl_shape* sh, void* const* 
     uint64_t short_max = wt / 2;
     const SegPlanCfg* cfg = nullptr;
     if (int st = segplan_config(pl, tile, 1, 0, 0, short_max, short_max, &cfg)) return st;
-    const std::string kname = "scl_reduce_seg<" + std::to_string(R) + ", 1>";
+    // Nearly all records: the form compiled for six blocks per SM instead of
+    // four (10^6 vectors of 1..199 floats 87.2 -> 79.9 us, 33333 of 2048..4096
+    // 85.5 -> 79.5; five 86.5, eight 90.6).  Its tiles are slower (71 -> 86 us),
+    // and one has eight records' elements.
+    const bool records = R == 32 && cfg->n_rec > 24 * cfg->tiles;
+    const std::string kname = "scl_reduce_seg<" + std::to_string(R) + (records ? ", 1, 6>" : ", 1>");
     CUfunction fn = find_kernel(p, kname);
     if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname + " missing");
     // partials after the first 256 bytes: the flat reduce keeps its ticket

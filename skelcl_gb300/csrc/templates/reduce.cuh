@@ -381,8 +381,8 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
 // plan numbered the tiles) they fold the segments of at most short_max
 // elements instead, one window of them per block (scl_reduce_window_run):
 // one launch for a whole segmented Reduce.
-template <int R, int MERGED = 0>
-__global__ void __launch_bounds__(256)
+template <int R, int MERGED = 0, int PER_SM = 0>
+__global__ void __launch_bounds__(256, PER_SM)
 scl_reduce_seg(const scl_T* in, scl_T* out, const scl_u64* seg_off,
                const unsigned int* tile_start, scl_u64 n_seg, int aligned, scl_C* partials,
                unsigned int* tickets, unsigned int* err, scl_u64 short_max,
