@@ -378,6 +378,12 @@ split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int part
   }
 }
 
+// Whether 16-byte stores fit every row of P: it may be a view that starts at
+// any element.
+__device__ __forceinline__ bool rows_aligned(const float* P, uint32_t N) {
+  return (N % 4u) == 0u && (reinterpret_cast<uintptr_t>(P) & 15u) == 0;
+}
+
 // A 128 x 128 tile's sums lie in the shared memory of the cluster's `ranks`
 // blocks (16-byte chunk c of row r at chunk c ^ (r % 32) of the row's 512
 // bytes): this block adds up its share of the rows, in block order, and stores
@@ -388,6 +394,7 @@ template <int THREADS>
 __device__ __forceinline__ void store_sums(uint32_t base, uint32_t ranks, uint32_t rank, uint32_t m0, uint32_t n0,
                                            uint32_t M, uint32_t N, float* P) {
   const uint32_t rows = BM / ranks, first = rank * rows;
+  const bool vec = rows_aligned(P, N);
   for (uint32_t i = threadIdx.x; i < rows * 32u; i += THREADS) {
     const uint32_t r = first + i / 32u, c = i % 32u;
     const uint32_t at = base + r * 512u + ((c ^ (r & 31u)) * 16u);
@@ -404,7 +411,7 @@ __device__ __forceinline__ void store_sums(uint32_t base, uint32_t ranks, uint32
     const uint32_t row = m0 + r, col = n0 + c * 4u;
     if (row < M) {
       float* dst = P + (uint64_t)row * N + col;
-      if ((N % 4u) == 0u && col + 4u <= N) {
+      if (vec && col + 4u <= N) {
         *reinterpret_cast<float4*>(dst) = v;
       } else {
         if (col < N) dst[0] = v.x;
@@ -643,7 +650,7 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
     } else if (ok) {
       const uint32_t row = m0 + (uint32_t)(q * 32 + lane);
       if (row < M) {
-        const bool vec = (N % 4u) == 0u;
+        const bool vec = rows_aligned(P, N);
 #pragma unroll
         for (int c = 0; c < CW / 32; ++c) {
           const uint32_t col0 = n0 + (uint32_t)(h * CW + c * 32);
@@ -1047,7 +1054,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
       // x 8192 245 -> 171 us, K = 4096 1.14 -> 1.11 ms).
       if (ok) {
         const uint32_t st = stage_out + (uint32_t)(warp - 2) * 2048u;
-        const bool vec = (g.N % 4u) == 0u;
+        const bool vec = rows_aligned(g.P, g.N);
         uint32_t m0, n0;
         place(t, &m0, &n0);
 #pragma unroll
