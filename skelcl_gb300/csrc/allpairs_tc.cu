@@ -769,15 +769,25 @@ struct PairArgs {
   uint32_t M, N, Kp, Mp, Np, epoch, spin_limit, tiles_n, tiles_m, group_m;
 };
 
-// Bounded wait for arrivals from both CTAs.
+// Bounded wait for arrivals from both CTAs.  ACQUIRE: for what they wrote to
+// shared memory (the operands' copies, read by MMAs that nothing else orders
+// after them); without it for the accumulators, which the tcgen05 fences on
+// either side of the hand-over order.
+template <bool ACQUIRE>
 __device__ __forceinline__ bool mbar_wait_cluster(uint32_t bar, uint32_t parity, uint32_t limit) {
   uint32_t polls = 0;
   for (;;) {
     uint32_t ok;
-    asm volatile(
-        "{ .reg .pred p; mbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;"
-        " selp.u32 %0, 1, 0, p; }"
-        : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    if (ACQUIRE)
+      asm volatile(
+          "{ .reg .pred p; mbarrier.test_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;"
+          " selp.u32 %0, 1, 0, p; }"
+          : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
+    else
+      asm volatile(
+          "{ .reg .pred p; mbarrier.test_wait.parity.relaxed.cluster.shared::cta.b64 p, [%1], %2;"
+          " selp.u32 %0, 1, 0, p; }"
+          : "=r"(ok) : "r"(bar), "r"(parity) : "memory");
     if (ok) return true;
     if (++polls > limit) return false;
     if (polls > 64) __nanosleep(32);
@@ -930,13 +940,13 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
             const uint32_t acc_i = grp & 1u, use = grp >> 1;
             const uint32_t dtm = tmem + acc_i * kPairCols;
             if (use > 0)
-              landed = mbar_wait_cluster(smem_u32(&bars->acc_empty[acc_i]), (use - 1) & 1u, g.spin_limit);
+              landed = mbar_wait_cluster<false>(smem_u32(&bars->acc_empty[acc_i]), (use - 1) & 1u, g.spin_limit);
             if constexpr (SMALLEST_FIRST) {
               // the whole drain group product by product, the smallest first,
               // as gemm_3xbf16_kernel does with its k-blocks of 64
 #pragma unroll
               for (int j = 0; j < SH::G; ++j)
-                landed = landed && mbar_wait_cluster(smem_u32(&bars->full[(it + j) % SH::STAGES]),
+                landed = landed && mbar_wait_cluster<true>(smem_u32(&bars->full[(it + j) % SH::STAGES]),
                                                      ((it + j) / SH::STAGES) & 1u, g.spin_limit);
               if (!landed) break;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -952,7 +962,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
 #pragma unroll
               for (int j = 0; j < SH::G; ++j) {
                 const uint32_t s = (it + j) % SH::STAGES, stage = base + s * SH::STAGE_BYTES;
-                landed = landed && mbar_wait_cluster(smem_u32(&bars->full[s]), ((it + j) / SH::STAGES) & 1u,
+                landed = landed && mbar_wait_cluster<true>(smem_u32(&bars->full[s]), ((it + j) / SH::STAGES) & 1u,
                                                      g.spin_limit);
                 if (!landed) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
