@@ -4,8 +4,8 @@
 // From a Reduce and a Zip:  P[i][j] = id (+) z(A[i][0], B[0][j]) (+) ...
 // (+) z(A[i][K-1], B[K-1][j]), folded in k order; extra arguments are the
 // Reduce's first, then the Zip's.  When the pair is x*y / x+y over float with
-// identity 0 the contraction runs on the tcgen05 tensor cores (FP32
-// operands split into FP16 or bf16 parts, FP32 accumulation); setPrecise(true) keeps it on the CUDA-core kernel.
+// identity 0 the contraction runs on the tcgen05 tensor cores (3xBF16 split,
+// FP32 accumulation); setPrecise(true) keeps it on the CUDA-core kernel.
 // From one user function f(lmatrix_t*, rmatrix_t*, dim, ...): P[i][j] =
 // f(row i of A, column j of B), with getElementFromRow / getElementFromColumn.
 #ifndef SKELCL_ALLPAIRS_H_

@@ -151,8 +151,7 @@ typedef struct scl_tuning {
                             tensor cores: output-tile rows per group of the
                             tile order (0: 16)                                */
   uint32_t items;        /* 16-byte vectors per thread (Map/Zip/Reduce/Scan);
-                            AllPairs tensor cores: bf16 parts, 2 or 3 (0: the
-                            default form for the shape)                        */
+                            AllPairs tensor cores: bf16 parts, 2 or 3 (0: 3)   */
   uint32_t tile_w;       /* Scan: tiles per SM; AllPairs tensor cores:
                             k-blocks per drain of 128-column tiles (1, 2, 4)  */
   uint32_t tile_h;       /* MapOverlap rows per thread / AllPairs tile columns */
@@ -164,7 +163,7 @@ typedef struct scl_tuning {
 #define SCL_VARIANT_SIMPLE 1u     /* one element per thread (reference shape) */
 #define SCL_VARIANT_VECTOR 2u     /* grid-stride 128-bit vectorised           */
 #define SCL_VARIANT_SIMT 3u       /* AllPairs: FP32 SIMT register tiles       */
-#define SCL_VARIANT_TC3XBF16 4u   /* AllPairs: tcgen05 contraction of parts  */
+#define SCL_VARIANT_TC3XBF16 4u   /* AllPairs: tcgen05 3xBF16 contraction     */
 #define SCL_VARIANT_TMA 5u        /* MapOverlap: TMA-staged tile              */
 #define SCL_VARIANT_LDST 6u       /* MapOverlap: cooperative-load tile        */
 

@@ -13,11 +13,11 @@
 // The reference's semantics (AllPairsKernel.cl:47-135: P = sum over k of
 // A[i][k]*B[k][j], identity 0) are kept; only the order of the FP32 sums
 // differs from the sequential fold of the CUDA-core kernel.
-// Products of 256-column tiles are by default taken from two FP16 parts
-// instead, three products in place of six (gemm_pair_kernel, split_tile;
-// the FP16 split with a scaled residual is Ootomo & Yokota, "Recovering
-// single precision accuracy from Tensor Cores while surpassing the FP32
-// theoretical peak performance", IJHPCA 2022).
+// Three parts hold every bit of an FP32 operand (24, of elements that are
+// neither tiny nor huge), so that products with one-hot rows and of whole
+// numbers below 2^12 are exact, as the sequential fold's are.  (Two FP16 parts
+// and three products ran 8192 x 4096 x 8192 in 1.1 ms against 2.0, but hold 22
+// or 23 bits: a quarter of all elements times 1 came out changed.)
 //
 // Shape of the bf16 kernel: 128 x 128 output tile per CTA.  Warp 0 (one thread) streams k-blocks
 // of 64 with TMA (3D tensor maps over the split parts, SWIZZLE_128B, one
@@ -35,7 +35,6 @@
 // memory before it returns.
 #include <cuda.h>
 #include <cuda_bf16.h>
-#include <cuda_fp16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -46,7 +45,6 @@
 namespace scl {
 namespace tc {
 
-enum Format { kBf16 = 0, kF16 = 1 };  // of the operands' parts
 constexpr int BM = 128;
 constexpr int MPAD = 256;                        // M padding: whole tiles of CTA pairs
 constexpr int NPAD = 256;                        // N padding: fits both tile widths
@@ -69,8 +67,8 @@ struct Shape {
   static constexpr uint32_t SBO = 8 * BK * 2;    // bytes between 8-row groups
   static constexpr uint64_t LAYOUT = BK == 64 ? 2u : 4u;  // SWIZZLE_128B : SWIZZLE_64B
   // Instruction descriptor, kind::f16: D = F32 (bits 4-5 = 1), A = B = BF16
-  // (bits 7-9 = 1, 10-12 = 1; 0: FP16), both K-major (bits 15, 16 = 0),
-  // N >> 3 in bits 17-22, M >> 4 in bits 24-28.
+  // (bits 7-9 = 1, 10-12 = 1), both K-major (bits 15, 16 = 0), N >> 3 in bits
+  // 17-22, M >> 4 in bits 24-28.
   static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) |
                                     ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
 };
@@ -155,50 +153,21 @@ __device__ __forceinline__ void raise(unsigned int* err) {
 }
 
 // One operand of the split pass: X, `rows` x K row-major (kmajor) or K x
-// `rows` row-major, into planes [part][rp][Kp] of 16-bit parts; FP16 parts
-// come with one unscale factor per row and 128-wide k-block ([k-block][rp]).
-// Only the first `rows` rows of a plane are written (the rest only reach
-// outputs that are not stored); k is zero-filled to Kp.
+// `rows` row-major, into planes [part][rp][Kp] of bf16 parts.  Only the first
+// `rows` rows of a plane are written (the rest only reach outputs that are
+// not stored); k is zero-filled to Kp.
 struct Operand {
   const float* x;
-  void* out;
-  float* unscale;
+  __nv_bfloat16* out;
   uint32_t rows, rp;
   int kmajor;
 };
 
-// FP16 parts of a 128-wide k-block.  A power of two brings the block's largest
-// |x| into [2^14, 2^15); hi = fp16(x s), lo = fp16((x s - hi) 2^11), so that
-// hi + 2^-11 lo holds 23 bits of every |x s| >= 2^-13 and every smaller
-// element to 2^-36, 2^-50 of the block's largest.  The products hi*hi + 2^-11
-// (lo*hi + hi*lo) then carry a relative error of at most about 2^-22 per term,
-// except where an element below 2^-13 meets an operand element that is itself
-// small or zero (with every element of the other block at least 2^-28 of its
-// largest, the 2^-50 is below 2^-22 of the block's sum of |a b|).  Nor there,
-// if at some k of every output both elements are at least 2, so that the sum
-// is at least 4 and the 2^-36 2^15 below 2^-23 of it: so it is where fewer
-// than an eighth of any row's elements, and fewer than seven eighths of any
-// column's, are below 2, or the other way round (zeros beside a few tiny
-// elements: 8192 x 4096 x 8192 with one of each 1.84 -> 1.10 ms).  The
-// remaining k-blocks, non-finite elements and blocks whose largest |x| lies
-// outside [2^-45, 2^46) are reported in `flags`, and the launch takes the bf16
-// parts instead.  flags: eight words per k-block, set to the launch's epoch, of
-// A (0 ..) and B (4 ..): a non-zero element below 2^-13, any element below it
-// (zeros included), a row with an eighth of its elements below 2, a row with
-// seven eighths of them (a row of zeros counts as neither); all of them where
-// out of range.
-constexpr int kScaleK = 128;
-constexpr int kFlagWords = 8;
-constexpr uint32_t kMaxKBlocks = 4096;  // k-blocks the flag area has room for
-constexpr int kMinExp = 82, kMaxExp = 172;  // biased exponents of 2^-45, 2^45
-
 // X tile of 64 rows x 128 k at (r0, k0): thread i handles rows i / 16 (+ 16,
 // + 32, + 48), k (i % 16) * 8 .. + 7, so sixteen neighbouring lanes hold a
 // row's k-block and store 256 contiguous bytes per part.
-template <int FMT>
 __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32_t Kp, uint32_t r0, uint32_t k0,
-                                           int parts, float (*tile)[65], unsigned int* flags,
-                                           unsigned int epoch, int flag0) {
+                                           int parts, float (*tile)[65]) {
   const uint64_t plane = (uint64_t)op.rp * Kp;
   const uint32_t R = op.rows;
   if (!op.kmajor) {
@@ -253,117 +222,35 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
 #pragma unroll
   for (int c = 0; c < 4; ++c) {
     const uint32_t row = r0 + threadIdx.x / 16 + 16 * c;
-    const bool stored = row < R && k < Kp;
-    const uint64_t o = (uint64_t)row * Kp + k;
-    if constexpr (FMT == kBf16) {
-      __align__(16) __nv_bfloat16 h[8], m[8], l[8];
+    __align__(16) __nv_bfloat16 h[8], m[8], l[8];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        h[e] = __float2bfloat16_rn(x[c][e]);
-        const float r1 = x[c][e] - __bfloat162float(h[e]);
-        m[e] = __float2bfloat16_rn(r1);
-        l[e] = __float2bfloat16_rn(r1 - __bfloat162float(m[e]));
-      }
-      if (stored) {
-        __nv_bfloat16* out = static_cast<__nv_bfloat16*>(op.out) + o;
-        *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
-        *reinterpret_cast<uint4*>(out + plane) = *reinterpret_cast<const uint4*>(m);
-        if (parts > 2) *reinterpret_cast<uint4*>(out + 2 * plane) = *reinterpret_cast<const uint4*>(l);
-      }
-    } else {
-      unsigned int mb = 0;  // largest |x| of the row's k-block, as bits (NaN above infinity)
-#pragma unroll
-      for (int e = 0; e < 8; ++e) mb = max(mb, __float_as_uint(x[c][e]) & 0x7fffffffu);
-      mb = __reduce_max_sync(0xffffu << (threadIdx.x & 16), mb);  // over the row's 16 lanes
-      const int eb = (int)(mb >> 23);
-      const bool in_range = mb == 0u || (eb >= kMinExp && eb <= kMaxExp);
-      const bool scaled = mb != 0u && in_range;
-      const float s = scaled ? __uint_as_float((unsigned int)(268 - eb) << 23) : 1.0f;  // 2^(14 - e)
-      __align__(16) __half h[8], l[8];
-      float least = 0x1p126f;
-#pragma unroll
-      for (int e = 0; e < 8; ++e) {
-        const float v = x[c][e] * s;
-        h[e] = __float2half_rn(v);
-        l[e] = __float2half_rn((v - __half2float(h[e])) * 2048.0f);
-        if (k + 8 <= K || k + e < K) least = fminf(least, fabsf(v));
-      }
-      const bool small = row < R && least < 0x1p-13f;
-      // the row's elements below 2 (2^-13 to 2^-14 of its largest), zeros past K
-      // taken off; a row of zeros has exact products
-      __half2 under = __float2half2_rn(0.0f);
-#pragma unroll
-      for (int e = 0; e < 8; e += 2)
-        under = __hadd2(under, __hlt2(__habs2(*reinterpret_cast<const __half2*>(h + e)), __float2half2_rn(2.0f)));
-      int low = (int)(__low2float(under) + __high2float(under));
-      if (k + 8 > K) low -= k < K ? (int)(k + 8 - K) : 8;
-      low = __reduce_add_sync(0xffffu << (threadIdx.x & 16), low);
-      if (mb == 0u) low = 0;
-      const int len = (int)(K - k0 < (uint32_t)kScaleK ? K - k0 : (uint32_t)kScaleK), eighth = len / 8;
-      if (stored) {
-        __half* out = static_cast<__half*>(op.out) + o;
-        *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
-        *reinterpret_cast<uint4*>(out + plane) = *reinterpret_cast<const uint4*>(l);
-        if (kc == 0)
-          op.unscale[(uint64_t)(k0 / kScaleK) * op.rp + row] =
-              scaled ? __uint_as_float((unsigned int)(eb - 14) << 23) : 1.0f;
-      }
-      const bool any = __any_sync(0xffffffffu, small);
-      bool any_nz = false;
-      if (any) {
-        bool small_nz = false;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) small_nz |= x[c][e] != 0.0f && fabsf(x[c][e] * s) < 0x1p-13f;
-        any_nz = __any_sync(0xffffffffu, small_nz);
-      }
-      const bool out_of_range = __any_sync(0xffffffffu, !in_range);
-      const bool some = __any_sync(0xffffffffu, low >= (eighth > 1 ? eighth : 1));
-      const bool many = __any_sync(0xffffffffu, low >= len - eighth);
-      if ((threadIdx.x & 31) == 0) {
-        unsigned int* f = flags + (uint64_t)(k0 / kScaleK) * kFlagWords;
-        if (any_nz) f[flag0] = epoch;
-        if (any) f[flag0 + 1] = epoch;
-        if (some) f[flag0 + 2] = epoch;
-        if (many) f[flag0 + 3] = epoch;
-        if (out_of_range)
-          for (int i = 0; i < kFlagWords; ++i) f[i] = epoch;
-      }
+    for (int e = 0; e < 8; ++e) {
+      h[e] = __float2bfloat16_rn(x[c][e]);
+      const float r1 = x[c][e] - __bfloat162float(h[e]);
+      m[e] = __float2bfloat16_rn(r1);
+      l[e] = __float2bfloat16_rn(r1 - __bfloat162float(m[e]));
+    }
+    if (row < R && k < Kp) {
+      __nv_bfloat16* out = op.out + ((uint64_t)row * Kp + k);
+      *reinterpret_cast<uint4*>(out) = *reinterpret_cast<const uint4*>(h);
+      *reinterpret_cast<uint4*>(out + plane) = *reinterpret_cast<const uint4*>(m);
+      if (parts > 2) *reinterpret_cast<uint4*>(out + 2 * plane) = *reinterpret_cast<const uint4*>(l);
     }
   }
 }
 
 // Splits both operands, one 64 x 128 tile per step (grid-stride over A's
-// tiles, then B's).  Bound by memory: reads 4 bytes, writes 4 (FP16) or 6
-// (bf16, three parts) per element.  A row-major operand's tiles are taken
-// along k, a transposed one's along its rows, so neighbouring blocks read
-// neighbouring memory.  With `verdict` (bf16 parts after an FP16 split) the
-// kernel first looks through the flags and leaves unless some k-block needs
-// the bf16 parts, which it reports to the contraction as *verdict = epoch.
-// (FP16: three blocks per SM, 80 registers; left to itself 128 and two blocks:
-// 8192 x 4096 x 8192 1.152 against 1.136 ms, 2560 x 512 x 2560 37.4 and 36.4 us.
-// bf16 parts: 64 registers by themselves.)
-template <int FMT>
-__global__ void __launch_bounds__(256, FMT == kF16 ? 3 : 0)
-split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int parts, unsigned int* flags,
-             unsigned int epoch, unsigned int* verdict) {
+// tiles, then B's).  Bound by memory: reads 4 bytes, writes 6 (three parts)
+// per element.  A row-major operand's tiles are taken along k, a transposed
+// one's along its rows, so neighbouring blocks read neighbouring memory.
+__global__ void __launch_bounds__(256)
+split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int parts) {
   __shared__ float tile[128][65];
   // the contraction's blocks may start setting up once every block here runs
   // (they wait for this grid's end before they read): 2-4 % of a small product
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   dependency_wait();
   const uint32_t kt = (Kp + 127) / 128;
-  if (FMT == kBf16 && verdict) {
-    bool bad = false;
-    for (uint32_t i = threadIdx.x; i < kt; i += 256) {
-      const uint4 f = *reinterpret_cast<const uint4*>(flags + (uint64_t)i * kFlagWords);
-      const uint4 g = *reinterpret_cast<const uint4*>(flags + (uint64_t)i * kFlagWords + 4);
-      const bool meet = (f.x == epoch && g.y == epoch) || (g.x == epoch && f.y == epoch);
-      const bool both_large = (f.z != epoch && g.w != epoch) || (f.w != epoch && g.z != epoch);
-      bad |= meet && !both_large;
-    }
-    if (!__syncthreads_or(bad ? 1 : 0)) return;
-    if (blockIdx.x == 0 && threadIdx.x == 0) *verdict = epoch;
-  }
   const uint32_t rta = (a.rows + 63) / 64, rtb = (b.rows + 63) / 64;
   const uint64_t na = (uint64_t)rta * kt, n = na + (uint64_t)rtb * kt;
   for (uint64_t t = blockIdx.x; t < n; t += gridDim.x) {
@@ -373,7 +260,7 @@ split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int part
     const uint32_t rt = second ? rtb : rta;
     const uint32_t r0 = (uint32_t)(op.kmajor ? i / kt : i % rt) * 64;
     const uint32_t k0 = (uint32_t)(op.kmajor ? i % kt : i / rt) * 128;
-    split_tile<FMT>(op, K, Kp, r0, k0, parts, tile, flags, epoch, second ? 4 : 0);
+    split_tile(op, K, Kp, r0, k0, parts, tile);
     if (n > gridDim.x) __syncthreads();  // (block-uniform: the tile is filled again)
   }
 }
@@ -700,73 +587,46 @@ gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constan
 }
 
 // ---- CTA pairs --------------------------------------------------------------------
-// The default form: 256 x 256 output tiles, each by a pair of CTAs
-// (cta_group::2, M = 256, N = 256, K = 16).  Each CTA of the pair holds 128
-// rows of A and 128 of the 256 columns of B per stage and the accumulators of
-// its 128 rows x 256 columns; the pair's first CTA issues the MMAs.  Two
-// 256-column accumulators in tensor memory alternate (ping-pong), drained by
-// 8 epilogue warps of 32 rows x 128 columns into FP32 registers.
-// FP16 parts (three products): k-blocks of 64, three stages of 64 KB per CTA,
-//   a drain per k-block that applies the rows' and columns' unscale factors
-//   (copied into a ring in shared memory beside the operands; products with
-//   powers of two, so exact).  The cross products go first, 2^11 too large;
-//   the first hi*hi MMA scales them down (scale-input-d = 11).
-// bf16 parts (six products, where the split reported values FP16 parts do not
-//   hold): k-blocks of 32, four stages of 48 KB, a drain every 64 of K; the
-//   products of a k-block together, or (SMALLEST_FIRST) of a drain's two, which
-//   is the order and so the bits of gemm_3xbf16_kernel's k-blocks of 64.
-// 8192 x 4096 x 8192, split included: 1.11 ms against 1.85 ms for six products
-// in gemm_3xbf16_kernel; without the drains' work 1.04 ms, at K = 16384 4.31
-// and 3.88 ms (three products at 1.54 and 1.71 of the 1.74 PFLOP/s bf16 a
-// long run sustains).  Bound by the tensor cores, then by the way round an
-// accumulator (MMAs, commit, drain, arrival from the other CTA).  A drain
-// every 128 of K ran 1.07 ms but doubled the error of positive operands
-// (4.6e-7 against 2.5e-7 for six products); two half-tiles of N = 128 with
-// their own accumulators 1.34 ms; 16 epilogue warps of 64 columns 1.25 ms;
-// release / acquire at cluster scope on the accumulators' barriers 1.69 ms
-// (the tcgen05 fences order what they hand over).
+// 256 x 256 output tiles, each by a pair of CTAs (cta_group::2, M = 256, N =
+// 256, K = 16): k-blocks of 32, four stages of 48 KB per CTA.  Each CTA of the
+// pair holds 128 rows of A and 128 of the 256 columns of B per stage and the
+// accumulators of its 128 rows x 256 columns; the pair's first CTA issues the
+// MMAs.  Two 256-column accumulators in tensor memory alternate (ping-pong),
+// drained every 64 of K by 8 epilogue warps of 32 rows x 128 columns into FP32
+// registers.  The products of a k-block of 32 follow one another as in
+// gemm_3xbf16_kernel's 256-column tiles, or (SMALLEST_FIRST) those of a drain's
+// two together as in its 128-column tiles: the same sums in the same order, so
+// the same bits.
+// Against gemm_3xbf16_kernel a pair reads each operand for twice the outputs.
+// Bound by the tensor cores, then by the way round an accumulator (MMAs, commit,
+// drain, arrival from the other CTA).  16 epilogue warps of 64 columns and two
+// half-tiles of N = 128 with their own accumulators were a tenth and a fifth
+// slower.
 // WALK: as many pairs as the device holds, each over several tiles, so that one
 // tile's way out overlaps the next one's products (allpairs_pair_launch says
 // when).
-// Normwise error against FP64 (2560 x K x 2048), here and with six bf16
-// products: normal operands K = 48 1.2e-7 / 2.1e-7, 128 1.4e-7 / 3.2e-7, 1024
-// 1.5e-7 / 3.2e-7, 4096 2.0e-7 / 3.5e-7; uniform in (0, 1) K = 48 1.4e-7 /
-// 1.9e-7, 4096 2.1e-7 / 2.6e-7.  Below K = 48 the six products are the more
-// exact (K = 32: 1.0e-7 / 0.6e-7), and stay.
-constexpr int kPairMinK = 48;
 constexpr int kPairCols = 256;  // tile columns; the tile has 2 * BM rows
 constexpr int kPairCW = 128;    // columns per epilogue warp
 constexpr int kPairThreads = 64 + 32 * 4 * (kPairCols / kPairCW);
-constexpr int kRing = 8;        // unscale slots: more than stages + accumulators in flight
-constexpr int kSlotBytes = (BM + kPairCols) * 4;
-
-template <int FMT>
 struct PairShape {
-  static constexpr int PARTS = FMT == kF16 ? 2 : 3;
-  static constexpr int STAGES = FMT == kF16 ? 3 : 4;
-  static constexpr int G = FMT == kF16 ? 1 : 2;  // k-blocks per drain
-  static constexpr int GS = 128 / (FMT == kF16 ? 64 : 32);  // k-blocks per unscale slot
-  static constexpr int BK = FMT == kF16 ? 64 : 32;
+  static constexpr int PARTS = 3;
+  static constexpr int STAGES = 4;
+  static constexpr int G = 2;  // k-blocks per drain
+  static constexpr int BK = 32;
   static constexpr int TILE = BM * BK * 2;       // bytes of one part of either operand per CTA
   static constexpr int STAGE_BYTES = 2 * PARTS * TILE;
   static constexpr uint32_t SBO = 8 * BK * 2;
-  static constexpr uint64_t LAYOUT = BK == 64 ? 2u : 4u;
-  static constexpr uint32_t IDESC = (1u << 4) | (FMT == kBf16 ? (1u << 7) | (1u << 10) : 0u) |
-                                    ((uint32_t)(kPairCols >> 3) << 17) | ((uint32_t)(2 * BM >> 4) << 24);
+  static constexpr uint64_t LAYOUT = 4u;         // SWIZZLE_64B
+  static constexpr uint32_t IDESC = (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(kPairCols >> 3) << 17) |
+                                    ((uint32_t)(2 * BM >> 4) << 24);
 };
 constexpr int kPairOut = 4 * (kPairCols / kPairCW) * 2048;  // an epilogue warp's way out
-constexpr size_t kPairSmem = (size_t)3 * 64 * 1024 + kRing * kSlotBytes + kPairOut + 1024;
-static_assert(PairShape<kF16>::STAGES * PairShape<kF16>::STAGE_BYTES == 3 * 64 * 1024 &&
-                  PairShape<kBf16>::STAGES * PairShape<kBf16>::STAGE_BYTES == 3 * 64 * 1024,
-              "both formats use the same stage ring");
+constexpr size_t kPairSmem = (size_t)PairShape::STAGES * PairShape::STAGE_BYTES + kPairOut + 1024;
 
 struct PairArgs {
   float* P;
-  const float* unscale_a;  // [k-block][Mp]
-  const float* unscale_b;  // [k-block][Np]
-  const unsigned int* verdict;
   unsigned int* err;
-  uint32_t M, N, Kp, Mp, Np, epoch, spin_limit, tiles_n, tiles_m, group_m;
+  uint32_t M, N, Kp, spin_limit, tiles_n, tiles_m, group_m;
 };
 
 // Bounded wait for arrivals from both CTAs.  ACQUIRE: for what they wrote to
@@ -800,16 +660,6 @@ __device__ __forceinline__ void commit_pair(uint32_t bar) {
       "tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
       :: "r"(bar), "h"((uint16_t)3) : "memory");
 }
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
 __device__ __forceinline__ uint64_t pack2(uint32_t lo, uint32_t hi) {
   uint64_t d;
   asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "r"(lo), "r"(hi));
@@ -821,15 +671,14 @@ struct PairBarriers {
   uint64_t empty[4];      // the MMAs reading a stage completed (each CTA)
   uint64_t acc_full[2];   // accumulator ready (each CTA)
   uint64_t acc_empty[2];  // accumulator drained by both CTAs' epilogues (first CTA)
-  uint64_t ring[kRing];   // unscale slot landed (each CTA)
   uint64_t drain;         // all issued MMAs completed (each CTA)
 };
 
-template <int FMT, bool WALK, bool SMALLEST_FIRST = false>
+template <bool WALK, bool SMALLEST_FIRST>
 __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensorMap& tmB, const PairArgs& g,
-                                          uint32_t base, uint32_t ring, uint32_t stage_out, PairBarriers* bars,
-                                          uint32_t tmem, uint32_t rank, int* s_fail) {
-  using SH = PairShape<FMT>;
+                                          uint32_t base, uint32_t stage_out, PairBarriers* bars, uint32_t tmem,
+                                          uint32_t rank, int* s_fail) {
+  using SH = PairShape;
   constexpr int EPI_WARPS = 4 * (kPairCols / kPairCW);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t nk = g.Kp / SH::BK, tiles = g.tiles_m * g.tiles_n;
@@ -848,7 +697,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
   // and MMAs overlap the last one's way out
   if (warp == 0) {
     // ---- TMA producer (both CTAs): its 128 rows of A and of B's columns, counted
-    //      on the first CTA's barrier, and the unscale factors of its outputs
+    //      on the first CTA's barrier
     if (lane == 0) {
       uint32_t m0, n0, it = 0;  // k-blocks so far
       bool landed = true;
@@ -883,26 +732,6 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
                    "r"((int)(n0 + rank * 128u)), "r"(p), "r"(first_fb)
                 : "memory");
           }
-          if (FMT == kF16 && kb % SH::GS == 0) {
-            // the slot was last read kRing slots ago, long drained: the MMAs of
-            // k-block it - STAGES, just waited for, began after the drain of
-            // k-block it - STAGES - 2
-            static_assert(kRing * SH::GS >= SH::STAGES + 2 + SH::GS, "a slot is reused after its drain");
-            const uint32_t grp = kb / SH::GS;
-            const uint32_t sg = it / SH::GS;  // a tile is a whole number of slots
-            const uint32_t slot = ring + (sg % kRing) * kSlotBytes, rb = smem_u32(&bars->ring[sg % kRing]);
-            asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;"
-                         :: "r"(rb), "r"((uint32_t)kSlotBytes) : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                :: "r"(slot), "l"(g.unscale_a + (uint64_t)grp * g.Mp + m0), "r"((uint32_t)(BM * 4)), "r"(rb)
-                : "memory");
-            asm volatile(
-                "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-                :: "r"(slot + BM * 4), "l"(g.unscale_b + (uint64_t)grp * g.Np + n0),
-                   "r"((uint32_t)(kPairCols * 4)), "r"(rb)
-                : "memory");
-          }
         }
       }
     }
@@ -911,7 +740,7 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
     if (lane == 0) {
       if (rank == 0) {
         // the products of one k-block: part pa of A times part pb of B
-        auto mma = [&](uint32_t dtm, uint32_t stage, int pa, int pb, bool fresh, bool scale_down) {
+        auto mma = [&](uint32_t dtm, uint32_t stage, int pa, int pb, bool fresh) {
           const uint64_t ad = smem_desc<SH>(stage + (uint32_t)(pa * SH::TILE));
           const uint64_t bd = smem_desc<SH>(stage + (uint32_t)((SH::PARTS + pb) * SH::TILE));
 #pragma unroll
@@ -919,20 +748,15 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
             // 16 elements = 32 bytes along K inside the swizzle row
             const uint64_t a = ad + (uint64_t)(ks * 2), b = bd + (uint64_t)(ks * 2);
             const uint32_t acc = fresh && ks == 0 ? 0u : 1u;
-            if (scale_down && ks == 0)
-              asm volatile(
-                  "{ .reg .pred p; setp.ne.b32 p, %4, 0;"
-                  " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p, 11; }"
-                  :: "r"(dtm), "l"(a), "l"(b), "r"(SH::IDESC), "r"(acc)
-                  : "memory");
-            else
-              asm volatile(
-                  "{ .reg .pred p; setp.ne.b32 p, %4, 0;"
-                  " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }"
-                  :: "r"(dtm), "l"(a), "l"(b), "r"(SH::IDESC), "r"(acc)
-                  : "memory");
+            asm volatile(
+                "{ .reg .pred p; setp.ne.b32 p, %4, 0;"
+                " tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p; }"
+                :: "r"(dtm), "l"(a), "l"(b), "r"(SH::IDESC), "r"(acc)
+                : "memory");
           }
         };
+        // lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi: smallest first
+        constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
         bool landed = true;
         uint32_t it = 0, grp = 0;  // k-blocks and drain groups so far
         for (uint32_t t = pair; landed && t < end; t += pairs) {
@@ -950,12 +774,11 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
                                                      ((it + j) / SH::STAGES) & 1u, g.spin_limit);
               if (!landed) break;
               asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-              constexpr int pa[6] = {2, 0, 1, 1, 0, 0}, pb[6] = {0, 2, 1, 0, 1, 0};
 #pragma unroll
               for (int q = 0; q < 6; ++q)
 #pragma unroll
                 for (int j = 0; j < SH::G; ++j)
-                  mma(dtm, base + (it + j) % SH::STAGES * SH::STAGE_BYTES, pa[q], pb[q], q == 0 && j == 0, false);
+                  mma(dtm, base + (it + j) % SH::STAGES * SH::STAGE_BYTES, pa[q], pb[q], q == 0 && j == 0);
 #pragma unroll
               for (int j = 0; j < SH::G; ++j) commit_pair(smem_u32(&bars->empty[(it + j) % SH::STAGES]));
             } else {
@@ -966,18 +789,8 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
                                                      g.spin_limit);
                 if (!landed) break;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (FMT == kF16) {  // lo*hi, hi*lo, hi*hi
-                  mma(dtm, stage, 1, 0, true, false);
-                  mma(dtm, stage, 0, 1, false, false);
-                  mma(dtm, stage, 0, 0, false, true);
-                } else {  // lo*hi, hi*lo, mid*mid, mid*hi, hi*mid, hi*hi: smallest first
-                  mma(dtm, stage, 2, 0, j == 0, false);
-                  mma(dtm, stage, 0, 2, false, false);
-                  mma(dtm, stage, 1, 1, false, false);
-                  mma(dtm, stage, 1, 0, false, false);
-                  mma(dtm, stage, 0, 1, false, false);
-                  mma(dtm, stage, 0, 0, false, false);
-                }
+#pragma unroll
+                for (int q = 0; q < 6; ++q) mma(dtm, stage, pa[q], pb[q], q == 0 && j == 0);
                 commit_pair(smem_u32(&bars->empty[s]));
               }
             }
@@ -1008,21 +821,6 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
       const uint32_t last = grp + nk / SH::G;
       for (; grp != last; ++grp) {
         const uint32_t acc_i = grp & 1u;
-        uint64_t sa = 0;
-        uint32_t sb = 0;
-        if (FMT == kF16) {
-          const uint32_t sg = grp / (SH::GS / SH::G);
-          const uint32_t slot = ring + (sg % kRing) * kSlotBytes;
-          if (!mbar_wait(smem_u32(&bars->ring[sg % kRing]), (sg / kRing) & 1u, g.spin_limit)) {
-            if (lane == 0) raise(g.err);
-            ok = false;
-            break;
-          }
-          uint32_t v;
-          asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(slot + (uint32_t)(q * 32 + lane) * 4u));
-          sa = pack2(v, v);
-          sb = slot + BM * 4 + tile_col * 4;
-        }
         if (!mbar_wait(smem_u32(&bars->acc_full[acc_i]), (grp >> 1) & 1u, g.spin_limit)) {
           if (lane == 0) raise(g.err);
           ok = false;
@@ -1034,22 +832,10 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
         for (int c = 0; c < kPairCW / 16; ++c) {
           uint32_t r[16];
           tmem_load16(tm + (uint32_t)(c * 16), r);
-          if (FMT == kF16) {
-            uint64_t f[8];
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
-            for (int j = 0; j < 4; ++j)
-              asm volatile("ld.shared.v2.u64 {%0, %1}, [%2];"
-                           : "=l"(f[2 * j]), "=l"(f[2 * j + 1]) : "r"(sb + (uint32_t)(c * 64 + j * 16)));
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              sum[c * 8 + j] = fma2(pack2(r[2 * j], r[2 * j + 1]), mul2(sa, f[j]), sum[c * 8 + j]);
-          } else {
-            asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-            for (int j = 0; j < 8; ++j)
-              asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[c * 8 + j]) : "l"(pack2(r[2 * j], r[2 * j + 1])));
-          }
+          for (int j = 0; j < 8; ++j)
+            asm("add.rn.f32x2 %0, %0, %1;" : "+l"(sum[c * 8 + j]) : "l"(pack2(r[2 * j], r[2 * j + 1])));
         }
         // accumulator drained: hand it back to the MMA issuer (one arrive per warp)
         asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
@@ -1111,11 +897,10 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
   static_assert(EPI_WARPS * 32 + 64 == kPairThreads, "");
 }
 
-// WALK: see pair_body.  BF16: bf16 parts alone, without a verdict of the split.
-template <bool WALK, bool BF16 = false>
+// WALK, SMALLEST_FIRST: see above.
+template <bool WALK, bool SMALLEST_FIRST>
 __global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kPairThreads, 1)
 gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                 const __grid_constant__ CUtensorMap tmA3, const __grid_constant__ CUtensorMap tmB3,
                  const PairArgs g) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
   __shared__ __align__(8) PairBarriers bars;
@@ -1123,7 +908,7 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
   __shared__ int s_fail;
   const int warp = threadIdx.x >> 5;
   const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;  // 1024-aligned stage ring
-  const uint32_t ring = base + 3 * 64 * 1024, stage_out = ring + kRing * kSlotBytes;
+  const uint32_t stage_out = base + PairShape::STAGES * PairShape::STAGE_BYTES;
   uint32_t rank;
   asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(rank));
   if (threadIdx.x == 0) {
@@ -1139,7 +924,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
       init(&bars.acc_full[a], 1);
       init(&bars.acc_empty[a], 2 * 4 * (kPairCols / kPairCW));
     }
-    for (int s = 0; s < kRing; ++s) init(&bars.ring[s], 1);
     init(&bars.drain, 1);
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -1149,18 +933,12 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::2.sync.aligned;" ::: "memory");
   }
   dependency_wait();
-  const bool f16 = !BF16 && *g.verdict != g.epoch;
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   cluster_sync();  // both CTAs' barriers are initialised, both hold tensor memory
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = tmem_slot;
-  if (BF16)
-    pair_body<kBf16, WALK, true>(tmA3, tmB3, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
-  else if (f16)
-    pair_body<kF16, WALK>(tmA, tmB, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
-  else
-    pair_body<kBf16, WALK>(tmA3, tmB3, g, base, ring, stage_out, &bars, tmem, rank, &s_fail);
+  pair_body<WALK, SMALLEST_FIRST>(tmA, tmB, g, base, stage_out, &bars, tmem, rank, &s_fail);
 
   // ---- teardown: wait for the copies a failed pipeline may still have in
   //      flight (bounded), then, both CTAs together, free the tensor memory
@@ -1170,10 +948,6 @@ gemm_pair_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant_
     for (int s = 0; s < 4; ++s) {
       mbar_wait(smem_u32(&bars.full[s]), 0, g.spin_limit);
       mbar_wait(smem_u32(&bars.full[s]), 1, g.spin_limit);
-    }
-    for (int s = 0; s < kRing; ++s) {
-      mbar_wait(smem_u32(&bars.ring[s]), 0, g.spin_limit);
-      mbar_wait(smem_u32(&bars.ring[s]), 1, g.spin_limit);
     }
   }
   __syncthreads();
@@ -1413,20 +1187,6 @@ size_t allpairs_tc_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int parts) 
   return (size_t)parts * (Mp + Np) * Kp * 2 + 1024;
 }
 
-// Head of the workspace, before the scratch: [verdict | flags], zero when the
-// workspace is made and written only with launch epochs.
-size_t allpairs_tc_head_bytes() { return 256 + (size_t)tc::kMaxKBlocks * tc::kFlagWords * 4; }
-// Scratch of the CTA-pair form: the planes of either format, then the unscale
-// factors.
-size_t allpairs_pair_scratch_bytes(uint32_t M, uint32_t N, uint32_t K) {
-  const uint64_t Mp = tc::round_up(M, tc::MPAD), Np = tc::round_up(N, tc::NPAD),
-                 Kp = tc::round_up(K, tc::kScaleK);
-  return (size_t)3 * (Mp + Np) * Kp * 2 + 1024 + (size_t)(Mp + Np) * (Kp / tc::kScaleK) * 4;
-}
-bool allpairs_pair_supported(uint32_t K) {
-  return K >= tc::kPairMinK && (K - 1) / tc::kScaleK < tc::kMaxKBlocks;
-}
-
 bool allpairs_tc_supported(uint32_t M, uint32_t N, uint32_t K, const void*, const void*,
                            const void*) {
   // the split arrays' row pitch (Kp * 2 bytes) and plane sizes stay far below
@@ -1436,14 +1196,13 @@ bool allpairs_tc_supported(uint32_t M, uint32_t N, uint32_t K, const void*, cons
 }
 
 static int encode_parts(CUtensorMap* tm, const void* base, uint64_t rows, uint64_t Kp, int parts,
-                        uint32_t box_rows, uint32_t box_k, tc::Format fmt) {
+                        uint32_t box_rows, uint32_t box_k) {
   cuuint64_t dims[3] = {Kp, rows, (cuuint64_t)parts};
   cuuint64_t strides[2] = {Kp * 2, rows * Kp * 2};
   cuuint32_t box[3] = {box_k, box_rows, 1};
   cuuint32_t estr[3] = {1, 1, 1};
   CUresult r = rt().drv.cuTensorMapEncodeTiled(
-      tm, fmt == tc::kF16 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT16 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3,
-      const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
+      tm, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 3, const_cast<void*>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,
       box_k == 64 ? CU_TENSOR_MAP_SWIZZLE_128B : CU_TENSOR_MAP_SWIZZLE_64B,
       CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return cu_fail(r, "cuTensorMapEncodeTiled(split parts)");
@@ -1480,15 +1239,15 @@ struct Split {
   uint32_t Mp, Np, Kp;
   tc::Operand a, b;
 };
-Split split_of(const float* A, const float* B, uint32_t M, uint32_t N, uint32_t K, uint32_t kpad, int parts,
-               int trans, void* scratch) {
+Split split_of(const float* A, const float* B, uint32_t M, uint32_t N, uint32_t K, int parts, int trans,
+               void* scratch) {
   Split s;
   s.Mp = tc::round_up(M, tc::MPAD);
   s.Np = tc::round_up(N, tc::NPAD);
-  s.Kp = tc::round_up(K, kpad);
-  uint16_t* base = reinterpret_cast<uint16_t*>(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
-  s.a = {A, base, nullptr, M, s.Mp, (trans & 1) ? 0 : 1};
-  s.b = {B, base + (size_t)parts * s.Mp * s.Kp, nullptr, N, s.Np, (trans & 2) ? 1 : 0};
+  s.Kp = tc::round_up(K, tc::KPAD);
+  __nv_bfloat16* base = reinterpret_cast<__nv_bfloat16*>(((uintptr_t)scratch + 1023) & ~(uintptr_t)1023);
+  s.a = {A, base, M, s.Mp, (trans & 1) ? 0 : 1};
+  s.b = {B, base + (size_t)parts * s.Mp * s.Kp, N, s.Np, (trans & 2) ? 1 : 0};
   return s;
 }
 uint64_t split_tiles(const Split& s) {
@@ -1522,7 +1281,7 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
   if (parts != 2 && parts != 3) return fail(SCL_ERR_ARG, "3xBF16: parts must be 2 or 3");
   if (scratch_bytes < allpairs_tc_scratch_bytes(M, N, K, parts))
     return fail(SCL_ERR_ARG, "3xBF16: scratch too small");
-  const Split sp = split_of(A, B, M, N, K, tc::KPAD, parts, trans, scratch);
+  const Split sp = split_of(A, B, M, N, K, parts, trans, scratch);
   const uint32_t Kp = sp.Kp;
   const uint32_t bn = wide ? 256 : 128, bk = wide ? 32 : 64;
   Tiles tiles;
@@ -1530,11 +1289,9 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
   const dim3 grid(tiles.m * tiles.n);
   const uint32_t tn = tiles.n, group_m = tiles.group;
   alignas(64) CUtensorMap tmA, tmB;
-  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, parts, tc::BM, bk, tc::kBf16)) return st;
-  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, parts, bn, bk, tc::kBf16)) return st;
-  unsigned int* none = nullptr;
-  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp,
-                                    parts, none, 0u, none);
+  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, parts, tc::BM, bk)) return st;
+  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, parts, bn, bk)) return st;
+  cudaError_t e = launch_overlapped(tc::split_kernel, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp, parts);
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
   if (wide) {
     // 128 x 256 tiles, k-blocks of 32: drains every 2 k-blocks (64 K, as the
@@ -1576,9 +1333,9 @@ uint64_t resident_pairs() {
     cfg.dynamicSmemBytes = tc::kPairSmem;
     cfg.attrs = &attr;
     cfg.numAttrs = 1;
-    if (cudaFuncSetAttribute(tc::gemm_pair_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    if (cudaFuncSetAttribute(tc::gemm_pair_kernel<true, false>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                              (int)tc::kPairSmem) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, tc::gemm_pair_kernel<true>, &cfg) != cudaSuccess || n < 1) {
+        cudaOccupancyMaxActiveClusters(&n, tc::gemm_pair_kernel<true, false>, &cfg) != cudaSuccess || n < 1) {
       cudaGetLastError();
       n = half;
     }
@@ -1586,6 +1343,16 @@ uint64_t resident_pairs() {
   }
   return (uint64_t)n;
 }
+}  // namespace
+
+namespace {
+// While a tile has few k-blocks, its start and its way out weigh more than its
+// products: each pair then walks over the tiles.  us, one tile per pair and
+// walking: 8192 x K x 8192 K = 64 124 / 64, 512 298 / 248, 1000 519 / 482, 2500
+// 1193 / 1178, 4096 1853 / 1904 (dealt out in advance, the tiles do not follow
+// the pairs' speeds); 2600 x K x 4000 K = 512 65.9 / 56.5, 1500 156 / 147; 2600 x
+// 3000 x 20000 1191 / 1216.
+bool pair_walks(uint64_t tiles, uint32_t Kp) { return Kp <= 2560 && tiles > resident_pairs(); }
 }  // namespace
 
 // One wave of 128 x 128 tiles (or of clusters that share one), few k-blocks a
@@ -1601,8 +1368,8 @@ int allpairs_fused_launch(const float* A, const float* B, float* P, uint32_t M, 
                           uint32_t group_rows, cudaStream_t stream, uint32_t spin_limit, unsigned int* err) {
   Tiles tiles;
   if (int st = tiles_of(M, N, tc::BM, 128, group_rows, &tiles)) return st;
-  const tc::Fused args = {{A, nullptr, nullptr, M, M, (trans & 1) ? 0 : 1},
-                          {B, nullptr, nullptr, N, N, (trans & 2) ? 1 : 0},
+  const tc::Fused args = {{A, nullptr, M, M, (trans & 1) ? 0 : 1},
+                          {B, nullptr, N, N, (trans & 2) ? 1 : 0},
                           P, err, M, N, K, spin_limit, tiles.n, tiles.group};
   const uint32_t split = split_of_k((uint64_t)tiles.m * tiles.n, tc::round_up(K, tc::KPAD));
   const dim3 grid(tiles.m * tiles.n * split);
@@ -1614,89 +1381,65 @@ int allpairs_fused_launch(const float* A, const float* B, float* P, uint32_t M, 
   return SCL_OK;
 }
 
-// CTA pairs: FP16 parts, with the bf16 parts as the device's fallback.
-// `head` (allpairs_tc_head_bytes) precedes the scratch; `epoch` differs from
-// every earlier launch's on this head, or the head was cleared before.
+// CTA pairs, three bf16 parts.  `small`: the products in the order of 128-column
+// tiles, else of 256-column ones.
 int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
-                         uint32_t group_rows, void* head, void* scratch, size_t scratch_bytes, unsigned int epoch,
-                         cudaStream_t stream, uint32_t spin_limit, unsigned int* err) {
-  if (scratch_bytes < allpairs_pair_scratch_bytes(M, N, K) || !allpairs_pair_supported(K))
+                         bool small, uint32_t group_rows, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                         uint32_t spin_limit, unsigned int* err) {
+  if (scratch_bytes < allpairs_tc_scratch_bytes(M, N, K, 3))
     return fail(SCL_ERR_ARG, "tensor-core AllPairs: scratch too small");
-  Split sp = split_of(A, B, M, N, K, tc::kScaleK, 2, trans, scratch);
-  const Split sp3 = split_of(A, B, M, N, K, tc::kScaleK, 3, trans, scratch);
+  const Split sp = split_of(A, B, M, N, K, 3, trans, scratch);
   const uint32_t Kp = sp.Kp;
-  float* unscale = reinterpret_cast<float*>(static_cast<uint16_t*>(sp3.b.out) + (size_t)3 * sp.Np * Kp);
-  sp.a.unscale = unscale;
-  sp.b.unscale = unscale + (size_t)sp.Mp * (Kp / tc::kScaleK);
-  unsigned int* verdict = static_cast<unsigned int*>(head);
-  unsigned int* flags = verdict + 64;
   Tiles tiles;
   if (int st = tiles_of(M, N, 2 * tc::BM, tc::kPairCols, group_rows, &tiles)) return st;
-  alignas(64) CUtensorMap tmA, tmB, tmA3, tmB3;
-  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, 2, tc::BM, 64, tc::kF16)) return st;
-  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, 2, 128, 64, tc::kF16)) return st;
-  if (int st = encode_parts(&tmA3, sp3.a.out, sp.Mp, Kp, 3, tc::BM, 32, tc::kBf16)) return st;
-  if (int st = encode_parts(&tmB3, sp3.b.out, sp.Np, Kp, 3, 128, 32, tc::kBf16)) return st;
-  unsigned int* none = nullptr;
-  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kF16>, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp, 2,
-                                    flags, epoch, none);
+  alignas(64) CUtensorMap tmA, tmB;
+  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, 3, tc::BM, 32)) return st;
+  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, 3, 128, 32)) return st;
+  cudaError_t e = launch_overlapped(tc::split_kernel, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp, 3);
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
-  const unsigned few = (unsigned)std::min<uint64_t>(split_tiles(sp), (uint64_t)rt().sm_count * 4);
-  e = launch_overlapped(tc::split_kernel<tc::kBf16>, dim3(few), dim3(256), 0, stream, sp3.a, sp3.b, K, Kp, 3, flags, epoch,
-                        verdict);
-  if (e != cudaSuccess) return cuda_fail(e, "split launch");
-  const tc::PairArgs args = {P,     sp.a.unscale, sp.b.unscale, verdict, err,        M,       N,      Kp,
-                             sp.Mp, sp.Np,        epoch,        spin_limit, tiles.n, tiles.m, tiles.group};
-  // With few k-blocks to a tile, its start and its way out weigh more than its
-  // products: each pair then walks over the tiles.  us, one tile per pair and
-  // walking, 8192 x K x 8192: K = 64 134 / 101, 256 171 / 126, 1000 347 / 328,
-  // 2048 579 / 579, 4096 1085 / 1100, 16384 4500 / 4680 (dealt out in advance,
-  // the tiles do not follow the pairs' speeds); 5000 x 100 x 5000 57 / 50; with
-  // 2.5 tiles to a pair (4000 x K x 3000) at K = 1000 81.5 / 82.5.
+  const tc::PairArgs args = {P, err, M, N, Kp, spin_limit, tiles.n, tiles.m, tiles.group};
   const uint64_t all = (uint64_t)tiles.m * tiles.n;
-  const bool walk = Kp <= 1024 && all > resident_pairs() * (Kp <= 512 ? 1 : 4);
-  e = launch_overlapped(walk ? tc::gemm_pair_kernel<true> : tc::gemm_pair_kernel<false>,
+  const bool walk = !small && pair_walks(all, Kp);
+  e = launch_overlapped(small  ? tc::gemm_pair_kernel<false, true>
+                        : walk ? tc::gemm_pair_kernel<true, false>
+                               : tc::gemm_pair_kernel<false, false>,
                         dim3((unsigned)(2 * (walk ? resident_pairs() : all))), dim3(tc::kPairThreads), tc::kPairSmem,
-                        stream, tmA, tmB, tmA3, tmB3, args);
+                        stream, tmA, tmB, args);
   if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
   return SCL_OK;
 }
 
-// CTA pairs, bf16 parts: where 128 x 128 tiles take two waves of the SMs and 256
-// x 256 tiles one of the pairs.  A k-block of 64 takes 1.2 us in the former
-// (its 96 KB per SM come at 12 TB/s, from L2) and 1.9 us in the latter, for
-// twice the outputs per SM, with the same products in the same order and so the
-// same bits.  us, 128 x 128 tiles and so, the split included: 2000 x K x 2000
-// K = 64 15.3 / 11.9, 500 32.1 / 24.8, 2000 90.1 / 71.8, 4000 166 / 132; 300 x
-// 1000 x 8000 55.8 / 47.3.
-bool allpairs_pair3_wins(uint32_t M, uint32_t N) {
+// Whether CTA pairs take the place of 128 x 128 tiles: where those take two
+// waves of the SMs and 256 x 256 tiles one of the pairs.  A k-block of 64 takes
+// 1.2 us in the former (its 96 KB per SM come at 12 TB/s, from L2) and 1.9 us in
+// the latter, for twice the outputs per SM, with the same products in the same
+// order and so the same bits.  us, 128 x 128 tiles and so, the split included:
+// 2000 x K x 2000 K = 64 15.3 / 11.9, 500 32.1 / 24.8, 2000 90.1 / 71.8, 4000
+// 166 / 132; 300 x 1000 x 8000 55.8 / 47.3.
+bool allpairs_pair_replaces_small(uint32_t M, uint32_t N) {
   const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u, pairs = resident_pairs();
   const uint64_t small = (uint64_t)((M + 127) / 128) * ((N + 127) / 128);
   const uint64_t large = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
   return small > sms && large <= pairs;
 }
-int allpairs_pair3_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
-                          uint32_t group_rows, void* scratch, size_t scratch_bytes, cudaStream_t stream,
-                          uint32_t spin_limit, unsigned int* err) {
-  if (scratch_bytes < allpairs_tc_scratch_bytes(M, N, K, 3))
-    return fail(SCL_ERR_ARG, "tensor-core AllPairs: scratch too small");
-  const Split sp = split_of(A, B, M, N, K, tc::KPAD, 3, trans, scratch);
-  const uint32_t Kp = sp.Kp;
-  Tiles tiles;
-  if (int st = tiles_of(M, N, 2 * tc::BM, tc::kPairCols, group_rows, &tiles)) return st;
-  alignas(64) CUtensorMap tmA, tmB;
-  if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, 3, tc::BM, 32, tc::kBf16)) return st;
-  if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, 3, 128, 32, tc::kBf16)) return st;
-  unsigned int* none = nullptr;
-  cudaError_t e = launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp,
-                                    3, none, 0u, none);
-  if (e != cudaSuccess) return cuda_fail(e, "split launch");
-  const tc::PairArgs args = {P,     nullptr, nullptr, none,       err,     M,       N,      Kp,
-                             sp.Mp, sp.Np,   0u,      spin_limit, tiles.n, tiles.m, tiles.group};
-  e = launch_overlapped(tc::gemm_pair_kernel<false, true>, dim3(2 * tiles.m * tiles.n), dim3(tc::kPairThreads),
-                        tc::kPairSmem, stream, tmA, tmB, tmA, tmB, args);
-  if (e != cudaSuccess) return cuda_fail(e, "tensor-core AllPairs launch");
-  return SCL_OK;
+
+// ... and of 128 x 256 tiles: nearly always.  us, 128 x 256 tiles and so, the
+// split included: 8192 x K x 8192 K = 64 167 / 64, 256 247 / 132, 1000 575 /
+// 482, 4096 2072 / 1902; 2560 x 512 x 2048 48.3 / 39.9; 4000 x 1000 x 3000 121 /
+// 104; 2500 x 1000 x 2305 109 / 75.  Not where the pairs' 256 rows hold so much
+// more padding that it shows: as rows take more pair tiles for their wide ones,
+// 1100 x K x 20000 (1.11) K = 512 139 / 113, 1500 321 / 320, 3000 604 / 618; 300
+// x K x 60000 (1.33) K = 256 113 / 92, 1500 405 / 437; 128 x K x 100000 (2) K =
+// 64 55 / 47, 512 171 / 180, 3000 821 / 978.  With as many waves the padding
+// costs nothing: 640 x 1500 x 7936 124 / 110.  A few rows write next to nothing,
+// and what is left is the pairs' start: 1 x 50 x 62000 20.7 / 23.7, 100 x 128 x
+// 39680 32.2 / 28.3.
+bool allpairs_pair_replaces_wide(uint32_t M, uint32_t N, uint32_t K) {
+  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u, pairs = resident_pairs();
+  const uint64_t wide = (uint64_t)((M + 127) / 128) * ((N + 255) / 256);
+  const uint64_t large = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
+  if ((K <= 128 && M >= 100) || (K <= 256 && 3 * large <= 2 * wide)) return true;
+  return 20 * large <= 11 * wide || (large + pairs - 1) / pairs <= (wide + sms - 1) / sms;
 }
 
 }  // namespace scl
@@ -1712,9 +1455,7 @@ extern "C" int scl_debug_allpairs_split(const float* A, const float* B, uint32_t
   if (!scratch) return SCL_OK;
   if (int st = require_init()) return st;
   if (!A || !B || scratch_bytes < need) return fail(SCL_ERR_ARG, "split: null operand or scratch too small");
-  const Split sp = split_of(A, B, M, N, K, tc::KPAD, parts, trans, scratch);
-  unsigned int* none = nullptr;
-  SCL_CUDA(launch_overlapped(tc::split_kernel<tc::kBf16>, split_grid(sp), dim3(256), 0, rt().stream, sp.a, sp.b, K, sp.Kp,
-                             parts, none, 0u, none));
+  const Split sp = split_of(A, B, M, N, K, parts, trans, scratch);
+  SCL_CUDA(launch_overlapped(tc::split_kernel, split_grid(sp), dim3(256), 0, rt().stream, sp.a, sp.b, K, sp.Kp, parts));
   return SCL_OK;
 }

@@ -147,7 +147,6 @@ struct Workspace {  // per-program scratch (reduce partials, scan tile status)
   void* scan_layout = nullptr;
   uint64_t scan_epoch = 0;
   uint64_t scan_used[2] = {0, 0};
-  uint32_t tc_epoch = 0;  // tensor-core AllPairs: eager launches made (see allpairs_tc.cu)
 };
 
 // Scan status layout (scan.cuh): three regions of `cap` tiles, each a

@@ -22,16 +22,11 @@ size_t allpairs_tc_scratch_bytes(uint32_t M, uint32_t N, uint32_t K, int parts);
 bool allpairs_fused_wins(uint32_t M, uint32_t N, uint32_t K, int trans);
 int allpairs_fused_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
                           uint32_t group_rows, cudaStream_t stream, uint32_t spin_limit, unsigned int* err);
-bool allpairs_pair3_wins(uint32_t M, uint32_t N);
-int allpairs_pair3_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
-                          uint32_t group_rows, void* scratch, size_t scratch_bytes, cudaStream_t stream,
-                          uint32_t spin_limit, unsigned int* err);
+bool allpairs_pair_replaces_small(uint32_t M, uint32_t N);
+bool allpairs_pair_replaces_wide(uint32_t M, uint32_t N, uint32_t K);
 int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, uint32_t N, uint32_t K, int trans,
-                         uint32_t group_rows, void* head, void* scratch, size_t scratch_bytes, unsigned int epoch,
-                         cudaStream_t stream, uint32_t spin_limit, unsigned int* err);
-size_t allpairs_pair_scratch_bytes(uint32_t M, uint32_t N, uint32_t K);
-size_t allpairs_tc_head_bytes();
-bool allpairs_pair_supported(uint32_t K);
+                         bool small, uint32_t group_rows, void* scratch, size_t scratch_bytes, cudaStream_t stream,
+                         uint32_t spin_limit, unsigned int* err);
 bool allpairs_tc_supported(uint32_t M, uint32_t N, uint32_t K, const void* A, const void* B,
                            const void* P);
 }  // namespace scl
@@ -951,9 +946,6 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
                     ((sh->flags & SCL_SHAPE_TRANS_RIGHT) ? 2 : 0);
   if (p->kind == SCL_KIND_ALLPAIRS) {
     const uint32_t want = tu ? tu->variant : SCL_VARIANT_AUTO;
-    // the workspace starts with the tensor-core form's flags, which must hold
-    // nothing but launch epochs: every other use begins after them
-    const size_t tc_head = allpairs_tc_head_bytes();
     if (p->tc_eligible && want != SCL_VARIANT_SIMT && extra_bytes == 0 &&
         allpairs_tc_supported(M, N, K, A, B, P)) {
       // tuning.tile_h: output-tile columns, 128 or 256; 0 takes 256 when the
@@ -962,14 +954,7 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
       const uint64_t wide_tiles = (uint64_t)((M + 127u) / 128u) * ((N + 255u) / 256u);
       const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
       const int wide = cols == 256u || (cols == 0u && wide_tiles >= sms) ? 1 : 0;
-      // tuning.items: 3 bf16 parts (6 products) or 2 (3 products); 0: 256-column
-      // tiles take CTA pairs with FP16 parts (3 products: 8192 x 4096 x 8192
-      // 1.11 ms against 1.85, normwise error 2.0e-7 against 3.5e-7; the device
-      // falls back to 3 bf16 parts for values FP16 parts do not hold) from
-      // K = 48 on, below which six products are the more exact; 128-column
-      // tiles keep 3 bf16 parts (drained per 64 of K, their normwise error,
-      // 1.1e-7, is below what FP16 parts gave there, 1.6e-7)
-      const bool pair = wide && !(tu && (tu->items || tu->tile_w > 1)) && allpairs_pair_supported(K);
+      // tuning.items == 2: two bf16 parts, 3 products; otherwise three parts, 6 products
       const int parts = (tu && tu->items == 2) ? 2 : 3;
       // (the fused form takes no workspace)
       const bool plain = cols == 0 && parts == 3 && !(tu && (tu->items || tu->tile_w));
@@ -978,39 +963,22 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
         return allpairs_fused_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans,
                                      tu ? tu->workgroup : 0u, rt().stream, spin_of(tu), rt().dev_err);
       }
-      const size_t need = pair ? allpairs_pair_scratch_bytes(M, N, K) : allpairs_tc_scratch_bytes(M, N, K, parts);
-      if (int st = ensure_workspace(p, tc_head + need)) return st;
-      char* scratch = static_cast<char*>(p->ws.ptr) + tc_head;
+      if (int st = ensure_workspace(p, allpairs_tc_scratch_bytes(M, N, K, parts))) return st;
       p->last_variant = SCL_VARIANT_TC3XBF16;
       // tuning.tile_w: k-blocks accumulated in tensor memory per drain of a
       // 128-column tile (1, 2 or 4)
       const int drain = (tu && tu->tile_w) ? (int)tu->tile_w : 1;
       // tuning.workgroup: output-tile rows per group of the tile order (0: 16)
       const uint32_t group_rows = tu ? tu->workgroup : 0u;
-      if (pair) {
-        // flags of the split are words that hold this launch's epoch: eager
-        // launches count up from 2; a recorded launch is replayed with the
-        // same one, so its graph clears the flags first
-        cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-        SCL_CUDA(cudaStreamIsCapturing(rt().stream, &capture));
-        unsigned int epoch = 1;
-        if (capture != cudaStreamCaptureStatusNone) {
-          SCL_CUDA(cudaMemsetAsync(p->ws.ptr, 0, tc_head, rt().stream));
-        } else {
-          if (++p->ws.tc_epoch < 2) p->ws.tc_epoch = 2;
-          epoch = p->ws.tc_epoch;
-        }
-        return allpairs_pair_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans, group_rows,
-                                    p->ws.ptr, scratch, p->ws.bytes - tc_head, epoch, rt().stream, spin_of(tu),
-                                    rt().dev_err);
-      }
-      // 128-column tiles in two waves, CTA pairs in one: the same products, the
-      // same bits (allpairs_pair3_launch)
-      if (!wide && plain && allpairs_pair3_wins(M, N))
-        return allpairs_pair3_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans, group_rows, scratch,
-                                     p->ws.bytes - tc_head, rt().stream, spin_of(tu), rt().dev_err);
+      // CTA pairs in place of either tile give the same bits; an explicit number
+      // of parts or of k-blocks per drain keeps the tiles
+      const bool pair = wide ? !(tu && (tu->items || tu->tile_w > 1)) && allpairs_pair_replaces_wide(M, N, K)
+                             : plain && allpairs_pair_replaces_small(M, N);
+      if (pair)
+        return allpairs_pair_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans, !wide, group_rows,
+                                    p->ws.ptr, p->ws.bytes, rt().stream, spin_of(tu), rt().dev_err);
       return allpairs_tc_launch((const float*)A, (const float*)B, (float*)P, M, N, K, parts, trans,
-                                drain, wide, group_rows, scratch, p->ws.bytes - tc_head, rt().stream,
+                                drain, wide, group_rows, p->ws.ptr, p->ws.bytes, rt().stream,
                                 spin_of(tu), rt().dev_err);
     }
     if (want == SCL_VARIANT_TC3XBF16)
@@ -1029,8 +997,8 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
       const size_t s0 = p->type_sizes[0], s1 = p->type_sizes[1];
       const size_t a_bytes = (trans & 1) ? ((size_t)M * K * s0 + 255) / 256 * 256 : 0;
       const size_t b_bytes = (trans & 2) ? (size_t)K * N * s1 : 0;
-      if (int st = ensure_workspace(p, tc_head + a_bytes + b_bytes)) return st;
-      char* ws = static_cast<char*>(p->ws.ptr) + tc_head;
+      if (int st = ensure_workspace(p, a_bytes + b_bytes)) return st;
+      char* ws = static_cast<char*>(p->ws.ptr);
       if (trans & 1) {
         if (int st = transpose_launch(A, ws, K, M, s0, rt().stream)) return st;
         A = ws;
