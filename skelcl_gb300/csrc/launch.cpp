@@ -242,18 +242,25 @@ int vec_width(size_t s0, size_t s1 = 1, size_t s2 = 1) {
   return 1;
 }
 
-// Blocks and threads of a flat Reduce over `units` loads, `items` of which a
-// thread keeps in flight: one block while its threads hold everything in one
-// round (no partials to combine: 1000..16000 floats 4.4 -> 2.8 us), then a
-// block per SM until their rounds are full, then as many as that takes, up to
-// what is resident (2^20 floats 6.5 -> 4.9 us, 300,000 5.7 -> 4.7, against a
-// block for every 256 loads: fewer partials, and blocks whose loads overlap).
+// Threads of a flat Reduce's blocks over `units` loads, and the blocks: one for
+// every 256 loads, up to what is resident.  Up to 512 loads are one block's where
+// the carries are narrow: a load to each of its threads, no partials to combine
+// (2000 ints 2.6 -> 1.4 us, of an operator with a division 4.1 -> 2.8).  Not with
+// FP64 carries, whose folds two SMs share (2000 floats 3.5 -> 2.3, but with the
+// division 14.5 -> 20.3; 1000 doubles 15.5 -> 22.6).  Fewer blocks with longer
+// folds were faster for sums of floats (16,000 4.1 -> 2.8 us, 2^20 6.2 -> 4.8) but
+// round more often in single precision before the carries, and an operator that
+// costs more waits for them (16,000 floats with the division 17.5 -> 25.0 us,
+// 4000 doubles 17.7 -> 40.6).
 constexpr uint32_t kReduceOneBlock = 512;
-uint64_t reduce_grid(uint64_t units, uint32_t wg, uint32_t items, uint64_t maxb) {
-  if (units <= (uint64_t)wg * items) return 1;
-  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
-  const uint64_t most = (units + wg - 1) / wg, full = (units + (uint64_t)wg * items - 1) / ((uint64_t)wg * items);
-  return std::min(maxb, std::max(full, std::min(most, sms)));
+uint32_t reduce_threads(scl_program* p, CUfunction fn, uint64_t units) {
+  return units > 256 && units <= kReduceOneBlock && p->carry_size > 0 && p->carry_size <= 4 &&
+                 max_threads(p, fn) >= (int)kReduceOneBlock
+             ? kReduceOneBlock
+             : 256;
+}
+uint64_t reduce_grid(uint64_t units, uint32_t wg, uint64_t maxb) {
+  return std::max<uint64_t>(1, std::min(maxb, (units + wg - 1) / wg));
 }
 
 // Tile of the CUDA-core AllPairs for M x N outputs.  A block takes its K steps
@@ -556,10 +563,9 @@ static int launch_reduce_impl(scl_program* p, const scl_shape* sh, void* const* 
   CUfunction fn = hot_kernel(p, items, kname);
   if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname() + " missing");
   const uint64_t units = aligned ? n / V : n;
-  const bool one_block = units <= (uint64_t)kReduceOneBlock * items && max_threads(p, fn) >= (int)kReduceOneBlock;
-  uint32_t wg = pick_block(tu, one_block ? kReduceOneBlock : 256);
+  uint32_t wg = pick_block(tu, reduce_threads(p, fn, units));
   wg = (wg + 31) / 32 * 32;
-  const uint64_t g = reduce_grid(units, wg, items, (uint64_t)max_resident_blocks(p, fn, (int)wg, 0));
+  const uint64_t g = reduce_grid(units, wg, (uint64_t)max_resident_blocks(p, fn, (int)wg, 0));
   const size_t part_off = 256;
   if (int st = ensure_workspace(p, part_off + g * csz)) return st;
   void* partials = (char*)p->ws.ptr + part_off;
@@ -593,10 +599,9 @@ static int launch_zipreduce(scl_program* p, const scl_shape* sh, void* const* bu
   CUfunction fn = hot_kernel(p, items, kname);
   if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname() + " missing");
   const uint64_t units = aligned ? n / V : n;
-  const bool one_block = units <= (uint64_t)kReduceOneBlock * items && max_threads(p, fn) >= (int)kReduceOneBlock;
-  uint32_t wg = pick_block(tu, one_block ? kReduceOneBlock : 256);
+  uint32_t wg = pick_block(tu, reduce_threads(p, fn, units));
   wg = (wg + 31) / 32 * 32;
-  const uint64_t g = reduce_grid(units, wg, items, (uint64_t)max_resident_blocks(p, fn, (int)wg, 0));
+  const uint64_t g = reduce_grid(units, wg, (uint64_t)max_resident_blocks(p, fn, (int)wg, 0));
   const size_t part_off = 256;
   if (int st = ensure_workspace(p, part_off + g * csz)) return st;
   void* partials = (char*)p->ws.ptr + part_off;
