@@ -343,7 +343,7 @@ struct SegPlanCfg {
 };
 // The window records of one pair of limits, shared by the tile shapes that
 // use it (device, 4 words each: first segment, end segment, first element,
-// elements).
+// elements with the longest segment's above them in the upper half).
 struct SegPlanRecords {
   uint64_t short_max = 0, window = 0, n_rec = 0;
   uint64_t* rec = nullptr;

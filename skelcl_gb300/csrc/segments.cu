@@ -524,7 +524,16 @@ int segplan_records(SegPlan* p, uint64_t short_max, uint64_t window, const SegPl
     p->host_off.swap(off);
   }
   std::vector<uint64_t> rec;
-  segplan_window_records(p->host_off.data(), p->n_seg, short_max, window, &rec);
+  const uint64_t* off = p->host_off.data();
+  segplan_window_records(off, p->n_seg, short_max, window, &rec);
+  // the kernels find the longest vector's length above the elements (below 2^32:
+  // a tile's)
+  for (size_t i = 0; i < rec.size(); i += 4) {
+    uint64_t longest = 0;
+    for (uint64_t s = rec[i]; s < rec[i + 1]; ++s)
+      if (off[s + 1] > off[s]) longest = std::max(longest, off[s + 1] - off[s]);
+    rec[i + 3] |= longest << 32;
+  }
   SegPlanRecords r;
   r.short_max = short_max;
   r.window = window;

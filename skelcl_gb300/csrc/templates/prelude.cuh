@@ -327,6 +327,10 @@ struct scl_vec_width {
                                 16 % S1 == 0 && 16 % S2 == 0) ? 16 / S : 1;
 };
 
+// Segment-plan windows: a record's elements, from its last word, whose upper half
+// holds the length of its longest vector.
+#define SCL_WIN_ELEMENTS(w) ((w) & 0xffffffffull)
+
 // Device-side status word: bit 0 = a bounded wait gave up.
 #define SCL_DEV_ERR_TIMEOUT 1u
 __device__ __forceinline__ void scl_raise(unsigned int* err, unsigned int bit) {

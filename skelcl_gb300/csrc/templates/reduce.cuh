@@ -276,15 +276,100 @@ scl_reduce_short(const scl_T* in, scl_T* out, const scl_u64* seg_off, scl_u64 n_
 // copies (element e0 + p at ts[p + shift]; bounded wait) while each thread
 // reads its first vector's offsets.  Then every vector is folded by a group of
 // G threads, G the power of two that gives the record's vectors all 256
-// threads: thread l of the group folds elements l, l + G, ... in order, a
-// warp's folds combine in a shuffle tree and a group's warps through shared
-// memory (a strided fold and a tree, as in the flat reduce; the operator is
-// taken to be commutative).  An empty vector
-// yields SCL_IDENTITY.  Folds in the element type.  10^6 vectors of 1..199
-// floats 0.143 -> 0.095 ms, 10^7 of 0..2 0.323 -> 0.049 ms, 3 * 10^5 of 200..399
-// 0.123 -> 0.079 ms against a thread per vector of up to 256 elements (about 40
+// threads: thread l of the group folds elements l, l + G, ... (in four chains
+// side by side where vectors are long or G is small: chains no longer than a
+// warp's, or a quarter of a vector of up to 256), a warp's folds combine in a
+// shuffle tree and a group's warps through shared memory (a strided fold and a
+// tree, as in the flat reduce; the operator is taken to be commutative).  A long
+// vector among so many that G < 8 is left to a warp: its few threads would hold
+// up the block, and their chains round more often (20,000 vectors of 4000 floats
+// beside 300 empty ones each 0.69 -> 0.08 ms).  An empty vector yields
+// SCL_IDENTITY.  Folds in the element type.  10^6 vectors of 1..199
+// floats 0.143 -> 0.082 ms, 10^7 of 0..2 0.323 -> 0.041 ms, 3 * 10^5 of 200..399
+// 0.123 -> 0.068 ms against a thread per vector of up to 256 elements (about 40
 // busy threads of a block's 256) and a warp per longer one.
 #define SCL_REDUCE_AHEAD 304
+// A vector is long from here on.  (Of single bytes a record holds four times as
+// many, and groups of few threads fold whole numbers as exactly as a warp: 32 %
+// faster for vectors of 200..399, 20 % slower for 500..1499.)
+constexpr bool kWinBytes = sizeof(scl_T) == 1;
+#define SCL_WIN_LONG (kWinBytes ? 512 : 256)
+// Elements first, first + step, ... below n (first < n) of v, in four chains
+// side by side.
+__device__ __forceinline__ scl_T scl_fold_chains(const scl_T* v, int first, int n, int step SCL_USER_PARAMS) {
+  scl_T acc = v[first];
+  int e = first + step;
+  if (e + 2 * step < n) {
+    scl_T c1 = v[e], c2 = v[e + step], c3 = v[e + 2 * step];
+    for (e += 3 * step; e + 3 * step < n; e += 4 * step) {
+      acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
+      c1 = SCL_FUNC(c1, v[e + step] SCL_OP_ARGS);
+      c2 = SCL_FUNC(c2, v[e + 2 * step] SCL_OP_ARGS);
+      c3 = SCL_FUNC(c3, v[e + 3 * step] SCL_OP_ARGS);
+    }
+    if (e < n) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
+    if (e + step < n) c1 = SCL_FUNC(c1, v[e + step] SCL_OP_ARGS);
+    if (e + 2 * step < n) c2 = SCL_FUNC(c2, v[e + 2 * step] SCL_OP_ARGS);
+    return SCL_FUNC(SCL_FUNC(acc, c1 SCL_OP_ARGS), SCL_FUNC(c2, c3 SCL_OP_ARGS) SCL_OP_ARGS);
+  }
+  for (; e < n; e += step) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
+  return acc;
+}
+
+// The folds of a record (elements e0 .. at ts) by groups of G = 2^glog < 32
+// threads in four chains each, and of the vectors too long for so few threads by
+// a warp each.  A function of its own: it keeps its registers off the other path.
+__device__ __noinline__ void scl_reduce_window_chains(scl_T* out, const scl_u64* seg_off, scl_u64 lo, scl_u64 top,
+                                                      scl_u64 e0, int len, const scl_T* ts, int glog,
+                                                      unsigned int longest SCL_USER_PARAMS) {
+  constexpr int B = 256;
+  const int G = 1 << glog, gl = (int)threadIdx.x & (G - 1), lane = threadIdx.x & 31;
+  const int most = kWinBytes ? SCL_WIN_LONG : (G >= 8 ? len : SCL_WIN_LONG);
+  for (scl_u64 base = lo; base < top; base += B >> glog) {
+    const scl_u64 sg = base + (threadIdx.x >> glog);
+    scl_u64 a = 0, b = 0;
+    if (sg < top) {
+      a = seg_off[sg];
+      b = seg_off[sg + 1];
+    }
+    const bool mine = sg < top && (b <= a || (a >= e0 && b <= e0 + (scl_u64)len));
+    const int nv = mine && b > a ? (int)(b - a) : 0;
+    scl_T acc = (scl_T)(SCL_IDENTITY);
+    if (gl < nv && nv <= most) acc = scl_fold_chains(ts + (int)(a - e0), gl, nv, G SCL_EXTRA_ARGS);
+    for (int off = G >> 1; off > 0; off >>= 1) {
+      // (threads of the group below nv hold a fold)
+      const scl_T o = scl_shfl_down(acc, off);
+      if (gl + off < G && gl + off < nv) acc = SCL_FUNC(acc, o SCL_OP_ARGS);
+    }
+    if (gl == 0 && mine && nv <= most) out[sg] = acc;
+  }
+  if ((int)longest <= most) return;  // (block-uniform)
+  // warp w takes the long ones of vectors lo + w, lo + w + 8, ... (an offset pair
+  // per lane)
+  for (scl_u64 g = lo + (threadIdx.x >> 5); g < top; g += B) {
+    const scl_u64 mine = g + (scl_u64)(B / 32 * lane);
+    scl_u64 a = 0, b = 0;
+    if (mine < top) {
+      a = seg_off[mine];
+      b = seg_off[mine + 1];
+    }
+    unsigned int todo =
+        __ballot_sync(0xffffffffu, b > a && b - a > (scl_u64)most && a >= e0 && b <= e0 + (scl_u64)len);
+    while (todo) {
+      const int k = __ffs((int)todo) - 1;
+      todo &= todo - 1u;
+      const int p = __shfl_sync(0xffffffffu, (int)(a - e0), k), n = __shfl_sync(0xffffffffu, (int)(b - a), k);
+      scl_T acc = scl_fold_chains(ts + p, lane, n, 32 SCL_EXTRA_ARGS);
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        const scl_T o = scl_shfl_down(acc, off);
+        if (lane + off < 32) acc = SCL_FUNC(acc, o SCL_OP_ARGS);
+      }
+      if (lane == 0) out[g + (scl_u64)(B / 32 * k)] = acc;
+    }
+  }
+}
+
 template <int WT>
 __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* out, const scl_u64* seg_off,
                                                       const scl_u64* win_rec, scl_u64 r, scl_u64 n_rec,
@@ -301,14 +386,16 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   const scl_u64 lo = win_rec[4 * r], top = win_rec[4 * r + 1], e0 = win_rec[4 * r + 2];
-  const scl_u64 ln = win_rec[4 * r + 3];
+  const scl_u64 w3 = win_rec[4 * r + 3], ln = SCL_WIN_ELEMENTS(w3);
   const int len = (int)(ln < (scl_u64)WT ? ln : (scl_u64)WT);  // (more only for bad offsets)
+  const unsigned int longest = (unsigned int)(w3 >> 32);
   // the record two per SM further on is asked into L2 ahead of its block, which
   // makes two dependent trips there (the record, then what it names): 10^6
   // vectors of 1..199 floats 95.4 -> 87.1 us (152 records ahead 89.1, 912 87.7)
   if (threadIdx.x == 32 && r + SCL_REDUCE_AHEAD < n_rec) {
     const scl_u64* nr = win_rec + 4 * (r + SCL_REDUCE_AHEAD);
-    const scl_u64 a0 = (scl_u64)in + nr[2] * sizeof(scl_T), l0 = nr[3] < (scl_u64)WT ? nr[3] : (scl_u64)WT;
+    const scl_u64 nl = SCL_WIN_ELEMENTS(nr[3]);
+    const scl_u64 a0 = (scl_u64)in + nr[2] * sizeof(scl_T), l0 = nl < (scl_u64)WT ? nl : (scl_u64)WT;
     scl_prefetch_l2(a0, a0 + l0 * sizeof(scl_T));
     scl_prefetch_l2((scl_u64)(seg_off + nr[0]), (scl_u64)(seg_off + nr[1] + 1));
   }
@@ -319,6 +406,7 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
   const int glog = 31 - __clz((int)share);
   const int G = 1 << glog, gl = (int)threadIdx.x & (G - 1);
   const scl_u64 step = (scl_u64)(B >> glog);
+  const bool chains = G < 32 && (longest > SCL_WIN_LONG || (G < 4 && longest >= 8));
   // this group's first vector's offsets are read while the copy lands
   scl_u64 sg = lo + (threadIdx.x >> glog);
   scl_u64 a = 0, b = 0;
@@ -336,6 +424,10 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
   }
   __syncthreads();
   if (!s_ok) return;
+  if (chains) {  // (block-uniform)
+    scl_reduce_window_chains(out, seg_off, lo, top, e0, len, ts + shift, glog, longest SCL_EXTRA_ARGS);
+    return;
+  }
   for (scl_u64 base = lo; base < top; base += step) {  // (block-uniform)
     // (outside the record only for offsets changed since the plan)
     const bool mine = sg < top && (b <= a || (a >= e0 && b <= e0 + (scl_u64)len));
@@ -350,8 +442,12 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
     scl_T acc = ident;
     if (gl < nv) {
       acc = v[gl];
+      if (G == 32) {  // (2048..4096 unsigned chars 32.2 -> 25.7 us, log-uniform floats 92 -> 88)
+        for (int e = gl + 32; e < nv; e += 32) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
+      } else {
 #pragma unroll 4
-      for (int e = gl + G; e < nv; e += G) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
+        for (int e = gl + G; e < nv; e += G) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
+      }
     }
     for (int off = G >= 32 ? 16 : G >> 1; off > 0; off >>= 1) {
       // (threads of the group below nv hold a fold)

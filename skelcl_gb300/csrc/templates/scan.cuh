@@ -755,11 +755,12 @@ __device__ __forceinline__ void scl_scan_window_run(const scl_T* in, scl_O* out,
   const scl_T ident = (scl_T)(SCL_IDENTITY);
   __shared__ W w;
   const scl_u64 lo = win_rec[4 * r], top = win_rec[4 * r + 1], e0 = win_rec[4 * r + 2];
-  const scl_u64 ln = win_rec[4 * r + 3];
+  const scl_u64 ln = SCL_WIN_ELEMENTS(win_rec[4 * r + 3]);
   const int len = (int)(ln < (scl_u64)TILE ? ln : (scl_u64)TILE);  // (more only for bad offsets)
   if (threadIdx.x == 32 && r + SCL_SCAN_AHEAD < n_rec) {  // (see SCL_SCAN_AHEAD)
     const scl_u64* nr = win_rec + 4 * (r + SCL_SCAN_AHEAD);
-    const scl_u64 a0 = (scl_u64)in + nr[2] * sizeof(scl_T), l0 = nr[3] < (scl_u64)TILE ? nr[3] : (scl_u64)TILE;
+    const scl_u64 nl = SCL_WIN_ELEMENTS(nr[3]);
+    const scl_u64 a0 = (scl_u64)in + nr[2] * sizeof(scl_T), l0 = nl < (scl_u64)TILE ? nl : (scl_u64)TILE;
     scl_prefetch_l2(a0, a0 + l0 * sizeof(scl_T));
     scl_prefetch_l2((scl_u64)(seg_off + nr[0]), (scl_u64)(seg_off + nr[1] + 1));
   }
