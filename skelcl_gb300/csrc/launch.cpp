@@ -291,6 +291,11 @@ int allpairs_tile(const scl_program* p, unsigned int M, unsigned int N) {
   return waves(2) >= 24 ? 3 : 2;
 }
 
+bool overlaps(const void* a, size_t abytes, const void* b, size_t bbytes) {
+  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
+  return a && b && x < y + bbytes && y < x + abytes;
+}
+
 uint32_t pick_block(const scl_tuning* t, uint32_t dflt) {
   uint32_t b = (t && t->workgroup) ? t->workgroup : dflt;
   if (b > 1024) b = 1024;
@@ -950,6 +955,9 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
   const int trans = ((sh->flags & SCL_SHAPE_TRANS_LEFT) ? 1 : 0) |
                     ((sh->flags & SCL_SHAPE_TRANS_RIGHT) ? 2 : 0);
   if (p->kind == SCL_KIND_ALLPAIRS) {
+    const size_t s0 = p->type_sizes[0], s1 = p->type_sizes[1], out_bytes = (size_t)M * N * p->type_sizes[2];
+    const bool in_place_a = overlaps(A, (size_t)M * K * s0, P, out_bytes),
+               in_place_b = overlaps(B, (size_t)K * N * s1, P, out_bytes);
     const uint32_t want = tu ? tu->variant : SCL_VARIANT_AUTO;
     if (p->tc_eligible && want != SCL_VARIANT_SIMT && extra_bytes == 0 &&
         allpairs_tc_supported(M, N, K, A, B, P)) {
@@ -961,9 +969,10 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
       const int wide = cols == 256u || (cols == 0u && wide_tiles >= sms) ? 1 : 0;
       // tuning.items == 2: two bf16 parts, 3 products; otherwise three parts, 6 products
       const int parts = (tu && tu->items == 2) ? 2 : 3;
-      // (the fused form takes no workspace)
+      // (the fused form takes no workspace, and reads the operands while other
+      // blocks store: an output in an operand's place needs the split before it)
       const bool plain = cols == 0 && parts == 3 && !(tu && (tu->items || tu->tile_w));
-      if (!wide && plain && allpairs_fused_wins(M, N, K, trans)) {
+      if (!wide && plain && !in_place_a && !in_place_b && allpairs_fused_wins(M, N, K, trans)) {
         p->last_variant = SCL_VARIANT_TC3XBF16;
         return allpairs_fused_launch((const float*)A, (const float*)B, (float*)P, M, N, K, trans,
                                      tu ? tu->workgroup : 0u, rt().stream, spin_of(tu), rt().dev_err);
@@ -996,20 +1005,23 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
       return fn ? SCL_OK : fail(SCL_ERR_LAUNCH, std::string("kernel ") + kAllPairsTiles[tile].kernel + " missing");
     };
     if (int st = get_kernel()) return st;
-    if (trans) {
+    const bool take_a = (trans & 1) || in_place_a, take_b = (trans & 2) || in_place_b;
+    if (take_a || take_b) {
       // CUDA-core kernel: transposed operands are first stored row-major in
-      // the program's workspace
-      const size_t s0 = p->type_sizes[0], s1 = p->type_sizes[1];
-      const size_t a_bytes = (trans & 1) ? ((size_t)M * K * s0 + 255) / 256 * 256 : 0;
-      const size_t b_bytes = (trans & 2) ? (size_t)K * N * s1 : 0;
+      // the program's workspace, and operands in whose place the output goes
+      // (its blocks share rows and columns) are copied there
+      const size_t a_bytes = take_a ? ((size_t)M * K * s0 + 255) / 256 * 256 : 0;
+      const size_t b_bytes = take_b ? (size_t)K * N * s1 : 0;
       if (int st = ensure_workspace(p, a_bytes + b_bytes)) return st;
       char* ws = static_cast<char*>(p->ws.ptr);
-      if (trans & 1) {
-        if (int st = transpose_launch(A, ws, K, M, s0, rt().stream)) return st;
+      if (take_a) {
+        if (!(trans & 1)) SCL_CUDA(cudaMemcpyAsync(ws, A, (size_t)M * K * s0, cudaMemcpyDeviceToDevice, rt().stream));
+        else if (int st = transpose_launch(A, ws, K, M, s0, rt().stream)) return st;
         A = ws;
       }
-      if (trans & 2) {
-        if (int st = transpose_launch(B, ws + a_bytes, N, K, s1, rt().stream)) return st;
+      if (take_b) {
+        if (!(trans & 2)) SCL_CUDA(cudaMemcpyAsync(ws + a_bytes, B, b_bytes, cudaMemcpyDeviceToDevice, rt().stream));
+        else if (int st = transpose_launch(B, ws + a_bytes, N, K, s1, rt().stream)) return st;
         B = ws + a_bytes;
       }
     }
@@ -1054,10 +1066,6 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
 // ---- exported launches: the autotuner in front of each skeleton -------------------
 namespace {
 
-bool overlaps(const void* a, size_t abytes, const void* b, size_t bbytes) {
-  const uintptr_t x = reinterpret_cast<uintptr_t>(a), y = reinterpret_cast<uintptr_t>(b);
-  return a && b && x < y + bbytes && y < x + abytes;
-}
 // extra arguments the user function cannot write through
 bool extras_are_values(const scl_program* p) {
   for (const Param& e : p->extra)
