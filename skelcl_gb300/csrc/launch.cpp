@@ -930,12 +930,16 @@ static int launch_mapoverlap_impl(scl_program* p, const scl_shape* sh, void* con
   CUfunction fn = hot_kernel(p, (uint32_t)PY, [&] { return kname(false); });
   if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname(false) + " missing");
   ArgPack pack;
-  pack.ptrs = {&in, &out, &rows, &cols};
+  int rows_out = 1;
+  pack.ptrs = {&in, &out, &rows, &cols, &rows_out};
   if (int st = pack_extra(p, fn, pack.ptrs.size(), (const unsigned char*)extra, extra_bytes, &pack))
     return st;
   p->last_variant = SCL_VARIANT_LDST;
-  // the tile's outputs pass through the window's place
-  return launch(fn, grid, block, std::max(win_bytes, (size_t)TH * 32 * obytes), pack);
+  // the tile's outputs pass through the window's place, if Local arguments leave
+  // room for outputs wider than the window
+  const size_t out_tile = (size_t)TH * 32 * obytes;
+  if (out_tile > win_bytes && (out_tile + 15) / 16 * 16 + pack.local_bytes > rt().smem_optin) rows_out = 0;
+  return launch(fn, grid, block, rows_out ? std::max(win_bytes, out_tile) : win_bytes, pack);
 }
 
 // ---- AllPairs -------------------------------------------------------------------
