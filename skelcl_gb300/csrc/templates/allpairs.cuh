@@ -52,6 +52,9 @@ __global__ void __launch_bounds__(BM / TM * (BN / TN), PER_SM)
 scl_allpairs_simt(const scl_L* A, const scl_Rt* B, scl_O* P, unsigned int M, unsigned int N,
                   unsigned int K, unsigned int tiles_n, int vec_b SCL_EXTRA_PARAMS) {
   SCL_EXTRA_SETUP
+  // operands are scalars (a zero of each is well-formed): vector types, which sit
+  // on the size of their components, would want other copies
+  static_assert(sizeof((scl_L)0) + sizeof((scl_Rt)0) > 0, "AllPairs: scalar operands");
   // wider values take tiles of at most four outputs per thread
   if constexpr (TM * TN > 4 && (sizeof(scl_L) > 4 || sizeof(scl_Rt) > 4 || sizeof(scl_O) > 4)) return;
   constexpr int BK = sizeof(scl_L) <= 4 && sizeof(scl_Rt) <= 4 ? BK4 : BK4 / 2;
