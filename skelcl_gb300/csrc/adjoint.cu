@@ -24,7 +24,7 @@ bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) ==
 
 // gx[i] = g (+ gx[i]); 16-byte accesses when gx is aligned
 template <typename T>
-__global__ void broadcast_kernel(const T* __restrict__ g, T* __restrict__ gx, uint64_t n, int acc,
+__global__ void broadcast_kernel(const T* g, T* gx, uint64_t n, int acc,
                                  int aligned) {
   constexpr int V = 16 / sizeof(T);
   dependency_wait();
@@ -52,7 +52,7 @@ __global__ void broadcast_kernel(const T* __restrict__ g, T* __restrict__ gx, ui
 
 // dst[i] += src[i]
 template <typename T>
-__global__ void accumulate_kernel(T* __restrict__ dst, const T* __restrict__ src, uint64_t n,
+__global__ void accumulate_kernel(T* dst, const T* src, uint64_t n,
                                   int aligned) {
   constexpr int V = 16 / sizeof(T);
   dependency_wait();
@@ -82,8 +82,8 @@ __global__ void accumulate_kernel(T* __restrict__ dst, const T* __restrict__ src
 
 // One edge pixel (y, x), any of them, by one warp: the lanes share the taps,
 // loop over the outside positions, and add their sums with shuffles.
-__device__ __forceinline__ void edge_pixel(const float* __restrict__ g, const float* __restrict__ w,
-                                           float* __restrict__ gin, int64_t rows, int64_t cols, int R, int64_t y,
+__device__ __forceinline__ void edge_pixel(const float* g, const float* w,
+                                           float* gin, int64_t rows, int64_t cols, int R, int64_t y,
                                            int64_t x) {
   const int lane = threadIdx.x & 31;
   const int64_t y0 = (y == 0) ? -R : y, y1 = (y == rows - 1) ? rows - 1 + R : y;
@@ -111,8 +111,8 @@ __device__ __forceinline__ void edge_pixel(const float* __restrict__ g, const fl
 }
 
 // A matrix of one row or one column: every pixel is an edge pixel.
-__global__ void line_edges_kernel(const float* __restrict__ g, const float* __restrict__ w,
-                                  float* __restrict__ gin, int64_t rows, int64_t cols, int R) {
+__global__ void line_edges_kernel(const float* g, const float* w,
+                                  float* gin, int64_t rows, int64_t cols, int R) {
   dependency_wait();
   const int64_t e = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   if (e >= rows * cols) return;  // whole warps leave together (blockDim is a multiple of 32)
@@ -132,7 +132,7 @@ __global__ void line_edges_kernel(const float* __restrict__ g, const float* __re
 // 7 us of a 629 us blur with its gradient, against a warp per pixel.
 constexpr int kEdgeThreads = 128;
 __global__ void __launch_bounds__(kEdgeThreads)
-stencil_edges_kernel(const float* __restrict__ g, const float* __restrict__ w, float* __restrict__ gin,
+stencil_edges_kernel(const float* g, const float* w, float* gin,
                      int64_t rows, int64_t cols, int R) {
   extern __shared__ float sums[];  // [line k][step along the edge]
   const int W = 2 * R + 1, side = blockIdx.y;

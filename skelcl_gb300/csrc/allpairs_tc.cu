@@ -327,7 +327,7 @@ __device__ __forceinline__ void store_sums(uint32_t base, uint32_t ranks, uint32
 template <int PARTS, int STAGES, int G, int BN_T, bool SPLIT = false>
 __global__ void __launch_bounds__(Shape<BN_T>::THREADS, 1)
 gemm_3xbf16_kernel(const __grid_constant__ CUtensorMap tmA, const __grid_constant__ CUtensorMap tmB,
-                   float* __restrict__ P, uint32_t M, uint32_t N, uint32_t Kp, uint32_t spin_limit,
+                   float* P, uint32_t M, uint32_t N, uint32_t Kp, uint32_t spin_limit,
                    unsigned int* err, uint32_t tiles_n, uint32_t group_m) {
   using SH = Shape<BN_T>;
   constexpr int BN = SH::BN, BK = SH::BK;

@@ -309,6 +309,9 @@ cudaError_t launch_overlapped(void (*kern)(KArgs...), dim3 grid, dim3 block, siz
   return launch_clustered(kern, 1u, grid, block, smem, stream, args...);
 }
 #ifdef __CUDACC__
+// (Parameters of such a kernel are not __restrict__: what it reads may change
+// until the wait ends, so its loads are neither invariant nor for the read-only
+// path.)
 __device__ __forceinline__ void dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
 

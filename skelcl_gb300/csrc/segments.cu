@@ -181,7 +181,7 @@ struct BroadcastChunk {
 };
 template <typename T>
 __global__ void __launch_bounds__(256)
-broadcast_segments_kernel(const T* __restrict__ g, T* __restrict__ gx, const uint64_t* __restrict__ off,
+broadcast_segments_kernel(const T* g, T* gx, const uint64_t* off,
                           uint64_t n_seg, uint64_t n_total, int acc, uint64_t run) {
   constexpr int WORDS = BroadcastChunk<T>::WORDS, CH = BroadcastChunk<T>::CH, V = 16 / sizeof(T);
   __shared__ unsigned int mask[WORDS];  // bit p: a segment starts at position p
@@ -342,7 +342,7 @@ broadcast_segments_kernel(const T* __restrict__ g, T* __restrict__ gx, const uin
 constexpr int kBroadcastWarp = 1024;
 template <typename T>
 __global__ void __launch_bounds__(256)
-broadcast_long_segments_kernel(const T* __restrict__ g, T* __restrict__ gx, const uint64_t* __restrict__ off,
+broadcast_long_segments_kernel(const T* g, T* gx, const uint64_t* off,
                           uint64_t n_seg, uint64_t n_total, int acc, int aligned) {
   constexpr int CH = kBroadcastWarp, V = 16 / sizeof(T);
   dependency_wait();
