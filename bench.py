@@ -596,11 +596,13 @@ def secondary(S, oracle, hbm_peak, args):
     res = {}
     rows_chk = np.arange(0, M, M // 16)
     ref = oracle.gemm_f64(A.reshape(M, K)[rows_chk], B.reshape(K, N))
-    # the tensor-core launches take 128 x 256 output tiles here (automatic
-    # choice); "_128col" repeats the 6-product one with 128 x 128 tiles
+    # "_default": what a launch without tuning takes (CTA pairs, six products);
+    # an explicit number of parts takes 128 x 256 output tiles of one CTA here,
+    # and "_128col" repeats the 6-product one with 128 x 128 tiles
     # (the tensor-core tiles are taken in groups of 16 tile rows; "_rowmajor"
     # repeats the 6-product launch in plain row-major tile order)
     for name, var, items, cols, group in (("fp32_simt", S.VARIANT_SIMT, 0, 0, 0),
+                                          ("tc_3xbf16_default", S.VARIANT_AUTO, 0, 0, 0),
                                           ("tc_3xbf16_6prod", S.VARIANT_TC3XBF16, 3, 0, 0),
                                           ("tc_3xbf16_6prod_rowmajor", S.VARIANT_TC3XBF16, 3, 0, 1),
                                           ("tc_3xbf16_6prod_128col", S.VARIANT_TC3XBF16, 3, 128, 0),
@@ -614,7 +616,7 @@ def secondary(S, oracle, hbm_peak, args):
                      # CUDA-core kernel: FP32 flops over the measured FP32 peak;
                      # tensor cores: the bf16 products' flops over the bf16 peak
                      "frac": round((2 * M * N * K if var == S.VARIANT_SIMT else
-                                    (6 if items == 3 else 3) * 2 * M * N * K) / ms / 1e9 /
+                                    (3 if items == 2 else 6) * 2 * M * N * K) / ms / 1e9 /
                                    (fp32_peak if var == S.VARIANT_SIMT else bf16_peak), 3),
                      "frac_of": "measured FP32 peak" if var == S.VARIANT_SIMT else
                                 "bf16 burst peak (MEASURED_PEAKS.json), bf16 products' flops",
@@ -635,6 +637,7 @@ def secondary(S, oracle, hbm_peak, args):
         prods = 6 if parts == 3 else 3
         res[name]["contraction_frac_of_bf16_peak"] = round(
             prods * 2 * M * N * K / (res[name]["ms"] - sms) / 1e9 / bf16_peak, 3)
+    res["speedup_default_over_simt"] = round(res["fp32_simt"]["ms"] / res["tc_3xbf16_default"]["ms"], 2)
     res["speedup_tc6_over_simt"] = round(res["fp32_simt"]["ms"] / res["tc_3xbf16_6prod"]["ms"], 2)
     res["speedup_tc3_over_simt"] = round(res["fp32_simt"]["ms"] / res["tc_3xbf16_3prod"]["ms"], 2)
     # backward of L = sum(G * P) as two AllPairs on transposed operands (tensor cores)
@@ -651,7 +654,7 @@ def secondary(S, oracle, hbm_peak, args):
     ref_b = oracle.gemm_f64(np.ascontiguousarray(A2[:, rb].T), hG)
     got_a = dgA.to_numpy().reshape(M, K)[ra].astype(np.float64)
     got_b = dgB.to_numpy().reshape(K, N)[rb].astype(np.float64)
-    res["backward_tc_3xbf16_6prod"] = {"fwd_ms": round(f_ms, 3), "dA_ms": round(a_ms, 3), "dB_ms": round(b_ms, 3),
+    res["backward_tc_3xbf16_default"] = {"fwd_ms": round(f_ms, 3), "dA_ms": round(a_ms, 3), "dB_ms": round(b_ms, 3),
                                        "fwd_plus_adjoint_over_fwd": round((f_ms + a_ms + b_ms) / f_ms, 3),
                                        "normwise_err_vs_fp64": {
                                            "dA": float(np.abs(got_a - ref_a).max() / np.abs(ref_a).max()),
