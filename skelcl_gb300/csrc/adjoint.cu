@@ -13,9 +13,8 @@ namespace {
 constexpr int kBlock = 256;
 
 int grid_for(uint64_t units) {
-  const int sm = rt().sm_count > 0 ? rt().sm_count : 148;
   uint64_t g = (units + kBlock - 1) / kBlock;
-  const uint64_t cap = (uint64_t)sm * 8;
+  const uint64_t cap = sm_count() * 8;
   if (g > cap) g = cap;
   return (int)(g < 1 ? 1 : g);
 }

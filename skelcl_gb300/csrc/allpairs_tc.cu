@@ -1217,7 +1217,7 @@ namespace {
 // us, 64 x 4096 x 512 (4 tiles) 72.9 -> 19.0 us; 256 x 256 x 256 with two
 // k-blocks each 11.2 -> 12.1 us.
 uint32_t split_of_k(uint64_t tiles, uint32_t Kp) {
-  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  const uint64_t sms = sm_count();
   uint32_t s = 1;
   while (s < 8 && tiles * s * 2 <= sms && Kp / 64 >= 8 * s) s *= 2;
   return s;
@@ -1322,7 +1322,7 @@ namespace {
 uint64_t resident_pairs() {
   int n = rt().pair_clusters;
   if (n == 0) {
-    const int half = (rt().sm_count > 0 ? rt().sm_count : 148) / 2;
+    const int half = (int)(sm_count() / 2);
     cudaLaunchAttribute attr{};
     attr.id = cudaLaunchAttributeClusterDimension;
     attr.val.clusterDim.x = 2;
@@ -1358,7 +1358,7 @@ bool pair_walks(uint64_t tiles, uint32_t Kp) { return Kp <= 2560 && tiles > resi
 // One wave of 128 x 128 tiles (or of clusters that share one), few k-blocks a
 // block: the operands split where they are used (gemm_fused_kernel).
 bool allpairs_fused_wins(uint32_t M, uint32_t N, uint32_t K, int trans) {
-  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  const uint64_t sms = sm_count();
   const uint64_t tiles = (uint64_t)((M + 127) / 128) * ((N + 127) / 128);
   const uint32_t all_k = (K + 63) / 64, split = split_of_k(tiles, tc::round_up(K, tc::KPAD));
   const bool strided = trans == 1;  // both operands
@@ -1417,7 +1417,7 @@ int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, u
 // 2000 x K x 2000 K = 64 15.3 / 11.9, 500 32.1 / 24.8, 2000 90.1 / 71.8, 4000
 // 166 / 132; 300 x 1000 x 8000 55.8 / 47.3.
 bool allpairs_pair_replaces_small(uint32_t M, uint32_t N) {
-  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u, pairs = resident_pairs();
+  const uint64_t sms = sm_count(), pairs = resident_pairs();
   const uint64_t small = (uint64_t)((M + 127) / 128) * ((N + 127) / 128);
   const uint64_t large = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
   return small > sms && large <= pairs;
@@ -1435,7 +1435,7 @@ bool allpairs_pair_replaces_small(uint32_t M, uint32_t N) {
 // and what is left is the pairs' start: 1 x 50 x 62000 20.7 / 23.7, 100 x 128 x
 // 39680 32.2 / 28.3.
 bool allpairs_pair_replaces_wide(uint32_t M, uint32_t N, uint32_t K) {
-  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u, pairs = resident_pairs();
+  const uint64_t sms = sm_count(), pairs = resident_pairs();
   const uint64_t wide = (uint64_t)((M + 127) / 128) * ((N + 255) / 256);
   const uint64_t large = (uint64_t)((M + 255) / 256) * ((N + 255) / 256);
   if ((K <= 128 && M >= 100) || (K <= 256 && 3 * large <= 2 * wide)) return true;

@@ -88,6 +88,8 @@ struct Runtime {
   Driver drv;
 };
 Runtime& rt();
+// The device's SMs (a GB300's while no device is open).
+inline uint64_t sm_count() { return rt().sm_count > 0 ? (uint64_t)rt().sm_count : 152u; }
 int require_init();
 
 // ---- CUDA-core AllPairs (templates/allpairs.cuh): its tiles, small to large ----

@@ -279,7 +279,7 @@ uint64_t reduce_grid(uint64_t units, uint32_t wg, uint64_t maxb) {
 // tiles 16 / 32 / 64: 97^2 10.6 / 35 / 132, 1400^2 409 / 417 / 513, 3000^2 1857
 // / 1876 / 1909; long 3000^2 478 / 314 / 317).
 int allpairs_tile(const scl_program* p, unsigned int M, unsigned int N) {
-  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  const uint64_t sms = sm_count();
   auto waves = [&](int tile) {
     const AllPairsTile& t = kAllPairsTiles[tile];
     return (((uint64_t)M + t.rows - 1) / t.rows * (((uint64_t)N + t.cols - 1) / t.cols) + sms - 1) / sms;
@@ -693,7 +693,7 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
   // 3.3, 100,000 5.6 -> 4.5, 620,000 6.5 -> 6.0, 800,000 6.5 and 6.5; doubles
   // 1000 6.0 -> 4.3, 300,000 8.4 -> 7.2, 400,000 8.7 and 8.9; unsigned char
   // 1000 8.6 -> 4.9)
-  const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+  const uint64_t sms = sm_count();
   if (staged && !(tu && (tu->items || tu->tile_w)) && sh->n_segments == 0 &&
       (n + 2048ull * V - 1) / (2048ull * V) <= sms / 2) R = 4;
   if (!staged && R == 6) R = 8;
@@ -969,7 +969,7 @@ extern "C" int scl_launch_allpairs(scl_program* p, const scl_shape* sh, void* co
       // 128 x 256 tiles still give every SM one
       const uint32_t cols = tu ? tu->tile_h : 0u;
       const uint64_t wide_tiles = (uint64_t)((M + 127u) / 128u) * ((N + 255u) / 256u);
-      const uint64_t sms = rt().sm_count > 0 ? (uint64_t)rt().sm_count : 148u;
+      const uint64_t sms = sm_count();
       const int wide = cols == 256u || (cols == 0u && wide_tiles >= sms) ? 1 : 0;
       // tuning.items == 2: two bf16 parts, 3 products; otherwise three parts, 6 products
       const int parts = (tu && tu->items == 2) ? 2 : 3;

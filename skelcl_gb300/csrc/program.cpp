@@ -313,7 +313,8 @@ int assemble(const scl_program_desc* d, scl_program* p, bool want_f64, Assembly*
     append_extra(ex, 0, &em, nullptr);
     p->extra = ex;
   }
-  s << "#define SCL_EXTRA_PARAMS " << em.params << "\n"
+  s << "#define SCL_SMS " << sm_count() << "\n"  // how far ahead memory is asked into L2
+    << "#define SCL_EXTRA_PARAMS " << em.params << "\n"
     << "#define SCL_USER_PARAMS " << em.user << "\n"
     << "#define SCL_EXTRA_SETUP SCL_GRID_DEPENDENCY_WAIT " << em.setup << "\n"
     << "#define SCL_EXTRA_ARGS " << em.args << "\n"

@@ -701,7 +701,7 @@ extern "C" int scl_adjoint_broadcast_segments(const void* g, void* gx, const uin
   }
   // one wave of blocks (6 per SM by their shared memory), each a run of chunks
   const uint64_t chunk = dtype == SCL_DTYPE_F32 ? BroadcastChunk<float>::CH : BroadcastChunk<double>::CH;
-  const uint64_t chunks = (n + chunk - 1) / chunk, wave = (uint64_t)rt().sm_count * 6;
+  const uint64_t chunks = (n + chunk - 1) / chunk, wave = sm_count() * 6;
   const uint64_t run = (chunks + wave - 1) / wave, blocks = (chunks + run - 1) / run;
   const dim3 grid((unsigned)blocks);
   SCL_CUDA(dtype == SCL_DTYPE_F32

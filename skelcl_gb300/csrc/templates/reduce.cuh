@@ -288,7 +288,7 @@ scl_reduce_short(const scl_T* in, scl_T* out, const scl_u64* seg_off, scl_u64 n_
 // floats 0.143 -> 0.082 ms, 10^7 of 0..2 0.323 -> 0.041 ms, 3 * 10^5 of 200..399
 // 0.123 -> 0.068 ms against a thread per vector of up to 256 elements (about 40
 // busy threads of a block's 256) and a warp per longer one.
-#define SCL_REDUCE_AHEAD 304
+#define SCL_REDUCE_AHEAD (2 * SCL_SMS)
 // A vector is long from here on.  (Of single bytes a record holds four times as
 // many, and groups of few threads fold whole numbers as exactly as a warp: 32 %
 // faster for vectors of 200..399, 20 % slower for 500..1499.)

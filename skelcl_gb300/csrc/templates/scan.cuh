@@ -55,14 +55,14 @@ typedef scl_T scl_O;
 #define SCL_EPILOGUE(v) (v)
 #endif
 
-// A staged tile asks for the tile this many after it to be brought into L2,
-// one per SM: its successors' copies then take an L2 round trip instead of one
-// through DRAM under load, and the look-back, which waits for the slowest of
-// its predecessors, ends sooner.  2^28 int 359.8 -> 332.3 us, 2^26 97.0 ->
+// A staged tile asks for the tile this many after it to be brought into L2, one
+// per SM (152 here): its successors' copies then take an L2 round trip instead
+// of one through DRAM under load, and the look-back, which waits for the slowest
+// of its predecessors, ends sooner.  2^28 int 359.8 -> 332.3 us, 2^26 97.0 ->
 // 89.6 (the transfers 317 and 79); 2^26 float 98.6 -> 94.5.  76 tiles ahead
 // 92.1 us at 2^26, 304 90.4, 912 (a whole wave of resident tiles) 104.1; asked
 // for before the tile's own copy, 94.5.
-#define SCL_SCAN_AHEAD 152
+#define SCL_SCAN_AHEAD SCL_SMS
 #define SCL_SCAN_B 256
 #define SCL_SCAN_W 8
 #define SCL_SLOT_STRIDE 16  // 64-bit words between tile slots (128 bytes)
