@@ -930,16 +930,20 @@ static int launch_mapoverlap_impl(scl_program* p, const scl_shape* sh, void* con
   CUfunction fn = hot_kernel(p, (uint32_t)PY, [&] { return kname(false); });
   if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + kname(false) + " missing");
   ArgPack pack;
-  int rows_out = 1;
-  pack.ptrs = {&in, &out, &rows, &cols, &rows_out};
+  pack.ptrs = {&in, &out, &rows, &cols};
   if (int st = pack_extra(p, fn, pack.ptrs.size(), (const unsigned char*)extra, extra_bytes, &pack))
     return st;
   p->last_variant = SCL_VARIANT_LDST;
   // the tile's outputs pass through the window's place, if Local arguments leave
   // room for outputs wider than the window
   const size_t out_tile = (size_t)TH * 32 * obytes;
-  if (out_tile > win_bytes && (out_tile + 15) / 16 * 16 + pack.local_bytes > rt().smem_optin) rows_out = 0;
-  return launch(fn, grid, block, rows_out ? std::max(win_bytes, out_tile) : win_bytes, pack);
+  if (out_tile > win_bytes && (out_tile + 15) / 16 * 16 + pack.local_bytes > rt().smem_optin) {
+    const std::string name = "scl_mapoverlap_ldst<" + std::to_string(PY) + ", 0>";
+    fn = hot_kernel(p, (uint32_t)PY | 1u << 17, [&] { return name; });
+    if (!fn) return fail(SCL_ERR_LAUNCH, "kernel " + name + " missing");
+    return launch(fn, grid, block, win_bytes, pack);
+  }
+  return launch(fn, grid, block, std::max(win_bytes, out_tile), pack);
 }
 
 // ---- AllPairs -------------------------------------------------------------------

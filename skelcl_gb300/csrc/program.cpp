@@ -372,11 +372,11 @@ int assemble(const scl_program_desc* d, scl_program* p, bool want_f64, Assembly*
       if (p->stencil_px == 4) {
         out->kernels = {"scl_mapoverlap_tma<4>"};
         out->lazy = {"scl_mapoverlap_ldst<4>", "scl_mapoverlap_tma<8>", "scl_mapoverlap_ldst<8>",
-                     "scl_mapoverlap_tma<16>"};
+                     "scl_mapoverlap_tma<16>", "scl_mapoverlap_ldst<4, 0>", "scl_mapoverlap_ldst<8, 0>"};
       } else {
         out->kernels = {"scl_mapoverlap_tma<8>"};
         out->lazy = {"scl_mapoverlap_ldst<4>", "scl_mapoverlap_tma<4>", "scl_mapoverlap_ldst<8>",
-                     "scl_mapoverlap_tma<16>"};
+                     "scl_mapoverlap_tma<16>", "scl_mapoverlap_ldst<4, 0>", "scl_mapoverlap_ldst<8, 0>"};
       }
       break;
     case SCL_KIND_ALLPAIRS:

@@ -173,11 +173,11 @@ __device__ __forceinline__ void scl_stage_registers(SCL_TYPE_0* win, const SCL_T
 // rows as well, not every SCL_PX-th element.  6000 x 5999 floats, clamped, R =
 // 1 108.4 -> 59.6 us, R = 5 280.5 -> 171.3 us against staging by a division per
 // element and stores SCL_PX elements apart (which remain where the outputs do
-// not fit beside Local arguments: without `rows_out`).
-template <int PY>
+// not fit beside Local arguments: ROWS_OUT 0, a kernel of its own since the
+// branch alone cost the others 3 to 13 %).
+template <int PY, int ROWS_OUT = 1>
 __global__ void __launch_bounds__(256)
-scl_mapoverlap_ldst(const SCL_TYPE_0* in, SCL_TYPE_1* out, scl_u64 rows, scl_u64 cols, int rows_out
-                    SCL_EXTRA_PARAMS) {
+scl_mapoverlap_ldst(const SCL_TYPE_0* in, SCL_TYPE_1* out, scl_u64 rows, scl_u64 cols SCL_EXTRA_PARAMS) {
   SCL_EXTRA_SETUP
   constexpr int TH = 8 * PY, WIN_H = TH + 2 * SCL_R;
   SCL_TYPE_0* win = reinterpret_cast<SCL_TYPE_0*>(scl_dyn_smem);  // WIN_H x SCL_WIN_W
@@ -199,7 +199,7 @@ scl_mapoverlap_ldst(const SCL_TYPE_0* in, SCL_TYPE_1* out, scl_u64 rows, scl_u64
   __syncthreads();
   SCL_TYPE_1 res[PY][SCL_PX];
   scl_compute_tile<PY>(win, res SCL_EXTRA_ARGS);
-  if (!rows_out) {
+  if constexpr (!ROWS_OUT) {
 #pragma unroll
     for (int p = 0; p < PY; ++p) {
       const scl_u64 y = y0 + ty * PY + p, x = x0 + (scl_u64)tx * SCL_PX;
