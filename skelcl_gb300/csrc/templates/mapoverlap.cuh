@@ -29,7 +29,7 @@ __device__ __forceinline__ scl_u64 scl_clampi(long long v, long long hi) {
 
 // Fill the positions of the window that lie outside the matrix: a warp takes a
 // row of the window at a time, all of it for a row outside, else the columns
-// left and right of the matrix.
+// left and right of the matrix, several loads in flight.
 template <int WIN_H>
 __device__ __forceinline__ void scl_patch_border(SCL_TYPE_0* win, long long x_org, long long y_org,
                                                  scl_u64 rows, scl_u64 cols) {
@@ -45,9 +45,10 @@ __device__ __forceinline__ void scl_patch_border(SCL_TYPE_0* win, long long x_or
     // (the clamped positions lie inside both the matrix and the window)
     const SCL_TYPE_0* from = win + (inside ? ly : (ly < top ? top : bottom - 1)) * SCL_WIN_W;
 #endif
-#pragma unroll 1
-    for (int lx = threadIdx.x; lx < SCL_WIN_W; lx += 32) {
-      if (inside && lx >= left && lx < right) continue;
+#pragma unroll
+    for (int c = 0; c < SCL_WIN_W; c += 32) {
+      const int lx = c + (int)threadIdx.x;
+      if (lx >= SCL_WIN_W || (inside && lx >= left && lx < right)) continue;
 #if SCL_PADDING == 1
       row[lx] = from[lx < left ? left : (lx >= right ? right - 1 : lx)];
 #else
@@ -87,41 +88,24 @@ __device__ __forceinline__ void scl_stage_element(SCL_TYPE_0* dst, const SCL_TYP
                : "memory");
 }
 
-// The window at (x_org, y_org), a warp per row, padded outside the matrix.
+// A window that lies inside the matrix, at (x_org, y_org), a warp per row.
 template <int WIN_H>
 __device__ __forceinline__ void scl_stage_window(SCL_TYPE_0* win, const SCL_TYPE_0* in, long long x_org,
-                                                 long long y_org, scl_u64 rows, scl_u64 cols, bool whole) {
+                                                 long long y_org, scl_u64 cols) {
   const int tx = threadIdx.x, ty = threadIdx.y;
-  if (whole) {
-    const SCL_TYPE_0* src = in + (scl_u64)(y_org + ty) * cols + (scl_u64)(x_org + tx);
-    SCL_TYPE_0* dst = win + ty * SCL_WIN_W + tx;
-    for (int ly = ty; ly < WIN_H; ly += 8, src += 8 * cols, dst += 8 * SCL_WIN_W) {
+  const SCL_TYPE_0* src = in + (scl_u64)(y_org + ty) * cols + (scl_u64)(x_org + tx);
+  SCL_TYPE_0* dst = win + ty * SCL_WIN_W + tx;
+  for (int ly = ty; ly < WIN_H; ly += 8, src += 8 * cols, dst += 8 * SCL_WIN_W) {
 #pragma unroll
-      for (int c = 0; c < SCL_WIN_W; c += 32)
-        if (c + 32 <= SCL_WIN_W || tx < SCL_WIN_W - c) scl_stage_element(dst + c, src + c);
-    }
-    return;
-  }
-  for (int ly = ty; ly < WIN_H; ly += 8) {
-    const long long gy = y_org + ly;
-    const bool row_in = gy >= 0 && gy < (long long)rows;
-    const SCL_TYPE_0* row = in + scl_clampi(gy, (long long)rows - 1) * cols;
-    for (int lx = tx; lx < SCL_WIN_W; lx += 32) {
-      const long long gx = x_org + lx;
-      const bool inside = row_in && gx >= 0 && gx < (long long)cols;
-#if SCL_PADDING == 1
-      (void)inside;
-      scl_stage_element(win + ly * SCL_WIN_W + lx, row + scl_clampi(gx, (long long)cols - 1));
-#else
-      if (inside) scl_stage_element(win + ly * SCL_WIN_W + lx, row + gx);
-      else win[ly * SCL_WIN_W + lx] = (SCL_TYPE_0)(SCL_NEUTRAL);
-#endif
-    }
+    for (int c = 0; c < SCL_WIN_W; c += 32)
+      if (c + 32 <= SCL_WIN_W || tx < SCL_WIN_W - c) scl_stage_element(dst + c, src + c);
   }
 }
 
-// The same through registers, for elements that cp.async does not take: the
-// loads of several rows are in flight before their stores.  Sobel on unsigned
+// The window through registers, padded outside the matrix, for elements that
+// cp.async does not take and for windows that reach outside (asynchronous copies
+// of the nearest elements: 20,000 x 33 floats, clamped, R = 1 14.0 us against 5.6):
+// the loads of several rows are in flight before their stores.  Sobel on unsigned
 // char, 1000 x 1001 7.0 -> 3.4 us, 3000 x 2999 15.5 -> 12.9, against loading and
 // storing an element at a time in border tiles and a row at a time elsewhere
 // (a window is a chain of 5 to 25 load latencies then).  Rows brought as words
@@ -188,8 +172,8 @@ scl_mapoverlap_ldst(const SCL_TYPE_0* in, SCL_TYPE_1* out, scl_u64 rows, scl_u64
   const bool whole = x_org >= 0 && y_org >= 0 && x_org + SCL_WIN_W <= (long long)cols && y_org + WIN_H <= (long long)rows;
   bool async = false;
   if constexpr (sized) {
-    async = (scl_u64)in % sizeof(SCL_TYPE_0) == 0;
-    if (async) scl_stage_window<WIN_H>(win, in, x_org, y_org, rows, cols, whole);
+    async = whole && (scl_u64)in % sizeof(SCL_TYPE_0) == 0;
+    if (async) scl_stage_window<WIN_H>(win, in, x_org, y_org, cols);
   }
   if (!async) {
     if (whole) scl_stage_registers<WIN_H, true>(win, in, x_org, y_org, rows, cols);
