@@ -98,6 +98,7 @@ __device__ __forceinline__ scl_pack<T, V * M> scl_load_lane(const T* p) {
     const scl_pack<T, V> q = scl_load<T, V>(p + m * V);
 #pragma unroll
     for (int e = 0; e < V; ++e) r.v[m * V + e] = q.v[e];
+  if constexpr (M == 1) return scl_load<T, V>(p);
   }
   return r;
 }
@@ -109,6 +110,10 @@ __device__ __forceinline__ void scl_store_lane(T* p, const scl_pack<T, V * M>& r
 #pragma unroll
     for (int e = 0; e < V; ++e) q.v[e] = r.v[m * V + e];
     scl_store<T, V>(p + m * V, q);
+  if constexpr (M == 1) {
+    scl_store<T, V>(p, r);
+    return;
+  }
   }
 }
 
