@@ -731,9 +731,13 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
     // and a record of short vectors fills 24 rows of the window scan, three
     // per warp (10^6 vectors of 1..199 floats 133 us; windows and segments of
     // half a tile, 17 rows, 154 us; segments of 3000 floats, now tiles, 333
-    // against 388 us)
-    if (int st = segplan_config(plan, tile, vg, ga, reverse ? 1 : 0, tile / 4, tile * 47 / 64,
-                                &pcfg)) return st;
+    // against 388 us).  A tile has half as many 8-byte elements, so half a tile
+    // of each there: as tiles of their own, 1025..2048 elements pay for a whole
+    // one (2 * 10^7 longs in vectors of 500..1499 128 -> 64 us, doubles 290 -> 150;
+    // longs in vectors of 1..199 59 -> 64)
+    const bool wide = tsz >= 8;
+    if (int st = segplan_config(plan, tile, vg, ga, reverse ? 1 : 0, wide ? tile / 2 : tile / 4,
+                                wide ? tile / 2 : tile * 47 / 64, &pcfg)) return st;
     tiles = pcfg->tiles;
   } else if (n_seg) {
     // an upper bound (the pre-pass has the count): tiles exist only for
@@ -810,11 +814,11 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
   if (plan) {
     // the blocks past the tiles take one window record of short segments
     // each; a record keeps its 16-byte phase in shared memory and is read in
-    // whole lane chunks, so it needs up to three vectors more than a tile
+    // whole lane chunks, so it needs up to a chunk more than a tile
     grid = tiles + pcfg->n_rec;
     if (grid == 0) return SCL_OK;  // (every vector is either a tile's or in a record)
     if (grid > 0x7fffffffull) return fail(SCL_ERR_ARG, "segmented scan: too many tiles");
-    smem += 48;
+    smem += 64;
   }
   if (prepass) {
     uint64_t* scratch = reinterpret_cast<uint64_t*>((char*)p->ws.ptr + total + seg_of + seg_ts);

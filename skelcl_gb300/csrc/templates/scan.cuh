@@ -89,31 +89,37 @@ constexpr bool kLocalPrefix = !scl_same<scl_C, scl_T>::value;
 // four-way bank conflicts): 2^25 doubles 344.5 -> 204.2 us (two vectors 243.7,
 // eight 260.3; floats with two 94.5 -> 102.8 at 2^26).
 constexpr int kLaneVectors = scl_same<scl_T, double>::value ? 4 : 1;
+// In a branch that folds: keeps the fold of doubles in the branch, which few
+// warps may take, where it would be made in any case and its result selected (2 *
+// 10^7 doubles in vectors of 1..199 156 -> 133 us).
+__device__ __forceinline__ void scl_costly_fold() {
+  if constexpr (kLaneVectors > 1) asm volatile("");
+}
 // A lane's vectors in shared memory.
 template <typename T, int V, int M>
 __device__ __forceinline__ scl_pack<T, V * M> scl_load_lane(const T* p) {
+  if constexpr (M == 1) return scl_load<T, V>(p);
   scl_pack<T, V * M> r;
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     const scl_pack<T, V> q = scl_load<T, V>(p + m * V);
 #pragma unroll
     for (int e = 0; e < V; ++e) r.v[m * V + e] = q.v[e];
-  if constexpr (M == 1) return scl_load<T, V>(p);
   }
   return r;
 }
 template <typename T, int V, int M>
 __device__ __forceinline__ void scl_store_lane(T* p, const scl_pack<T, V * M>& r) {
+  if constexpr (M == 1) {
+    scl_store<T, V>(p, r);
+    return;
+  }
 #pragma unroll
   for (int m = 0; m < M; ++m) {
     scl_pack<T, V> q;
 #pragma unroll
     for (int e = 0; e < V; ++e) q.v[e] = r.v[m * V + e];
     scl_store<T, V>(p + m * V, q);
-  if constexpr (M == 1) {
-    scl_store<T, V>(p, r);
-    return;
-  }
   }
 }
 
@@ -509,8 +515,9 @@ __device__ __forceinline__ void scl_scan_short_run(const scl_T* in, scl_O* out, 
 // ---- windows of short segments (planned segmented Scan) --------------------
 // One block takes one window record r of the plan, {first vector, end vector,
 // first element, elements}: consecutive vectors of at most a quarter of a
-// tile that start in one window of 47/64 of a tile, all but the last ending
-// inside it, so that the record fits in one staged tile.
+// tile that start in one window of 47/64 of a tile (half a tile of each for
+// elements of 8 bytes and more), all but the last ending inside it, so that the
+// record fits in one staged tile.
 // The record's elements come into shared memory by bulk asynchronous copies
 // (element e0 + p at ts[p + shift]; bounded wait) while the threads mark, in
 // a bit mask, where the vectors start in logical order (their last elements
@@ -530,7 +537,9 @@ __device__ __forceinline__ void scl_scan_short_run(const scl_T* in, scl_O* out, 
 template <typename T, int TILE>
 struct scl_win {
   static constexpr int V = scl_vec_width<sizeof(T)>::value;
-  static constexpr int E = 2 * V;           // elements per lane and row
+  // elements per lane and row (more of doubles, as in a staged tile: 2 * 10^7 in
+  // vectors of 1..199 170 -> 150 us)
+  static constexpr int E = (kLaneVectors > 1 ? 4 : 2) * V;
   static constexpr int ROW = 32 * E;
   static constexpr int ROWS = TILE / ROW + 1;  // (a record keeps its 16-byte phase)
   unsigned int mask[ROWS * ROW / 32];       // bit p: a vector starts at ts[p]
@@ -618,13 +627,13 @@ __device__ __forceinline__ void scl_win_scan(T* ts, unsigned int P, const T& ide
     T x[E];  // in logical order
     unsigned int hd = 0;
     if (j < chunks) {
-      const scl_pack<T, V> p0 = scl_load<T, V>(ts + pos);
-      const scl_pack<T, V> p1 = scl_load<T, V>(ts + pos + V);
+      scl_pack<T, V> p[E / V];
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        x[REV ? E - 1 - e : e] = p0.v[e];
-        x[REV ? V - 1 - e : V + e] = p1.v[e];
-      }
+      for (int c = 0; c < E / V; ++c) p[c] = scl_load<T, V>(ts + pos + c * V);
+#pragma unroll
+      for (int e = 0; e < V; ++e)
+#pragma unroll
+        for (int c = 0; c < E / V; ++c) x[REV ? E - 1 - c * V - e : c * V + e] = p[c].v[e];
       hd = w.mask[pos >> 5] >> (pos & 31u);
       if (REV) hd = __brev(hd << (32 - E));
       else if (E < 32) hd &= (1u << (E & 31)) - 1u;
@@ -642,17 +651,19 @@ __device__ __forceinline__ void scl_win_scan(T* ts, unsigned int P, const T& ide
     if (lane != 0) {
 #pragma unroll
       for (int e = 0; e < E; ++e)
-        if (e < first) x[e] = SCL_FUNC(cin, x[e] SCL_OP_ARGS);
+        if (e < first) {
+          scl_costly_fold();
+          x[e] = SCL_FUNC(cin, x[e] SCL_OP_ARGS);
+        }
     }
     if (j < chunks) {
-      scl_pack<T, V> p0, p1;
+      scl_pack<T, V> p[E / V];
 #pragma unroll
-      for (int e = 0; e < V; ++e) {
-        p0.v[e] = x[REV ? E - 1 - e : e];
-        p1.v[e] = x[REV ? V - 1 - e : V + e];
-      }
-      scl_store<T, V>(ts + pos, p0);
-      scl_store<T, V>(ts + pos + V, p1);
+      for (int e = 0; e < V; ++e)
+#pragma unroll
+        for (int c = 0; c < E / V; ++c) p[c].v[e] = x[REV ? E - 1 - c * V - e : c * V + e];
+#pragma unroll
+      for (int c = 0; c < E / V; ++c) scl_store<T, V>(ts + pos + c * V, p[c]);
     }
     const int fl = starts ? __ffs((int)starts) - 1 : 0;
     const int fe = __shfl_sync(0xffffffffu, first, fl);
@@ -688,7 +699,10 @@ __device__ __forceinline__ T scl_win_at(const T* ts, unsigned int p, unsigned in
   const unsigned int l = REV ? (P + W::E - 1) / W::E * W::E - 1 - p : p;
   const unsigned int row = l / W::ROW;
   T v = ts[p];
-  if ((int)(l % W::ROW) < w.head[row]) v = SCL_FUNC(w.carry[row], v SCL_OP_ARGS);
+  if ((int)(l % W::ROW) < w.head[row]) {
+    scl_costly_fold();
+    v = SCL_FUNC(w.carry[row], v SCL_OP_ARGS);
+  }
   return v;
 }
 
@@ -715,7 +729,10 @@ __device__ __forceinline__ void scl_scan_window_store(scl_T* ts, scl_u64 e0, int
       const scl_T c = w.carry[row];
 #pragma unroll
       for (int e = 0; e < V; ++e)
-        if (REV ? d > -e : d > e) v.v[e] = SCL_FUNC(c, v.v[e] SCL_OP_ARGS);
+        if (REV ? d > -e : d > e) {
+          scl_costly_fold();
+          v.v[e] = SCL_FUNC(c, v.v[e] SCL_OP_ARGS);
+        }
     }
     scl_pack<scl_O, V> m;
     if (inclusive) {
