@@ -692,10 +692,13 @@ static int launch_scan_impl(scl_program* p, const scl_shape* sh, void* const* bu
   // tile's own steps are what such a call waits for (us, floats 1000 4.2 ->
   // 3.3, 100,000 5.6 -> 4.5, 620,000 6.5 -> 6.0, 800,000 6.5 and 6.5; doubles
   // 1000 6.0 -> 4.3, 300,000 8.4 -> 7.2, 400,000 8.7 and 8.9; unsigned char
-  // 1000 8.6 -> 4.9)
+  // 1000 8.6 -> 4.9).  64-bit whole numbers, whose look-back is the longer part,
+  // gain up to one to four SMs (65,536 5.6 -> 4.8, 150,000 6.2 -> 5.9, 200,000 6.4
+  // and 6.3, 250,000 6.4 -> 7.5)
   const uint64_t sms = sm_count();
   if (staged && !(tu && (tu->items || tu->tile_w)) && sh->n_segments == 0 &&
-      (n + 2048ull * V - 1) / (2048ull * V) <= sms / 2) R = 4;
+      (n + 2048ull * V - 1) / (2048ull * V) <= sms / (tsz > 4 && p->type_names[0] != "double" ? 4 : 2))
+    R = 4;
   if (!staged && R == 6) R = 8;
   size_t smem = staged ? (size_t)R * 256 * V * tsz : 0;
   if (staged && smem + 2048 > rt().smem_optin) {
