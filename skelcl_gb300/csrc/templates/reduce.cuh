@@ -278,20 +278,25 @@ scl_reduce_short(const scl_T* in, scl_T* out, const scl_u64* seg_off, scl_u64 n_
 // G threads, G the power of two that gives the record's vectors all 256
 // threads: thread l of the group folds elements l, l + G, ... (in four chains
 // side by side where vectors are long or G is small: chains no longer than a
-// warp's, or a quarter of a vector of up to 256), a warp's folds combine in a
-// shuffle tree and a group's warps through shared memory (a strided fold and a
-// tree, as in the flat reduce; the operator is taken to be commutative).  A long
-// vector among so many that G < 8 is left to a warp: its few threads would hold
-// up the block, and their chains round more often (20,000 vectors of 4000 floats
-// beside 300 empty ones each 0.69 -> 0.08 ms).  An empty vector yields
-// SCL_IDENTITY.  Folds in the element type.  10^6 vectors of 1..199
-// floats 0.143 -> 0.082 ms, 10^7 of 0..2 0.323 -> 0.041 ms, 3 * 10^5 of 200..399
-// 0.123 -> 0.068 ms against a thread per vector of up to 256 elements (about 40
-// busy threads of a block's 256) and a warp per longer one.
+// warp's, or a quarter of a vector of up to 256), the group's folds combine in a
+// shuffle tree (a strided fold and a tree, as in the flat reduce; the operator is
+// taken to be commutative).  A long vector among so many that G < 8 is left to a
+// warp: its few threads would hold up the block, and their chains round more
+// often (20,000 vectors of 4000 floats beside 300 empty ones each 0.69 -> 0.08
+// ms).  An empty vector yields SCL_IDENTITY.  Folds in the element type.  10^6
+// vectors of 1..199 floats 0.143 -> 0.081 ms, 10^7 of 0..2 0.323 -> 0.041 ms,
+// 3.3 * 10^5 of 200..399 0.134 -> 0.075 ms against a thread per vector of up to
+// 256 elements (about 40 busy threads of a block's 256) and a warp per longer one.
+// A warp takes each vector of a record that has at most eight (groups of two and
+// more warps waited for one another: 10^5 vectors of 500..1499 floats 75.6 -> 64.7
+// us, of doubles 69 -> 58 a fifth of it), and of one of up to 32 whose vectors
+// are long (450 elements on average) or uneven (the longest over three times the
+// average: 40,000 log-uniform of 1..4096 floats 20.4 -> 15.5 us, of shorts 18.8 ->
+// 11.8; even ones of 200..399 floats 14.6 by groups, 15.3 by warps).
 #define SCL_REDUCE_AHEAD (2 * SCL_SMS)
-// A vector is long from here on.  (Of single bytes a record holds four times as
-// many, and groups of few threads fold whole numbers as exactly as a warp: 32 %
-// faster for vectors of 200..399, 20 % slower for 500..1499.)
+// A vector among many is long from here on.  (Of single bytes a record holds four
+// times as many, and groups of few threads fold whole numbers as exactly as a
+// warp: 32 % faster for vectors of 200..399.)
 constexpr bool kWinBytes = sizeof(scl_T) == 1;
 #define SCL_WIN_LONG (kWinBytes ? 512 : 256)
 // Elements first, first + step, ... below n (first < n) of v, in four chains
@@ -370,7 +375,8 @@ __device__ __noinline__ void scl_reduce_window_chains(scl_T* out, const scl_u64*
   }
 }
 
-template <int WT>
+// (CHAINS: a warp's fold of a vector in four chains too.)
+template <int WT, bool CHAINS>
 __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* out, const scl_u64* seg_off,
                                                       const scl_u64* win_rec, scl_u64 r, scl_u64 n_rec,
                                                       scl_T* ts, unsigned int spin_limit,
@@ -379,7 +385,6 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
   const scl_T ident = (scl_T)(SCL_IDENTITY);
   __shared__ __align__(8) unsigned long long bar;
   __shared__ int s_ok;
-  __shared__ scl_T s_part[B / 32];
   const unsigned int bar_s = (unsigned int)__cvta_generic_to_shared(&bar);
   if (threadIdx.x == 0) {
     asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" :: "r"(bar_s));
@@ -406,9 +411,11 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
   const int glog = 31 - __clz((int)share);
   const int G = 1 << glog, gl = (int)threadIdx.x & (G - 1);
   const scl_u64 step = (scl_u64)(B >> glog);
-  const bool chains = G < 32 && (longest > SCL_WIN_LONG || (G < 4 && longest >= 8));
+  const unsigned int few = nvec < B ? (unsigned int)nvec : B;
+  const bool warps = G >= 32 || (G >= 8 && ((unsigned int)len >= 450u * few || longest * few > 3u * (unsigned int)len));
+  const bool chains = longest > SCL_WIN_LONG || (G < 4 && longest >= 8);
   // this group's first vector's offsets are read while the copy lands
-  scl_u64 sg = lo + (threadIdx.x >> glog);
+  scl_u64 sg = lo + (threadIdx.x >> (warps ? 5 : glog));
   scl_u64 a = 0, b = 0;
   if (sg < top) {
     a = seg_off[sg];
@@ -424,6 +431,35 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
   }
   __syncthreads();
   if (!s_ok) return;
+  if (warps) {  // (block-uniform; sg, a, b are the warp's first vector)
+    const int lane = threadIdx.x & 31;
+    for (; sg < top; sg += B / 32) {
+      // (outside the record only for offsets changed since the plan)
+      const bool mine = b <= a || (a >= e0 && b <= e0 + (scl_u64)len);
+      const int nv = mine && b > a ? (int)(b - a) : 0;
+      const scl_T* v = ts + (nv ? (int)(a - e0) + shift : 0);
+      const scl_u64 cur = sg;
+      if (sg + B / 32 < top) {
+        a = seg_off[sg + B / 32];
+        b = seg_off[sg + B / 32 + 1];
+      }
+      scl_T acc = ident;
+      if constexpr (CHAINS) {
+        if (lane < nv) acc = scl_fold_chains(v, lane, nv, 32 SCL_EXTRA_ARGS);
+      } else if (lane < nv) {
+        acc = v[lane];
+        for (int e = lane + 32; e < nv; e += 32) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
+      }
+#pragma unroll
+      for (int off = 16; off > 0; off >>= 1) {
+        // (lanes below nv hold a fold)
+        const scl_T o = scl_shfl_down(acc, off);
+        if (lane + off < 32 && lane + off < nv) acc = SCL_FUNC(acc, o SCL_OP_ARGS);
+      }
+      if (lane == 0 && mine) out[cur] = acc;
+    }
+    return;
+  }
   if (chains) {  // (block-uniform)
     scl_reduce_window_chains(out, seg_off, lo, top, e0, len, ts + shift, glog, longest SCL_EXTRA_ARGS);
     return;
@@ -442,28 +478,26 @@ __device__ __forceinline__ void scl_reduce_window_run(const scl_T* in, scl_T* ou
     scl_T acc = ident;
     if (gl < nv) {
       acc = v[gl];
-      if (G == 32) {  // (2048..4096 unsigned chars 32.2 -> 25.7 us, log-uniform floats 92 -> 88)
-        for (int e = gl + 32; e < nv; e += 32) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
-      } else {
 #pragma unroll 4
-        for (int e = gl + G; e < nv; e += G) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
-      }
+      for (int e = gl + G; e < nv; e += G) acc = SCL_FUNC(acc, v[e] SCL_OP_ARGS);
     }
-    for (int off = G >= 32 ? 16 : G >> 1; off > 0; off >>= 1) {
+    for (int off = G >> 1; off > 0; off >>= 1) {
       // (threads of the group below nv hold a fold)
       const scl_T o = scl_shfl_down(acc, off);
-      if ((gl & 31) + off < (G < 32 ? G : 32) && gl + off < nv) acc = SCL_FUNC(acc, o SCL_OP_ARGS);
-    }
-    if (G > 32) {  // (block-uniform)
-      const int warp = threadIdx.x >> 5;
-      if ((threadIdx.x & 31) == 0) s_part[warp] = acc;
-      __syncthreads();
-      if (gl == 0)
-        for (int k = 1; k < (G >> 5) && k * 32 < nv; ++k) acc = SCL_FUNC(acc, s_part[warp + k] SCL_OP_ARGS);
-      __syncthreads();
+      if (gl + off < G && gl + off < nv) acc = SCL_FUNC(acc, o SCL_OP_ARGS);
     }
     if (gl == 0 && mine) out[cur] = acc;
   }
+}
+
+// A function of its own beside the tiles, whose registers and order of loads its
+// code would change (250 log-uniform vectors of 64..2^20 floats 12.3 us, inlined
+// 13.8, with CHAINS 15.7).
+template <int WT>
+__device__ __noinline__ void scl_reduce_window_apart(const scl_T* in, scl_T* out, const scl_u64* seg_off,
+                                                     const scl_u64* win_rec, scl_u64 r, scl_u64 n_rec, scl_T* ts,
+                                                     unsigned int spin_limit, unsigned int* err SCL_USER_PARAMS) {
+  scl_reduce_window_run<WT, false>(in, out, seg_off, win_rec, r, n_rec, ts, spin_limit, err SCL_EXTRA_ARGS);
 }
 
 // Segmented Reduce (no counterpart in the reference): out[s] = the fold of
@@ -493,8 +527,13 @@ scl_reduce_seg(const scl_T* in, scl_T* out, const scl_u64* seg_off,
   if constexpr (MERGED != 0) {
     if (blockIdx.x >= nt) {  // (block-uniform: the whole block takes the window role)
       constexpr int WT = 8 * 256 * scl_vec_width<sizeof(scl_T)>::value;  // 32 KB of elements
-      scl_reduce_window_run<WT>(in, out, seg_off, win_rec, blockIdx.x - nt, gridDim.x - nt,
-                                reinterpret_cast<scl_T*>(scl_dyn_smem), spin_limit, err SCL_EXTRA_ARGS);
+      scl_T* ts = reinterpret_cast<scl_T*>(scl_dyn_smem);
+      if constexpr (PER_SM != 0)
+        scl_reduce_window_run<WT, true>(in, out, seg_off, win_rec, blockIdx.x - nt, gridDim.x - nt, ts, spin_limit,
+                                        err SCL_EXTRA_ARGS);
+      else
+        scl_reduce_window_apart<WT>(in, out, seg_off, win_rec, blockIdx.x - nt, gridDim.x - nt, ts, spin_limit,
+                                    err SCL_EXTRA_ARGS);
       return;
     }
   }

@@ -40,3 +40,23 @@ def test_wide_scan_windows(scl, dtype, pattern, shift, items):
                     tuning=S.Tuning(items=items))
         assert np.array_equal(out.to_numpy()[shift:], want.astype(dtype)), flags
     plan.release()
+
+
+@pytest.mark.parametrize("dtype", [np.float32, np.uint8, np.int16, np.float64])
+@pytest.mark.parametrize("pattern", [[4096, 0, 4095], [512] * 8, [455] * 9, [500] * 7 + [0, 33],  # a warp each
+                                     [4000] + [3] * 20, [900] + [31, 32, 33] * 6,                 # uneven
+                                     [300] * 15, [128] * 31 + [130], [4000] + [1] * 31])          # groups
+@pytest.mark.parametrize("shift", [0, 1])
+def test_reduce_records(scl, dtype, pattern, shift):
+    off = segments(pattern, 60_000, 7)
+    n, o = int(off[-1]), off.astype(np.int64)
+    x = np.random.default_rng(8).integers(0, 9, n + shift).astype(dtype)
+    c = np.concatenate([[0], np.cumsum(x[shift:].astype(np.int64))])
+    want = (c[o[1:]] - c[o[:-1]]).astype(dtype)
+    t = S.CL_TYPE[np.dtype(dtype)]
+    red = S.Program(S.KIND_REDUCE, f"{t} func({t} x, {t} y){{ return x + y; }}", [t], identity="0")
+    base, out = S.DeviceArray.from_numpy(x), S.DeviceArray(len(want), dtype)
+    plan = S.SegPlan(S.DeviceArray.from_numpy(off), n)
+    red.launch([base.view(shift, n), out], n=n, segments=plan)
+    assert np.array_equal(out.to_numpy(), want)
+    plan.release()
