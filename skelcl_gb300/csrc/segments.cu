@@ -685,8 +685,11 @@ extern "C" int scl_adjoint_broadcast_segments(const void* g, void* gx, const uin
   // a warp per 1024 elements walks long segments at the speed of plain stores,
   // but spends 40 instructions an element on short ones: 10^8 floats in
   // vectors of 100 on average 123 us against 81 for the chunks, of 300 64
-  // against 70, of 1500 62 against 70
-  const bool long_segments = n / n_segments >= 200;
+  // against 70, of 1500 62 against 70.  Of doubles, whose chunks have half as many
+  // elements, plain stores win from 48 on (10^7 in vectors of 32 on average 37
+  // against 27, of 50 26.3 / 26.9, of 100 15.7 / 26.4), added ones later (of 50 59
+  // against 32, of 150 37 / 31)
+  const bool long_segments = n / n_segments >= (dtype == SCL_DTYPE_F64 && !acc ? 48u : 200u);
   if (long_segments) {
     const uint64_t blocks = (n + 8 * kBroadcastWarp - 1) / (8 * kBroadcastWarp);
     if (blocks > 0x7fffffffull) return fail(SCL_ERR_ARG, "segmented broadcast: vector too large");

@@ -60,3 +60,21 @@ def test_reduce_records(scl, dtype, pattern, shift):
     red.launch([base.view(shift, n), out], n=n, segments=plan)
     assert np.array_equal(out.to_numpy(), want)
     plan.release()
+
+
+@pytest.mark.parametrize("dtype,code", [(np.float32, S.DTYPE_F32), (np.float64, S.DTYPE_F64)])
+@pytest.mark.parametrize("mean", [47, 48, 199, 200])
+@pytest.mark.parametrize("shift", [0, 1])
+def test_broadcast_forms(scl, dtype, code, mean, shift):
+    lens = np.random.default_rng(9).permutation(np.tile([0, 1, mean - 1, mean, mean + 1, 2 * mean - 1, 2 * mean], 300))
+    off = np.concatenate([[0], np.cumsum(lens)]).astype(np.uint64)
+    n = int(off[-1])
+    assert n // len(lens) == mean
+    rng = np.random.default_rng(10)
+    g, x = rng.integers(-99, 100, len(lens)).astype(dtype), rng.integers(-99, 100, n + shift).astype(dtype)
+    dg, doff = S.DeviceArray.from_numpy(g), S.DeviceArray.from_numpy(off)
+    for acc in (0, 1):
+        gx = S.DeviceArray.from_numpy(x)
+        S.check(S.lib().scl_adjoint_broadcast_segments(dg.ptr, gx.view(shift, n).ptr, doff.ptr, len(lens), n, code, acc))
+        assert np.array_equal(gx.to_numpy()[shift:], np.repeat(g, lens) + (x[shift:] if acc else 0)), acc
+        assert np.array_equal(gx.to_numpy()[:shift], x[:shift])
