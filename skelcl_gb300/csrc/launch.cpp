@@ -278,6 +278,11 @@ uint64_t reduce_grid(uint64_t units, uint32_t wg, uint64_t maxb) {
 // instructions) is what counts, and an even share of it (double x * y, K = 128,
 // tiles 16 / 32 / 64: 97^2 10.6 / 35 / 132, 1400^2 409 / 417 / 513, 3000^2 1857
 // / 1876 / 1909; long 3000^2 478 / 314 / 317).
+// Where the large tile takes half as many waves, whole numbers take it: its 8 x 8
+// outputs share their loads better and a multiplication is not its bound (int x *
+// y, K = 128, tiles 64 / 64 x 128: 1400^2 22.5 / 21.0, 1600^2 27.4 / 30.3, 1800^2
+// 32.9 / 31.0, 2400^2 52.3 / 47.2; float |x - y| 23.8 / 24.3, 29.6 / 33.6, 35.4 /
+// 34.5, 57.1 / 57.3).
 int allpairs_tile(const scl_program* p, unsigned int M, unsigned int N) {
   const uint64_t sms = sm_count();
   auto waves = [&](int tile) {
@@ -288,6 +293,7 @@ int allpairs_tile(const scl_program* p, unsigned int M, unsigned int N) {
   if (waves(0) <= 2) return 0;
   if (waves(1) <= 3 || l > 4 || r > 4 || o > 4) return 1;
   if (l < 4 || r < 4) return 10 * waves(2) >= 17 * waves(3) ? 3 : 2;
+  if (waves(2) >= 4 && 10 * waves(2) >= 18 * waves(3) && p->type_names[2] != "float") return 3;
   return waves(2) >= 24 ? 3 : 2;
 }
 
