@@ -326,10 +326,11 @@ int scl_launch_scan_noalloc(scl_program* prog, const scl_shape* shape,
  *      window of short segments (up to 2048 four-byte elements for a Scan,
  *      which scans a window's segments together; up to 4096 for a Reduce,
  *      which gives each segment a share of the block's threads).  The plan
- *      keeps, per tile
- *      shape, which tiles belong to which segment (and each tile's segment)
- *      and the windows; the first launch with a tile shape builds them (four
- *      small launches and a read-back of the offsets), so make it before
+ *      keeps, per tile shape, which tiles belong to which segment (and each
+ *      tile's segment) and the windows with their longest segments, and in
+ *      host memory the offsets (8 bytes a segment), read back once; the first
+ *      launch with a tile shape builds them (four small launches and that
+ *      read-back), so make it before
  *      capturing a graph.  Later changes to the caller's offsets are not
  *      seen: release the plan and create another. */
 int scl_segplan_create(const uint64_t* seg_offsets, uint64_t n_segments, uint64_t n,
