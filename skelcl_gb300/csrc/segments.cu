@@ -484,28 +484,40 @@ void free_plan(SegPlan* p) {
 // record spans less than window + short_max elements.  Records whose segments
 // are all empty stay (the Reduce writes their identities); windows that own
 // no segment get none.  `off` holds n_seg + 1 clamped offsets.
-void segplan_window_records(const uint64_t* off, uint64_t n_seg, uint64_t short_max, uint64_t window,
-                            std::vector<uint64_t>* rec) {
-  rec->clear();
+// each(first, end, first element, elements, longest segment's length).
+template <typename Each>
+static void walk_window_records(const uint64_t* off, uint64_t n_seg, uint64_t short_max, uint64_t window,
+                                const Each& each) {
   for (uint64_t sg = 0; sg < n_seg;) {
     const uint64_t e0 = off[sg];
     uint64_t lo = e0, hi = off[sg + 1];  // the segment at hand
-    if (hi > lo && hi - lo > short_max) {
+    uint64_t len = hi > lo ? hi - lo : 0;
+    if (len > short_max) {
       ++sg;
       continue;
     }
     const uint64_t w0 = e0 / window * window;
-    uint64_t top = sg + 1, last = hi > lo ? hi : lo;
+    uint64_t top = sg + 1, last = lo + len, longest = len;
     while (top < n_seg) {
       lo = hi;
       hi = off[top + 1];
-      if (lo - w0 >= window || (hi > lo && hi - lo > short_max)) break;
-      last = hi > lo ? hi : lo;
+      len = hi > lo ? hi - lo : 0;
+      if (lo - w0 >= window || len > short_max) break;
+      last = lo + len;
+      longest = std::max(longest, len);
       ++top;
     }
-    rec->insert(rec->end(), {sg, top, e0, last > e0 ? last - e0 : 0});
+    each(sg, top, e0, last > e0 ? last - e0 : 0, longest);
     sg = top;
   }
+}
+void segplan_window_records(const uint64_t* off, uint64_t n_seg, uint64_t short_max, uint64_t window,
+                            std::vector<uint64_t>* rec) {
+  rec->clear();
+  walk_window_records(off, n_seg, short_max, window,
+                      [&](uint64_t first, uint64_t end, uint64_t e0, uint64_t elements, uint64_t) {
+                        rec->insert(rec->end(), {first, end, e0, elements});
+                      });
 }
 
 namespace {
@@ -524,16 +536,12 @@ int segplan_records(SegPlan* p, uint64_t short_max, uint64_t window, const SegPl
     p->host_off.swap(off);
   }
   std::vector<uint64_t> rec;
-  const uint64_t* off = p->host_off.data();
-  segplan_window_records(off, p->n_seg, short_max, window, &rec);
   // the kernels find the longest vector's length above the elements (below 2^32:
   // a tile's)
-  for (size_t i = 0; i < rec.size(); i += 4) {
-    uint64_t longest = 0;
-    for (uint64_t s = rec[i]; s < rec[i + 1]; ++s)
-      if (off[s + 1] > off[s]) longest = std::max(longest, off[s + 1] - off[s]);
-    rec[i + 3] |= longest << 32;
-  }
+  walk_window_records(p->host_off.data(), p->n_seg, short_max, window,
+                      [&](uint64_t first, uint64_t end, uint64_t e0, uint64_t elements, uint64_t longest) {
+                        rec.insert(rec.end(), {first, end, e0, elements | longest << 32});
+                      });
   SegPlanRecords r;
   r.short_max = short_max;
   r.window = window;
