@@ -846,8 +846,9 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
       }
       // The sums leave 16 columns at a time through shared memory (16-byte chunk
       // c of row r at chunk c ^ (r / 2 % 4)), four lanes to a row, so that a
-      // store covers 64 bytes of eight rows instead of 16 bytes of 32 (8192 x 256
-      // x 8192 245 -> 171 us, K = 4096 1.14 -> 1.11 ms).
+      // store covers 64 bytes of eight rows instead of 16 bytes of 32 (with three
+      // products in place of six, 8192 x 256 x 8192 245 -> 171 us, K = 4096 1.14 ->
+      // 1.11 ms).
       if (ok) {
         const uint32_t st = stage_out + (uint32_t)(warp - 2) * 2048u;
         const bool vec = rows_aligned(g.P, g.N);
@@ -876,8 +877,9 @@ __device__ __forceinline__ void pair_body(const CUtensorMap& tmA, const CUtensor
               if (row < g.M && col < g.N) *reinterpret_cast<float4*>(g.P + (uint64_t)row * g.N + col) = v;
             }
           } else {
-            // sixteen lanes to a row: 8000 x 256 x 8001 212 -> 166 us, 2001 x 1000
-            // x 2003 48 -> 41 against four 4-byte stores of four lanes to a row
+            // sixteen lanes to a row: 8000 x 256 x 8001 212 -> 166 us (three
+            // products), 2001 x 1000 x 2003 48 -> 41 against four 4-byte stores of
+            // four lanes to a row
             const uint32_t cc = (uint32_t)(lane & 15), col = col0 + cc;
 #pragma unroll 4
             for (int i = 0; i < 16; ++i) {
