@@ -163,9 +163,10 @@ struct Operand {
   int kmajor;
 };
 
-// X tile of 64 rows x 128 k at (r0, k0): thread i handles rows i / 16 (+ 16,
-// + 32, + 48), k (i % 16) * 8 .. + 7, so sixteen neighbouring lanes hold a
-// row's k-block and store 256 contiguous bytes per part.
+// X tile of 64 rows x KT k (128, or 64: split_depth) at (r0, k0): KT / 8
+// neighbouring lanes hold 8 consecutive k each of a row and store 2 * KT
+// contiguous bytes per part.
+template <int KT>
 __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32_t Kp, uint32_t r0, uint32_t k0,
                                            int parts, float (*tile)[65]) {
   const uint64_t plane = (uint64_t)op.rp * Kp;
@@ -175,15 +176,15 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
     // it (r0 and R multiples of 4: a load is wholly in or out)
     if ((R % 4u) == 0 && (reinterpret_cast<uintptr_t>(op.x) & 15u) == 0) {
       const uint32_t c4 = threadIdx.x % 16, kr = threadIdx.x / 16;
-      float4 q[8];
+      float4 q[KT / 16];
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < KT / 16; ++i) {
         const uint32_t k = k0 + kr + 16 * i, n = r0 + c4 * 4;
         q[i] = (k < K && n < R) ? *reinterpret_cast<const float4*>(op.x + (uint64_t)k * R + n)
                                 : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
-      for (int i = 0; i < 8; ++i) {
+      for (int i = 0; i < KT / 16; ++i) {
         float* t = &tile[kr + 16 * i][c4 * 4];
         t[0] = q[i].x;
         t[1] = q[i].y;
@@ -192,7 +193,7 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
       }
     } else {
 #pragma unroll 8
-      for (int i = threadIdx.x; i < 128 * 64; i += 256) {
+      for (int i = threadIdx.x; i < KT * 64; i += 256) {
         const uint32_t kk = (uint32_t)i / 64, nn = (uint32_t)i % 64;
         const uint32_t k = k0 + kk, n = r0 + nn;
         tile[kk][nn] = (k < K && n < R) ? op.x[(uint64_t)k * R + n] : 0.0f;
@@ -201,11 +202,12 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
     __syncthreads();
   }
   const bool vec = op.kmajor && (K % 4u) == 0 && (reinterpret_cast<uintptr_t>(op.x) & 15u) == 0;
-  const uint32_t kc = (threadIdx.x % 16) * 8, k = k0 + kc;
-  float x[4][8];
+  constexpr int LANES = KT / 8, AT_ONCE = 256 / LANES, PASSES = 64 / AT_ONCE;
+  const uint32_t kc = (threadIdx.x % LANES) * 8, k = k0 + kc;
+  float x[PASSES][8];
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const uint32_t rr = threadIdx.x / 16 + 16 * c, row = r0 + rr;
+  for (int c = 0; c < PASSES; ++c) {
+    const uint32_t rr = threadIdx.x / LANES + AT_ONCE * c, row = r0 + rr;
     if (!op.kmajor) {
 #pragma unroll
       for (int e = 0; e < 8; ++e) x[c][e] = tile[kc + e][rr];
@@ -220,8 +222,8 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
     }
   }
 #pragma unroll
-  for (int c = 0; c < 4; ++c) {
-    const uint32_t row = r0 + threadIdx.x / 16 + 16 * c;
+  for (int c = 0; c < PASSES; ++c) {
+    const uint32_t row = r0 + threadIdx.x / LANES + AT_ONCE * c;
     __align__(16) __nv_bfloat16 h[8], m[8], l[8];
 #pragma unroll
     for (int e = 0; e < 8; ++e) {
@@ -239,18 +241,19 @@ __device__ __forceinline__ void split_tile(const Operand& op, uint32_t K, uint32
   }
 }
 
-// Splits both operands, one 64 x 128 tile per step (grid-stride over A's
-// tiles, then B's).  Bound by memory: reads 4 bytes, writes 6 (three parts)
+// Splits both operands, one 64 x KT tile per step (grid-stride over A's tiles,
+// then B's).  Bound by memory: reads 4 bytes, writes 6 (three parts)
 // per element.  A row-major operand's tiles are taken along k, a transposed
 // one's along its rows, so neighbouring blocks read neighbouring memory.
+template <int KT>
 __global__ void __launch_bounds__(256)
 split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int parts) {
-  __shared__ float tile[128][65];
+  __shared__ float tile[KT][65];
   // the contraction's blocks may start setting up once every block here runs
   // (they wait for this grid's end before they read): 2-4 % of a small product
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
   dependency_wait();
-  const uint32_t kt = (Kp + 127) / 128;
+  const uint32_t kt = (Kp + KT - 1) / KT;
   const uint32_t rta = (a.rows + 63) / 64, rtb = (b.rows + 63) / 64;
   const uint64_t na = (uint64_t)rta * kt, n = na + (uint64_t)rtb * kt;
   for (uint64_t t = blockIdx.x; t < n; t += gridDim.x) {
@@ -259,8 +262,8 @@ split_kernel(const Operand a, const Operand b, uint32_t K, uint32_t Kp, int part
     const uint64_t i = second ? t - na : t;
     const uint32_t rt = second ? rtb : rta;
     const uint32_t r0 = (uint32_t)(op.kmajor ? i / kt : i % rt) * 64;
-    const uint32_t k0 = (uint32_t)(op.kmajor ? i % kt : i / rt) * 128;
-    split_tile(op, K, Kp, r0, k0, parts, tile);
+    const uint32_t k0 = (uint32_t)(op.kmajor ? i % kt : i / rt) * KT;
+    split_tile<KT>(op, K, Kp, r0, k0, parts, tile);
     if (n > gridDim.x) __syncthreads();  // (block-uniform: the tile is filled again)
   }
 }
@@ -1252,10 +1255,22 @@ Split split_of(const float* A, const float* B, uint32_t M, uint32_t N, uint32_t 
   s.b = {B, base + (size_t)parts * s.Mp * s.Kp, N, s.Np, (trans & 2) ? 1 : 0};
   return s;
 }
-uint64_t split_tiles(const Split& s) {
-  return (uint64_t)((s.a.rows + 63) / 64 + (s.b.rows + 63) / 64) * ((s.Kp + 127) / 128);
+// k of a tile of the split pass: 64 (more blocks an SM, and none half empty where
+// Kp is an odd number of 64s), but 128 for operands of over 2^25 elements, whose
+// stores go to memory and want to be long.  us of a call, 128 / 64: 2000 x K x
+// 2000 K = 64 10.8 / 10.0, 1000 39.0 / 37.6; 1 x K x 62000 K = 16 18.5 / 14.9, 192
+// 41.3 / 37.7, 4096 664 / 680; 100 x 4096 x 39680 518 / 533.
+uint32_t split_depth(const Split& s) {
+  const uint64_t elements = ((uint64_t)s.a.rows + s.b.rows) * s.Kp;
+  return elements < (1ull << 25) || (s.Kp % 128 == 64 && s.Kp <= 320) ? 64 : 128;
 }
-dim3 split_grid(const Split& s) { return dim3((unsigned)std::min<uint64_t>(split_tiles(s), 0x7fffffffull)); }
+cudaError_t launch_split(const Split& s, uint32_t K, int parts, cudaStream_t stream) {
+  const uint32_t depth = split_depth(s);
+  const uint64_t tiles = (uint64_t)((s.a.rows + 63) / 64 + (s.b.rows + 63) / 64) * ((s.Kp + depth - 1) / depth);
+  return launch_overlapped(depth == 64 ? tc::split_kernel<64> : tc::split_kernel<128>,
+                           dim3((unsigned)std::min<uint64_t>(tiles, 0x7fffffffull)), dim3(256), 0, stream, s.a, s.b, K,
+                           s.Kp, parts);
+}
 
 // The output tiles (rows x cols each), numbered in groups of tile rows; the
 // default is a group whose rows of A and columns of B for one wave of one
@@ -1293,7 +1308,7 @@ int allpairs_tc_launch(const float* A, const float* B, float* P, uint32_t M, uin
   alignas(64) CUtensorMap tmA, tmB;
   if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, parts, tc::BM, bk)) return st;
   if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, parts, bn, bk)) return st;
-  cudaError_t e = launch_overlapped(tc::split_kernel, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp, parts);
+  cudaError_t e = launch_split(sp, K, parts, stream);
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
   if (wide) {
     // 128 x 256 tiles, k-blocks of 32: drains every 2 k-blocks (64 K, as the
@@ -1397,7 +1412,7 @@ int allpairs_pair_launch(const float* A, const float* B, float* P, uint32_t M, u
   alignas(64) CUtensorMap tmA, tmB;
   if (int st = encode_parts(&tmA, sp.a.out, sp.Mp, Kp, 3, tc::BM, 32)) return st;
   if (int st = encode_parts(&tmB, sp.b.out, sp.Np, Kp, 3, 128, 32)) return st;
-  cudaError_t e = launch_overlapped(tc::split_kernel, split_grid(sp), dim3(256), 0, stream, sp.a, sp.b, K, Kp, 3);
+  cudaError_t e = launch_split(sp, K, 3, stream);
   if (e != cudaSuccess) return cuda_fail(e, "split launch");
   const tc::PairArgs args = {P, err, M, N, Kp, spin_limit, tiles.n, tiles.m, tiles.group};
   const uint64_t all = (uint64_t)tiles.m * tiles.n;
@@ -1458,6 +1473,6 @@ extern "C" int scl_debug_allpairs_split(const float* A, const float* B, uint32_t
   if (int st = require_init()) return st;
   if (!A || !B || scratch_bytes < need) return fail(SCL_ERR_ARG, "split: null operand or scratch too small");
   const Split sp = split_of(A, B, M, N, K, parts, trans, scratch);
-  SCL_CUDA(launch_overlapped(tc::split_kernel, split_grid(sp), dim3(256), 0, rt().stream, sp.a, sp.b, K, sp.Kp, parts));
+  SCL_CUDA(launch_split(sp, K, parts, rt().stream));
   return SCL_OK;
 }
